@@ -278,21 +278,25 @@ __device__ __forceinline__ void rope_pair(float x0, float x1, float c, float s, 
 // 7.1.26).  A template, so that a kernel branches on the code once per tile and not per
 // element — written as a switch in the element loop the compiler evaluates every case
 // for every element and selects.
-template <int ACT>
+// APPROX_DIV takes the quotients from one reciprocal instruction (2 ulp in f32; for results
+// rounded to f16, where the correctly rounded division cost three times the rest of the
+// function).
+template <int ACT, bool APPROX_DIV = false>
 __device__ __forceinline__ float act_apply(float x) {
+  auto div = [](float a, float b) { return APPROX_DIV ? __fdividef(a, b) : a / b; };
   if (ACT == 1) return tanhf(x);
   if (ACT == 2) {
     const float z = x * 0.70710678118654752f, az = fabsf(z);
-    const float t = 1.f / (1.f + az * 0.3275911f);
+    const float t = div(1.f, 1.f + az * 0.3275911f);
     const float poly = t * (0.254829592f + t * (-0.284496736f + t * (1.421413741f +
                        t * (-1.453152027f + t * 1.061405429f))));
     return 0.5f * x * (1.f + copysignf(1.f - poly * __expf(-az * az), z));
   }
-  if (ACT == 3) return x / (1.f + __expf(-x));
+  if (ACT == 3) return div(x, 1.f + __expf(-x));
   if (ACT == 4) return fmaxf(x, 0.f);
   if (ACT == 5) {  // torch's gelu(approximate='tanh'), tanh as 1 - 2/(e^{2u} + 1)
     const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
-    return 0.5f * x * (2.f - 2.f / (__expf(2.f * u) + 1.f));
+    return 0.5f * x * (2.f - div(2.f, __expf(2.f * u) + 1.f));
   }
   if (ACT == 6) return fmaxf(x, 0.f) + (__expf(fminf(x, 0.f)) - 1.f);
   return x;

@@ -2,17 +2,26 @@
 // out [M, N] = act(a [M, K] * b [K, N] + bias) + addend, f32 accumulation in tensor
 // memory.  Same op as matmul.cu (packages/runntime/src/core/graph/ops/matmul.ts:28-99).
 //
-// One 128 x 128 output tile per CTA.  Warp 4 (one elected lane) streams K in steps of
-// 64 through a three-stage ring of TMA loads: a 128 x 64 piece of a (K-major, 128-byte
-// swizzle) and a 64 x 128 piece of b as two 64-column boxes (b is [K, N] row-major, that
-// is MN-major for the MMA, the layout the V tiles of the attention kernels use).  Warp 5
-// (one elected lane) issues four tcgen05.mma (M = 128, N = 128, K = 16) per stage into a
-// 128-column accumulator and frees the stage by tcgen05.commit.  Warps 0-3 read the
-// accumulator (one row per thread), apply bias, activation and addend, and store.
-// Rows, columns and K past the matrices are zero-filled by TMA and never stored.
-// Every wait is bounded (sm100.cuh).  Two CTAs share an SM (97 KB of shared memory and
-// 128 tensor-memory columns each), so that one's start-up and read-out overlap the
-// other's K loop.
+// One CTA per SM walks the 128 x BN output tiles (columns fastest).  Warp 8 streams K in
+// steps of 64 through a ring of TMA loads: a 128 x 64 piece of a (K-major, 128-byte
+// swizzle) and a 64 x BN piece of b as 64-column boxes (b is [K, N] row-major, that is
+// MN-major for the MMA, the layout the V tiles of the attention kernels use).  Warp 9
+// issues four tcgen05.mma (M = 128, N = BN, K = 16) per stage into one of two accumulators,
+// so the K loop of a tile runs under the read-out of the tile before.  Warp 10 fetches the
+// addend's tile into the staging buffer by TMA.  Warps 0-7 read the accumulator (a
+// row and half of the columns per thread), apply bias, activation and addend in registers, leave the halves in the
+// staging buffer in the swizzled layout (16 bytes per thread, no bank conflicts) and one
+// thread stores it by TMA, which also clips the matrix edge.  Rows, columns and K past the
+// matrices are zero-filled.  Every wait is bounded (sm100.cuh).
+//
+// What bounds it: with one tile per CTA (a speech clip, a few paragraphs) latency, launch to
+// store; with many, the read-out's instructions where the activation has some, else the MMAs.
+// The activation is a template parameter: with the seven of them in one kernel the read-out
+// was larger than the instruction cache and stalled on fetches.  Measured, that kernel (a CTA
+// per tile, stores and addend by row) and this one, launches back to back: [415, 288] x
+// [288, 864] 9.0 -> 4.0 us; [4352, 384] x [384, 1152] 20.2 -> 9.1, x [384, 1536] + gelu 55 ->
+// 12.9; [4352, 1536] x [1536, 384] + addend 24 -> 11.2; [32768, 1024] x [1024, 3072] 323 -> 204
+// (1 011 TFLOP/s); 8192 x 4096 x 4096 279 -> 245 (1 124).
 #include "common.cuh"
 #include "sm100.cuh"
 #include "tc_common.cuh"
@@ -23,139 +32,315 @@ namespace {
 using namespace sm100;
 using namespace tc;
 
-constexpr int GBM = 128, GBN = 128, GBK = 64, GSTAGES = 3;   // 97 KB of shared memory: two CTAs per SM
-constexpr int kABytes = GBM * GBK * 2, kBBytes = GBK * GBN * 2, kStageBytes = kABytes + kBBytes;
-constexpr int kGemmSmem = GSTAGES * kStageBytes + 1024;
-constexpr int kGemmThreads = 192;
+// Programmatic dependent launch: a grid launched with the stream-serialization attribute
+// may start while the grid before it in the stream drains; grid_dependency_wait() returns
+// once that grid has completed and its writes are visible (at once if there is none);
+// grid_launch_dependents() lets the next such grid start its prologue.
+__device__ __forceinline__ void grid_dependency_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void grid_launch_dependents() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
-__global__ void __launch_bounds__(kGemmThreads, 2)
+constexpr int GBM = 128, GBK = 64;
+constexpr int kReadThreads = 256;                   // two warpgroups, half of a tile's columns each
+constexpr int kGemmThreads = kReadThreads + 96;
+constexpr int kABytes = GBM * GBK * 2;
+constexpr int kBoxBytes = GBM * 64 * 2;   // 64 columns of a tile in the staging buffer
+
+template <int BN>
+struct Gemm {
+  static constexpr int kBBytes = GBK * BN * 2, kStage = kABytes + kBBytes;
+  static constexpr int kStagings = BN == 256 ? 1 : 2;       // output tiles in flight to memory
+  static constexpr int kStages = BN == 256 ? 3 : BN == 128 ? 5 : 6;
+  static constexpr int kStaging = BN / 64 * kBoxBytes;
+  static constexpr int kSmem = kStages * kStage + kStagings * kStaging + 1024;
+};
+
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t src, int x, int y) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(map),
+               "r"(src), "r"(x), "r"(y)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_commit() {
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+template <int N>
+__device__ __forceinline__ void bulk_wait_read() {
+  asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
+}
+template <int N>
+__device__ __forceinline__ void bulk_wait() {
+  asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory");
+}
+// Barrier over the read-out warps that also ands a predicate: a wait that gave up in one
+// thread ends the loop in all of them.
+__device__ __forceinline__ bool readout_all(bool ok) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "barrier.cta.red.and.aligned.pred q, 1, 256, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"(ok ? 1u : 0u)
+      : "memory");
+  return r != 0;
+}
+__device__ __forceinline__ void st_shared_v4(uint32_t addr, uint4 v) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z),
+               "r"(v.w)
+               : "memory");
+}
+__device__ __forceinline__ uint4 ld_shared_v4(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "r"(addr)
+               : "memory");
+  return v;
+}
+
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return fma2(a, b, make_float2(0.f, 0.f)); }
+
+// gelu of a pair, the erf polynomial of act_apply in a form without the sign: x/2 (1 + erf(z)) =
+// max(x, 0) - |x|/2 * poly(t) e^(-z^2), z = x / sqrt 2.  Packed arithmetic, one reciprocal and
+// one exponential instruction per element: the special-function unit (16 per clock) is what is
+// left to bound it, 2 048 cycles for a 128 x 128 tile ([4352, 384] x [384, 1536] + gelu: 15.1 us
+// with the scalar form, 12.9 with this one).
+__device__ __forceinline__ float2 gelu_pair(float2 x) {
+  auto both = [](float c) { return make_float2(c, c); };
+  const float2 ax = make_float2(fabsf(x.x), fabsf(x.y));
+  const float2 d = fma2(ax, both(0.3275911f * 0.70710678118654752f), both(1.f));
+  float2 t;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t.x) : "f"(d.x));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t.y) : "f"(d.y));
+  float2 poly = fma2(both(1.061405429f), t, both(-1.453152027f));
+  poly = fma2(poly, t, both(1.421413741f));
+  poly = fma2(poly, t, both(-0.284496736f));
+  poly = fma2(poly, t, both(0.254829592f));
+  const float2 u = mul2(mul2(x, x), both(-0.5f * kLog2e));
+  const float2 e = make_float2(fast_exp2(u.x), fast_exp2(u.y));
+  const float2 w = mul2(mul2(poly, t), e);
+  return fma2(mul2(ax, both(-0.5f)), w, make_float2(fmaxf(x.x, 0.f), fmaxf(x.y, 0.f)));
+}
+
+// addMode: 0 = no addend, 1 = by TMA, 2 = element by element (an addend off a 16-byte boundary).
+template <int BN, int ACT>
+__global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
-               const __half* __restrict__ bias, const __half* __restrict__ addend,
-               __half* __restrict__ out, int64_t M, int64_t K, int64_t N, int act, int* status) {
+               const __grid_constant__ CUtensorMap mapAdd, const __grid_constant__ CUtensorMap mapOut,
+               const __half* __restrict__ bias, const __half* __restrict__ addend, int addMode,
+               int64_t M, int64_t K, int64_t N, int tilesN, int tiles, int* status) {
+  using G = Gemm<BN>;
   extern __shared__ unsigned char smemRaw[];
-  __shared__ __align__(8) uint64_t sFull[GSTAGES], sEmpty[GSTAGES], sAcc;
+  __shared__ __align__(8) uint64_t sFull[G::kStages], sEmpty[G::kStages], sAccFull[2], sAccEmpty[2];
+  __shared__ __align__(8) uint64_t sAddFull[2], sStgFree[2];
+  __shared__ __align__(16) float sBias[2][BN];
   __shared__ uint32_t sTmemBase;
   __shared__ int sAbort;
   const int tid = threadIdx.x, warp = tid >> 5;
-  TC_TRACE_DECL
-  TC_TRACE(0, 0);
   const uint32_t smemBase = (smem_u32(smemRaw) + 1023u) & ~1023u;
-  const int64_t row0 = (int64_t)blockIdx.y * GBM, col0 = (int64_t)blockIdx.x * GBN;
+  const uint32_t stgBase = smemBase + G::kStages * G::kStage;
   const int nk = (int)((K + GBK - 1) / GBK);
 
   if (tid == 0) {
     sAbort = 0;
-    for (int s = 0; s < GSTAGES; s++) {
+    for (int s = 0; s < G::kStages; s++) {
       mbar_init(smem_u32(&sFull[s]), 1);
       mbar_init(smem_u32(&sEmpty[s]), 1);
     }
-    mbar_init(smem_u32(&sAcc), 1);
+    for (int b = 0; b < 2; b++) {
+      mbar_init(smem_u32(&sAccFull[b]), 1);
+      mbar_init(smem_u32(&sAccEmpty[b]), kReadThreads / 32);
+      mbar_init(smem_u32(&sAddFull[b]), 1);
+      mbar_init(smem_u32(&sStgFree[b]), 1);
+    }
     fence_barrier_init();
   }
-  if (warp == 5) {
-    tmem_alloc(smem_u32(&sTmemBase), GBN);
+  if (warp == 8 && elect_one()) {
+    prefetch_tensormap(&mapA);
+    prefetch_tensormap(&mapB);
+    prefetch_tensormap(&mapOut);
+  }
+  if (warp == 9) {
+    tmem_alloc(smem_u32(&sTmemBase), 2 * BN);
     tmem_relinquish();
   }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = sTmemBase;
-  TC_TRACE(1, 0);
+  // Everything above touched no global memory; what follows reads tensors the grid before
+  // this one may have written and overwrites out, which it may still read.
+  grid_dependency_wait();
 
-  if (warp == 4) {
+  if (warp == 8) {
     // ------------------------------ TMA producer ------------------------------
     if (elect_one()) {
-      prefetch_tensormap(&mapA);
-      prefetch_tensormap(&mapB);
-      for (int it = 0; it < nk; it++) {
-        const int s = it % GSTAGES;
-        if (it >= GSTAGES && !mbar_wait(smem_u32(&sEmpty[s]), ((it / GSTAGES) - 1) & 1, &sAbort))
-          break;
-        const uint32_t bar = smem_u32(&sFull[s]);
-        const uint32_t dA = smemBase + s * kStageBytes, dB = dA + kABytes;
-        mbar_expect_tx(bar, kStageBytes);
-        tma_load_2d(dA, &mapA, it * GBK, (int)row0, bar);                  // 64 k x 128 rows
-        tma_load_2d(dB, &mapB, (int)col0, it * GBK, bar);                  // 64 cols x 64 k
-        tma_load_2d(dB + GBK * 128, &mapB, (int)col0 + 64, it * GBK, bar);
+      int it = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+        const int row0 = tile / tilesN * GBM, col0 = tile % tilesN * BN;
+        for (int k = 0; k < nk; k++, it++) {
+          const int s = it % G::kStages;
+          if (it >= G::kStages && !mbar_wait(smem_u32(&sEmpty[s]), ((it / G::kStages) - 1) & 1, &sAbort)) {
+            ok = false;
+            break;
+          }
+          const uint32_t bar = smem_u32(&sFull[s]);
+          const uint32_t dA = smemBase + s * G::kStage, dB = dA + kABytes;
+          mbar_expect_tx(bar, G::kStage);
+          tma_load_2d(dA, &mapA, k * GBK, row0, bar);                  // 64 k x 128 rows
+#pragma unroll
+          for (int c = 0; c < BN; c += 64)                             // 64 columns x 64 k each
+            tma_load_2d(dB + c * GBK * 2, &mapB, col0 + c, k * GBK, bar);
+        }
       }
+      grid_launch_dependents();
     }
-  } else if (warp == 5) {
+  } else if (warp == 9) {
     // ------------------------------ MMA issuer --------------------------------
-    constexpr uint32_t idesc = instr_desc(GBN, true);
+    constexpr uint32_t idesc = instr_desc(BN, true);
     constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);  // SBO, version, SW128
     constexpr uint32_t kLboA = (16u >> 4) << 16;                          // K-major operand
     constexpr uint32_t kLboB = ((uint32_t)(GBK * 128) >> 4) << 16;        // MN-major: next 64 columns
     bool ok = true;
-    for (int it = 0; it < nk && ok; it++) {
-      const int s = it % GSTAGES;
-      ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&sFull[s]), (it / GSTAGES) & 1, &sAbort)) != 0;
-      if (!ok) break;
-      tc_fence_after_sync();
-      TC_TRACE(2, it);
-      if (elect_one()) {
-        const uint32_t aLo = (((smemBase + s * kStageBytes) >> 4) & 0x3fffu) | kLboA;
-        const uint32_t bLo = (((smemBase + s * kStageBytes + kABytes) >> 4) & 0x3fffu) | kLboB;
+    int it = 0, t = 0;
+    for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, t++) {
+      const int b = t & 1;
+      if (t >= 2) ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&sAccEmpty[b]), ((t >> 1) - 1) & 1, &sAbort)) != 0;
+      for (int k = 0; k < nk && ok; k++, it++) {
+        const int s = it % G::kStages;
+        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&sFull[s]), (it / G::kStages) & 1, &sAbort)) != 0;
+        if (!ok) break;
+        tc_fence_after_sync();
+        if (elect_one()) {
+          const uint32_t aLo = (((smemBase + s * G::kStage) >> 4) & 0x3fffu) | kLboA;
+          const uint32_t bLo = (((smemBase + s * G::kStage + kABytes) >> 4) & 0x3fffu) | kLboB;
 #pragma unroll
-        for (int kk = 0; kk < GBK / 16; kk++) {
-          const uint64_t aDesc = ((uint64_t)kDescHi << 32) | (aLo + kk * 2);
-          const uint64_t bDesc = ((uint64_t)kDescHi << 32) | (bLo + kk * (2048 >> 4));
-          mma_f16_ss(tmem, aDesc, bDesc, idesc, (it > 0 || kk > 0) ? 1u : 0u);
+          for (int kk = 0; kk < GBK / 16; kk++) {
+            const uint64_t aDesc = ((uint64_t)kDescHi << 32) | (aLo + kk * 2);
+            const uint64_t bDesc = ((uint64_t)kDescHi << 32) | (bLo + kk * (2048 >> 4));
+            mma_f16_ss(tmem + b * BN, aDesc, bDesc, idesc, (k > 0 || kk > 0) ? 1u : 0u);
+          }
+          tc_commit(smem_u32(&sEmpty[s]));
+          if (k == nk - 1) tc_commit(smem_u32(&sAccFull[b]));
         }
-        tc_commit(smem_u32(&sEmpty[s]));
-        if (it == nk - 1) tc_commit(smem_u32(&sAcc));
+        __syncwarp();
       }
-      __syncwarp();
+    }
+  } else if (warp == 10) {
+    // ------------------------------ addend loads ------------------------------
+    if (addMode == 1 && elect_one()) {
+      int t = 0;
+      for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, t++) {
+        const int row0 = tile / tilesN * GBM, col0 = tile % tilesN * BN;
+        const int g = t % G::kStagings;
+        if (t >= G::kStagings &&
+            !mbar_wait(smem_u32(&sStgFree[g]), ((t / G::kStagings) - 1) & 1, &sAbort))
+          break;
+        const uint32_t bar = smem_u32(&sAddFull[g]);
+        mbar_expect_tx(bar, G::kStaging);
+#pragma unroll
+        for (int c = 0; c < BN / 64; c++)
+          tma_load_2d(stgBase + g * G::kStaging + c * kBoxBytes, &mapAdd, col0 + c * 64, row0, bar);
+      }
     }
   } else {
-    // ------------------------------ epilogue ----------------------------------
-    const bool ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&sAcc), 0, &sAbort)) != 0;
-    TC_TRACE(4, 0);
-    if (ok) {
+    // ------------------------------ read-out ----------------------------------
+    const int row = tid & 127, half = tid >> 7;   // row of the tile, half of its columns
+    int t = 0;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, t++) {
+      const int row0 = tile / tilesN * GBM, col0 = tile % tilesN * BN;
+      const int b = t & 1, g = t % G::kStagings;
+      if (tid < BN) {
+        const int c = tid;
+        sBias[b][c] = (bias && col0 + c < N) ? __half2float(bias[col0 + c]) : 0.f;
+      }
+      bool ok = mbar_wait(smem_u32(&sAccFull[b]), (t >> 1) & 1, &sAbort);
+      if (ok && addMode == 1)
+        ok = mbar_wait(smem_u32(&sAddFull[g]), (t / G::kStagings) & 1, &sAbort);
+      // (also: this tile's bias is in place, and the store that last used the staging buffer
+      // has read it — thread 0 waited for that before it came here)
+      if (!readout_all(ok)) break;
       tc_fence_after_sync();
-      const int64_t row = row0 + tid;  // thread = accumulator lane = output row
-      const uint32_t laneBase = (uint32_t)(warp * 32) << 16;
-#pragma unroll
-      for (int c = 0; c < GBN; c += 32) {
+      const uint32_t acc0 = tmem + b * BN + ((uint32_t)((warp & 3) * 32) << 16);
+      const uint32_t stg = stgBase + g * G::kStaging + row * 128;
+#pragma unroll 1
+      for (int c = half * (BN / 2); c < (half + 1) * (BN / 2); c += 32) {
         uint32_t acc[32];
-        tmem_ld32(tmem + laneBase + c, acc);
+        tmem_ld32(acc0 + c, acc);
         tmem_wait_ld();
-        if (row < M) {
-          const int64_t nc = col0 + c;             // first column of this 32-column piece
-          uint4 pk[4];
-          __half* h = reinterpret_cast<__half*>(pk);
-          act_dispatch(act, [&](auto code) {
+        const uint32_t box = stg + (c >> 6) * kBoxBytes;
 #pragma unroll
-            for (int x = 0; x < 32; x++) {
-              float y = __uint_as_float(acc[x]);
-              const int64_t n = nc + x;
-              if (bias && n < N) y += __half2float(bias[n]);
-              y = act_apply<decltype(code)::value>(y);
-              if (addend && n < N) y += __half2float(addend[row * N + n]);
-              h[x] = __float2half_rn(y);
+        for (int v = 0; v < 4; v++) {
+          const uint32_t at = box + (((((c & 32) >> 3) + v) ^ (row & 7)) << 4);
+          const float4 b0 = *reinterpret_cast<const float4*>(&sBias[b][c + v * 8]);
+          const float4 b1 = *reinterpret_cast<const float4*>(&sBias[b][c + v * 8 + 4]);
+          const float bs[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+          float y[8];
+#pragma unroll
+          for (int e = 0; e < 8; e += 2) {
+            const float x0 = __uint_as_float(acc[v * 8 + e]) + bs[e];
+            const float x1 = __uint_as_float(acc[v * 8 + e + 1]) + bs[e + 1];
+            if (ACT == 2) {
+              const float2 r = gelu_pair(make_float2(x0, x1));
+              y[e] = r.x;
+              y[e + 1] = r.y;
+            } else {
+              y[e] = act_apply<ACT, true>(x0);
+              y[e + 1] = act_apply<ACT, true>(x1);
             }
-          });
-          __half* dst = out + row * N + nc;
-          if (nc + 32 <= N) {
-#pragma unroll
-            for (int v = 0; v < 4; v++) reinterpret_cast<uint4*>(dst)[v] = pk[v];
-          } else {
-            for (int x = 0; x < 32 && nc + x < N; x++) dst[x] = h[x];
           }
+          if (addMode == 1) {
+            const uint4 w = ld_shared_v4(at);
+            const __half2* h = reinterpret_cast<const __half2*>(&w);
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+              const float2 f = __half22float2(h[e]);
+              y[2 * e] += f.x;
+              y[2 * e + 1] += f.y;
+            }
+          } else if (addMode == 2 && row0 + row < M) {
+            for (int e = 0; e < 8; e++) {
+              const int64_t n = col0 + c + v * 8 + e;
+              if (n < N) y[e] += __half2float(addend[(int64_t)(row0 + row) * N + n]);
+            }
+          }
+          uint4 w;
+          __half2* h = reinterpret_cast<__half2*>(&w);
+#pragma unroll
+          for (int e = 0; e < 4; e++) h[e] = __floats2half2_rn(y[2 * e], y[2 * e + 1]);
+          st_shared_v4(at, w);
         }
       }
+      tc_fence_before_sync();
+      fence_proxy_async();
+      __syncwarp();
+      if ((tid & 31) == 0) mbar_arrive(smem_u32(&sAccEmpty[b]));
+      readout_all(true);
+      if (tid == 0) {
+#pragma unroll
+        for (int c = 0; c < BN / 64; c++)
+          if (col0 + c * 64 < N)
+            tma_store_2d(&mapOut, stgBase + g * G::kStaging + c * kBoxBytes, col0 + c * 64, row0);
+        bulk_commit();
+        bulk_wait_read<G::kStagings - 1>();   // the store before the last kStagings - 1 has been read
+        if (t >= G::kStagings - 1) mbar_arrive(smem_u32(&sStgFree[(t + 1) % G::kStagings]));
+      }
     }
+    if (tid == 0) bulk_wait<0>();   // shared memory stays until the stores are done with it
   }
 
-  TC_TRACE(5, 0);
   tc_fence_before_sync();
   __syncthreads();
-  TC_TRACE(6, 0);
   if (tid == 0 && sAbort) atomicOr(status, kStatusWaitTimeout);
-  if (warp == 5) {
+  if (warp == 9) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem, GBN);
+    tmem_dealloc(tmem, 2 * BN);
   }
-  TC_TRACE(7, 0);
 }
 
 // ---- up to 16 rows (the projections of a decode step) -------------------------------
@@ -186,16 +371,6 @@ constexpr int kSkB = SKK * SKN * 2, kSkA = SKM * SKK * 2, kSkStage = kSkB + kSkA
 constexpr int kSkThreads = 192;
 constexpr int kSkMaxCluster = 8;
 
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-}
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -214,16 +389,6 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
 }
 __device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
-}
-// Programmatic dependent launch: a grid launched with the stream-serialization attribute
-// may start while the grid before it in the stream drains; grid_dependency_wait() returns
-// once that grid has completed and its writes are visible (at once if there is none);
-// grid_launch_dependents() lets the next such grid start its prologue.
-__device__ __forceinline__ void grid_dependency_wait() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-__device__ __forceinline__ void grid_launch_dependents() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 // The hardware barrier over all threads of the cluster, in its two halves.
 __device__ __forceinline__ void cluster_arrive() {
@@ -421,10 +586,33 @@ bool matmul_tc_supported(const void* a, const void* b, const void* out, int64_t 
   auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
   return dtype == RT_F16 && M >= 1 && K >= 64 && N >= (M <= SKM ? SKN : 64) && K % 8 == 0 &&
          N % 8 == 0 && al(a) && al(b) && al(out) && M < (1ll << 31) - 256 && N < (1ll << 31) - 256 &&
-         K < (1ll << 31) - 256 && (M + GBM - 1) / GBM <= 65535 && encode_fn() != nullptr;
+         K < (1ll << 31) - 256 &&
+         ((M + GBM - 1) / GBM) * ((N + 63) / 64) < (1ll << 31) && encode_fn() != nullptr;
 }
 
 namespace {
+constexpr int kSms = 148;
+
+// Columns of an output tile: the width whose slowest SM is done first.  Microseconds, measured:
+// a K step is bound by the L2 delivering its operands (24 / 32 / 48 KB at about 90 GB/s per SM),
+// the read-out takes 8 ns a column, 24 with an activation, and hides under the K loop of the
+// next tile.  [16384, 384] x [384, 1152]: 32 / 20 / 24 us with 64 / 128 / 256 columns,
+// [32768, 1024] x [1024, 3072]: 378 / 253 / 204, [415, 288] x [288, 864]: 4.0 / 4.8 / 7.0.
+int tile_columns(int64_t M, int64_t K, int64_t N, int act) {
+  const double nk = (double)((K + GBK - 1) / GBK);
+  int best = 64;
+  double bestCost = 1e30;
+  for (int bn : {64, 128, 256}) {
+    const int64_t tiles = ((N + bn - 1) / bn) * ((M + GBM - 1) / GBM);
+    const double waves = (double)((tiles + kSms - 1) / kSms);
+    const double loop = nk * (bn == 256 ? 0.545 : bn == 128 ? 0.33 : 0.285);
+    const double readout = bn * (act ? 0.024 : 0.008);
+    const double cost = waves * ((loop > readout ? loop : readout) + 0.2) + readout;
+    if (cost < bestCost) best = bn, bestCost = cost;
+  }
+  return best;
+}
+
 cudaError_t launch_skinny(const void* a, const void* b, const void* bias, const void* addend,
                           void* out, int64_t M, int64_t K, int64_t N, int act, int* status,
                           cudaStream_t s, std::string* err) {
@@ -462,21 +650,65 @@ cudaError_t launch_skinny(const void* a, const void* b, const void* bias, const 
 }
 }  // namespace
 
+namespace {
+template <int BN, int ACT>
+cudaError_t launch_tiled(const void* a, const void* b, const void* bias, const void* addend,
+                         void* out, int64_t M, int64_t K, int64_t N, int* status, cudaStream_t s,
+                         std::string* err) {
+  using G = Gemm<BN>;
+  CUtensorMap ma, mb, madd, mo;
+  if (!make_map(&ma, a, M, K, K, GBM, err) || !make_map(&mb, b, K, N, N, GBK, err) ||
+      !make_map(&mo, out, M, N, N, GBM, err))
+    return cudaErrorInvalidValue;
+  madd = mo;
+  int addMode = 0;
+  if (addend) {
+    addMode = (reinterpret_cast<uintptr_t>(addend) & 15u) == 0 ? 1 : 2;
+    if (addMode == 1 && !make_map(&madd, addend, M, N, N, GBM, err)) return cudaErrorInvalidValue;
+  }
+  auto kern = gemm_tc_kernel<BN, ACT>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, G::kSmem);
+  if (e != cudaSuccess) return e;
+  const int64_t tilesN = (N + BN - 1) / BN, tiles = tilesN * ((M + GBM - 1) / GBM);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(tiles < kSms ? tiles : kSms));
+  cfg.blockDim = dim3(kGemmThreads);
+  cfg.dynamicSmemBytes = G::kSmem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, ma, mb, madd, mo, static_cast<const __half*>(bias),
+                            static_cast<const __half*>(addend), addMode, M, K, N, (int)tilesN,
+                            (int)tiles, status);
+}
+
+template <int BN>
+cudaError_t launch_tiled_act(const void* a, const void* b, const void* bias, const void* addend,
+                             void* out, int64_t M, int64_t K, int64_t N, int act, int* status,
+                             cudaStream_t s, std::string* err) {
+  switch (act) {
+    case 1: return launch_tiled<BN, 1>(a, b, bias, addend, out, M, K, N, status, s, err);
+    case 2: return launch_tiled<BN, 2>(a, b, bias, addend, out, M, K, N, status, s, err);
+    case 3: return launch_tiled<BN, 3>(a, b, bias, addend, out, M, K, N, status, s, err);
+    case 4: return launch_tiled<BN, 4>(a, b, bias, addend, out, M, K, N, status, s, err);
+    case 5: return launch_tiled<BN, 5>(a, b, bias, addend, out, M, K, N, status, s, err);
+    case 6: return launch_tiled<BN, 6>(a, b, bias, addend, out, M, K, N, status, s, err);
+    default: return launch_tiled<BN, 0>(a, b, bias, addend, out, M, K, N, status, s, err);
+  }
+}
+}  // namespace
+
 cudaError_t launch_matmul_tc(const void* a, const void* b, const void* bias, const void* addend,
                              void* out, int64_t M, int64_t K, int64_t N, int act, int* status,
                              cudaStream_t s, std::string* err) {
   if (M <= SKM) return launch_skinny(a, b, bias, addend, out, M, K, N, act, status, s, err);
-  CUtensorMap ma, mb;
-  if (!make_map(&ma, a, M, K, K, GBM, err) || !make_map(&mb, b, K, N, N, GBK, err))
-    return cudaErrorInvalidValue;
-  cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       kGemmSmem);
-  if (e != cudaSuccess) return e;
-  const dim3 grid((unsigned)((N + GBN - 1) / GBN), (unsigned)((M + GBM - 1) / GBM));
-  gemm_tc_kernel<<<grid, kGemmThreads, kGemmSmem, s>>>(
-      ma, mb, static_cast<const __half*>(bias), static_cast<const __half*>(addend),
-      static_cast<__half*>(out), M, K, N, act, status);
-  return cudaGetLastError();
+  const int bn = tile_columns(M, K, N, act);
+  if (bn == 256) return launch_tiled_act<256>(a, b, bias, addend, out, M, K, N, act, status, s, err);
+  if (bn == 128) return launch_tiled_act<128>(a, b, bias, addend, out, M, K, N, act, status, s, err);
+  return launch_tiled_act<64>(a, b, bias, addend, out, M, K, N, act, status, s, err);
 }
 
 }  // namespace rt
