@@ -660,6 +660,16 @@ int rt_local_attention(rt_ctx* ctx, const void* qkv, const float* rel, const flo
       reinterpret_cast<uintptr_t>(rel) % 16 || reinterpret_cast<uintptr_t>(qScale) % 16)
     return fail(ctx, RT_INVALID_ARGUMENT,
                 "localAttention: tensors must start on a four-element boundary");
+  if (ctx->useTc && rt::local_attn_tc_supported(qkv, rel, out, rows, heads, headDim, dtype)) {
+    std::string err;
+    cudaError_t e = rt::launch_local_attn_tc(qkv, rel, qScale, out, rows, heads, headDim, window, kScale,
+                                             softcap, ctx->statusDev, ctx->stream, &err);
+    if (e != cudaSuccess)
+      return fail(ctx, RT_EXECUTION_FAILED, "local_attn_tc launch: %s %s", cudaGetErrorString(e),
+                  err.c_str());
+    ctx->launches++;
+    return RT_OK;
+  }
   RT_CUDA(ctx, rt::launch_local_attn(qkv, rel, qScale, out, rows, heads, headDim, window, kScale,
                                      softcap, dtype, ctx->stream));
   ctx->launches++;

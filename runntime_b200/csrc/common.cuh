@@ -365,6 +365,12 @@ cudaError_t launch_argmax_dot(const void* w, const void* x, float* out, int64_t 
 cudaError_t launch_local_attn(const void* qkv, const float* rel, const float* qScale, void* out,
                               int64_t rows, int heads, int hd, int window, float kScale,
                               float softcap, int dtype, cudaStream_t s);
+// ... on the tensor cores (f16, head sizes 64 and 128).
+bool local_attn_tc_supported(const void* qkv, const float* rel, const void* out, int64_t rows,
+                             int heads, int hd, int dtype);
+cudaError_t launch_local_attn_tc(const void* qkv, const float* rel, const float* qScale, void* out,
+                                 int64_t rows, int heads, int hd, int window, float kScale,
+                                 float softcap, int* status, cudaStream_t s, std::string* err);
 cudaError_t launch_softmax(const void* x, void* out, const float* segs, int64_t rows, int64_t cols,
                            int64_t wl, int64_t wr, int dtype, cudaStream_t s);
 cudaError_t launch_slice(const void* x, void* out, int64_t rows, int64_t srcColBytes,
