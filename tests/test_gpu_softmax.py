@@ -107,3 +107,29 @@ def test_matmul_attention_path_agrees_with_the_fused_op(ex):
                                dict(qHeads=heads, kvHeads=heads, headDim=hd, windowLeft=8,
                                     windowRight=8, segments=S)), ex).reshape(t, hd)
     assert np.all(np.abs(fused - viaMatmul) <= 2e-5 + 1e-4 * np.abs(viaMatmul))
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f16"])
+@pytest.mark.parametrize("shift,outShift", [(0, 0), (3, 3), (1, 5), (4, 0), (2, 1)])
+@pytest.mark.parametrize("rows,cols", [(2, 5), (5, 33), (3, 2051), (2050, 67), (2049, 2307)])
+def test_rows_that_start_anywhere(ex, dtype, shift, outShift, rows, cols):
+    """x and out `shift` elements into an allocation: chunks of 16 bytes, 8 bytes or one
+    element, ragged ends on either side; nothing outside the rows is written."""
+    import ctypes as C
+    import torch
+    from runntime_b200._lib import DTYPE_CODE, check
+    td = torch.float16 if dtype == "f16" else torch.float32
+    x = 8 * oracle.random_f32(rows * cols, 4)
+    x = oracle.round_f16(x) if dtype == "f16" else x
+    src = torch.zeros(rows * cols + 16, dtype=td, device="cuda")
+    src[shift:shift + rows * cols] = torch.from_numpy(x).to("cuda", td)
+    out = torch.full((rows * cols + 16,), 7.0, dtype=td, device="cuda")
+    torch.cuda.synchronize()
+    es = src.element_size()
+    check(ex._lib.rt_softmax(ex.ctx, C.c_void_p(src.data_ptr() + shift * es),
+                             C.c_void_p(out.data_ptr() + outShift * es), None, rows, cols, 0, 0,
+                             DTYPE_CODE[dtype]), ex.ctx)
+    ex.sync()
+    got = out.float().cpu().numpy()
+    close(got[outShift:outShift + rows * cols], oracle.softmax_ref(x.reshape(rows, cols)), dtype)
+    assert (got[:outShift] == 7).all() and (got[outShift + rows * cols:] == 7).all()
