@@ -68,7 +68,8 @@ RT_API int rt_ctx_set_stream(rt_ctx* ctx, void* cuda_stream, int external);
 /* Context options.  RT_OPT_PREFILL_TC (default 1): route eligible f16 prefill
  * shapes to a tensor-core kernel of the library's choice (head sizes 64, 128,
  * 256 and the narrow heads: one 128-row query tile per thread block whose key
- * tiles alternate between two softmax warpgroups).  0 sends every prefill to the FP32-pipe kernel; 2 forces one tile
+ * tiles alternate between two softmax warpgroups).  0 sends every prefill, f32
+ * ones too, to the FP32-pipe kernel; 2 forces one tile
  * with one warpgroup, 3 two tiles per block, 4 the alternating form, 5 the
  * alternating form on pairs of thread blocks that share every K/V tile, 6 the
  * alternating form as one persistent thread block per SM over a queue of query
@@ -155,8 +156,9 @@ RT_API int rt_attn(rt_ctx* ctx, const rt_attn_args* args);
 
 /* Which kernel rt_attn would run for these arguments: writes a short static
  * name into *route: "decode", "prefill_simt" (FP32 pipes), or one of the
- * tensor-core kernels "prefill_tc3" (the default), "prefill_tc3_pair",
- * "prefill_tc4", "prefill_tc2", "prefill_tc" (see RT_OPT_PREFILL_TC). */
+ * tensor-core kernels "prefill_tc3" (the default for f16), "prefill_tc3_pair",
+ * "prefill_tc4", "prefill_tc2", "prefill_tc" (see RT_OPT_PREFILL_TC) and
+ * "prefill_f32_tc" (f32). */
 RT_API int rt_attn_route(rt_ctx* ctx, const rt_attn_args* args, const char** route);
 
 /* ---- batched single-token decode over KV caches -----------------------------
