@@ -3,9 +3,9 @@
 //
 // Every f32 operand x is split into hi + lo, each a tf32 number (11 bits): x = hi + lo to 2^-23, and
 // a product is hi hi' + hi lo' + lo hi', 2^-22 short of exact at worst.  The tensor core adds into its
-// accumulator less carefully than an FMA does, so no accumulator lives long: scores add 64 columns of
-// the head before they join the f32 sum (hi hi' apart from the 2^-11 smaller cross terms), and the
-// output of 16 keys joins the f32 output in the FMA that rescales it.  Against 64-bit
+// accumulator less carefully than an FMA does, so no accumulator lives long: scores add 32 columns of
+// the head before they join the f32 sum (hi hi' apart from the 2^-11 smaller cross terms), and 16 keys
+// are added, their cross terms first, before they join the f32 output.  Against 64-bit
 // products: 4.6e-7 of the norm at head size 256 (1.5e-6 for sequential f32 sums), 2.6e-7 to 3.7e-7 below.
 //
 // A CTA of eight warps owns 32 query rows of one query head and walks 128-key tiles of the union of
@@ -358,29 +358,33 @@ prefill_f32_tc_kernel(const AttnParams p, int tilesPerSeq) {
       const float* sV = advance() + (keySet * 16 + 2 * t4) * S::kVPitch + 32 * colSet + 4 * g;
       const int block = c * S::kKeySets + keySet;   // sixteen keys of the tile
       if (t * BK + block * 16 >= span) continue;
-      float f[2][4][4];
+      uint32_t ph[2][2][4], pl[2][2][4];   // [8 keys][row set]
+      float ev[2][2][4];                   // [8 keys][key 2 t4, 2 t4 + 1]
 #pragma unroll
       for (int n = 0; n < 2; n++) {
         const uint4* fp = sP + (block * 2 + n) * 128 + lane;
-        const uint4 h0 = fp[0], l0 = fp[32], h1 = fp[64], l1 = fp[96];
-        const uint32_t ph[2][4] = {{h0.x, h0.y, h0.z, h0.w}, {h1.x, h1.y, h1.z, h1.w}};
-        const uint32_t pl[2][4] = {{l0.x, l0.y, l0.z, l0.w}, {l1.x, l1.y, l1.z, l1.w}};
-        const float4 v0 = *reinterpret_cast<const float4*>(sV + n * 8 * S::kVPitch);
-        const float4 v1 = *reinterpret_cast<const float4*>(sV + (n * 8 + 1) * S::kVPitch);
-        const float e0[4] = {v0.x, v0.y, v0.z, v0.w}, e1[4] = {v1.x, v1.y, v1.z, v1.w};
-        // MMA column g of tile j is column 4 g + j of the warp's 32
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-          uint32_t vh0, vl0, vh1, vl1;
-          split(e0[j], vh0, vl0);
-          split(e1[j], vh1, vl1);
+        for (int a = 0; a < 2; a++) {
+          *reinterpret_cast<uint4*>(ph[n][a]) = fp[64 * a];
+          *reinterpret_cast<uint4*>(pl[n][a]) = fp[64 * a + 32];
+          *reinterpret_cast<float4*>(ev[n][a]) = *reinterpret_cast<const float4*>(sV + (n * 8 + a) * S::kVPitch);
+        }
+      }
+      float f[2][4][4];
+      // MMA column g of tile j is column 4 g + j of the warp's 32; the small products first
 #pragma unroll
-          for (int a = 0; a < 2; a++) {
-            if (n == 0) mma_tf32_first(f[a][j], pl[a], vh0, vh1);
-            else mma_tf32(f[a][j], pl[a], vh0, vh1);
-            mma_tf32(f[a][j], ph[a], vl0, vl1);
-            mma_tf32(f[a][j], ph[a], vh0, vh1);
-          }
+      for (int j = 0; j < 4; j++) {
+        uint32_t vh[2][2], vl[2][2];
+#pragma unroll
+        for (int n = 0; n < 2; n++) split(ev[n][0][j], vh[n][0], vl[n][0]), split(ev[n][1][j], vh[n][1], vl[n][1]);
+#pragma unroll
+        for (int a = 0; a < 2; a++) {
+          mma_tf32_first(f[a][j], pl[0][a], vh[0][0], vh[0][1]);
+          mma_tf32(f[a][j], ph[0][a], vl[0][0], vl[0][1]);
+          mma_tf32(f[a][j], pl[1][a], vh[1][0], vh[1][1]);
+          mma_tf32(f[a][j], ph[1][a], vl[1][0], vl[1][1]);
+          mma_tf32(f[a][j], ph[0][a], vh[0][0], vh[0][1]);
+          mma_tf32(f[a][j], ph[1][a], vh[1][0], vh[1][1]);
         }
       }
 #pragma unroll
