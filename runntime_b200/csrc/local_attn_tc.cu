@@ -4,25 +4,28 @@
 // A CTA takes 64 consecutive rows of one head: TMA brings their q rows and the K and V rows
 // they see (64 + WP, WP = 16 or 32 rows of halo before them; rows before the first are
 // zero-filled) into shared memory, 128-byte swizzled.  Each of four warps owns 16 rows and
-// 16 + WP keys and stays in registers from the scores to the output:
+// 16 + WP keys:
 //     S = q' K^T,  R = q' rel^T,  s_ij = cap tanh((kScale S_ij + R_i,i-j) / cap),  O = P V,
-// with mma.sync m16n8k16, the scores' fragments becoming the A operand of P V.  R is one row
-// of distances per query; it goes through shared memory to be read along the diagonals.
+// with mma.sync m16n8k16.  R is one row of distances per query; the scores go through shared
+// memory to where a lane finds them by (row, distance), as R's fragments lie, so that the soft cap
+// and the exponential run on 16 or 32 elements of a row and not on its 32 or 48 keys, and
+// the probabilities come back as the A operand of P V.  A CTA stays with its head and walks its row
+// tiles, so that the bias rows are split once.
 //
 // (mma.sync and not tcgen05: the contraction is a band.  A 128-row tcgen05 tile would compute
 // 128 x 160 scores for the 12 or 32 each row uses and take them through tensor memory, while
-// at 16 rows a warp computes 32 or 48 per row and nothing leaves its registers; the tensor
-// time is a third of the HBM time either way.)
+// at 16 rows a warp computes 32 or 48 per row; the tensor time is a third of the HBM time
+// either way.)
 //
 // Precision is that of f32 products: q' = q qScale and rel are f32, P is f32.  Each is scaled
 // by a power of two per row and split into two halves hi + lo, 22 bits, and multiplied in two
 // (three for R) MMAs with f32 accumulation; K and V are halves already.  No operand can
 // overflow: the scale puts the row's largest element at 2^13.
 //
-// What bounds it: latency and instructions, about 2 800 per warp and 16 rows, of which 250 tensor
-// or ldmatrix (ncu: issue slots 40 % busy at 12 warps per SM, DRAM 30 %).  [32769, 3 x 8 x 128],
-// window 12: 528 us for one warp per row on the FP32 pipes (local_attn.cu) -> 98 us; the slab and
-// the output at the copy rate are 42 us.
+// What bounds it: instructions, about 1 700 per warp and 16 rows, at 12 warps per SM.
+// [32769, 3 x 8 x 128], window 12: 528 us for one warp per row on the FP32 pipes (local_attn.cu), 98 us
+// with the soft cap on the scores' own fragments and the bias rows split for every tile, 74 us; the
+// slab and the output at the copy rate are 40 us.
 #include "common.cuh"
 #include "sm100.cuh"
 #include "tc_common.cuh"
@@ -84,19 +87,50 @@ struct Local {
   static constexpr int kKeys = kRows + WP;              // staged K and V rows
   static constexpr int kQBytes = kRows * HD * 2, kKBytes = kKeys * HD * 2;
   static constexpr int kRelBytes = WP * HD * 2;         // one half of the split bias rows
-  static constexpr int kSkew = WP + 7;                  // row pitch of R: eight banks from row to row on a diagonal
-  static constexpr int kSkewBytes = 4 * 16 * kSkew * 4;
+  // A warp's scores [16][16 + WP] f32, then its probabilities as halves hi and lo, eight rows at
+  // two places each: in the warp's own q rows (of each 64-column box) where these are long enough.
+  static constexpr int kScorePitch = (WP == 16 ? 40 : 56) * 4;  // float2 stores of four rows: distinct banks
+  static constexpr int kProbPitch = WP == 16 ? 80 : 112;        // 16-byte pieces of eight rows: distinct banks
+  static constexpr bool kOwn = HD < 128;
+  static constexpr int kEight = kOwn ? 8 * kScorePitch : kRows * 128;   // from rows 0..7 to rows 8..15
   static constexpr int kQ = 0, kK = kQBytes, kV = kK + kKBytes, kRelHi = kV + kKBytes,
-                       kRelLo = kRelHi + kRelBytes, kSkewAt = kRelLo + kRelBytes,
-                       kSmem = kSkewAt + kSkewBytes + 1024;
+                       kRelLo = kRelHi + kRelBytes, kScratch = kRelLo + kRelBytes,
+                       kSmem = kScratch + (kOwn ? 4 * 2 * 8 * kScorePitch : 0) + 1024;
+  static_assert(16 * kProbPitch <= 8 * kScorePitch && (kOwn || 8 * kScorePitch <= 16 * 128), "fits its place");
 };
+
+// One row of one head from global memory, by one warp: rows whose tile holds numbers that are not
+// finite, which a probability of zero or a low half would turn into NaN.
+template <int HD>
+__device__ __noinline__ void exact_row(const __half* qkv, const float* rel, const float* qScale, __half* out,
+                                       int64_t t, int h, int heads, int window, float kScale, float softcap) {
+  const int lane = threadIdx.x & 31;
+  const int64_t width = (int64_t)heads * HD, col = (int64_t)h * HD;
+  const int n = (int)min((int64_t)window, t + 1);
+  float mine = -3.402823466e38f;     // lane j: the score j rows back
+  for (int j = 0; j < n; j++) {
+    float s = 0.f;
+    for (int x = lane; x < HD; x += 32)
+      s = fmaf(__half2float(qkv[t * 3 * width + col + x]) * qScale[x],
+               fmaf(__half2float(qkv[(t - j) * 3 * width + width + col + x]), kScale, rel[j * width + col + x]), s);
+    s = softcap * tanhf(warp_sum(s) / softcap);
+    if (lane == j) mine = s;
+  }
+  const float m = warp_max(mine), e = lane < n ? expf(mine - m) : 0.f, inv = 1.f / warp_sum(e);
+  for (int x = lane; x < HD; x += 32) {
+    float acc = 0.f;
+    for (int j = 0; j < n; j++)
+      acc = fmaf(__shfl_sync(0xffffffffu, e, j), __half2float(qkv[(t - j) * 3 * width + 2 * width + col + x]), acc);
+    out[t * width + col + x] = __float2half_rn(acc * inv);
+  }
+}
 
 template <int HD, int WP>
 __global__ void __launch_bounds__(kLocalThreads, 3)
 local_attn_tc_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapKV,
-                     const float* __restrict__ rel, const float* __restrict__ qScale,
-                     __half* __restrict__ out, int64_t rows, int heads, int window, float kScale,
-                     float softcap, int* status) {
+                     const __half* __restrict__ qkv, const float* __restrict__ rel,
+                     const float* __restrict__ qScale, __half* __restrict__ out, int64_t rows, int heads,
+                     int window, float kScale, float softcap, int* status) {
   using L = Local<HD, WP>;
   constexpr int NT = (16 + WP) / 8, KS = HD / 16;       // key tiles of a warp, steps of the head
   extern __shared__ unsigned char smemRaw[];
@@ -107,22 +141,26 @@ local_attn_tc_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
   const int g = lane >> 2, t4 = lane & 3;               // fragment row and column pair
   const uint32_t base = (smem_u32(smemRaw) + 1023u) & ~1023u;
   unsigned char* const generic = smemRaw + (base - smem_u32(smemRaw));
-  const int h = (int)(blockIdx.x % (unsigned)heads);
-  const int64_t t0 = (int64_t)(blockIdx.x / (unsigned)heads) * kRows;
+  const int h = (int)(blockIdx.x % (unsigned)heads);    // the launcher makes the grid a multiple of heads
   const int width = heads * HD;
+  const int64_t tiles = (rows + kRows - 1) / kRows, step = gridDim.x / (unsigned)heads;
+  const uint32_t bar = smem_u32(&sFull);
 
-  if (tid == 0) {
-    sAbort = 0;
-    mbar_init(smem_u32(&sFull), 1);
-    fence_barrier_init();
-    const uint32_t bar = smem_u32(&sFull);
+  auto load = [&](int64_t tile) {
     mbar_expect_tx(bar, L::kQBytes + 2 * L::kKBytes);
 #pragma unroll
     for (int c = 0; c < HD; c += 64) {
-      tma_load_2d(base + L::kQ + c * 2 * kRows, &mapQ, h * HD + c, (int)t0, bar);
-      tma_load_2d(base + L::kK + c * 2 * L::kKeys, &mapKV, width + h * HD + c, (int)t0 - WP, bar);
-      tma_load_2d(base + L::kV + c * 2 * L::kKeys, &mapKV, 2 * width + h * HD + c, (int)t0 - WP, bar);
+      const int t0 = (int)(tile * kRows);
+      tma_load_2d(base + L::kQ + c * 2 * kRows, &mapQ, h * HD + c, t0, bar);
+      tma_load_2d(base + L::kK + c * 2 * L::kKeys, &mapKV, width + h * HD + c, t0 - WP, bar);
+      tma_load_2d(base + L::kV + c * 2 * L::kKeys, &mapKV, 2 * width + h * HD + c, t0 - WP, bar);
     }
+  };
+  if (tid == 0) {
+    sAbort = 0;
+    mbar_init(bar, 1);
+    fence_barrier_init();
+    load(blockIdx.x / (unsigned)heads);
   }
   // Bias rows, split into halves: a warp per distance.
   for (int j = warp; j < WP; j += 4) {
@@ -152,178 +190,205 @@ local_attn_tc_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
   }
   for (int x = tid; x < HD; x += kLocalThreads) sScale[x] = qScale[x];
   __syncthreads();
-  const bool ok = mbar_wait(smem_u32(&sFull), 0, &sAbort);
-  if (!__syncthreads_and(ok)) {
-    if (tid == 0) atomicOr(status, kStatusWaitTimeout);
-    return;
-  }
 
-  // q' = q qScale of rows g and g + 8 of the warp's 16, as A fragments: largest magnitude of a
-  // row first, then scaled and split.
   const int r0 = warp * 16;
-  uint32_t qh[KS][4], ql[KS][4];
-  float mx[2] = {0.f, 0.f};
-  auto scaled = [&](uint32_t w, int x) {
-    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w));
-    return make_float2(f.x * sScale[x], f.y * sScale[x + 1]);
-  };
+  unsigned char* const scratch =
+      generic + (L::kOwn ? L::kScratch + warp * 2 * 8 * L::kScorePitch : L::kQ + r0 * 128);
+  float* const score0 = reinterpret_cast<float*>(scratch + g * L::kScorePitch);   // row g; row g + 8 is kEight on
+  uint32_t parity = 0;
+  for (int64_t tile = blockIdx.x / (unsigned)heads; tile < tiles; tile += step, parity ^= 1) {
+    const int64_t t0 = tile * kRows;
+    const bool ok = __all_sync(0xffffffffu, mbar_wait(bar, parity, &sAbort));
+    if (ok) {
+      // q' = q qScale of rows g and g + 8 of the warp's 16, as A fragments: largest magnitude of a
+      // row first, then scaled and split.
+      uint32_t qh[KS][4], ql[KS][4];
+      float2 qf[KS][4];
+      float mx[2] = {0.f, 0.f};
 #pragma unroll
-  for (int k = 0; k < KS; k++) {
-    ldmatrix4(base + L::kQ + piece(r0 + (lane & 15), 2 * k + (lane >> 4), kRows), qh[k]);
+      for (int k = 0; k < KS; k++) {
+        ldmatrix4(base + L::kQ + piece(r0 + (lane & 15), 2 * k + (lane >> 4), kRows), qh[k]);
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const float2 f = scaled(qh[k][i], k * 16 + (i >> 1) * 8 + t4 * 2);
-      mx[i & 1] = fmaxf(mx[i & 1], fmaxf(fabsf(f.x), fabsf(f.y)));
-    }
-  }
-  float qsc[2], qinv[2];
-#pragma unroll
-  for (int i = 0; i < 2; i++) {
-    mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 1));
-    mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 2));
-    qsc[i] = row_scale(mx[i], qinv[i]);
-  }
-#pragma unroll
-  for (int k = 0; k < KS; k++)
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const float2 f = scaled(qh[k][i], k * 16 + (i >> 1) * 8 + t4 * 2);
-      split2(f.x * qsc[i & 1], f.y * qsc[i & 1], qh[k][i], ql[k][i]);
-    }
-
-  // R [16, WP], to shared memory in its natural order (row, distance).
-  float* const skew = reinterpret_cast<float*>(generic + L::kSkewAt) + warp * 16 * L::kSkew;
-#pragma unroll
-  for (int n = 0; n < WP / 8; n += 2) {
-    float r[2][4] = {};
-#pragma unroll
-    for (int k = 0; k < KS; k++) {
-      const uint32_t at = piece(n * 8 + (lane & 7) + ((lane >> 4) << 3), 2 * k + ((lane >> 3) & 1), WP);
-      uint32_t bh[4], bl[4];
-      ldmatrix4(base + L::kRelHi + at, bh);
-      ldmatrix4(base + L::kRelLo + at, bl);
-#pragma unroll
-      for (int e = 0; e < 2; e++) {
-        mma16816(r[e], qh[k], bh[2 * e], bh[2 * e + 1]);
-        mma16816(r[e], qh[k], bl[2 * e], bl[2 * e + 1]);
-        mma16816(r[e], ql[k], bh[2 * e], bh[2 * e + 1]);
-      }
-    }
-#pragma unroll
-    for (int e = 0; e < 2; e++)
-#pragma unroll
-      for (int i = 0; i < 4; i++) {
-        const int j = (n + e) * 8 + t4 * 2 + (i & 1);
-        skew[(g + (i >> 1) * 8) * L::kSkew + j] = r[e][i] * (qinv[i >> 1] * sRelInv[j]);
-      }
-  }
-  __syncwarp();
-
-  // Scores of the warp's keys (staged rows r0 .. r0 + 16 + WP), soft cap, mask.
-  float s[NT][4];
-  float m[2] = {-3.402823466e38f, -3.402823466e38f};
-  const float kq[2] = {qinv[0] * kScale, qinv[1] * kScale};
-  const int64_t firstKey = t0 - WP + r0;
-#pragma unroll
-  for (int n = 0; n < NT; n += 2) {
-#pragma unroll
-    for (int e = 0; e < 2; e++)
-#pragma unroll
-      for (int i = 0; i < 4; i++) s[n + e][i] = 0.f;
-    if (WP - (8 * n + 15) >= window) {   // both tiles lie before every row's window
-#pragma unroll
-      for (int e = 0; e < 2; e++)
-#pragma unroll
-        for (int i = 0; i < 4; i++) s[n + e][i] = -3.402823466e38f;
-      continue;
-    }
-#pragma unroll
-    for (int k = 0; k < KS; k++) {
-      uint32_t b[4];
-      ldmatrix4(base + L::kK + piece(r0 + n * 8 + (lane & 7) + ((lane >> 4) << 3),
-                                     2 * k + ((lane >> 3) & 1), L::kKeys), b);
-#pragma unroll
-      for (int e = 0; e < 2; e++) {
-        mma16816(s[n + e], qh[k], b[2 * e], b[2 * e + 1]);
-        mma16816(s[n + e], ql[k], b[2 * e], b[2 * e + 1]);
-      }
-    }
-#pragma unroll
-    for (int e = 0; e < 2; e++)
-#pragma unroll
-      for (int i = 0; i < 4; i++) {
-        const int row = g + (i >> 1) * 8, c = (n + e) * 8 + t4 * 2 + (i & 1), dist = row + WP - c;
-        const bool seen = dist >= 0 && dist < window && firstKey + c >= 0;
-        float x = -3.402823466e38f;
-        if (seen) {
-          x = fmaf(s[n + e][i], kq[i >> 1], skew[row * L::kSkew + dist]);
-          x = softcap * tanhf(x / softcap);
-          m[i >> 1] = fmaxf(m[i >> 1], x);
+        for (int i = 0; i < 4; i++) {
+          const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&qh[k][i]));
+          const float2 sc = *reinterpret_cast<const float2*>(&sScale[k * 16 + (i >> 1) * 8 + t4 * 2]);
+          qf[k][i] = make_float2(f.x * sc.x, f.y * sc.y);
+          mx[i & 1] = fmaxf(mx[i & 1], fmaxf(fabsf(qf[k][i].x), fabsf(qf[k][i].y)));
         }
-        s[n + e][i] = x;
       }
-  }
-  float sum[2] = {0.f, 0.f};
+      float qsc[2], qinv[2];
 #pragma unroll
-  for (int i = 0; i < 2; i++) {
-    m[i] = fmaxf(m[i], __shfl_xor_sync(0xffffffffu, m[i], 1));
-    m[i] = fmaxf(m[i], __shfl_xor_sync(0xffffffffu, m[i], 2));
-  }
+      for (int i = 0; i < 2; i++) {
+        mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 1));
+        mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 2));
+        qsc[i] = row_scale(mx[i], qinv[i]);
+      }
 #pragma unroll
-  for (int n = 0; n < NT; n++)
+      for (int k = 0; k < KS; k++)
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const float x = s[n][i];
-      s[n][i] = x > -3e38f ? expf(x - m[i >> 1]) : 0.f;
-      sum[i >> 1] += s[n][i];
-    }
-#pragma unroll
-  for (int i = 0; i < 2; i++) {
-    sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], 1);
-    sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], 2);
-  }
+        for (int i = 0; i < 4; i++)
+          split2(qf[k][i].x * qsc[i & 1], qf[k][i].y * qsc[i & 1], qh[k][i], ql[k][i]);
 
-  // O = P V: tiles n and n + 1 of the scores are one k-step's A fragment.
-  float o[HD / 8][4];
+      // R [16, WP]: this lane has rows g (0, 1) and g + 8 (2, 3), distances 8 n + 2 t4 and the next.
+      float r[WP / 8][4];
 #pragma unroll
-  for (int x = 0; x < HD / 8; x++)
+      for (int n = 0; n < WP / 8; n += 2) {
 #pragma unroll
-    for (int i = 0; i < 4; i++) o[x][i] = 0.f;
+        for (int e = 0; e < 2; e++)
 #pragma unroll
-  for (int n = 0; n < NT; n += 2) {
-    if (WP - (8 * n + 15) >= window) continue;
-    uint32_t ph[4], pl[4];
+          for (int i = 0; i < 4; i++) r[n + e][i] = 0.f;
 #pragma unroll
-    for (int i = 0; i < 4; i++)
-      split2(s[n + (i >> 1)][(i & 1) * 2], s[n + (i >> 1)][(i & 1) * 2 + 1], ph[i], pl[i]);
+        for (int k = 0; k < KS; k++) {
+          const uint32_t at = piece(n * 8 + (lane & 7) + ((lane >> 4) << 3), 2 * k + ((lane >> 3) & 1), WP);
+          uint32_t bh[4], bl[4];
+          ldmatrix4(base + L::kRelHi + at, bh);
+          ldmatrix4(base + L::kRelLo + at, bl);
 #pragma unroll
-    for (int x = 0; x < HD / 8; x += 2) {
-      uint32_t b[4];
-      ldmatrix4_trans(base + L::kV + piece(r0 + n * 8 + (lane & 15), x + (lane >> 4), L::kKeys), b);
+          for (int e = 0; e < 2; e++) {
+            mma16816(r[n + e], qh[k], bh[2 * e], bh[2 * e + 1]);
+            mma16816(r[n + e], qh[k], bl[2 * e], bl[2 * e + 1]);
+            mma16816(r[n + e], ql[k], bh[2 * e], bh[2 * e + 1]);
+          }
+        }
+      }
+      __syncwarp();      // the warp's q rows are in registers: their place is free
+
+      // Scores of the warp's keys (staged rows r0 .. r0 + 16 + WP), to where a lane finds the keys
+      // at its own distances.
 #pragma unroll
-      for (int e = 0; e < 2; e++) {
-        mma16816(o[x + e], ph, b[2 * e], b[2 * e + 1]);
-        mma16816(o[x + e], pl, b[2 * e], b[2 * e + 1]);
+      for (int n = 0; n < NT; n += 2) {
+        if (WP - (8 * n + 15) >= window) continue;   // both tiles lie before every row's window
+        float s[2][4] = {};
+#pragma unroll
+        for (int k = 0; k < KS; k++) {
+          uint32_t b[4];
+          ldmatrix4(base + L::kK + piece(r0 + n * 8 + (lane & 7) + ((lane >> 4) << 3),
+                                         2 * k + ((lane >> 3) & 1), L::kKeys), b);
+#pragma unroll
+          for (int e = 0; e < 2; e++) {
+            mma16816(s[e], qh[k], b[2 * e], b[2 * e + 1]);
+            mma16816(s[e], ql[k], b[2 * e], b[2 * e + 1]);
+          }
+        }
+#pragma unroll
+        for (int e = 0; e < 2; e++)
+#pragma unroll
+          for (int i = 0; i < 2; i++)
+            *reinterpret_cast<float2*>(score0 + i * (L::kEight / 4) + (n + e) * 8 + t4 * 2) =
+                make_float2(s[e][2 * i], s[e][2 * i + 1]);
+      }
+      __syncwarp();
+
+      // Soft cap, mask and softmax by (row, distance).
+      float m[2] = {-3.402823466e38f, -3.402823466e38f}, sum[2] = {0.f, 0.f};
+#pragma unroll
+      for (int n = 0; n < WP / 8; n++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const int row = g + (i >> 1) * 8, dist = n * 8 + t4 * 2 + (i & 1);
+          float x = -3.402823466e38f;
+          if (dist < window && dist <= t0 + r0 + row) {
+            const float dot = score0[(i >> 1) * (L::kEight / 4) + row + WP - dist];
+            x = fmaf(dot, qinv[i >> 1] * kScale, r[n][i] * (qinv[i >> 1] * sRelInv[dist]));
+            x = softcap * tanhf(x / softcap);
+            m[i >> 1] = fmaxf(m[i >> 1], x);
+          }
+          r[n][i] = x;
+        }
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        m[i] = fmaxf(m[i], __shfl_xor_sync(0xffffffffu, m[i], 1));
+        m[i] = fmaxf(m[i], __shfl_xor_sync(0xffffffffu, m[i], 2));
+      }
+      __syncwarp();      // every score is read: its place takes the probabilities
+#pragma unroll
+      for (int i = lane; i < 2 * 16 * L::kProbPitch / 16; i += 32) {
+        constexpr int kPieces = 16 * L::kProbPitch / 16;
+        *reinterpret_cast<uint4*>(scratch + (i / kPieces) * L::kEight + i % kPieces * 16) = make_uint4(0, 0, 0, 0);
+      }
+      __syncwarp();
+#pragma unroll
+      for (int n = 0; n < WP / 8; n++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const int row = g + (i >> 1) * 8, dist = n * 8 + t4 * 2 + (i & 1);
+          if (dist < window && dist <= t0 + r0 + row) {
+            const float pe = expf(r[n][i] - m[i >> 1]);
+            sum[i >> 1] += pe;
+            __half* at = reinterpret_cast<__half*>(scratch + (i >> 1) * L::kEight + g * L::kProbPitch) + row + WP - dist;
+            const __half hi = __float2half_rn(pe);
+            *at = hi;
+            at[8 * L::kProbPitch / 2] = __float2half_rn(pe - __half2float(hi));
+          }
+        }
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], 1);
+        sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], 2);
+      }
+      __syncwarp();
+
+      // O = P V, sixteen keys at a time.
+      float o[HD / 8][4];
+#pragma unroll
+      for (int x = 0; x < HD / 8; x++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) o[x][i] = 0.f;
+#pragma unroll
+      for (int n = 0; n < NT; n += 2) {
+        if (WP - (8 * n + 15) >= window) continue;
+        uint32_t ph[4], pl[4];
+        const uint32_t at = smem_u32(scratch) + ((lane >> 3) & 1) * L::kEight + (lane & 7) * L::kProbPitch +
+                            (n + (lane >> 4)) * 16;
+        ldmatrix4(at, ph);
+        ldmatrix4(at + 8 * L::kProbPitch, pl);
+#pragma unroll
+        for (int x = 0; x < HD / 8; x += 2) {
+          uint32_t b[4];
+          ldmatrix4_trans(base + L::kV + piece(r0 + n * 8 + (lane & 15), x + (lane >> 4), L::kKeys), b);
+#pragma unroll
+          for (int e = 0; e < 2; e++) {
+            mma16816(o[x + e], ph, b[2 * e], b[2 * e + 1]);
+            mma16816(o[x + e], pl, b[2 * e], b[2 * e + 1]);
+          }
+        }
+      }
+      __syncwarp();      // the probabilities are read: q's place takes the output
+
+      // Through the warp's own q rows to whole 16-byte pieces of output rows.
+      const float inv[2] = {1.f / sum[0], 1.f / sum[1]};   // distance 0 always exists: sum >= 1
+      bool odd = false;
+#pragma unroll
+      for (int x = 0; x < HD / 8; x++)
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+          const float a = o[x][2 * i] * inv[i], b = o[x][2 * i + 1] * inv[i];
+          odd |= !(fabsf(a) + fabsf(b) < INFINITY);
+          *reinterpret_cast<__half2*>(generic + L::kQ + piece(r0 + g + i * 8, x, kRows) + t4 * 4) =
+              __floats2half2_rn(a, b);
+        }
+      odd = __any_sync(0xffffffffu, odd);
+#pragma unroll
+      for (int i = lane; i < 16 * HD / 8; i += 32) {
+        const int rr = i / (HD / 8), c = i % (HD / 8);
+        const int64_t row = t0 + r0 + rr;
+        if (row < rows)
+          *reinterpret_cast<uint4*>(out + row * width + (int64_t)h * HD + c * 8) =
+              *reinterpret_cast<const uint4*>(generic + L::kQ + piece(r0 + rr, c, kRows));
+      }
+      if (odd) {
+        __syncwarp();
+        for (int i = 0; i < 16 && t0 + r0 + i < rows; i++)
+          exact_row<HD>(qkv, rel, qScale, out, t0 + r0 + i, h, heads, window, kScale, softcap);
       }
     }
-  }
-
-  // Through the warp's own q rows (read long ago) to whole 16-byte pieces of output rows.
-  const float inv[2] = {1.f / sum[0], 1.f / sum[1]};   // distance 0 always exists: sum >= 1
-#pragma unroll
-  for (int x = 0; x < HD / 8; x++)
-#pragma unroll
-    for (int i = 0; i < 2; i++)
-      *reinterpret_cast<__half2*>(generic + L::kQ + piece(r0 + g + i * 8, x, kRows) + t4 * 4) =
-          __floats2half2_rn(o[x][2 * i] * inv[i], o[x][2 * i + 1] * inv[i]);
-  __syncwarp();
-#pragma unroll
-  for (int i = lane; i < 16 * HD / 8; i += 32) {
-    const int r = i / (HD / 8), c = i % (HD / 8);
-    const int64_t row = t0 + r0 + r;
-    if (row < rows)
-      *reinterpret_cast<uint4*>(out + row * width + (int64_t)h * HD + c * 8) =
-          *reinterpret_cast<const uint4*>(generic + L::kQ + piece(r0 + r, c, kRows));
+    // Everyone is done with the tile; what the threads wrote into it comes before the next copy.
+    fence_proxy_async();
+    if (!__syncthreads_and(ok)) {
+      if (tid == 0) atomicOr(status, kStatusWaitTimeout);
+      return;
+    }
+    if (tid == 0 && tile + step < tiles) load(tile + step);
   }
 }
 
@@ -340,9 +405,13 @@ cudaError_t launch(const void* qkv, const float* rel, const float* qScale, void*
   auto kern = local_attn_tc_kernel<HD, WP>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kSmem);
   if (e != cudaSuccess) return e;
-  const int64_t blocks = (rows + kRows - 1) / kRows * heads;
-  kern<<<(unsigned)blocks, kLocalThreads, L::kSmem, s>>>(mq, mkv, rel, qScale, static_cast<__half*>(out),
-                                                         rows, heads, window, kScale, softcap, status);
+  // As many blocks of a head as are resident at once (three per SM): each splits its head's bias
+  // rows once and walks every step-th tile.
+  const int64_t tiles = (rows + kRows - 1) / kRows, most = 3 * 148 / heads;
+  const int64_t perHead = tiles < most ? tiles : most < 1 ? 1 : most;
+  kern<<<(unsigned)(perHead * heads), kLocalThreads, L::kSmem, s>>>(
+      mq, mkv, static_cast<const __half*>(qkv), rel, qScale, static_cast<__half*>(out), rows, heads, window, kScale,
+      softcap, status);
   return cudaGetLastError();
 }
 
