@@ -235,7 +235,7 @@ int run_decode(rt_ctx* ctx, rt::DecodeParams& p, int dtype) {
   p.counters = ctx->counters;
   p.status = ctx->statusDev;
   RT_CUDA(ctx, rt::launch_decode(p, dtype, ctx->stream));
-  ctx->launches++;
+  ctx->launches += p.mergeAfter ? 2 : 1;
   return RT_OK;
 }
 

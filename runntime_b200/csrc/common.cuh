@@ -107,6 +107,7 @@ struct DecodeParams {
   int32_t kvPerCta;     // kv heads handled by one CTA
   int32_t keySlots;     // keys processed concurrently by one CTA
   int32_t stages;       // smem ring depth (bulk path)
+  int32_t mergeAfter;   // the splits are merged by a second launch
   int32_t lanesPerRow;  // threads that share one (key, head) pair, each a slice of the head (1, 2, 4)
   // fused rope (null tables = off) and row strides of q / kNew / vNew, in elements
   const float* ropeCos;
@@ -339,7 +340,7 @@ cudaError_t launch_prefill_tc3(const AttnParams& p, bool pair, int* status, cuda
 bool prefill_tc4_supported(const AttnParams& p, int dtype);
 cudaError_t launch_prefill_tc4(const AttnParams& p, int* status, int* work, int smCount,
                                cudaStream_t s, std::string* err);
-// Fills kvPerCta/keySlots/stages/splits; returns false with a message when the shape cannot run.
+// Fills kvPerCta/keySlots/stages/splits/mergeAfter; returns false with a message when the shape cannot run.
 bool plan_decode(DecodeParams& p, int dtype, int smCount, std::string* err);
 cudaError_t launch_decode(const DecodeParams& p, int dtype, cudaStream_t s);
 cudaError_t launch_merge_partials(const float* partials, int parts, int64_t units, int hd,

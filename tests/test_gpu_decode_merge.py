@@ -1,0 +1,41 @@
+"""The merge of a decode launch's key splits: more splits than lanes, more (head, split) weights
+than fit at once, odd head sizes (single columns), splits that see no key, partials out."""
+import numpy as np
+import pytest
+
+import oracle
+from gpu_harness import ex  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f16"])
+@pytest.mark.parametrize("splits", [2, 17, 33, 64])
+@pytest.mark.parametrize("heads,kvHeads,hd", [(8, 8, 36), (3, 1, 37), (64, 1, 128), (200, 1, 8), (5, 5, 1)])
+def test_against_the_oracle(ex, dtype, splits, heads, kvHeads, hd):
+    import torch
+    from runntime_b200.engine import decode_batched
+    batch, rows = 3, 150
+    lens = [150, 1, 70]          # with 64 splits most hold no key of a short sequence
+    td = torch.float16 if dtype == "f16" else torch.float32
+    g = torch.Generator().manual_seed(splits * hd)
+    q, k, v = (torch.randn(*s, generator=g).to(td) for s in
+               ((batch, heads * hd), (batch, rows, kvHeads * hd), (batch, rows, kvHeads * hd)))
+    q = (q * hd ** -0.5).to(td)
+    dq, dk, dv = q.cuda(), k.cuda(), v.cuda()
+    out = torch.empty_like(dq)
+    part = torch.empty(batch, heads, 2 + hd, device="cuda")
+    dl = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    kw = dict(dtype=dtype, batch=batch, cacheRows=rows, qHeads=heads, kvHeads=kvHeads, headDim=hd,
+              kvLen=rows, kvLens=dl, splits=splits)
+    decode_batched(ex, dq, out, dk, dv, **kw)
+    decode_batched(ex, dq, out, dk, dv, partialsOut=part, **kw)
+    ex.sync()
+    for b, n in enumerate(lens):
+        want = oracle.sdpa_ref(q[b:b + 1].float().numpy(), k[b, :n].float().numpy(), v[b, :n].float().numpy(),
+                               qHeads=heads, kvHeads=kvHeads, headDim=hd)
+        oracle.assert_close(out[b].float().cpu().numpy(), np.asarray(want).reshape(-1), dtype, f"out {b}")
+        p = part[b].cpu().numpy()
+        assert (p[:, 1] > 0).all()
+        oracle.assert_close((p[:, 2:] / p[:, 1:2]).reshape(-1), np.asarray(want).reshape(-1), dtype, f"partials {b}")
