@@ -173,6 +173,44 @@ __device__ __forceinline__ void process_key(const T* kp, const T* vp, const floa
   }
 }
 
+// Two keys of one head at once (heads without a rotation: 36 and 52 columns): q is read once for
+// both, and their two dot products and updates are independent instruction streams, which a block
+// alone on its SM has too few warps to do without.
+template <typename T, int HDP, int VEC>
+__device__ __forceinline__ void process_two(const T* ka, const T* va, const T* kb, const T* vb, const float* qv,
+                                            float& m, float& l, float (&acc)[HDP]) {
+  static_assert(VEC == 4, "q in pieces of four");
+  float a0 = 0.f, a1 = 0.f, b0 = 0.f, b1 = 0.f;
+#pragma unroll
+  for (int i = 0; i < HDP / VEC; i++) {
+    float fa[VEC], fb[VEC];
+    Loader<T, VEC>::load(ka + i * VEC, fa);
+    Loader<T, VEC>::load(kb + i * VEC, fb);
+    const float4 q = *reinterpret_cast<const float4*>(qv + i * VEC);
+    a0 = fmaf(q.x, fa[0], a0), a1 = fmaf(q.y, fa[1], a1), a0 = fmaf(q.z, fa[2], a0), a1 = fmaf(q.w, fa[3], a1);
+    b0 = fmaf(q.x, fb[0], b0), b1 = fmaf(q.y, fb[1], b1), b0 = fmaf(q.z, fb[2], b0), b1 = fmaf(q.w, fb[3], b1);
+  }
+  const float sa = (a0 + a1) * kLog2e, sb = (b0 + b1) * kLog2e;  // log2 domain
+  const float mn = fmaxf(sa, sb);
+  if (mn > m) {
+    const float c = fast_exp2(m - mn);
+    l *= c;
+#pragma unroll
+    for (int x = 0; x < HDP; x++) acc[x] *= c;
+    m = mn;
+  }
+  const float pa = fast_exp2(sa - m), pb = fast_exp2(sb - m);
+  l += pa + pb;
+#pragma unroll
+  for (int i = 0; i < HDP / VEC; i++) {
+    float fa[VEC], fb[VEC];
+    Loader<T, VEC>::load(va + i * VEC, fa);
+    Loader<T, VEC>::load(vb + i * VEC, fb);
+#pragma unroll
+    for (int e = 0; e < VEC; e++) acc[i * VEC + e] = fmaf(pa, fa[e], fmaf(pb, fb[e], acc[i * VEC + e]));
+  }
+}
+
 // The same for a thread that owns W = hd / R columns of the (key, head) pair, R = 2 or 4
 // adjacent lanes sharing the pair (head size 64 and 128: a whole 128-wide row per thread
 // costs 512 bytes of every stage and 128 accumulator registers, so few keys fit a tile
@@ -726,7 +764,8 @@ decode_kernel(const DecodeParams p) {
 
   bool ok = true;
   int it = 0;
-  if constexpr (R > 1) {
+  constexpr bool PAIRS = BULK && (R > 1 || (EXACT && !ROT && VEC == 4));
+  if constexpr (PAIRS) {
     // Tiles two at a time while the ring is deep enough to keep copies in flight behind them.
     if (stages >= 4) {
       for (; it + 1 < ntiles; it += 2) {
@@ -742,7 +781,12 @@ decode_kernel(const DecodeParams p) {
         if (active) {
           const int off = slot * sliceElems + kvl * hd + sub * W;
           const int vOff = tileBytes / (int)sizeof(T);
-          if (slot < nkb)
+          if constexpr (R == 1) {
+            if (slot < nkb)
+              process_two<T, HDP, VEC>(aK + off, aK + vOff + off, bK + off, bK + vOff + off, qv, m, l, acc);
+            else
+              process_key<T, HDP, EXACT, VEC, QSMEM>(aK + off, aK + vOff + off, qv, hd, m, l, acc, rot);
+          } else if (slot < nkb)
             process_key_pair<T, W, VEC, R>(aK + off, aK + vOff + off, bK + off, bK + vOff + off, qr, m,
                                            l, acc, rot, groupMask);
           else
@@ -1137,20 +1181,23 @@ bool plan_decode(DecodeParams& p, int dtype, int smCount, std::string* err) {
       nmax = nmax < 1 ? 1 : nmax > p.cacheRows ? p.cacheRows : nmax;
     }
     if (!p.useRange && p.wl < nmax) nmax = (int64_t)p.wl + 1;
-    int64_t maxS = nmax / (4ll * keySlots);  // at least four tiles per split
-    if (maxS > 32) maxS = 32;
+    int64_t maxS = nmax / keySlots;   // at least one tile per split
+    if (maxS > 64) maxS = 64;
     if (maxS < 1) maxS = 1;
-    // Cost in units of one tile's streaming time: every CTA pays a fixed set-up,
+    // Cost in eighths of one tile's streaming time: every CTA pays a fixed set-up,
     // pipeline-fill and merge cost (about three tiles' worth, measured), CTAs run in
-    // waves of `resident` at a time, and splitting adds the partials pass.  Measured
-    // on B200: with at least one wave of sequences, not splitting is fastest.
+    // waves of `resident` at a time, and splitting adds the partials pass, three tiles and an
+    // eighth per split.  Measured on B200: with at least one wave of sequences, not splitting is
+    // fastest; alone, a sequence of 415 keys takes 12.9 / 10.2 / 9.1 us in 1 / 3 / 13 splits, one of
+    // 1250 keys 28.3 / 10.4 / 12.2 in 1 / 20 / 39, one of 4096 keys x 32 heads of 128 50 / 35 in
+    // 32 / 64.
     const int64_t resident = (int64_t)smCount * ctasPerSm;
     int best = 1;
     int64_t bestCost = INT64_MAX;
     for (int s = 1; s <= maxS; s++) {
       const int64_t tilesPerCta = (nmax + (int64_t)s * keySlots - 1) / ((int64_t)s * keySlots);
       const int64_t waves = (ctas * s + resident - 1) / resident;
-      const int64_t cost = waves * (3 + tilesPerCta) + (s > 1 ? 3 : 0);
+      const int64_t cost = 8 * waves * (3 + tilesPerCta) + (s > 1 ? 24 + s : 0);
       if (cost < bestCost) {
         bestCost = cost;
         best = s;
@@ -1305,7 +1352,13 @@ int rt_attn_decode_noalloc(const rt_decode_args* a, void* cuda_stream) {
   if (!plan_decode(p, a->dtype, smCount, &err)) return static_fail(RT_INVALID_ARGUMENT, err);
   const size_t zBlocks = (size_t)(p.kvHeads + p.kvPerCta - 1) / p.kvPerCta;
   const size_t sets = p.hasSecond ? 2 : 1;
-  const size_t needFloats = p.splits > 1 ? sets * p.batch * p.splits * p.qHeads * (2 + p.hd) : 0;
+  const size_t perSplit = sets * p.batch * p.qHeads * (2 + p.hd);
+  const size_t fit = kStaticScratchFloats / perSplit;
+  if (a->splits == 0 && (size_t)p.splits > fit && fit >= 2) {
+    p.splits = (int)fit;   // the plan's own choice: as many as the area holds
+    if (!plan_decode(p, a->dtype, smCount, &err)) return static_fail(RT_INVALID_ARGUMENT, err);
+  }
+  const size_t needFloats = p.splits > 1 ? p.splits * perSplit : 0;
   const size_t needCounters = p.splits > 1 ? sets * p.batch * zBlocks : 0;
   if (needFloats > kStaticScratchFloats || needCounters > kStaticCounters)
     return static_fail(
