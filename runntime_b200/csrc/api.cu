@@ -393,10 +393,11 @@ int rt_buf_download(rt_ctx* ctx, const void* device_ptr, size_t offset, void* ho
 // 0 = FP32-pipe kernel, 1 = tensor cores, one query tile per CTA, 2 = two tiles per CTA,
 // 3 = one tile with two softmax warpgroups on alternate key tiles, 4 = the same in pairs of
 // CTAs that share every K/V tile, 5 = the persistent form of 3 (one CTA per SM, units
-// overlapping), 6 = f32 on the tensor cores.
+// overlapping), 6 = f32 on the tensor cores, 7 = packed short segments.
 static int prefill_kernel_of(const rt_ctx* ctx, const rt::AttnParams& p, int dtype) {
   if (!ctx->useTc) return 0;
   if (rt::prefill_f32_tc_supported(p, dtype)) return 6;
+  if (ctx->useTc == 1 && rt::prefill_mma_supported(p, dtype)) return 7;
   const bool tc3 = rt::prefill_tc3_supported(p, dtype);
   if (ctx->useTc == 6 && rt::prefill_tc4_supported(p, dtype)) return 5;
   if (ctx->useTc == 5 && rt::prefill_tc3_pair_supported(p, dtype)) return 4;
@@ -415,7 +416,7 @@ static int prefill_kernel_of(const rt_ctx* ctx, const rt::AttnParams& p, int dty
 static const char* route_of(const rt_ctx* ctx, const rt_attn_args* a) {
   if (a->qLen == 1) return "decode";
   const int k = prefill_kernel_of(ctx, to_params(a), a->dtype);
-  return k == 6 ? "prefill_f32_tc" : k == 5 ? "prefill_tc4" : k == 4 ? "prefill_tc3_pair" : k == 3 ? "prefill_tc3" : k == 2 ? "prefill_tc2" : k == 1 ? "prefill_tc" : "prefill_simt";
+  return k == 7 ? "prefill_mma" : k == 6 ? "prefill_f32_tc" : k == 5 ? "prefill_tc4" : k == 4 ? "prefill_tc3_pair" : k == 3 ? "prefill_tc3" : k == 2 ? "prefill_tc2" : k == 1 ? "prefill_tc" : "prefill_simt";
 }
 
 int rt_attn_route(rt_ctx* ctx, const rt_attn_args* args, const char** route) {
@@ -454,7 +455,9 @@ int rt_attn(rt_ctx* ctx, const rt_attn_args* a) {
   }
   const rt::AttnParams p = to_params(a);
   const int kernel = prefill_kernel_of(ctx, p, a->dtype);
-  if (kernel == 6) {
+  if (kernel == 7) {
+    RT_CUDA(ctx, rt::launch_prefill_mma(p, ctx->stream));
+  } else if (kernel == 6) {
     RT_CUDA(ctx, rt::launch_prefill_f32_tc(p, ctx->stream));
   } else if (kernel != 0) {
     std::string err;
