@@ -20,6 +20,7 @@ struct rt_ctx {
   unsigned* counters;
   size_t counterCount;
   int* statusDev;
+  int* statusHost;   // pinned: the status word comes back on the stream, without a second wait
   int64_t launches;
   int useTc;
   int waitPolls;   // polls of the cross-GPU merge's wait before it gives up
@@ -275,6 +276,7 @@ int rt_ctx_create(int device, rt_ctx** out) {
   ctx->waitPolls = 1 << 20;   // about a second with the kernel's sleeps
   if ((e = cudaSetDevice(device)) != cudaSuccess ||
       (e = cudaStreamCreateWithFlags(&ctx->own, cudaStreamNonBlocking)) != cudaSuccess ||
+      (e = cudaMallocHost(&ctx->statusHost, sizeof(int))) != cudaSuccess ||
       (e = cudaMalloc(&ctx->statusDev, kStatusWords * sizeof(int))) != cudaSuccess ||
       (e = cudaMemset(ctx->statusDev, 0, kStatusWords * sizeof(int))) != cudaSuccess) {
     delete ctx;
@@ -291,10 +293,12 @@ int rt_ctx_destroy(rt_ctx* ctx) {
   if (ctx->scratch) cudaFree(ctx->scratch);
   if (ctx->counters) cudaFree(ctx->counters);
   cudaFree(ctx->statusDev);
+  cudaFreeHost(ctx->statusHost);
   cudaStreamDestroy(ctx->own);
   ctx->scratch = nullptr;
   ctx->counters = nullptr;
   ctx->statusDev = nullptr;
+  ctx->statusHost = nullptr;
   ctx->magic = kDead;
   std::lock_guard<std::mutex> lock(gGraveyardMutex);
   gGraveyard.push_back(ctx);
@@ -331,11 +335,10 @@ const char* rt_last_error(const rt_ctx* ctx) {
   return tlsError.c_str();
 }
 
-int rt_sync(rt_ctx* ctx) {
-  RT_ENTER(ctx);
+// Waits for the stream and for the copy of the status word that is on it; what the word says.
+static int finish(rt_ctx* ctx) {
   RT_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  int status = 0;
-  RT_CUDA(ctx, cudaMemcpy(&status, ctx->statusDev, sizeof(int), cudaMemcpyDeviceToHost));
+  const int status = *ctx->statusHost;
   if (status != 0) {
     // (with the status word, the work counter of the persistent prefill kernel, which a
     // block that gave up never rewound)
@@ -351,6 +354,16 @@ int rt_sync(rt_ctx* ctx) {
                       "per-sequence cache pointer is not 16-byte aligned");
   }
   return RT_OK;
+}
+
+static cudaError_t copy_status(rt_ctx* ctx) {
+  return cudaMemcpyAsync(ctx->statusHost, ctx->statusDev, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
+}
+
+int rt_sync(rt_ctx* ctx) {
+  RT_ENTER(ctx);
+  RT_CUDA(ctx, copy_status(ctx));
+  return finish(ctx);
 }
 
 int64_t rt_launch_count(const rt_ctx* ctx) {
@@ -385,9 +398,10 @@ int rt_buf_upload(rt_ctx* ctx, void* device_ptr, size_t offset, const void* host
 int rt_buf_download(rt_ctx* ctx, const void* device_ptr, size_t offset, void* host, size_t bytes) {
   RT_ENTER(ctx);
   if (!device_ptr || !host) return fail(ctx, RT_INVALID_ARGUMENT, "rt_buf_download: NULL pointer");
+  RT_CUDA(ctx, copy_status(ctx));   // ahead of the data, whose copy to pageable memory waits
   RT_CUDA(ctx, cudaMemcpyAsync(host, static_cast<const char*>(device_ptr) + offset, bytes,
                                cudaMemcpyDeviceToHost, ctx->stream));
-  return rt_sync(ctx);
+  return finish(ctx);
 }
 
 // 0 = FP32-pipe kernel, 1 = tensor cores, one query tile per CTA, 2 = two tiles per CTA,

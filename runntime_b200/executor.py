@@ -159,7 +159,9 @@ class CudaExecutor:
     def dispatch(self, node: Value, inputs: Sequence[DeviceBuffer], out: DeviceBuffer,
                  extras: Optional[dict] = None) -> None:
         op = node.pending.op
-        if op == "attn":
+        if op == "matmul":
+            self._dispatch_matmul(node, inputs, out)
+        elif op == "attn":
             self._dispatch_attn(node, inputs, out, extras)
         elif op == "writeRows":
             self._dispatch_write_rows(node, inputs)
@@ -169,36 +171,20 @@ class CudaExecutor:
             self._dispatch_slice(node, inputs, out)
         elif op == "softmax":
             self._dispatch_softmax(node, inputs, out)
-        elif op == "matmul":
-            hasBias, hasAddend, act, baseRow, _ = (int(v) for v in node.pending.attrs)
-            ins = node.pending.inputs
-            m, k = ins[0].shape.dims
-            bRows, n = ins[1].shape.dims
-            nxt = 2
-            bias = addend = None
-            if hasBias:
-                bias = C.c_void_p(inputs[nxt].ptr)
-                nxt += 1
-            if hasAddend:
-                addend = C.c_void_p(inputs[nxt].ptr)
-            check(self._lib.rt_matmul(self.ctx, C.c_void_p(inputs[0].ptr), C.c_void_p(inputs[1].ptr),
-                                      bias, addend, C.c_void_p(out.ptr), m, k, n, bRows, baseRow,
-                                      act, DTYPE_CODE[node.shape.dtype]), self.ctx)
-            self.dispatches.append("matmul")
         elif op == "argmaxDot":
             wV = node.pending.inputs[0]
             rows, cols = wV.shape.dims
-            check(self._lib.rt_argmax_dot(self.ctx, C.c_void_p(inputs[0].ptr),
-                                          C.c_void_p(inputs[1].ptr), C.c_void_p(out.ptr), rows,
-                                          cols, DTYPE_CODE[wV.shape.dtype]), self.ctx)
+            ctx = self.ctx
+            check(self._lib.rt_argmax_dot(ctx, inputs[0].ptr, inputs[1].ptr, out.ptr, rows, cols,
+                                          DTYPE_CODE[wV.shape.dtype]), ctx)
             self.dispatches.append("argmaxDot")
         elif op == "localAttention":
             heads, hd, window, kScale, softcap = node.pending.attrs
+            ctx = self.ctx
             check(self._lib.rt_local_attention(
-                self.ctx, C.c_void_p(inputs[0].ptr), C.c_void_p(inputs[1].ptr),
-                C.c_void_p(inputs[2].ptr), C.c_void_p(out.ptr), node.shape.dims[0], int(heads),
-                int(hd), int(window), float(kScale), float(softcap),
-                DTYPE_CODE[node.shape.dtype]), self.ctx)
+                ctx, inputs[0].ptr, inputs[1].ptr, inputs[2].ptr, out.ptr, node.shape.dims[0],
+                int(heads), int(hd), int(window), float(kScale), float(softcap),
+                DTYPE_CODE[node.shape.dtype]), ctx)
             self.dispatches.append("localAttention")
         else:
             raise RunntimeError("INVALID_ARGUMENT", f"dispatch: no kernel for op '{op}'")
@@ -220,6 +206,17 @@ class CudaExecutor:
                 v.markReleased("released by releaseValues")
 
     # -- per-op encoders -----------------------------------------------------------
+    def _dispatch_matmul(self, node, inputs, out):
+        hasBias, hasAddend, act, baseRow, _ = node.pending.attrs
+        a, b = node.pending.inputs[:2]
+        m, k = a.shape.dims
+        bRows, n = b.shape.dims
+        ctx = self.ctx
+        check(self._lib.rt_matmul(ctx, inputs[0].ptr, inputs[1].ptr, inputs[2].ptr if hasBias else None,
+                                  inputs[2 + int(hasBias)].ptr if hasAddend else None, out.ptr, m, k, n,
+                                  bRows, int(baseRow), int(act), DTYPE_CODE[node.shape.dtype]), ctx)
+        self.dispatches.append("matmul")
+
     def _dispatch_attn(self, node, inputs, out, extras):
         a = node.pending.attrs
         qHeads, kvHeads, hd, wl, wr, qPosOffset, hasSinks, hasSegs, maxSegment, packed = (
@@ -260,31 +257,26 @@ class CudaExecutor:
             check(self._lib.rt_attn_decode(self.ctx, C.byref(d)), self.ctx)
             self.dispatches.append("decode+rope+append" if "ropeCos" in fused else "decode+append")
             return
-        args = AttnArgs()
-        args.q, args.k, args.v, args.out = q.ptr, k.ptr, v.ptr, out.ptr
-        args.sinks = sinks.ptr if sinks else None
-        args.segments = segs.ptr if segs else None
-        args.dtype = DTYPE_CODE[node.shape.dtype]
-        args.qkvPacked = packed
-        args.qLen, args.kvLen = qLen, kvLen
-        args.qHeads, args.kvHeads, args.headDim = qHeads, kvHeads, hd
-        args.windowLeft, args.windowRight, args.maxSegment = wl, wr, maxSegment
-        args.qPosOffset = qPosOffset
+        # (fields in the order of the structure)
+        args = AttnArgs(q.ptr, k.ptr, v.ptr, out.ptr, sinks.ptr if sinks else None,
+                        segs.ptr if segs else None, DTYPE_CODE[node.shape.dtype], packed, qLen, kvLen,
+                        qHeads, kvHeads, hd, wl, wr, maxSegment, qPosOffset)
         if len(a) > 10 and a[10]:
             args.hasKeyBias, args.biasStart, args.biasEnd = 1, int(a[11]), int(a[12])
             args.biasValue = float(a[13])
+        ctx = self.ctx
         route = C.c_char_p()
-        check(self._lib.rt_attn_route(self.ctx, C.byref(args), C.byref(route)), self.ctx)
-        check(self._lib.rt_attn(self.ctx, C.byref(args)), self.ctx)
+        check(self._lib.rt_attn_route(ctx, C.byref(args), C.byref(route)), ctx)
+        check(self._lib.rt_attn(ctx, C.byref(args)), ctx)
         self.dispatches.append(route.value.decode())
 
     def _dispatch_rope(self, node, inputs, out):
         xV = node.pending.inputs[0]
         headDim, srcStart, width = (int(a) for a in node.pending.attrs)
         rows, cols = xV.shape.dims
-        check(self._lib.rt_rope(self.ctx, C.c_void_p(inputs[0].ptr), C.c_void_p(inputs[1].ptr),
-                                C.c_void_p(inputs[2].ptr), C.c_void_p(out.ptr), rows, cols,
-                                headDim, srcStart, width, DTYPE_CODE[xV.shape.dtype]), self.ctx)
+        ctx = self.ctx
+        check(self._lib.rt_rope(ctx, inputs[0].ptr, inputs[1].ptr, inputs[2].ptr, out.ptr, rows, cols,
+                                headDim, srcStart, width, DTYPE_CODE[xV.shape.dtype]), ctx)
         self.dispatches.append("rope")
 
     def _dispatch_softmax(self, node, inputs, out):
@@ -304,8 +296,9 @@ class CudaExecutor:
         rows, cols = xV.shape.dims
         start, end = (int(a) for a in node.pending.attrs)
         box = (start, end, 0, cols) if node.pending.op == "sliceRows" else (0, rows, start, end)
-        check(self._lib.rt_slice(self.ctx, C.c_void_p(inputs[0].ptr), C.c_void_p(out.ptr), rows,
-                                 cols, *box, DTYPE_CODE[xV.shape.dtype]), self.ctx)
+        ctx = self.ctx
+        check(self._lib.rt_slice(ctx, inputs[0].ptr, out.ptr, rows, cols, *box,
+                                 DTYPE_CODE[xV.shape.dtype]), ctx)
         self.dispatches.append(node.pending.op)
 
     def _dispatch_write_rows(self, node, inputs):
@@ -326,14 +319,16 @@ def _collect_pending(targets: Sequence[Value]) -> List[Value]:
     seen = set()
 
     def visit(v: Value) -> None:
-        if v.state == "released":
+        # (the fields behind Value.state, which is asked once per edge of the graph)
+        if v._released is not None:
             op = v.pending.op if v.pending else "upload"
-            raise RuntimeError(f"evalValues: '{op}': {v.releasedReason}")
-        if v.state == "materialized" or id(v) in seen:
+            raise RuntimeError(f"evalValues: '{op}': {v._released}")
+        if v._buffer is not None or v in seen:
             return
-        seen.add(id(v))
+        seen.add(v)
         for i in v.pending.inputs:
-            visit(i)
+            if i._buffer is None or i._released is not None:
+                visit(i)
         order.append(v)
 
     for t in targets:
@@ -347,6 +342,8 @@ def _fusable_appends(order: List[Value], targets: Sequence[Value]) -> Dict[int, 
     appends at that position used by nothing else in this evaluation.  The plan
     also names the rope / slice nodes feeding q and the new rows that the kernel
     can absorb ("elided": used once, not targets, rope over the same tables)."""
+    if not any(n.pending.op == "writeRows" for n in order):
+        return {}
     uses: Dict[int, int] = {}
     for n in order:
         for i in n.pending.inputs:
@@ -422,51 +419,66 @@ def _fused_extras(f: dict) -> dict:
 def evalValues(targets: Sequence[Value], ex: CudaExecutor) -> None:
     """Dispatches every pending node the targets depend on, once, in dependency
     order; intermediates go back to the pool after their last consumer."""
+    # Values are compared and hashed by identity, so they are the keys themselves.
     order = _collect_pending(targets)
-    produced = {id(v) for v in order}
-    target_ids = {id(t) for t in targets}
     fuse = _fusable_appends(order, targets)
-    skipped = {id(w) for f in fuse.values() for w in (f["k"], f["v"])}
+    skipped = {w for f in fuse.values() for w in (f["k"], f["v"])}
     # Nodes a fused kernel computes on the fly: never dispatched, they stay pending.
-    elided = {id(w) for f in fuse.values() for w in f["elided"]}
-    remaining: Dict[int, int] = {}
+    elided = {w for f in fuse.values() for w in f["elided"]}
+    # Readers left of every value made here; targets have one that never reads.
+    left: Dict[Value, int] = dict.fromkeys(order, 0)
+    for t in targets:
+        if t in left:
+            left[t] = 1
     for n in order:
         for i in set(n.pending.inputs):
-            remaining[id(i)] = remaining.get(id(i), 0) + 1
+            if i in left:
+                left[i] += 1
     aliased = set()
     for node in order:
-        if id(node) in elided:
+        if node in elided:
             continue
         p = node.pending
-        ins = [None if id(i) in elided else i.buffer for i in p.inputs]
+        if elided:
+            ins = [None if i in elided else i.buffer for i in p.inputs]
+        else:
+            ins = [i.buffer for i in p.inputs]
+        consumed = p.inputs
         if p.op in IN_PLACE_OPS:
             out = ins[0]
-            aliased.add(id(node))
-            if id(node) not in skipped:
+            aliased.add(node)
+            if node not in skipped:
                 ex.dispatch(node, ins, out)
+            node.setMaterialized(out)
+            if node in skipped:
+                continue  # its inputs are read by the fused kernel: released after that one
         else:
             out = ex.acquireOutput(node.shape)
-            extras = None
-            if id(node) in fuse:
-                extras = {"fusedAppend": _fused_extras(fuse[id(node)])}
-            ex.dispatch(node, ins, out, extras)
-        node.setMaterialized(out)
-        if id(node) in skipped:
-            continue  # its inputs are read by the fused kernel: released after that one
-        consumed = [p.inputs]
-        if id(node) in fuse:
-            f = fuse[id(node)]
-            consumed += [f["k"].pending.inputs, f["v"].pending.inputs]
-            consumed += [w.pending.inputs for w in f["elided"]]
-        for group in consumed:
-            for i in set(group):
-                remaining[id(i)] -= 1
-                if (remaining[id(i)] == 0 and id(i) in produced and id(i) not in target_ids):
-                    if id(i) in aliased or id(i) in elided:
-                        continue  # a view of a caller-owned buffer / never materialized
-                    ex.releaseOutput(i.buffer, i.shape)
-                    i.markReleased()
+            f = fuse.get(id(node)) if fuse else None
+            ex.dispatch(node, ins, out, {"fusedAppend": _fused_extras(f)} if f else None)
+            node.setMaterialized(out)
+            if f:
+                _release(f["k"].pending.inputs, left, aliased, elided, ex, after=p.inputs)
+                _release(f["v"].pending.inputs, left, aliased, elided, ex)
+                for w in f["elided"]:
+                    _release(w.pending.inputs, left, aliased, elided, ex)
+                continue
+        _release(consumed, left, aliased, elided, ex)
     ex.submit()
+
+
+def _release(inputs, left, aliased, elided, ex, after=()) -> None:
+    """One reader less of each of a node's inputs; those that nobody reads any more go back."""
+    for group in (after, inputs):
+        for i in set(group):
+            n = left.get(i)
+            if n is None:
+                continue
+            left[i] = n = n - 1
+            if n == 0 and i not in aliased and i not in elided:
+                # (views of a caller-owned buffer and values never materialized stay)
+                ex.releaseOutput(i.buffer, i.shape)
+                i.markReleased()
 
 
 def toArray(value: Value, ex: CudaExecutor) -> np.ndarray:

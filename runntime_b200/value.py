@@ -3,16 +3,14 @@ pending op (packages/runntime/src/core/graph/value.ts:123-200).  Calling ops
 only links nodes; reading a result evaluates what it depends on."""
 from __future__ import annotations
 
-from dataclasses import dataclass
-from typing import Optional, Sequence, Tuple
+from typing import NamedTuple, Optional, Sequence, Tuple
 
 
 def elemBytes(dtype: str) -> int:
     return 2 if dtype == "f16" else 4
 
 
-@dataclass(frozen=True)
-class ValueMeta:
+class ValueMeta(NamedTuple):
     elems: int
     dtype: str = "f32"
     dims: Optional[Tuple[int, ...]] = None
@@ -22,8 +20,7 @@ def matrix(rows: int, cols: int, dtype: str = "f32") -> ValueMeta:
     return ValueMeta(rows * cols, dtype, (rows, cols))
 
 
-@dataclass(frozen=True)
-class PendingOp:
+class PendingOp(NamedTuple):
     op: str
     inputs: Tuple["Value", ...]
     scalar: Optional[float] = None
@@ -40,6 +37,8 @@ class DeviceBuffer:
 
 
 class Value:
+    __slots__ = ("shape", "_buffer", "pending", "_released", "__weakref__", "__dict__")
+
     def __init__(self, shape: ValueMeta, buffer: Optional[DeviceBuffer],
                  pending: Optional[PendingOp]):
         self.shape = shape
