@@ -764,7 +764,8 @@ decode_kernel(const DecodeParams p) {
 
   bool ok = true;
   int it = 0;
-  constexpr bool PAIRS = BULK && (R > 1 || (EXACT && !ROT && VEC == 4));
+  // (f32 tiles are too large for a ring of four of them)
+  constexpr bool PAIRS = BULK && (R > 1 || (EXACT && !ROT && VEC == 4 && sizeof(T) == 2));
   if constexpr (PAIRS) {
     // Tiles two at a time while the ring is deep enough to keep copies in flight behind them.
     if (stages >= 4) {
