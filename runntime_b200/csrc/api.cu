@@ -626,6 +626,11 @@ int rt_matmul(rt_ctx* ctx, const void* a, const void* b, const void* bias, const
     ctx->launches++;
     return RT_OK;
   }
+  if (ctx->useTc && rt::matmul_f32_tc_supported(a, bp, addend, out, m, k, n, dtype)) {
+    RT_CUDA(ctx, rt::launch_matmul_f32_tc(a, bp, bias, addend, out, m, k, n, activation, ctx->stream));
+    ctx->launches++;
+    return RT_OK;
+  }
   const size_t need = rt::matmul_scratch_need(m, k, n, dtype);
   if (need) {
     const int s = ensure_scratch(ctx, need, 1);

@@ -367,6 +367,11 @@ bool matmul_tc_supported(const void* a, const void* b, const void* out, int64_t 
 cudaError_t launch_matmul_tc(const void* a, const void* b, const void* bias, const void* addend,
                              void* out, int64_t M, int64_t K, int64_t N, int act, int* status,
                              cudaStream_t s, std::string* err);
+// f32 matmul on the tensor cores (more than 16 rows, K and N multiples of four, 16-byte tensors).
+bool matmul_f32_tc_supported(const void* a, const void* b, const void* addend, const void* out, int64_t M,
+                             int64_t K, int64_t N, int dtype);
+cudaError_t launch_matmul_f32_tc(const void* a, const void* b, const void* bias, const void* addend, void* out,
+                                 int64_t M, int64_t K, int64_t N, int act, cudaStream_t s);
 cudaError_t launch_argmax_dot(const void* w, const void* x, float* out, int64_t V, int64_t N,
                               int dtype, unsigned long long* scratch, cudaStream_t s);
 cudaError_t launch_local_attn(const void* qkv, const float* rel, const float* qScale, void* out,

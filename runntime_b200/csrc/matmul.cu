@@ -11,7 +11,8 @@
 //    row pieces of b (8 or 16 bytes per lane) while the few rows of a come from L1;
 //    the warps' sums meet in shared memory.  b is read once (twice for M > 8).
 //  - tiled (any M): 64 x 64 output tile per block, 16-deep K steps through shared memory,
-//    4 x 4 outputs per thread.  This is the general fallback, not a tensor-core GEMM.
+//    4 x 4 outputs per thread.  This is the general fallback for shapes that the tensor-core
+//    kernels (matmul_tc.cu, matmul_f32_tc.cu) do not take.
 #include <cfloat>
 #include <type_traits>
 #include "common.cuh"
