@@ -22,7 +22,8 @@
 // (three for R) MMAs with f32 accumulation; K and V are halves already.  No operand can
 // overflow: the scale puts the row's largest element at 2^13.
 //
-// What bounds it: instructions, about 1 700 per warp and 16 rows, at 12 warps per SM.
+// What bounds it: instructions, about 1 900 per warp and 16 rows, at 12 warps per SM (issue slots 43 %
+// busy, DRAM 40 %).
 // [32769, 3 x 8 x 128], window 12: 528 us for one warp per row on the FP32 pipes (local_attn.cu), 98 us
 // with the soft cap on the scores' own fragments and the bias rows split for every tile, 74 us; the
 // slab and the output at the copy rate are 40 us.

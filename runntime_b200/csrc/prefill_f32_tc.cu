@@ -6,7 +6,8 @@
 // accumulator less carefully than an FMA does, so no accumulator lives long: scores add 32 columns of
 // the head before they join the f32 sum (hi hi' apart from the 2^-11 smaller cross terms), and 16 keys
 // are added, their cross terms first, before they join the f32 output.  Against 64-bit
-// products: 4.6e-7 of the norm at head size 256 (1.5e-6 for sequential f32 sums), 2.6e-7 to 3.7e-7 below.
+// products: 4.2e-7 to 4.8e-7 of the norm at head size 256 (1.5e-6 to 1.7e-6 for sequential f32 sums),
+// 1.9e-7 to 3.0e-7 below (2.4e-7 to 9.1e-7).
 //
 // A CTA of eight warps owns 32 query rows of one query head and walks 128-key tiles of the union of
 // its rows' bands.  For the scores a warp takes all rows and 16 of the keys, for the output all
@@ -17,9 +18,10 @@
 //
 // Why not prefill_simt.cu: two-wide FMAs with three different operands run at 48 of the
 // 73 TFLOP/s, tf32 MMAs at 275, 92 in threes.
-// What bounds it: instructions and latency with two warps per scheduler (a third of them MMAs), and the
-// last row tiles.  8 sequences of 92..484 rows, 3 heads of 256 on one K/V head (2.4 GFLOP, 27 us at
-// 92 TFLOP/s): 583 us for 16-row tiles of scalar FMAs, 155 for prefill_simt.cu, 102 here.
+// What bounds it: instructions and latency with two warps per scheduler (8.7 instructions per MMA, the
+// MMA pipe 32 % of active cycles), and the last row tiles.  8 sequences of 92..484 rows, 3 heads of
+// 256 on one K/V head (2.4 GFLOP, 27 us at 92 TFLOP/s): 583 us for 16-row tiles of scalar FMAs, 155
+// for prefill_simt.cu, 102 here.
 //
 // Numbers that are not finite (an input's infinity times another's low part is NaN where the
 // product should be infinite) show in the output: such row tiles are computed again by
