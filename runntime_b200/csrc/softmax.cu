@@ -5,33 +5,57 @@
 // packages/runntime/src/core/kernels/reduce/softmax.ts:111-186).
 //
 // HBM-bound: one read of the kept scores and one write of the row.  A row is handled by one
-// warp (eight rows per CTA) or by one CTA.  Memory is touched in
-// 16-byte chunks at 16-byte addresses wherever the row starts: a row of an odd width begins in
-// the middle of a chunk, and only its first and last chunk go element by element.  The zeros
-// outside the kept range need no statistics, so they are stored while the first chunk of scores
-// is on its way; then a running (max, sum) per thread, and a second look at the kept scores
-// (L1/L2 by then) writes exp(x - max) / sum.
+// warp (narrow rows, eight per CTA) or by one CTA; the first pass keeps a running (max, sum) per
+// thread, the second re-reads the row (it is in L1/L2 by then) and writes exp(x - max) / sum.
 //
-// Measured, f16 [6007, 6007] with 24 segments (75 MB, 11 us at the copy rate): 55.3 us with
-// odd rows element by element, 20.5 us in chunks.
+// Rows that start on four elements are taken four at a time.  Any other row begins in the middle of
+// a 16-byte chunk: memory is still touched in 16-byte chunks at 16-byte addresses, only the row's
+// first and last chunk go element by element, and the zeros outside the kept range, which need no
+// statistics, are stored while the first scores are on their way.  Element by element, chunks, us: f16
+// [6007, 6007] with 24 segments (75 MB, 11 us at the copy rate) 55.5, 20.8 (55.3, 24.6 through the
+// operator), with one 74.6, 71.9; f32
+// 51.4, 31.0 with 24.  On aligned rows the quads are the faster ones: f16 [12288, 12288] with 2
+// segments 119 against 141, [2500, 2500] with 3 12.4 against 18.7.
 #include "common.cuh"
 
 namespace rt {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kAhead = 4;
-// One warp per row for narrow rows, and wherever there are rows enough to fill the chip with
-// warps: no block-wide reduction, and the idle lanes of a narrow kept range cost one warp
-// instead of eight (f16 [6007, 6007], 24 segments: 28.7 us with a CTA per row,
-// 20.5 with a warp).
-constexpr int kWarpRowCols = 2048, kWarpRows = 2048;
+constexpr int kAhead = 2, kCtas = 5;
+// One warp per row up to kWarpRowCols columns, one CTA beyond.  Of that CTA one warp alone takes a
+// kept range of up to kWarpKept columns, without a block barrier, while all of them store the
+// zeros (f16 [6007, 6007], 24 segments: 28.7 us with all warps on the kept range, 20.8).
+constexpr int kWarpRowCols = 2048, kWarpKept = 1024;
 constexpr float kNegMax = -3.402823466e38f;
 
-// N elements that are read and written together.
-template <typename T, int N>
-struct alignas(N * sizeof(T)) Chunk {
-  T e[N];
+template <typename T>
+struct Quad;
+template <>
+struct Quad<float> {
+  using type = float4;
+  static __device__ __forceinline__ void unpack(const float4& v, float (&f)[4]) {
+    f[0] = v.x, f[1] = v.y, f[2] = v.z, f[3] = v.w;
+  }
+  static __device__ __forceinline__ float4 pack(const float (&f)[4]) {
+    return make_float4(f[0], f[1], f[2], f[3]);
+  }
+};
+template <>
+struct Quad<__half> {
+  using type = uint2;
+  static __device__ __forceinline__ void unpack(const uint2& v, float (&f)[4]) {
+    const __half2* h = reinterpret_cast<const __half2*>(&v);
+    const float2 a = __half22float2(h[0]), b = __half22float2(h[1]);
+    f[0] = a.x, f[1] = a.y, f[2] = b.x, f[3] = b.y;
+  }
+  static __device__ __forceinline__ uint2 pack(const float (&f)[4]) {
+    uint2 v;
+    __half2* h = reinterpret_cast<__half2*>(&v);
+    h[0] = __floats2half2_rn(f[0], f[1]);
+    h[1] = __floats2half2_rn(f[2], f[3]);
+    return v;
+  }
 };
 
 __device__ __forceinline__ void combine(float& m, float& s, float m2, float s2) {
@@ -40,14 +64,13 @@ __device__ __forceinline__ void combine(float& m, float& s, float m2, float s2) 
   m = mNew;
 }
 
-// WARP: one warp per row, else one CTA per row.  V: elements per chunk.
-template <typename T, bool WARP, int V>
+// Rows that start on four elements: quads.  WARP: one warp per row, else one CTA per row.
+template <typename T, bool WARP>
 __global__ void __launch_bounds__(kThreads)
-softmax_kernel(const T* __restrict__ x, T* __restrict__ out, const float* __restrict__ segs,
+softmax_quad_kernel(const T* __restrict__ x, T* __restrict__ out, const float* __restrict__ segs,
                int64_t rows, int64_t cols, int64_t wl, int64_t wr) {
-  using C = Chunk<T, V>;
-  // chunk and column numbers: the launcher takes V > 1 only for rows shorter than 2^31
-  using I = std::conditional_t<V == 1, int64_t, int>;
+  using Q = Quad<T>;
+  using QV = typename Q::type;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t row = WARP ? (int64_t)blockIdx.x * (kThreads / 32) + warp : (int64_t)blockIdx.x;
   if (row >= rows) return;  // uniform per warp (WARP) or per CTA
@@ -55,12 +78,119 @@ softmax_kernel(const T* __restrict__ x, T* __restrict__ out, const float* __rest
   const int span = WARP ? 32 : kThreads;
 
   // Kept columns [lo, hi).
-  int64_t lo64 = 0, hi64 = cols;
+  int64_t lo = 0, hi = cols;
   if (segs) {
     const int64_t s0 = (int64_t)segs[2 * row], s1 = (int64_t)segs[2 * row + 1];
-    lo64 = max(s0, row - min(row, wl));
-    hi64 = min(s1, row + min(cols - row, wr + 1));
+    lo = max(s0, row - min(row, wl));
+    hi = min(s1, row + min(cols - row, wr + 1));
   }
+
+  const T* xr = x + row * cols;
+  T* orow = out + row * cols;
+  float m = kNegMax, s = 0.f;
+  // Quads of columns [q0, q1) touch the kept range; only the first and the last of them
+  // can hold masked columns (32-bit column arithmetic: the launcher takes this path only for
+  // rows shorter than 2^31).
+  const int lo32 = (int)lo, hi32 = (int)hi;
+  const int q0 = lo32 >> 2, q1 = hi32 > lo32 ? (hi32 + 3) >> 2 : q0;
+  const QV* xq = reinterpret_cast<const QV*>(xr);
+  {
+    for (int i = q0 + t; i < q1; i += span) {
+      float f[4];
+      Q::unpack(xq[i], f);
+      const int j = i * 4;
+      const bool inner = j >= lo32 && j + 4 <= hi32;
+      if (!inner) {
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+          if (j + e < lo32 || j + e >= hi32) f[e] = kNegMax;
+      }
+      // one running-sum rescale per quad instead of per element: five exponentials for four columns
+      const float mNew = fmaxf(m, fmaxf(fmaxf(f[0], f[1]), fmaxf(f[2], f[3])));
+      float add = 0.f;
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        const float pe = __expf(f[e] - mNew);
+        add += (inner || (j + e >= lo32 && j + e < hi32)) ? pe : 0.f;
+      }
+      s = s * __expf(m - mNew) + add;
+      m = mNew;
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    combine(m, s, __shfl_xor_sync(0xffffffffu, m, o), __shfl_xor_sync(0xffffffffu, s, o));
+  if (!WARP) {
+    __shared__ float sM[kThreads / 32], sS[kThreads / 32];
+    if (lane == 0) sM[warp] = m, sS[warp] = s;
+    __syncthreads();
+    m = sM[0], s = sS[0];
+#pragma unroll
+    for (int w = 1; w < kThreads / 32; w++) combine(m, s, sM[w], sS[w]);
+  }
+  const float inv = s > 0.f ? 1.f / s : 0.f;
+
+  {
+    QV* oq = reinterpret_cast<QV*>(orow);
+    const int nq = (int)(cols >> 2);
+    // zeros either side of the kept range: stores only
+    const float z4[4] = {0.f, 0.f, 0.f, 0.f};
+    const QV zero = Q::pack(z4);
+#pragma unroll 4
+    for (int i = t; i < q0; i += span) oq[i] = zero;
+#pragma unroll 4
+    for (int i = q1 + t; i < nq; i += span) oq[i] = zero;
+    for (int i = q0 + t; i < q1; i += span) {
+      float f[4];
+      Q::unpack(xq[i], f);
+      const int j = i * 4;
+      if (j >= lo32 && j + 4 <= hi32) {
+#pragma unroll
+        for (int e = 0; e < 4; e++) f[e] = __expf(f[e] - m) * inv;
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+          f[e] = (j + e >= lo32 && j + e < hi32) ? __expf(f[e] - m) * inv : 0.f;
+      }
+      oq[i] = Q::pack(f);
+    }
+  }
+}
+
+// N elements that are read and written together.
+template <typename T, int N>
+struct alignas(N * sizeof(T)) Chunk {
+  T e[N];
+};
+
+// Who works on a row: a warp; all warps of a CTA; or one warp on the kept columns while all warps
+// store the zeros.
+enum class By { Warp, Cta, WarpInCta };
+
+// Kept columns [lo, hi) of a row.
+__device__ __forceinline__ void kept_range(const float* segs, int64_t row, int64_t cols, int64_t wl, int64_t wr,
+                                           int64_t& lo, int64_t& hi) {
+  lo = 0, hi = cols;
+  if (segs) {
+    const int64_t s0 = (int64_t)segs[2 * row], s1 = (int64_t)segs[2 * row + 1];
+    lo = max(s0, row - min(row, wl));
+    hi = min(s1, row + min(cols - row, wr + 1));
+  }
+}
+
+// One row.  V: elements per chunk.
+template <typename T, By BY, int V>
+__device__ __forceinline__ void softmax_row(const T* __restrict__ x, T* __restrict__ out, int64_t row, int64_t cols,
+                                            int64_t lo64, int64_t hi64, float* sM, float* sS) {
+  using C = Chunk<T, V>;
+  // chunk and column numbers: the launcher takes V > 1 only for rows shorter than 2^31
+  using I = std::conditional_t<V == 1, int64_t, int>;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int t = BY == By::Cta ? threadIdx.x : lane;      // for the kept columns
+  const int span = BY == By::Cta ? kThreads : 32;
+  const int zt = BY == By::Warp ? lane : threadIdx.x;    // for the zeros
+  const int zspan = BY == By::Warp ? 32 : kThreads;
+  const bool keeps = BY != By::WarpInCta || warp == 0;
 
   // The row begins `mis` elements into its first chunk (the same for x and out: see the
   // launcher), so column j is element (j + mis) % V of chunk (j + mis) / V.
@@ -102,21 +232,23 @@ softmax_kernel(const T* __restrict__ x, T* __restrict__ out, const float* __rest
     for (int u = 0; u < kAhead; u++)
       if (c + u * span < q1) ahead[u] = load(c + u * span);
   };
-  loadAhead(q0 + t);
+  if (keeps) loadAhead(q0 + t);
   {
     C zero;
 #pragma unroll
     for (int e = 0; e < V; e++) zero.e[e] = from_f32<T>(0.f);
     const I left = min(q0, w1), right = max(q1, w0);
 #pragma unroll 4
-    for (I c = w0 + t; c < left; c += span) oc[c] = zero;
+    for (I c = w0 + zt; c < left; c += zspan) oc[c] = zero;
 #pragma unroll 4
-    for (I c = right + t; c < w1; c += span) oc[c] = zero;
-    if (V > 1 && t < 2) {   // the row's ragged chunks, where no kept column is in them
-      const I c = t == 0 ? 0 : nc - 1;
+    for (I c = right + zt; c < w1; c += zspan) oc[c] = zero;
+    if (V > 1 && zt < 2) {   // the row's ragged chunks, where no kept column is in them
+      const I c = zt == 0 ? 0 : nc - 1;
       if ((c < w0 || c >= w1) && (c < q0 || c >= q1)) store(c, zero);
     }
   }
+
+  if (!keeps) return;
 
   float m = kNegMax, s = 0.f;
   for (I c = q0 + t; c < q1; c += kAhead * span) {
@@ -144,16 +276,21 @@ softmax_kernel(const T* __restrict__ x, T* __restrict__ out, const float* __rest
       m = mNew;
     }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-    combine(m, s, __shfl_xor_sync(0xffffffffu, m, o), __shfl_xor_sync(0xffffffffu, s, o));
-  if (!WARP) {
-    __shared__ float sM[kThreads / 32], sS[kThreads / 32];
+  // one exponential per thread and one per warp: the maxima first, then the sums brought to them
+  const float top = warp_max(m);
+  s = warp_sum(s * __expf(m - top));
+  m = top;
+  if (BY == By::Cta) {
+    constexpr int kWarps = kThreads / 32;
     if (lane == 0) sM[warp] = m, sS[warp] = s;
     __syncthreads();
-    m = sM[0], s = sS[0];
+    const float mw = sM[lane % kWarps];
+    m = mw;
 #pragma unroll
-    for (int w = 1; w < kThreads / 32; w++) combine(m, s, sM[w], sS[w]);
+    for (int o = kWarps / 2; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    s = sS[lane % kWarps] * __expf(mw - m);
+#pragma unroll
+    for (int o = kWarps / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   }
   const float inv = s > 0.f ? 1.f / s : 0.f;
 
@@ -176,14 +313,36 @@ softmax_kernel(const T* __restrict__ x, T* __restrict__ out, const float* __rest
 }
 
 template <typename T, int V>
+__global__ void __launch_bounds__(kThreads, kCtas)
+softmax_cta_kernel(const T* __restrict__ x, T* __restrict__ out, const float* __restrict__ segs, int64_t cols,
+                   int64_t wl, int64_t wr) {
+  __shared__ float sM[kThreads / 32], sS[kThreads / 32];
+  int64_t lo, hi;
+  kept_range(segs, blockIdx.x, cols, wl, wr, lo, hi);
+  if (hi - lo <= kWarpKept) softmax_row<T, By::WarpInCta, V>(x, out, blockIdx.x, cols, lo, hi, nullptr, nullptr);
+  else softmax_row<T, By::Cta, V>(x, out, blockIdx.x, cols, lo, hi, sM, sS);
+}
+
+template <typename T, int V>
+__global__ void __launch_bounds__(kThreads, kCtas)
+softmax_warp_kernel(const T* __restrict__ x, T* __restrict__ out, const float* __restrict__ segs, int64_t rows,
+                    int64_t cols, int64_t wl, int64_t wr) {
+  const int64_t row = (int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  int64_t lo, hi;
+  kept_range(segs, row, cols, wl, wr, lo, hi);
+  softmax_row<T, By::Warp, V>(x, out, row, cols, lo, hi, nullptr, nullptr);
+}
+
+template <typename T, int V>
 cudaError_t softmax_chunked(const T* x, T* out, const float* segs, int64_t rows, int64_t cols,
                             int64_t wl, int64_t wr, cudaStream_t s) {
-  const bool warpRows = cols <= kWarpRowCols || rows >= kWarpRows;
+  const bool warpRows = cols <= kWarpRowCols;
   const int64_t blocks = warpRows ? (rows + kThreads / 32 - 1) / (kThreads / 32) : rows;
   if (blocks > 0x7fffffffll) return cudaErrorInvalidValue;
   const unsigned g = (unsigned)blocks;
-  if (warpRows) softmax_kernel<T, true, V><<<g, kThreads, 0, s>>>(x, out, segs, rows, cols, wl, wr);
-  else softmax_kernel<T, false, V><<<g, kThreads, 0, s>>>(x, out, segs, rows, cols, wl, wr);
+  if (warpRows) softmax_warp_kernel<T, V><<<g, kThreads, 0, s>>>(x, out, segs, rows, cols, wl, wr);
+  else softmax_cta_kernel<T, V><<<g, kThreads, 0, s>>>(x, out, segs, cols, wl, wr);
   return cudaGetLastError();
 }
 
@@ -194,6 +353,15 @@ cudaError_t softmax_typed(const void* x, void* out, const float* segs, int64_t r
                           int64_t wl, int64_t wr, cudaStream_t s) {
   auto* xi = static_cast<const T*>(x);
   auto* oi = static_cast<T*>(out);
+  const uintptr_t both = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out);
+  if (cols % 4 == 0 && cols < (1ll << 31) - 8 && both % (4 * sizeof(T)) == 0) {
+    const bool warpRows = cols <= kWarpRowCols;
+    const int64_t blocks = warpRows ? (rows + kThreads / 32 - 1) / (kThreads / 32) : rows;
+    if (blocks > 0x7fffffffll) return cudaErrorInvalidValue;
+    if (warpRows) softmax_quad_kernel<T, true><<<(unsigned)blocks, kThreads, 0, s>>>(xi, oi, segs, rows, cols, wl, wr);
+    else softmax_quad_kernel<T, false><<<(unsigned)blocks, kThreads, 0, s>>>(xi, oi, segs, rows, cols, wl, wr);
+    return cudaGetLastError();
+  }
   const uintptr_t apart = reinterpret_cast<uintptr_t>(x) ^ reinterpret_cast<uintptr_t>(out);
   const bool shortRows = cols < (1ll << 31) - 4096;
   if (shortRows && apart % 16 == 0) return softmax_chunked<T, 16 / sizeof(T)>(xi, oi, segs, rows, cols, wl, wr, s);
