@@ -439,6 +439,7 @@ prefill_f32_tc_kernel(const AttnParams p, int tilesPerSeq) {
 #pragma unroll
         for (int w = 0; w < kWarps; w++) sum += sSum[w][r];
         const float invL = sum > 0.f ? 1.f / sum : 0.f;  // empty band -> zeros
+        odd |= !(sum < INFINITY);   // a NaN score: the sum says so whatever its parts did to the output
 #pragma unroll
         for (int half = 0; half < 2; half++) {
           const int x = 32 * colSet + 8 * t4 + 4 * half, e = 2 * i + half;

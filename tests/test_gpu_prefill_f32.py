@@ -78,3 +78,37 @@ def test_values_past_the_split(ex, route, value):
     oracle.assert_close(got[finite], want[finite], "f32", "finite part")
     seen = got[40:, 5]
     assert (np.sign(seen) == np.sign(value)).all() and (np.abs(seen) > 1e30).all()
+
+
+def scores_ref(q, k, v):
+    """Causal attention of one head in f64: a score of -inf weighs nothing, a row with one of
+    +inf or NaN is NaN."""
+    import torch
+    q, k, v = (torch.from_numpy(x).double() for x in (q, k, v))
+    return torch.stack([torch.softmax(k[:i + 1] @ q[i], 0) @ v[:i + 1] for i in range(len(q))]).numpy()
+
+
+def check_marked(ex, route, hd, where, value):
+    """Column 5 of row 40 of q, k or v is `value`: the rows that see it are what the op's
+    definition gives, NaN where it is NaN; the others have nothing to do with it."""
+    import runntime_b200 as rt
+    rng = np.random.default_rng(hd)
+    x = {c: rng.standard_normal((90, hd)).astype(np.float32) * s for c, s in zip("qkv", (0.3, 0.3, 1))}
+    x[where][40, 5] = value
+    with np.errstate(all="ignore"):
+        want = scores_ref(x["q"], x["k"], x["v"])
+    got = rt.toArray(rt.sdpa(*(ex.upload(x[c], [90, hd]) for c in "qkv"),
+                             dict(qHeads=1, kvHeads=1, headDim=hd, windowLeft=np.inf, windowRight=0)), ex)
+    assert ex.dispatches[-1] == route
+    got = got.reshape(90, hd)
+    assert (np.isnan(got) == np.isnan(want)).all()
+    finite = np.isfinite(want)
+    assert not finite.all() or (where == "k" and value == -np.inf)
+    oracle.assert_close(got[finite], want[finite], "f32", f"{where} {value}")
+
+
+@pytest.mark.parametrize("hd", [32, 52, 128, 256])
+@pytest.mark.parametrize("where", ["q", "k"])
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
+def test_scores_that_are_not_finite(ex, route, hd, where, value):
+    check_marked(ex, route, hd, where, value)
