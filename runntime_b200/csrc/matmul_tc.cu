@@ -22,6 +22,7 @@
 // [288, 864] 9.0 -> 4.0 us; [4352, 384] x [384, 1152] 20.2 -> 9.1, x [384, 1536] + gelu 55 ->
 // 12.9; [4352, 1536] x [1536, 384] + addend 24 -> 11.2; [32768, 1024] x [1024, 3072] 323 -> 204
 // (1 011 TFLOP/s); 8192 x 4096 x 4096 279 -> 245 (1 124).
+#include <cfloat>
 #include "common.cuh"
 #include "sm100.cuh"
 #include "tc_common.cuh"
@@ -108,10 +109,11 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return fma2(a, b, m
 // max(x, 0) - |x|/2 * poly(t) e^(-z^2), z = x / sqrt 2.  Packed arithmetic, one reciprocal and
 // one exponential instruction per element: the special-function unit (16 per clock) is what is
 // left to bound it, 2 048 cycles for a 128 x 128 tile ([4352, 384] x [384, 1536] + gelu: 15.1 us
-// with the scalar form, 12.9 with this one).
+// with the scalar form, 12.9 with this one).  +inf stays +inf: |x| ends at the largest finite number
+// above zero, where the second term is an exact zero, and -inf is NaN as in x * 0.
 __device__ __forceinline__ float2 gelu_pair(float2 x) {
   auto both = [](float c) { return make_float2(c, c); };
-  const float2 ax = make_float2(fabsf(x.x), fabsf(x.y));
+  const float2 ax = make_float2(fabsf(fminf(x.x, FLT_MAX)), fabsf(fminf(x.y, FLT_MAX)));
   const float2 d = fma2(ax, both(0.3275911f * 0.70710678118654752f), both(1.f));
   float2 t;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t.x) : "f"(d.x));

@@ -53,3 +53,29 @@ def test_tiles(ex, m, k, n, act, bias, addend):
 @pytest.mark.parametrize("m,k,n", [(8300, 64, 1000), (130, 64, 136)])
 def test_addend_off_a_16_byte_boundary(ex, m, k, n):
     run(ex, m, k, n, None, True, True, shift=1)
+
+
+@pytest.mark.parametrize("act", [None, "tanh", "gelu", "silu", "relu", "geluTanh", "elu"])
+def test_activations_do_not_depend_on_the_row_count(ex, act):
+    """Sums at the ends of the range, infinite ones and NaN: 17 rows (this kernel) answer as 16 do
+    (the cluster kernel, whole divisions).  Finite results may differ by one rounding to f16."""
+    import numpy as np
+    import runntime_b200 as rt
+    ends = [np.inf, -np.inf, np.nan, 65504, -65504, 1e4, -1e4, 90, -90, 88, -88, 44, -44, 9, -9, 1, -1, 0, -0.0, 1e-7]
+    bias = np.zeros(128, np.float32)
+    bias[:len(ends)] = ends
+    rows = []
+    for m in (16, 17):
+        opts = dict(bias=ex.upload(bias, [128], "f16"))
+        if act:
+            opts["activation"] = act
+        y = rt.matmul(ex.upload(np.zeros((m, 64)), [m, 64], "f16"), ex.upload(np.zeros((64, 128)), [64, 128], "f16"),
+                      opts)
+        rows.append(rt.toArray(y, ex).reshape(m, 128))
+    few, many = rows[0][0], rows[1][-1]
+    assert (np.isnan(few) == np.isnan(many)).all(), (few, many)
+    assert (few[np.isinf(few) | np.isinf(many)] == many[np.isinf(few) | np.isinf(many)]).all(), (few, many)
+    finite = np.isfinite(few)
+    # (below 2^-14 halves are 2^-24 apart)
+    few, many = few[finite], many[finite]
+    assert (np.abs(few - many) <= 2.0 ** -10 * np.abs(few) + 2.0 ** -24).all(), (few, many)
