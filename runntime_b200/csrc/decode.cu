@@ -417,6 +417,8 @@ __device__ __noinline__ void merge_splits(int hd, int splits, int qHeads, const 
   }
 }
 
+constexpr float kGivenUp = -1.f;   // in the place of a split's row sum: a wait of its block ran out
+
 template <typename T, int HDP, bool EXACT, int VEC, bool BULK, int R = 1>
 __global__ void __launch_bounds__(BULK ? kConsumers + 32 : kConsumers, HDP / R <= 64 ? 2 : 1)
 decode_kernel(const DecodeParams p) {
@@ -853,6 +855,10 @@ decode_kernel(const DecodeParams p) {
   if (sAbortSeen) {
     // A wait ran out: record it, let copies in flight land, leave.
     if (tid == 0) atomicOr(p.status, kStatusWaitTimeout);
+    if (p.mergeAfter) {   // a row sum that no block leaves: the merge launch writes nothing for these heads
+      float* sums = p.scratch + (((int64_t)by * p.splits + split) * p.qHeads + kvh0 * group) * (2 + hd) + 1;
+      for (int hh = tid; hh < hqReal; hh += kConsumers) sums[hh * (2 + hd)] = kGivenUp;
+    }
     for (int i = 0; i < 64; i++) __nanosleep(4000);
     return;
   }
@@ -966,15 +972,16 @@ merge_kernel(const DecodeParams p) {
     const float M = warp_max(fmaxf(m0, m1));
     const float w0 = fast_exp2(m0 - M), w1 = fast_exp2(m1 - M);
     const float L = warp_sum(fmaf(l0, w0, l1 * w1));
+    const bool givenUp = __any_sync(0xffffffffu, l0 == kGivenUp || l1 == kGivenUp);
     sW[lane] = w0, sW[lane + 32] = w1;
     if (lane == 0) {
-      sInv = L > 0.f ? 1.f / L : 0.f;
-      if (partials) partials[0] = L > 0.f ? M * 0.6931471805599453f : kNegSeed, partials[1] = L;
+      sInv = givenUp ? kGivenUp : L > 0.f ? 1.f / L : 0.f;
+      if (partials && !givenUp) partials[0] = L > 0.f ? M * 0.6931471805599453f : kNegSeed, partials[1] = L;
     }
   }
   __syncthreads();
   const int x = threadIdx.x;
-  if (x >= hd) return;
+  if (x >= hd || sInv == kGivenUp) return;
   float o = 0.f;
 #pragma unroll 16
   for (int s = 0; s < splits; s++) o = fmaf(__ldcg(src + s * ss + 2 + x), sW[s], o);
