@@ -80,6 +80,15 @@ int enter(rt_ctx* ctx) {
 const char* dtype_name(int d) { return d == RT_F16 ? "f16" : "f32"; }
 int elem_size(int d) { return d == RT_F16 ? 2 : 4; }
 
+bool capturing(cudaStream_t stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &status) != cudaSuccess) {
+    cudaGetLastError();   // the legacy stream beside another stream's capture
+    return false;
+  }
+  return status != cudaStreamCaptureStatusNone;
+}
+
 int ensure_scratch(rt_ctx* ctx, size_t bytes, size_t counters) {
   if (bytes > ctx->scratchBytes) {
     // The old block may still be read by enqueued work.
@@ -223,14 +232,24 @@ rt::AttnParams to_params(const rt_attn_args* a) {
 
 int run_decode(rt_ctx* ctx, rt::DecodeParams& p, int dtype) {
   std::string err;
+  const bool chosen = p.splits <= 0;   // by the plan, not by the caller
   if (!rt::plan_decode(p, dtype, ctx->smCount, &err))
     return fail(ctx, RT_INVALID_ARGUMENT, "%s", err.c_str());
-  const int zBlocks = (p.kvHeads + p.kvPerCta - 1) / p.kvPerCta;
   if (p.splits > 1) {
     const size_t sets = p.hasSecond ? 2 : 1;   // a second attention has its own partials and counters
-    const size_t bytes = sets * p.batch * p.splits * p.qHeads * (2 + p.hd) * sizeof(float);
-    int s = ensure_scratch(ctx, bytes, sets * p.batch * zBlocks);
-    if (s != RT_OK) return s;
+    const size_t perSplit = sets * p.batch * p.qHeads * (2 + p.hd) * sizeof(float);
+    const size_t counters = sets * p.batch * ((p.kvHeads + p.kvPerCta - 1) / p.kvPerCta);
+    const bool grows = p.splits * perSplit > ctx->scratchBytes || counters > ctx->counterCount;
+    if (chosen && grows && capturing(ctx->stream)) {
+      // Nothing can be allocated under a capture: as many splits as the scratch at hand holds.
+      const size_t fit = counters > ctx->counterCount ? 0 : ctx->scratchBytes / perSplit;
+      p.splits = fit > 1 ? (int)fit : 1;
+      if (!rt::plan_decode(p, dtype, ctx->smCount, &err))
+        return fail(ctx, RT_INVALID_ARGUMENT, "%s", err.c_str());
+    } else {
+      const int s = ensure_scratch(ctx, p.splits * perSplit, counters);
+      if (s != RT_OK) return s;
+    }
   }
   p.scratch = ctx->scratch;
   p.counters = ctx->counters;

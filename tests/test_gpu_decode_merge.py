@@ -39,3 +39,45 @@ def test_against_the_oracle(ex, dtype, splits, heads, kvHeads, hd):
         p = part[b].cpu().numpy()
         assert (p[:, 1] > 0).all()
         oracle.assert_close((p[:, 2:] / p[:, 1:2]).reshape(-1), np.asarray(want).reshape(-1), dtype, f"partials {b}")
+
+
+@pytest.mark.parametrize("batch,heads,hd,rows", [(1, 8, 36, 100), (1, 8, 52, 415), (4, 32, 128, 700)])
+def test_a_first_call_under_capture_needs_no_allocation(batch, heads, hd, rows):
+    """A graph is captured before the context has any scratch for splits, and once more with
+    too little of it."""
+    import torch
+    import runntime_b200 as rt
+    from runntime_b200.engine import decode_batched
+    w = heads * hd
+    g = torch.Generator().manual_seed(rows)
+    q, k, v = (torch.randn(*s, generator=g).half() for s in ((batch, w), (batch, rows, w), (batch, rows, w)))
+    q = (q * hd ** -0.5).half()
+    dq, dk, dv = q.cuda(), k.cuda(), v.cuda()
+    out = torch.empty_like(dq)
+    e = rt.CudaExecutor(0)
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    try:
+        e.setStream(stream.cuda_stream)
+        call = lambda n: decode_batched(e, dq, out, dk, dv, dtype="f16", batch=batch, cacheRows=rows,  # noqa: E731
+                                        qHeads=heads, kvHeads=heads, headDim=hd, kvLen=n)
+        for warm in (None, 1):
+            if warm:    # scratch for a shorter call than the one captured
+                decode_batched(e, dq, out, dk, dv, dtype="f16", batch=1, cacheRows=rows, qHeads=heads,
+                               kvHeads=heads, headDim=hd, kvLen=rows, splits=2)
+                e.sync()
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=stream):
+                call(rows)
+            out.fill_(7)
+            torch.cuda.synchronize()
+            graph.replay()
+            torch.cuda.synchronize()
+            got = out.float().cpu().numpy()
+            for b in range(batch):
+                want = oracle.sdpa_ref(q[b:b + 1].float().numpy(), k[b].float().numpy(), v[b].float().numpy(),
+                                       qHeads=heads, kvHeads=heads, headDim=hd)
+                oracle.assert_close(got[b], np.asarray(want).reshape(-1), "f16", f"warm {warm} {b}")
+            del graph
+    finally:
+        e.dispose()
