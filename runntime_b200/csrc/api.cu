@@ -19,6 +19,11 @@ struct rt_ctx {
   size_t scratchBytes;
   unsigned* counters;
   size_t counterCount;
+  struct Outgrown {
+    void* block;
+    size_t clear;   // bytes to clear after a wait that ran out: all of counters, none of scratch
+  };
+  std::vector<Outgrown> outgrown;   // smaller scratch and counters of before
   int* statusDev;
   int* statusHost;   // pinned: the status word comes back on the stream, without a second wait
   int64_t launches;
@@ -89,26 +94,29 @@ bool capturing(cudaStream_t stream) {
   return status != cudaStreamCaptureStatusNone;
 }
 
+// Blocks that are outgrown stay until the context goes: enqueued work may still use them, and a CUDA graph
+// that the caller captured uses its own on every replay.  Each is at least half as large again as
+// the one before, so all of them together are at most twice the newest.  (The waits refuse to grow under a
+// capture, into which the clearing of new counters would go.)
 int ensure_scratch(rt_ctx* ctx, size_t bytes, size_t counters) {
   if (bytes > ctx->scratchBytes) {
-    // The old block may still be read by enqueued work.
     RT_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    if (ctx->scratch) RT_CUDA(ctx, cudaFree(ctx->scratch));
-    ctx->scratch = nullptr;
-    ctx->scratchBytes = 0;
-    size_t want = bytes + bytes / 2;
-    RT_CUDA(ctx, cudaMalloc(&ctx->scratch, want));
+    const size_t want = bytes + bytes / 2;
+    float* fresh = nullptr;
+    RT_CUDA(ctx, cudaMalloc(&fresh, want));
+    if (ctx->scratch) ctx->outgrown.push_back({ctx->scratch, 0});
+    ctx->scratch = fresh;
     ctx->scratchBytes = want;
   }
   if (counters > ctx->counterCount) {
     RT_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    if (ctx->counters) RT_CUDA(ctx, cudaFree(ctx->counters));
-    ctx->counters = nullptr;
-    ctx->counterCount = 0;
-    size_t want = counters * 2;
-    RT_CUDA(ctx, cudaMalloc(&ctx->counters, want * sizeof(unsigned)));
-    RT_CUDA(ctx, cudaMemsetAsync(ctx->counters, 0, want * sizeof(unsigned), ctx->stream));
+    const size_t want = counters * 2;
+    unsigned* fresh = nullptr;
+    RT_CUDA(ctx, cudaMalloc(&fresh, want * sizeof(unsigned)));
+    if (ctx->counters) ctx->outgrown.push_back({ctx->counters, ctx->counterCount * sizeof(unsigned)});
+    ctx->counters = fresh;
     ctx->counterCount = want;
+    RT_CUDA(ctx, cudaMemsetAsync(ctx->counters, 0, want * sizeof(unsigned), ctx->stream));
   }
   return RT_OK;
 }
@@ -311,6 +319,8 @@ int rt_ctx_destroy(rt_ctx* ctx) {
   cudaStreamSynchronize(ctx->stream);
   if (ctx->scratch) cudaFree(ctx->scratch);
   if (ctx->counters) cudaFree(ctx->counters);
+  for (const auto& o : ctx->outgrown) cudaFree(o.block);
+  ctx->outgrown.clear();
   cudaFree(ctx->statusDev);
   cudaFreeHost(ctx->statusHost);
   cudaStreamDestroy(ctx->own);
@@ -365,6 +375,8 @@ static int finish(rt_ctx* ctx) {
     // A block that gave up never counted itself in: the arrival counters of the split
     // merge are no longer zero, and the next split launch would pick the wrong last block.
     if (ctx->counters) cudaMemset(ctx->counters, 0, ctx->counterCount * sizeof(unsigned));
+    for (const auto& o : ctx->outgrown)
+      if (o.clear) cudaMemset(o.block, 0, o.clear);
     return fail(ctx, RT_EXECUTION_FAILED,
                 "a kernel reported status 0x%x (%s)", status,
                 (status & rt::kStatusWaitTimeout)

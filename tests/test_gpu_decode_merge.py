@@ -81,3 +81,42 @@ def test_a_first_call_under_capture_needs_no_allocation(batch, heads, hd, rows):
             del graph
     finally:
         e.dispose()
+
+
+def test_a_graph_keeps_its_scratch_when_a_larger_call_needs_more():
+    import torch
+    import runntime_b200 as rt
+    from runntime_b200.engine import decode_batched
+    heads, hd, rows, w = 8, 36, 415, 288
+    g = torch.Generator().manual_seed(9)
+    q, k, v = (torch.randn(*s, generator=g).half() for s in ((1, w), (rows, w), (rows, w)))
+    q = (q * hd ** -0.5).half()
+    dq, dk, dv = q.cuda(), k.cuda(), v.cuda()
+    out = torch.empty_like(dq)
+    e = rt.CudaExecutor(0)
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    try:
+        e.setStream(stream.cuda_stream)
+        kw = dict(dtype="f16", cacheRows=rows, qHeads=heads, kvHeads=heads, headDim=hd, kvLen=rows)
+        decode_batched(e, dq, out, dk, dv, batch=1, splits=13, **kw)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            decode_batched(e, dq, out, dk, dv, batch=1, splits=13, **kw)
+        n = 64
+        many = [x.expand(n, *x.shape).contiguous() for x in (dq.view(-1), dk, dv)]
+        torch.cuda.synchronize()
+        for splits in (13, 60):     # two larger scratches
+            decode_batched(e, many[0], torch.empty_like(many[0]), many[1], many[2], batch=n, splits=splits, **kw)
+        e.sync()
+        taken = [torch.full((1 << 18,), 7.0, device="cuda") for _ in range(8)]   # freed memory would be theirs
+        out.fill_(7)
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        want = oracle.sdpa_ref(*(x.float().numpy() for x in (q, k, v)), qHeads=heads, kvHeads=heads, headDim=hd)
+        oracle.assert_close(out.float().cpu().numpy().reshape(-1), np.asarray(want).reshape(-1), "f16", "replayed")
+        assert all(bool((t == 7).all()) for t in taken)
+        del graph
+    finally:
+        e.dispose()
