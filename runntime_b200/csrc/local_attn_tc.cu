@@ -18,9 +18,10 @@
 // either way.)
 //
 // Precision is that of f32 products: q' = q qScale and rel are f32, P is f32.  Each is scaled
-// by a power of two per row and split into two halves hi + lo, 22 bits, and multiplied in two
-// (three for R) MMAs with f32 accumulation; K and V are halves already.  No operand can
-// overflow: the scale puts the row's largest element at 2^13.
+// by a power of two (per row; P, whose largest is one, by 2^13) and split into two halves hi + lo,
+// 22 bits, and multiplied in two (three for R) MMAs with f32 accumulation; K and V are halves
+// already.  No operand can overflow: the scale puts the row's largest element at 2^13.  (Without a scale
+// P had an absolute 2^-25 in place of 22 bits: a key that weighs e^-12 was off by 2^-9 of itself.)
 //
 // What bounds it: instructions, about 1 900 per warp and 16 rows, at 12 warps per SM (issue slots 43 %
 // busy, DRAM 40 %).
@@ -38,6 +39,7 @@ using namespace sm100;
 using namespace tc;
 
 constexpr int kRows = 64, kLocalThreads = 128;
+constexpr float kProbScale = 8192.f;   // 2^13
 
 __device__ __forceinline__ void ldmatrix4(uint32_t addr, uint32_t (&r)[4]) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
@@ -317,9 +319,9 @@ local_attn_tc_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
             const float pe = expf(r[n][i] - m[i >> 1]);
             sum[i >> 1] += pe;
             __half* at = reinterpret_cast<__half*>(scratch + (i >> 1) * L::kEight + g * L::kProbPitch) + row + WP - dist;
-            const __half hi = __float2half_rn(pe);
+            const __half hi = __float2half_rn(pe * kProbScale);
             *at = hi;
-            at[8 * L::kProbPitch / 2] = __float2half_rn(pe - __half2float(hi));
+            at[8 * L::kProbPitch / 2] = __float2half_rn(fmaf(pe, kProbScale, -__half2float(hi)));
           }
         }
 #pragma unroll
@@ -357,7 +359,8 @@ local_attn_tc_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
       __syncwarp();      // the probabilities are read: q's place takes the output
 
       // Through the warp's own q rows to whole 16-byte pieces of output rows.
-      const float inv[2] = {1.f / sum[0], 1.f / sum[1]};   // distance 0 always exists: sum >= 1
+      // distance 0 always exists: sum >= 1
+      const float inv[2] = {1.f / (sum[0] * kProbScale), 1.f / (sum[1] * kProbScale)};
       bool odd = false;
 #pragma unroll
       for (int x = 0; x < HD / 8; x++)

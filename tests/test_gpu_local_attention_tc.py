@@ -58,3 +58,33 @@ def test_operands_past_the_range_of_a_half(ex, window):
     one when the soft cap of 2^24 leaves it as it is — so a cap that decides by sign instead."""
     check(ex, 200, 2, 128, window, softcap=4.0, qs=2.0 ** -20, rs=2.0 ** 20)
     check(ex, 200, 2, 128, window, softcap=4.0, qs=2.0 ** 16, rs=2.0 ** -20, kScale=2.0 ** -16)
+
+
+@pytest.mark.parametrize("hd,window", [(64, 12), (128, 32)])
+@pytest.mark.parametrize("apart", [6, 9, 12, 14])
+def test_a_key_that_weighs_little(ex, hd, window, apart):
+    """The row's own key outweighs the others by e^apart and has a value of zero: what is left is the
+    others' weight times values near the top of the range."""
+    import torch
+    import runntime_b200 as rt
+    rows, softcap = 100, 1e4
+    g = torch.Generator(device="cuda").manual_seed(apart)
+    qkv = torch.zeros(rows, 3 * hd, device="cuda")
+    qkv[:, 0] = 1
+    qkv[::2, 2 * hd:] = (torch.rand(rows // 2, hd, generator=g, device="cuda") + 0.5) * 3e4
+    qkv = qkv.half()
+    rel = torch.zeros(window, hd, device="cuda")
+    rel[0, 0] = apart
+    rel[2::2, 0] = torch.rand(window // 2 - 1, generator=g, device="cuda")
+    qScale = torch.ones(hd, device="cuda")
+    torch.cuda.synchronize()
+    wrap = lambda t, d: ex.wrap(t.data_ptr(), t.shape, d, keepalive=t)  # noqa: E731
+    y = rt.localAttention(wrap(qkv, "f16"), wrap(rel, "f32"), wrap(qScale, "f32"),
+                          dict(heads=1, headDim=hd, window=window, kScale=1.0, softcap=softcap))
+    got = torch.from_numpy(rt.toArray(y, ex)).cuda().double().view(rows, hd)[1::2]
+    ex.releaseValues([y])
+    want = want_of(qkv, rel, qScale, 1, hd, window, 1.0, softcap)[1::2]
+    # half an ulp of the result, and 2^-17 of it: scores up to 14 in f32 are off by 2^-20, tanhf and
+    # the exponential by a few 2^-24 of theirs (tanhf's argument times the cap: 2 ulp of the score)
+    bad = (got - want).abs() > (2.0 ** -11 + 2.0 ** -17) * want.abs() + 2.0 ** -25
+    assert not bool(bad.any()), f"{int(bad.sum())} of {bad.numel()} off, by up to {float(((got - want) / want).abs().max()):.2g} of the result"
