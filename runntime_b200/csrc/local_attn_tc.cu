@@ -138,7 +138,8 @@ local_attn_tc_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
   constexpr int NT = (16 + WP) / 8, KS = HD / 16;       // key tiles of a warp, steps of the head
   extern __shared__ unsigned char smemRaw[];
   __shared__ __align__(8) uint64_t sFull;
-  __shared__ float sRelInv[WP], sScale[HD];
+  __shared__ float sRelInv[WP];
+  __shared__ __align__(8) float sScale[HD];             // read in pairs
   __shared__ int sAbort;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t4 = lane & 3;               // fragment row and column pair
