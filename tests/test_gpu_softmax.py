@@ -133,3 +133,37 @@ def test_rows_that_start_anywhere(ex, dtype, shift, outShift, rows, cols):
     got = out.float().cpu().numpy()
     close(got[outShift:outShift + rows * cols], oracle.softmax_ref(x.reshape(rows, cols)), dtype)
     assert (got[:outShift] == 7).all() and (got[outShift + rows * cols:] == 7).all()
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f16"])
+@pytest.mark.parametrize("wl,wr", [(INF, INF), (1100, 3), (0, 0)])
+@pytest.mark.parametrize("n,shift,outShift", [(2049, 0, 0), (2051, 3, 3), (2051, 4, 0), (2051, 2, 1), (2052, 0, 0)])
+def test_masked_rows_of_a_block(ex, dtype, n, shift, outShift, wl, wr):
+    """Rows of more than 2048 columns: kept ranges of up to 1024 columns belong to one warp of the
+    block, longer ones to all of it, and all of it stores the zeros.  Ranges of no, one, 1024 and
+    1025 columns that begin or end in the row's first or last 16 bytes or beside them; nothing of
+    what the output held is left, and nothing around it is written."""
+    import ctypes as C
+    import torch
+    from runntime_b200._lib import DTYPE_CODE, WINDOW_INF, check
+    ends = [(0, 0), (5, 5), (n, n), (0, 1), (n - 1, n), (n // 2, n // 2 + 1)]
+    for kept in (1023, 1024, 1025, n - 1, n):
+        ends += [(at, at + kept) for at in (0, 1, 3, 7, 8, n - kept - 9, n - kept - 8, n - kept - 1, n - kept)
+                 if at >= 0 and at + kept <= n]
+    segs = np.array([ends[r % len(ends)] for r in range(n)], np.float32)
+    td = torch.float16 if dtype == "f16" else torch.float32
+    x = 8 * oracle.random_f32(n * n, 7)
+    x = oracle.round_f16(x) if dtype == "f16" else x
+    src = torch.zeros(n * n + 16, dtype=td, device="cuda")
+    src[shift:shift + n * n] = torch.from_numpy(x).to("cuda", td)
+    out = torch.full((n * n + 16,), 7.0, dtype=td, device="cuda")
+    dev = torch.from_numpy(segs).cuda()
+    torch.cuda.synchronize()
+    es = src.element_size()
+    check(ex._lib.rt_softmax(ex.ctx, C.c_void_p(src.data_ptr() + shift * es),
+                             C.c_void_p(out.data_ptr() + outShift * es), C.c_void_p(dev.data_ptr()), n, n,
+                             *(WINDOW_INF if w == INF else w for w in (wl, wr)), DTYPE_CODE[dtype]), ex.ctx)
+    ex.sync()
+    got = out.float().cpu().numpy()
+    close(got[outShift:outShift + n * n], oracle.softmax_ref(x.reshape(n, n), segs, wl, wr), dtype)
+    assert (got[:outShift] == 7).all() and (got[outShift + n * n:] == 7).all()
