@@ -18,7 +18,7 @@ LIB = os.path.join(HERE, "librt_attn.so")
 SOURCES = ["api.cu", "prefill_simt.cu", "prefill_f32_tc.cu", "prefill_mma.cu", "prefill_tc.cu", "prefill_tc2.cu", "prefill_tc3.cu", "prefill_tc4.cu", "decode.cu", "exchange.cu", "misc.cu", "softmax.cu",
            "local_attn.cu", "local_attn_tc.cu", "matmul.cu",
            "matmul_tc.cu", "matmul_f32_tc.cu"]
-HEADERS = ["common.cuh", "sm100.cuh", "tc_common.cuh", "exact_row.cuh", os.path.join(ROOT, "include", "rt_attn.h")]
+HEADERS = ["common.cuh", "sm100.cuh", "tc_common.cuh", "tf32.cuh", "exact_row.cuh", os.path.join(ROOT, "include", "rt_attn.h")]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

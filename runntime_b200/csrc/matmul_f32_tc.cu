@@ -15,6 +15,7 @@
 // A result that is not finite is computed again in whole f32 products (see exact_row.cuh).
 #include "common.cuh"
 #include "sm100.cuh"
+#include "tf32.cuh"
 
 namespace rt {
 namespace {
@@ -25,30 +26,6 @@ constexpr int TM = 64, TN = 64, TK = 32, kThreads = 128, kStages = 3;
 constexpr int kAPitch = TK + 8, kBPitch = TN + 4;
 constexpr int kAFloats = TM * kAPitch, kStage = kAFloats + TK * kBPitch;
 constexpr int kSmem = 4 * kStages * kStage;
-
-__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
-      "{%8, %9}, {%0, %1, %2, %3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void mma_tf32_first(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
-      "{%8, %9}, {%10, %10, %10, %10};"
-      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
-}
-__device__ __forceinline__ void split(float x, uint32_t& hi, uint32_t& lo) {
-  hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
-  lo = __float_as_uint(x - __uint_as_float(hi)) + 0x1000u;
-}
-__device__ __forceinline__ void copy_async16(float* dst, const float* src, bool read) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sm100::smem_u32(dst)), "l"(src),
-               "r"(read ? 16 : 0)
-               : "memory");
-}
 
 __global__ void __launch_bounds__(kThreads, 3)
 matmul_f32_tc_kernel(const float* __restrict__ a, const float* __restrict__ b, const float* __restrict__ bias,

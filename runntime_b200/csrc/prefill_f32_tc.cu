@@ -23,12 +23,13 @@
 // 256 on one K/V head (2.4 GFLOP, 27 us at 92 TFLOP/s): 583 us for 16-row tiles of scalar FMAs, 155
 // for prefill_simt.cu, 102 here.
 //
-// Numbers that are not finite (an input's infinity times another's low part is NaN where the
-// product should be infinite) show in the output: such row tiles are computed again by
-// whole f32 products.
+// A product with an infinity or a NaN is NaN here (tf32.cuh), where the op's definition may have an
+// infinite score that weighs nothing: a row tile with a row sum or an output that is not finite
+// is computed again by whole f32 products.
 #include "common.cuh"
 #include "exact_row.cuh"
 #include "sm100.cuh"
+#include "tf32.cuh"
 
 namespace rt {
 namespace {
@@ -51,32 +52,6 @@ struct F32Tc {
   static constexpr int kCtas = HDP == 32 ? 2 : 1;             // per SM
   static_assert((kKeySets - 1) * BQ * HDP <= kStages * kStage, "the other key sets' rows fit the ring");
 };
-
-__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
-      "{%8, %9}, {%0, %1, %2, %3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-// ... and into zeros.
-__device__ __forceinline__ void mma_tf32_first(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
-      "{%8, %9}, {%10, %10, %10, %10};"
-      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
-}
-// x = hi + lo, both rounded to the 11 bits that the tensor core reads.
-__device__ __forceinline__ void split(float x, uint32_t& hi, uint32_t& lo) {
-  hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
-  lo = __float_as_uint(x - __uint_as_float(hi)) + 0x1000u;
-}
-__device__ __forceinline__ void copy_async16(float* dst, const float* src, bool read) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sm100::smem_u32(dst)), "l"(src),
-               "r"(read ? 16 : 0)
-               : "memory");
-}
 
 // Which row tile block number u of a padded batch takes: the tiles of the longest sequence first
 // (its last rows first: under a causal mask they are the longest), those past the sequences' ends
@@ -439,7 +414,7 @@ prefill_f32_tc_kernel(const AttnParams p, int tilesPerSeq) {
 #pragma unroll
         for (int w = 0; w < kWarps; w++) sum += sSum[w][r];
         const float invL = sum > 0.f ? 1.f / sum : 0.f;  // empty band -> zeros
-        odd |= !(sum < INFINITY);   // a NaN score: the sum says so whatever its parts did to the output
+        odd |= !(sum < INFINITY);   // (1 / sum is not asked for a NaN sum, and 0 leaves nothing of it)
 #pragma unroll
         for (int half = 0; half < 2; half++) {
           const int x = 32 * colSet + 8 * t4 + 4 * half, e = 2 * i + half;

@@ -53,3 +53,23 @@ def test_values_past_the_split(ex, value):
         big = np.abs(w32) > 1e30
         assert big.any() and (np.sign(got[9][big]) == np.sign(w32[big])).all()
         assert np.allclose(got[9][:4], w32[:4], rtol=1e-5)
+
+
+@pytest.mark.parametrize("where", ["a", "b"])
+@pytest.mark.parametrize("bits", [0x7fffffff, 0xffffffff, 0x7fc00000, 0x7f800001])
+def test_every_nan_stays_one(ex, where, bits):
+    """0x7fffffff is the NaN that GPU arithmetic makes: an earlier operator's NaN is the next
+    projection's too."""
+    import runntime_b200 as rt
+    rng = np.random.default_rng(6)
+    x = dict(a=rng.standard_normal((40, 64)).astype(np.float32), b=rng.standard_normal((64, 48)).astype(np.float32))
+    want = x["a"].astype(np.float64) @ x["b"].astype(np.float64)
+    x[where][9, 7] = np.uint32(bits).view(np.float32)
+    got = rt.toArray(rt.matmul(ex.upload(x["a"], [40, 64]), ex.upload(x["b"], [64, 48])), ex).reshape(40, 48)
+    hit = np.zeros((40, 48), bool)
+    if where == "a":
+        hit[9] = True
+    else:
+        hit[:, 7] = True
+    assert np.isnan(got[hit]).all()
+    assert np.allclose(got[~hit], want[~hit], rtol=1e-5, atol=1e-5)

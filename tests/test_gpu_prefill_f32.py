@@ -112,3 +112,11 @@ def check_marked(ex, route, hd, where, value):
 @pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
 def test_scores_that_are_not_finite(ex, route, hd, where, value):
     check_marked(ex, route, hd, where, value)
+
+
+@pytest.mark.parametrize("hd", [32, 256])
+@pytest.mark.parametrize("where", ["q", "k", "v"])
+@pytest.mark.parametrize("bits", [0x7fffffff, 0xffffffff, 0x7f800001])
+def test_every_nan_stays_one(ex, route, hd, where, bits):
+    """0x7fffffff is the NaN that GPU arithmetic makes."""
+    check_marked(ex, route, hd, where, np.uint32(bits).view(np.float32))
