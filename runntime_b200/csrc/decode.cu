@@ -8,7 +8,8 @@
 // private online softmax over the keys of its slot in f32 registers.  At the
 // end the slots of a head are merged with a log-sum-exp; with more than one
 // split the per-split (m, l, acc) partials go to scratch and the last CTA to
-// arrive for the sequence merges them — no second launch, no waiting.
+// arrive for the sequence merges them, without waiting, or, where they are more than
+// one CTA reads in a few microseconds, a second launch does (see plan_decode).
 //
 // The KV-cache append is fused: the new K/V row is stored to the cache by the
 // CTA of split 0 and attended to straight from its source.
@@ -457,7 +458,7 @@ decode_kernel(const DecodeParams p) {
   const int aCacheRows = sec ? p.s2.cacheRows : p.cacheRows;
   const int aKvLen = sec ? p.s2.kvLen : p.kvLen;
   const int aWl = sec ? p.s2.wl : p.wl;
-  const int hd = p.hd;
+  const int hd = EXACT ? HDP : p.hd;
   const int group = p.qHeads / p.kvHeads;
   const int kvh0 = zb * p.kvPerCta;
   const int nkv = min(p.kvPerCta, p.kvHeads - kvh0);
