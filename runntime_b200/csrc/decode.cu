@@ -458,7 +458,7 @@ decode_kernel(const DecodeParams p) {
   const int aCacheRows = sec ? p.s2.cacheRows : p.cacheRows;
   const int aKvLen = sec ? p.s2.kvLen : p.kvLen;
   const int aWl = sec ? p.s2.wl : p.wl;
-  const int hd = EXACT ? HDP : p.hd;
+  const int hd = p.hd;
   const int group = p.qHeads / p.kvHeads;
   const int kvh0 = zb * p.kvPerCta;
   const int nkv = min(p.kvPerCta, p.kvHeads - kvh0);
@@ -912,8 +912,9 @@ decode_kernel(const DecodeParams p) {
       rowF[hh * stride + 1] = sum;
     }
   }
-  for (int i = tid; i < hqReal * hd; i += kConsumers) {
-    const int hh = i / hd, x = i - hh * hd;
+  const int cols = EXACT ? HDP : hd;   // (a constant to divide by, where there is one)
+  for (int i = tid; i < hqReal * cols; i += kConsumers) {
+    const int hh = i / cols, x = i - hh * cols;
     const float* r = sM + (hh * R + x / W) * MS + 1 + x % W;
     float o = 0.f;
 #pragma unroll 8
