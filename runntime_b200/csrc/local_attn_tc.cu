@@ -21,7 +21,9 @@
 // by a power of two (per row; P, whose largest is one, by 2^13) and split into two halves hi + lo,
 // 22 bits, and multiplied in two (three for R) MMAs with f32 accumulation; K and V are halves
 // already.  No operand can overflow: the scale puts the row's largest element at 2^13.  (Without a scale
-// P had an absolute 2^-25 in place of 22 bits: a key that weighs e^-12 was off by 2^-9 of itself.)
+// P had an absolute 2^-25 in place of 22 bits: a key that weighs e^-12 was off by 2^-9 of itself.)  The
+// tensor core adds into its accumulator less carefully than an FMA does, so the products of halves hi are
+// added 32 columns at a time, the 2^-11 smaller ones apart.
 //
 // What bounds it: instructions, about 1 900 per warp and 16 rows, at 12 warps per SM (issue slots 43 %
 // busy, DRAM 40 %).
@@ -59,6 +61,14 @@ __device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], 
       "{%8, %9}, {%0, %1, %2, %3};"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// ... into zeros.
+__device__ __forceinline__ void mma16816_first(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, "
+      "{%8, %9}, {%10, %10, %10, %10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
 }
 __device__ __forceinline__ uint32_t pack2(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
 // Two f32 values as halves hi and what is left of them as halves lo.
@@ -136,6 +146,7 @@ local_attn_tc_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                      int window, float kScale, float softcap, int* status) {
   using L = Local<HD, WP>;
   constexpr int NT = (16 + WP) / 8, KS = HD / 16;       // key tiles of a warp, steps of the head
+  constexpr int kSteps = 2;                             // that an accumulator adds up before it joins the f32 sum
   extern __shared__ unsigned char smemRaw[];
   __shared__ __align__(8) uint64_t sFull;
   __shared__ float sRelInv[WP];
@@ -237,10 +248,7 @@ local_attn_tc_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
       float r[WP / 8][4];
 #pragma unroll
       for (int n = 0; n < WP / 8; n += 2) {
-#pragma unroll
-        for (int e = 0; e < 2; e++)
-#pragma unroll
-          for (int i = 0; i < 4; i++) r[n + e][i] = 0.f;
+        float d[2][4], small[2][4];
 #pragma unroll
         for (int k = 0; k < KS; k++) {
           const uint32_t at = piece(n * 8 + (lane & 7) + ((lane >> 4) << 3), 2 * k + ((lane >> 3) & 1), WP);
@@ -249,11 +257,21 @@ local_attn_tc_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
           ldmatrix4(base + L::kRelLo + at, bl);
 #pragma unroll
           for (int e = 0; e < 2; e++) {
-            mma16816(r[n + e], qh[k], bh[2 * e], bh[2 * e + 1]);
-            mma16816(r[n + e], qh[k], bl[2 * e], bl[2 * e + 1]);
-            mma16816(r[n + e], ql[k], bh[2 * e], bh[2 * e + 1]);
+            if (k % kSteps == 0) mma16816_first(d[e], qh[k], bh[2 * e], bh[2 * e + 1]);
+            else mma16816(d[e], qh[k], bh[2 * e], bh[2 * e + 1]);
+            if (k == 0) mma16816_first(small[e], qh[k], bl[2 * e], bl[2 * e + 1]);
+            else mma16816(small[e], qh[k], bl[2 * e], bl[2 * e + 1]);
+            mma16816(small[e], ql[k], bh[2 * e], bh[2 * e + 1]);
+            if (k % kSteps == kSteps - 1) {
+#pragma unroll
+              for (int i = 0; i < 4; i++) r[n + e][i] = k < kSteps ? d[e][i] : r[n + e][i] + d[e][i];
+            }
           }
         }
+#pragma unroll
+        for (int e = 0; e < 2; e++)
+#pragma unroll
+          for (int i = 0; i < 4; i++) r[n + e][i] += small[e][i];
       }
       __syncwarp();      // the warp's q rows are in registers: their place is free
 
@@ -262,7 +280,7 @@ local_attn_tc_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
 #pragma unroll
       for (int n = 0; n < NT; n += 2) {
         if (WP - (8 * n + 15) >= window) continue;   // both tiles lie before every row's window
-        float s[2][4] = {};
+        float s[2][4], d[2][4], small[2][4];
 #pragma unroll
         for (int k = 0; k < KS; k++) {
           uint32_t b[4];
@@ -270,8 +288,14 @@ local_attn_tc_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                                          2 * k + ((lane >> 3) & 1), L::kKeys), b);
 #pragma unroll
           for (int e = 0; e < 2; e++) {
-            mma16816(s[e], qh[k], b[2 * e], b[2 * e + 1]);
-            mma16816(s[e], ql[k], b[2 * e], b[2 * e + 1]);
+            if (k % kSteps == 0) mma16816_first(d[e], qh[k], b[2 * e], b[2 * e + 1]);
+            else mma16816(d[e], qh[k], b[2 * e], b[2 * e + 1]);
+            if (k == 0) mma16816_first(small[e], ql[k], b[2 * e], b[2 * e + 1]);
+            else mma16816(small[e], ql[k], b[2 * e], b[2 * e + 1]);
+            if (k % kSteps == kSteps - 1) {
+#pragma unroll
+              for (int i = 0; i < 4; i++) s[e][i] = k < kSteps ? d[e][i] : s[e][i] + d[e][i];
+            }
           }
         }
 #pragma unroll
@@ -279,7 +303,7 @@ local_attn_tc_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
 #pragma unroll
           for (int i = 0; i < 2; i++)
             *reinterpret_cast<float2*>(score0 + i * (L::kEight / 4) + (n + e) * 8 + t4 * 2) =
-                make_float2(s[e][2 * i], s[e][2 * i + 1]);
+                make_float2(s[e][2 * i] + small[e][2 * i], s[e][2 * i + 1] + small[e][2 * i + 1]);
       }
       __syncwarp();
 
@@ -332,7 +356,7 @@ local_attn_tc_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
       }
       __syncwarp();
 
-      // O = P V, sixteen keys at a time.
+      // O = P V, sixteen keys at a time, the small products first.
       float o[HD / 8][4];
 #pragma unroll
       for (int x = 0; x < HD / 8; x++)
@@ -352,8 +376,8 @@ local_attn_tc_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
           ldmatrix4_trans(base + L::kV + piece(r0 + n * 8 + (lane & 15), x + (lane >> 4), L::kKeys), b);
 #pragma unroll
           for (int e = 0; e < 2; e++) {
-            mma16816(o[x + e], ph, b[2 * e], b[2 * e + 1]);
             mma16816(o[x + e], pl, b[2 * e], b[2 * e + 1]);
+            mma16816(o[x + e], ph, b[2 * e], b[2 * e + 1]);
           }
         }
       }
