@@ -446,11 +446,13 @@ cudaError_t launch(const void* qkv, const float* rel, const float* qScale, void*
 
 }  // namespace
 
-// f16, heads of 64 or 128, tensors on 16-byte boundaries, coordinates within 31 bits.
+// f16, heads of 64 or 128, tensors on 16-byte boundaries, coordinates within 31 bits, more than a few
+// rows: a block's set-up, bias rows split among it, takes 5 to 12 us by window and head, a warp per row on
+// the FP32 pipes (local_attn.cu) 5 to 7 for one to eight rows and 7 to 14 for twelve.
 bool local_attn_tc_supported(const void* qkv, const float* rel, const void* out, int64_t rows,
                              int heads, int hd, int dtype) {
   auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
-  return dtype == RT_F16 && (hd == 64 || hd == 128) && al(qkv) && al(rel) && al(out) &&
+  return dtype == RT_F16 && (hd == 64 || hd == 128) && rows > 8 && al(qkv) && al(rel) && al(out) &&
          3ll * heads * hd < (1ll << 31) && (rows + kRows) * heads < (1ll << 31) && encode_fn() != nullptr;
 }
 

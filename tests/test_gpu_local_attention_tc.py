@@ -88,3 +88,11 @@ def test_a_key_that_weighs_little(ex, hd, window, apart):
     # the exponential by a few 2^-24 of theirs (tanhf's argument times the cap: 2 ulp of the score)
     bad = (got - want).abs() > (2.0 ** -11 + 2.0 ** -17) * want.abs() + 2.0 ** -25
     assert not bool(bad.any()), f"{int(bad.sum())} of {bad.numel()} off, by up to {float(((got - want) / want).abs().max()):.2g} of the result"
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("rows", [2, 8, 9])
+def test_a_few_rows(ex, rows, hd):
+    """Either side of the count from which the tensor cores take the call."""
+    check(ex, rows, 5, hd, 12)
+    check(ex, rows, 5, hd, 32)
