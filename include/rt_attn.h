@@ -158,8 +158,8 @@ RT_API int rt_attn(rt_ctx* ctx, const rt_attn_args* args);
  * name into *route: "decode", "prefill_simt" (FP32 pipes), or one of the
  * tensor-core kernels "prefill_tc3" (the default for f16), "prefill_tc3_pair",
  * "prefill_tc4", "prefill_tc2", "prefill_tc" (see RT_OPT_PREFILL_TC),
- * "prefill_f32_tc" (f32) and "prefill_mma" (f16, packed short segments, heads up
- * to 32). */
+ * "prefill_f32_tc" (f32; batches of short sequences go to the FP32 pipes) and
+ * "prefill_mma" (f16, packed short segments, heads up to 32). */
 RT_API int rt_attn_route(rt_ctx* ctx, const rt_attn_args* args, const char** route);
 
 /* ---- batched single-token decode over KV caches -----------------------------

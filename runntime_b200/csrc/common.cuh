@@ -319,6 +319,9 @@ __device__ __forceinline__ void act_dispatch(int act, F&& f) {
 
 // Launchers (defined one per .cu).  Each returns a cudaError_t from the launch.
 cudaError_t launch_prefill_simt(const AttnParams& p, int dtype, cudaStream_t s);
+// ... in 16-row pieces, for rows that see few keys and rows off four-element boundaries.
+bool prefill_rows_better(const AttnParams& p, int dtype);
+cudaError_t launch_prefill_rows(const AttnParams& p, int dtype, cudaStream_t s);
 // f32 on the tensor cores (head sizes up to 256, rows on 16-byte boundaries).
 bool prefill_f32_tc_supported(const AttnParams& p, int dtype);
 cudaError_t launch_prefill_f32_tc(const AttnParams& p, cudaStream_t s);

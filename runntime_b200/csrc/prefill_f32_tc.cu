@@ -1,5 +1,6 @@
 // f32 prefill attention on the tensor cores (mma.sync, tf32), head sizes up to 256 that are a
-// multiple of four, rows that start on 16 bytes; everything else is prefill_simt.cu's.
+// multiple of four, rows that start on 16 bytes; prefill_rows.cu takes batches of short sequences,
+// prefill_simt.cu everything else.
 //
 // Every f32 operand x is split into hi + lo, each a tf32 number (11 bits): x = hi + lo to 2^-23, and
 // a product is hi hi' + hi lo' + lo hi', 2^-22 short of exact at worst.  The tensor core adds into its

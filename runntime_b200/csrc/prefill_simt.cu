@@ -1,6 +1,7 @@
 // General prefill attention on the FP32 pipes: every option of the 'attn' op,
-// f32 or f16 storage, any head size up to 512.  It takes the shapes that the tensor-core
-// kernels do not: rows that do not start on 16 bytes, head sizes outside theirs.
+// f32 or f16 storage, head sizes up to 512 that are a multiple of four, rows that start on four
+// elements.  It takes the shapes that the tensor-core kernels do not; prefill_rows.cu takes the rest,
+// and rows that see few keys.
 //
 // A CTA owns 32 query rows of one query head and walks the 64-key tiles of the union of its
 // rows' bands.  K (64 keys x 64 columns at a time) and V
@@ -94,14 +95,13 @@ struct Shape {
   static constexpr int kCtas = HDP <= 64 ? 3 : HDP <= 256 ? 2 : 1;  // per SM
 };
 
-// VEC: rows of q, k and v can be read four elements at a time.
-template <typename T, int HDP, bool VEC>
+template <typename T, int HDP>
 __global__ void __launch_bounds__(kThreads, Shape<HDP>::kCtas)
 prefill_simt_kernel(const AttnParams p, int tilesPerSeq) {
   using S = Shape<HDP>;
   constexpr int NP = 2 * S::kQuads;          // column pairs of the output per lane and row
   constexpr int NJ = BK / 32;                // keys per lane
-  constexpr bool ASYNC = VEC && sizeof(T) == 4;
+  constexpr bool ASYNC = sizeof(T) == 4;
   extern __shared__ __align__(16) float smem[];
   float* sQ = smem;                          // [BQ][kQPitch]
   float* sP = sQ + BQ * S::kQPitch;          // [BQ][PS]
@@ -133,22 +133,13 @@ prefill_simt_kernel(const AttnParams p, int tilesPerSeq) {
     sEnd[tid] = end;
   }
   // q, with zeros in the columns past the head and the rows past the tensor
-  const int hdUp = (hd + 3) & ~3;
-  if (VEC) {
-    constexpr int Q4 = HDP / 4;
-    for (int i = tid; i < BQ * Q4; i += kThreads) {
-      const int r = i / Q4, x = (i % Q4) * 4;
-      if (x >= hd) continue;
-      const bool in = row0 + r < rowEnd;
-      *reinterpret_cast<float4*>(sQ + r * S::kQPitch + x) =
-          in ? load4(q + (row0 + r) * p.qStride + x) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-  } else {
-    for (int i = tid; i < BQ * hdUp; i += kThreads) {
-      const int r = i / hdUp, x = i - r * hdUp;
-      sQ[r * S::kQPitch + x] =
-          (row0 + r < rowEnd && x < hd) ? to_f32<T>(q[(row0 + r) * p.qStride + x]) : 0.f;
-    }
+  constexpr int Q4 = HDP / 4;
+  for (int i = tid; i < BQ * Q4; i += kThreads) {
+    const int r = i / Q4, x = (i % Q4) * 4;
+    if (x >= hd) continue;
+    const bool in = row0 + r < rowEnd;
+    *reinterpret_cast<float4*>(sQ + r * S::kQPitch + x) =
+        in ? load4(q + (row0 + r) * p.qStride + x) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   __syncthreads();
 
@@ -178,36 +169,26 @@ prefill_simt_kernel(const AttnParams p, int tilesPerSeq) {
       const T* src = isK ? k + k0 * p.kvStride : v + k0 * p.kvStride;
       const int r0 = isK ? 0 : (fillPart - kChunks) * S::kVRows;
       const int x0 = isK ? fillPart * S::kDims : 0;
-      if (VEC) {
-        constexpr int KW = S::kDims / 4, VW = HDP / 4;
-        constexpr int NK = BK * KW / kThreads, NV = S::kVRows * VW / kThreads;
-        auto piece = [&](int r, int x, int pitch) {
-          const bool in = r0 + r < nk;
-          float* d = dst + r * pitch + x;
-          const T* s = in ? src + (r0 + r) * p.kvStride + x0 + x : src;
-          if (ASYNC) copy_async16(d, s, in);
-          else *reinterpret_cast<float4*>(d) = in ? load4(s) : make_float4(0.f, 0.f, 0.f, 0.f);
-        };
-        if (isK) {
+      constexpr int KW = S::kDims / 4, VW = HDP / 4;
+      constexpr int NK = BK * KW / kThreads, NV = S::kVRows * VW / kThreads;
+      auto piece = [&](int r, int x, int pitch) {
+        const bool in = r0 + r < nk;
+        float* d = dst + r * pitch + x;
+        const T* s = in ? src + (r0 + r) * p.kvStride + x0 + x : src;
+        if (ASYNC) copy_async16(d, s, in);
+        else *reinterpret_cast<float4*>(d) = in ? load4(s) : make_float4(0.f, 0.f, 0.f, 0.f);
+      };
+      if (isK) {
 #pragma unroll
-          for (int i = 0; i < NK; i++) {
-            const int idx = tid + i * kThreads, r = idx / KW, x = (idx % KW) * 4;
-            if (x0 + x < hd) piece(r, x, S::kKeyPitch);
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < NV; i++) {
-            const int idx = tid + i * kThreads, r = idx / VW, x = (idx % VW) * 4;
-            if (x < hd) piece(r, x, HDP);
-          }
+        for (int i = 0; i < NK; i++) {
+          const int idx = tid + i * kThreads, r = idx / KW, x = (idx % KW) * 4;
+          if (x0 + x < hd) piece(r, x, S::kKeyPitch);
         }
       } else {
-        const int rows = isK ? BK : S::kVRows, pitch = isK ? S::kKeyPitch : HDP;
-        const int width = isK ? min(S::kDims, hdUp - x0) : hd;
-        for (int i = tid; i < rows * width; i += kThreads) {
-          const int r = i / width, x = i - r * width;
-          dst[r * pitch + x] = (r0 + r < nk && x0 + x < hd)
-                                   ? to_f32<T>(src[(r0 + r) * p.kvStride + x0 + x]) : 0.f;
+#pragma unroll
+        for (int i = 0; i < NV; i++) {
+          const int idx = tid + i * kThreads, r = idx / VW, x = (idx % VW) * 4;
+          if (x < hd) piece(r, x, HDP);
         }
       }
       if (++fillPart == perTile) fillPart = 0, fillTile++;
@@ -257,7 +238,7 @@ prefill_simt_kernel(const AttnParams p, int tilesPerSeq) {
     for (int kc = 0; kc < kChunks; kc++) {
       const float* sK = advance() + lane * S::kKeyPitch;
       const float* sq = qRow + kc * S::kDims;
-      const int steps = min(S::kDims, hdUp - kc * S::kDims) >> 2;
+      const int steps = min(S::kDims, hd - kc * S::kDims) >> 2;
       auto dots = [&](auto n) {   // the first n x 32 keys of the tile
 #pragma unroll 4
         for (int x = 0; x < steps; x++) {
@@ -350,7 +331,7 @@ prefill_simt_kernel(const AttnParams p, int tilesPerSeq) {
 
   T* __restrict__ out = static_cast<T*>(p.out) + (int64_t)h * hd;
   const int64_t qw = (int64_t)p.qHeads * hd;
-  const bool out4 = VEC && reinterpret_cast<uintptr_t>(p.out) % (4 * sizeof(T)) == 0;
+  const bool out4 = reinterpret_cast<uintptr_t>(p.out) % (4 * sizeof(T)) == 0;
   bool odd = false;   // something that is not finite
 #pragma unroll
   for (int i = 0; i < kRows; i++) {
@@ -387,9 +368,9 @@ prefill_simt_kernel(const AttnParams p, int tilesPerSeq) {
   }
 }
 
-template <typename T, int HDP, bool VEC>
+template <typename T, int HDP>
 cudaError_t launch(const AttnParams& p, cudaStream_t s) {
-  auto kern = prefill_simt_kernel<T, HDP, VEC>;
+  auto kern = prefill_simt_kernel<T, HDP>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape<HDP>::kSmem);
   if (e != cudaSuccess) return e;
   const int64_t perSeq = p.seqStride > 0 ? (p.seqStride + BQ - 1) / BQ : 0;
@@ -398,27 +379,28 @@ cudaError_t launch(const AttnParams& p, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-// Four elements at a time where every row of q, k and v of every head starts at such a boundary.
-template <typename T, int HDP>
-cudaError_t launch_aligned(const AttnParams& p, cudaStream_t s) {
+// Every row of q, k and v of every head starts on four elements.  Without that this kernel's loads, one
+// element each and a division for its place, cost more than its tiles save: [300, 8 x 33] f32 64 us, 42
+// in 16-row pieces (prefill_rows.cu), [1000, 8 x 129] 707 and 715.
+bool by_fours(const AttnParams& p, uintptr_t bytes) {
   const uintptr_t bases = reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.k) |
                           reinterpret_cast<uintptr_t>(p.v);
-  const bool vec = p.hd % 4 == 0 && p.qStride % 4 == 0 && p.kvStride % 4 == 0 && bases % (4 * sizeof(T)) == 0;
-  return vec ? launch<T, HDP, true>(p, s) : launch<T, HDP, false>(p, s);
+  return p.hd % 4 == 0 && p.qStride % 4 == 0 && p.kvStride % 4 == 0 && bases % bytes == 0;
 }
 
 template <typename T>
 cudaError_t dispatch_hd(const AttnParams& p, cudaStream_t s) {
-  if (p.hd <= 32) return launch_aligned<T, 32>(p, s);
-  if (p.hd <= 64) return launch_aligned<T, 64>(p, s);
-  if (p.hd <= 128) return launch_aligned<T, 128>(p, s);
-  if (p.hd <= 256) return launch_aligned<T, 256>(p, s);
-  return launch_aligned<T, 512>(p, s);
+  if (p.hd <= 32) return launch<T, 32>(p, s);
+  if (p.hd <= 64) return launch<T, 64>(p, s);
+  if (p.hd <= 128) return launch<T, 128>(p, s);
+  if (p.hd <= 256) return launch<T, 256>(p, s);
+  return launch<T, 512>(p, s);
 }
 
 }  // namespace
 
 cudaError_t launch_prefill_simt(const AttnParams& p, int dtype, cudaStream_t s) {
+  if (!by_fours(p, dtype == RT_F16 ? 8 : 16) || prefill_rows_better(p, dtype)) return launch_prefill_rows(p, dtype, s);
   return dtype == RT_F16 ? dispatch_hd<__half>(p, s) : dispatch_hd<float>(p, s);
 }
 
