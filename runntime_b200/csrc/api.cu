@@ -442,8 +442,8 @@ int rt_buf_download(rt_ctx* ctx, const void* device_ptr, size_t offset, void* ho
 static int prefill_kernel_of(const rt_ctx* ctx, const rt::AttnParams& p, int dtype) {
   if (!ctx->useTc) return 0;
   if (rt::prefill_f32_tc_supported(p, dtype)) return rt::prefill_rows_better(p, dtype) ? 0 : 6;
-  if (ctx->useTc == 1 && rt::prefill_mma_supported(p, dtype)) return 7;
   const bool tc3 = rt::prefill_tc3_supported(p, dtype);
+  if (ctx->useTc == 1 && rt::prefill_mma_supported(p, dtype, tc3)) return 7;
   if (ctx->useTc == 6 && rt::prefill_tc4_supported(p, dtype)) return 5;
   if (ctx->useTc == 5 && rt::prefill_tc3_pair_supported(p, dtype)) return 4;
   if ((ctx->useTc == 4 || ctx->useTc == 5) && tc3) return 3;

@@ -325,8 +325,9 @@ cudaError_t launch_prefill_rows(const AttnParams& p, int dtype, cudaStream_t s);
 // f32 on the tensor cores (head sizes up to 256, rows on 16-byte boundaries).
 bool prefill_f32_tc_supported(const AttnParams& p, int dtype);
 cudaError_t launch_prefill_f32_tc(const AttnParams& p, cudaStream_t s);
-// f16, packed segments known to be short, heads of up to 32 columns.
-bool prefill_mma_supported(const AttnParams& p, int dtype);
+// f16, packed segments known to be short, heads of up to 32 columns.  other: the tcgen05 kernel takes
+// the call as well.
+bool prefill_mma_supported(const AttnParams& p, int dtype, bool other);
 cudaError_t launch_prefill_mma(const AttnParams& p, cudaStream_t s);
 bool prefill_tc_supported(const AttnParams& p, int dtype);
 cudaError_t launch_prefill_tc(const AttnParams& p, int dtype, int* status, cudaStream_t s,
