@@ -27,6 +27,12 @@ constexpr int kAhead = 2, kCtas = 5;
 // kept range of up to kWarpKept columns, without a block barrier, while all of them store the
 // zeros (f16 [6007, 6007], 24 segments: 28.7 us with all warps on the kept range, 20.8).
 constexpr int kWarpRowCols = 2048, kWarpKept = 1024;
+// A warp's rows that start anywhere go element by element where they have no mask or are narrow: between
+// the ragged ends there are too few chunks to pay for them, and an exponential per element costs
+// less than the registers of eight.  f16, chunks and elements, us: [70000, 3] 39.2, 19.4, [20000, 515] 31.3, 17.3,
+// [2047, 2047] without segments 13.4, 8.9; [515, 515] in 5 segments 3.9, 3.5, [1001, 1001] in 5 4.2, 4.4,
+// [2047, 2047] in 5 6.2, 8.5.
+constexpr int kElementCols = 768;
 constexpr float kNegMax = -3.402823466e38f;
 
 template <typename T>
@@ -323,6 +329,30 @@ softmax_cta_kernel(const T* __restrict__ x, T* __restrict__ out, const float* __
   else softmax_row<T, By::Cta, V>(x, out, blockIdx.x, cols, lo, hi, sM, sS);
 }
 
+// A row by a warp, element by element.
+template <typename T, bool MASKED>
+__global__ void __launch_bounds__(kThreads)
+softmax_element_kernel(const T* __restrict__ x, T* __restrict__ out, const float* __restrict__ segs, int64_t rows,
+                       int64_t cols, int64_t wl, int64_t wr) {
+  const int lane = threadIdx.x & 31;
+  const int64_t row = (int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+  if (row >= rows) return;
+  int64_t lo = 0, hi = cols;
+  if (MASKED) kept_range(segs, row, cols, wl, wr, lo, hi);
+  const T* xr = x + row * cols;
+  T* orow = out + row * cols;
+  float m = kNegMax, s = 0.f;
+  for (int64_t j = lo + lane; j < hi; j += 32) combine(m, s, to_f32<T>(xr[j]), 1.f);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    combine(m, s, __shfl_xor_sync(0xffffffffu, m, o), __shfl_xor_sync(0xffffffffu, s, o));
+  const float inv = s > 0.f ? 1.f / s : 0.f;
+  for (int64_t j = lane; j < cols; j += 32) {
+    const bool kept = !MASKED || (j >= lo && j < hi);
+    orow[j] = from_f32<T>(kept ? __expf(to_f32<T>(xr[j]) - m) * inv : 0.f);
+  }
+}
+
 template <typename T, int V>
 __global__ void __launch_bounds__(kThreads, kCtas)
 softmax_warp_kernel(const T* __restrict__ x, T* __restrict__ out, const float* __restrict__ segs, int64_t rows,
@@ -360,6 +390,14 @@ cudaError_t softmax_typed(const void* x, void* out, const float* segs, int64_t r
     if (blocks > 0x7fffffffll) return cudaErrorInvalidValue;
     if (warpRows) softmax_quad_kernel<T, true><<<(unsigned)blocks, kThreads, 0, s>>>(xi, oi, segs, rows, cols, wl, wr);
     else softmax_quad_kernel<T, false><<<(unsigned)blocks, kThreads, 0, s>>>(xi, oi, segs, rows, cols, wl, wr);
+    return cudaGetLastError();
+  }
+  if (cols <= (segs ? kElementCols : kWarpRowCols)) {
+    const int64_t blocks = (rows + kThreads / 32 - 1) / (kThreads / 32);
+    if (blocks > 0x7fffffffll) return cudaErrorInvalidValue;
+    const unsigned g = (unsigned)blocks;
+    if (segs) softmax_element_kernel<T, true><<<g, kThreads, 0, s>>>(xi, oi, segs, rows, cols, wl, wr);
+    else softmax_element_kernel<T, false><<<g, kThreads, 0, s>>>(xi, oi, segs, rows, cols, wl, wr);
     return cudaGetLastError();
   }
   const uintptr_t apart = reinterpret_cast<uintptr_t>(x) ^ reinterpret_cast<uintptr_t>(out);

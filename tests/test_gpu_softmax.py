@@ -167,3 +167,18 @@ def test_masked_rows_of_a_block(ex, dtype, n, shift, outShift, wl, wr):
     got = out.float().cpu().numpy()
     close(got[outShift:outShift + n * n], oracle.softmax_ref(x.reshape(n, n), segs, wl, wr), dtype)
     assert (got[:outShift] == 7).all() and (got[outShift + n * n:] == 7).all()
+
+
+@pytest.mark.parametrize("dtype", ["f32", "f16"])
+@pytest.mark.parametrize("n", [511, 767, 769, 2047])
+@pytest.mark.parametrize("parts", [1, 2, 3])
+def test_masked_rows_of_a_warp(ex, dtype, n, parts):
+    """Rows that start anywhere, on either side of the width up to which they go element by element."""
+    import runntime_b200 as rt
+    x = 8 * oracle.random_f32(n * n, 5)
+    x = (oracle.round_f16(x) if dtype == "f16" else x).reshape(n, n)
+    at = [n * p // parts for p in range(parts + 1)]
+    segs = np.array([[at[r * parts // n], at[r * parts // n + 1]] for r in range(n)], np.float32)
+    segs[3], segs[4], segs[5] = (0, n // 2), (n // 2 - 1, n), (n, n)
+    got = rt.toArray(rt.softmax(ex.upload(x, [n, n], dtype), dict(segments=ex.upload(segs, [n, 2]))), ex)
+    close(got, oracle.softmax_ref(x, segs), dtype)
