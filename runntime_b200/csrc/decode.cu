@@ -418,8 +418,6 @@ __device__ __noinline__ void merge_splits(int hd, int splits, int qHeads, const 
   }
 }
 
-constexpr float kGivenUp = -1.f;   // in the place of a split's row sum: a wait of its block ran out
-
 template <typename T, int HDP, bool EXACT, int VEC, bool BULK, int R = 1>
 __global__ void __launch_bounds__(BULK ? kConsumers + 32 : kConsumers, HDP / R <= 64 ? 2 : 1)
 decode_kernel(const DecodeParams p) {
@@ -855,10 +853,11 @@ decode_kernel(const DecodeParams p) {
   named_barrier_sync(1, kConsumers);
   if (sAbortSeen) {
     // A wait ran out: record it, let copies in flight land, leave.
-    if (tid == 0) atomicOr(p.status, kStatusWaitTimeout);
-    if (p.mergeAfter) {   // a row sum that no block leaves: the merge launch writes nothing for these heads
-      float* sums = p.scratch + (((int64_t)by * p.splits + split) * p.qHeads + kvh0 * group) * (2 + hd) + 1;
-      for (int hh = tid; hh < hqReal; hh += kConsumers) sums[hh * (2 + hd)] = kGivenUp;
+    if (tid == 0) {
+      atomicOr(p.status, kStatusWaitTimeout);
+      // (the arrival counter, which the blocks leave alone then, and which is cleared with the status
+      // word: the merge launch writes nothing for these heads)
+      if (p.mergeAfter) p.counters[by * gridDim.z + zb] = 1;
     }
     for (int i = 0; i < 64; i++) __nanosleep(4000);
     return;
@@ -961,7 +960,10 @@ __global__ void __launch_bounds__(kMergeThreads)
 merge_kernel(const DecodeParams p) {
   __shared__ float sW[64], sInv;
   const int h = blockIdx.x, b = blockIdx.y, hd = p.hd, stride = 2 + hd, splits = p.splits;
+  const int zBlocks = (p.kvHeads + p.kvPerCta - 1) / p.kvPerCta;
+  const int zb = h / (p.qHeads / p.kvHeads) / p.kvPerCta;
   asm volatile("griddepcontrol.wait;" ::: "memory");   // the attention's partials are complete
+  if (__ldcg(p.counters + b * zBlocks + zb) != 0) return;   // a block gave up: its rows are no partials
   const int64_t row = (int64_t)b * p.qHeads + h;
   const float* src = p.scratch + ((int64_t)b * splits * p.qHeads + h) * stride;
   const int64_t ss = (int64_t)p.qHeads * stride;       // between splits
@@ -974,16 +976,15 @@ merge_kernel(const DecodeParams p) {
     const float M = warp_max(fmaxf(m0, m1));
     const float w0 = fast_exp2(m0 - M), w1 = fast_exp2(m1 - M);
     const float L = warp_sum(fmaf(l0, w0, l1 * w1));
-    const bool givenUp = __any_sync(0xffffffffu, l0 == kGivenUp || l1 == kGivenUp);
     sW[lane] = w0, sW[lane + 32] = w1;
     if (lane == 0) {
-      sInv = givenUp ? kGivenUp : L > 0.f ? 1.f / L : 0.f;
-      if (partials && !givenUp) partials[0] = L > 0.f ? M * 0.6931471805599453f : kNegSeed, partials[1] = L;
+      sInv = L > 0.f ? 1.f / L : 0.f;
+      if (partials) partials[0] = L > 0.f ? M * 0.6931471805599453f : kNegSeed, partials[1] = L;
     }
   }
   __syncthreads();
   const int x = threadIdx.x;
-  if (x >= hd || sInv == kGivenUp) return;
+  if (x >= hd) return;
   float o = 0.f;
 #pragma unroll 16
   for (int s = 0; s < splits; s++) o = fmaf(__ldcg(src + s * ss + 2 + x), sW[s], o);
