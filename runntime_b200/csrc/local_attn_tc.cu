@@ -23,9 +23,9 @@
 // already.  No operand can overflow: the scale puts the row's largest element at 2^13.  (Without a scale
 // P had an absolute 2^-25 in place of 22 bits: a key that weighs e^-12 was off by 2^-9 of itself.)  The
 // tensor core adds into its accumulator less carefully than an FMA does, so the products of halves hi are
-// added 32 columns at a time, the 2^-11 smaller ones apart.
+// added 32 columns at a time (64 in the widest form), the 2^-11 smaller ones apart.
 //
-// What bounds it: instructions, about 1 900 per warp and 16 rows, at 12 warps per SM (issue slots 43 %
+// What bounds it: instructions, about 2 000 per warp and 16 rows, at 12 warps per SM (issue slots 46 %
 // busy, DRAM 40 %).
 // [32769, 3 x 8 x 128], window 12: 528 us for one warp per row on the FP32 pipes (local_attn.cu), 98 us
 // with the soft cap on the scores' own fragments and the bias rows split for every tile, 74 us; the
@@ -146,7 +146,9 @@ local_attn_tc_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                      int window, float kScale, float softcap, int* status) {
   using L = Local<HD, WP>;
   constexpr int NT = (16 + WP) / 8, KS = HD / 16;       // key tiles of a warp, steps of the head
-  constexpr int kSteps = 2;                             // that an accumulator adds up before it joins the f32 sum
+  // Steps that an accumulator adds up before it joins the f32 sum.  (The widest form has no registers for
+  // the sums of two: 4 bytes spilled, [9000, 3 x 8 x 128] with a window of 32 4 % slower.)
+  constexpr int kSteps = HD == 128 && WP == 32 ? 4 : 2;
   extern __shared__ unsigned char smemRaw[];
   __shared__ __align__(8) uint64_t sFull;
   __shared__ float sRelInv[WP];
