@@ -275,8 +275,8 @@ int piece_bytes(const AttnParams& p) {
 // measurement against the tcgen05 kernel's 128-row blocks, us here and there, heads of 32: 39 segments
 // of 512 keys, 12 heads 125 and 133, 2 heads 30 and 29; 17 of 350, 4 heads 22 and 25.  Shorter ones where
 // a row has fewer than 64 bytes to move and the launch is not many blocks (heads of 20, 50 segments of 400, 2
-// heads 36 and 33, 12 heads 135 and 141) and where the other kernel's blocks leave a third of the SMs idle, so
-// that one of them is all of its time (23 of 256, 2 heads 10.2 and 9.2, 46 of 128 7.2 and 8.2).  With fewer
+// heads 36 and 33, 12 heads 135 and 141) and where the other kernel's blocks leave a fifth of the SMs idle, so
+// that one of them is all of its time (23 of 256, 2 heads 10.2 and 9.2, 32 of 400, one head 20.5 and 15.3).  With fewer
 // blocks of both: one segment of 256 7.7 and 8.6, of 500 12.5 and 12.  Where the tcgen05 kernel does not take
 // the call the FP32 pipes would: 5 of 400, one head of 20: 58.
 // Wider heads stay there: 8 segments of 300 keys, 8 heads of 36, in 64 padded columns 25 and 22.
@@ -285,7 +285,7 @@ bool prefill_mma_supported(const AttnParams& p, int dtype, bool other) {
   const int64_t mine = (p.qLen + BQ - 1) / BQ * p.qHeads, theirs = (p.qLen + 127) / 128 * p.qHeads;
   const int most = !other                                ? 512
                    : mine < kSms                         ? 256
-                   : theirs < 100                        ? 128
+                   : theirs < 120                        ? 128
                    : p.hd <= 24 && theirs < 3 * kSms     ? 384
                                                          : 512;
   return dtype == RT_F16 && p.hd <= HDP && p.segs && p.maxSegment > 0 && p.maxSegment <= most &&
