@@ -69,7 +69,8 @@ RT_API int rt_ctx_set_stream(rt_ctx* ctx, void* cuda_stream, int external);
  * shapes to a tensor-core kernel of the library's choice (head sizes 64, 128,
  * 256 and the narrow heads: one 128-row query tile per thread block whose key
  * tiles alternate between two softmax warpgroups).  0 sends every prefill, f32
- * ones too, to the FP32-pipe kernel; 2 forces one tile
+ * ones too, to the FP32-pipe kernel, and matmul and
+ * localAttention to theirs; 2 forces one tile
  * with one warpgroup, 3 two tiles per block, 4 the alternating form, 5 the
  * alternating form on pairs of thread blocks that share every K/V tile, 6 the
  * alternating form as one persistent thread block per SM over a queue of query
@@ -165,7 +166,8 @@ RT_API int rt_attn_route(rt_ctx* ctx, const rt_attn_args* args, const char** rou
 /* ---- batched single-token decode over KV caches -----------------------------
  * The decode step of the KV-cache engine (packages/runntime/src/zoo/moonshine/
  * decoder.ts:58-76,105-109; transcriber.ts:111-118,161-203) for `batch`
- * independent sequences in one launch.  The reference runs one sequence per
+ * independent sequences in one call: one launch, and a second, small one where the
+ * partials of the key splits are many.  The reference runs one sequence per
  * call; batch = 1 is that call.
  *
  * kCache/vCache: `batch` caches of [cacheRows, kvHeads*headDim] each,
@@ -189,7 +191,7 @@ RT_API int rt_attn_route(rt_ctx* ctx, const rt_attn_args* args, const char** rou
  * gathered by the caller; with batch 1 that is the reference's cosRow/sinRow).
  * Together with the row strides this lets q, kNew and vNew point into the one
  * fused qkv row the projection wrote, so a decoder layer's rope x 2, slice,
- * writeRows x 2 and attention (decoder.ts:58-76) become one launch.
+ * writeRows x 2 and attention (decoder.ts:58-76) become one call.
  *
  * partialsOut != NULL: instead of `out`, writes un-normalised partials
  * f32 [batch, qHeads, 2+headDim] = (m, l, acc) per head for a later

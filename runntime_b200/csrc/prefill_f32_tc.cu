@@ -20,7 +20,8 @@
 // Why not prefill_simt.cu: two-wide FMAs with three different operands run at 48 of the
 // 73 TFLOP/s, tf32 MMAs at 275, 92 in threes.
 // What bounds it: instructions and latency with two warps per scheduler (8.7 instructions per MMA, the
-// MMA pipe 32 % of active cycles), and the last row tiles.  8 sequences of 92..484 rows, 3 heads of
+// MMA pipe 32 % of active cycles), and the last row tiles; at head sizes up to 32 also the registers, 128 for
+// two CTAs per SM, of which 356 bytes a thread spill.  8 sequences of 92..484 rows, 3 heads of
 // 256 on one K/V head (2.4 GFLOP, 27 us at 92 TFLOP/s): 583 us for 16-row tiles of scalar FMAs, 155
 // for prefill_simt.cu, 102 here.
 //

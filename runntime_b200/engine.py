@@ -158,7 +158,7 @@ class KvCacheEngine:
         """One decoder-layer step from the fused projection's rows
         qkv [batch, (qHeads + 2*kvHeads)*headDim] (columns q|k|v, un-rotated): rope
         on q and k at each sequence's position, append, causal attend — the six
-        dispatches of packages/runntime/src/zoo/moonshine/decoder.ts:66-76 in one launch."""
+        dispatches of packages/runntime/src/zoo/moonshine/decoder.ts:66-76 in one call."""
         qw, kvw = self.qHeads * self.headDim, self.kvHeads * self.headDim
         es = qkv.element_size()
         base = qkv.data_ptr()

@@ -75,6 +75,7 @@ def test_activations_do_not_depend_on_the_row_count(ex, act):
     few, many = rows[0][0], rows[1][-1]
     assert (np.isnan(few) == np.isnan(many)).all(), (few, many)
     assert (few[np.isinf(few) | np.isinf(many)] == many[np.isinf(few) | np.isinf(many)]).all(), (few, many)
+    assert act not in ("gelu", "geluTanh", "silu") or many[0] == np.inf
     finite = np.isfinite(few)
     # (below 2^-14 halves are 2^-24 apart)
     few, many = few[finite], many[finite]
