@@ -57,7 +57,8 @@ __device__ __forceinline__ void row_band(const AttnParams& p, int64_t row, int64
     if (s0 > lo) lo = s0;
     if (s1 < end) end = s1;
   } else if (p.seqStride > 0) {
-    const int64_t b = row / p.seqStride;
+    // (a 64-bit division takes some 350 cycles, and blocks start with this one)
+    const int64_t b = (row >> 32) == 0 ? (int64_t)((uint32_t)row / (uint32_t)p.seqStride) : row / p.seqStride;
     const int64_t r = row - b * p.seqStride;
     const int64_t len = p.seqLens[b];
     if (r >= len) {

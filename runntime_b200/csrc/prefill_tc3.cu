@@ -12,10 +12,17 @@
 //     from,
 //   - the P V issuer accumulates O += P(j) V(j) in tile order as the halves of P arrive.
 // The running maximum is shared by the two warpgroups through shared memory: the
-// reference point of a row moves only when its maximum has grown by more than 2^8
+// reference point of a row moves only when its maximum has grown by more than 2^13
 // (rare after the first tile), and the "max phases" of consecutive tiles are
 // ordered by a per-warp counter, so both warpgroups always exponentiate against
 // the same reference point and the accumulator is rescaled by exactly one of them.
+// Up to head size 128 a tile's exponentials start before its max phase, against the
+// reference point last seen, and the maximum is gathered beside them; if the point has
+// moved, what was computed is computed again before anything is published.  (Together with
+// cheaper waits: 64 x 8192 rows causal, 8 heads of 128, 9440 -> 9220 us, the power limit
+// being what is left there; 16 x 2048 rows in a +-512 window 164 -> 140; head size 256,
+// where the one S buffer makes the order of the max phases matter more and the maximum
+// comes first, 32 sequences in that window 162 -> 139.)
 //
 // Head sizes: 64 and 128 (two S buffers), 256 (the accumulator takes half of tensor
 // memory, so there is ONE S buffer — free again as soon as its scores are in a warpgroup's
@@ -55,15 +62,6 @@ namespace {
 using namespace sm100;
 using namespace tc;
 
-#ifndef RT_TC3_WIDE_STORES
-#define RT_TC3_WIDE_STORES 1  // 32-byte stores in the read-out where the rows allow
-#endif
-#ifndef RT_TC3_CHECK_EMPTY
-#define RT_TC3_CHECK_EMPTY 1   // look a padded batch's length up before asking for the Q tile
-#endif
-#ifndef RT_TC3_RELAXED
-#define RT_TC3_RELAXED 0
-#endif
 constexpr int kThreads3 = 384;
 constexpr int kRegsSoftmax3 = 216, kRegsOther3 = 64;  // 2*128*216 + 128*64 <= 384*168
 constexpr int BK3 = 128;
@@ -192,13 +190,74 @@ constexpr uint32_t instr_desc_pair(int n, bool bMnMajor) {
   return (instr_desc(n, bMnMajor) & ~(0x1fu << 24)) | ((uint32_t)(256 >> 4) << 24);
 }
 
+// Waits (bounded) until the counter at `addr` has reached `want`; an acquire load pairs with the
+// release store of the warp that moved it.  The lanes of the warp agree on the outcome.
+__device__ __forceinline__ bool counter_poll_warp(uint32_t addr, int want, volatile int* abortFlag) {
+  bool reached = false;
+  for (int i = 0; i < (1 << 22); i++) {
+    int v;
+    asm volatile("ld.acquire.cta.shared::cta.s32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    if (v >= want) {
+      reached = true;
+      break;
+    }
+    if ((i & 63) == 63 && *abortFlag) break;
+  }
+  return __all_sync(0xffffffffu, reached);
+}
+
+// First and last key that four of the 128 rows from `row0` on see (lane, lane + 32, ...;
+// INT_MAX and -1 if none): row_band, with the loads of all four rows ahead of the first use
+// and no branch between them (row by row, each load waiting for the branch before it, this took
+// 2100 cycles at the start of every unit).
+__device__ __forceinline__ void rows_range(const AttnParams& p, int64_t row0, int lane, int& first, int& last) {
+  constexpr int kRows = BM / 32;
+  int64_t s0[kRows], s1[kRows];
+  if (p.segs) {
+    float a[kRows], b[kRows];
+#pragma unroll
+    for (int i = 0; i < kRows; i++) {
+      const int64_t row = min(row0 + lane + 32 * i, p.qLen - 1);
+      a[i] = p.segs[2 * row];
+      b[i] = p.segs[2 * row + 1];
+    }
+#pragma unroll
+    for (int i = 0; i < kRows; i++) s0[i] = (int64_t)a[i], s1[i] = (int64_t)b[i] - 1;
+  } else if (p.seqStride > 0) {
+    int len[kRows];
+#pragma unroll
+    for (int i = 0; i < kRows; i++) {
+      const uint32_t row = (uint32_t)min(row0 + lane + 32 * i, p.qLen - 1);   // (qLen is below 2^31)
+      const uint32_t b = row / (uint32_t)p.seqStride;
+      s0[i] = (int64_t)b * p.seqStride;
+      len[i] = p.seqLens[b];
+    }
+#pragma unroll
+    for (int i = 0; i < kRows; i++)
+      s1[i] = row0 + lane + 32 * i - s0[i] < len[i] ? s0[i] + len[i] - 1 : -1;
+  } else {
+#pragma unroll
+    for (int i = 0; i < kRows; i++) s0[i] = 0, s1[i] = p.kvLen - 1;
+  }
+  first = INT_MAX;
+  last = -1;
+#pragma unroll
+  for (int i = 0; i < kRows; i++) {
+    const int64_t row = row0 + lane + 32 * i, pos = p.qPosOffset + row;
+    const int64_t lo = max(max(pos - p.wl, s0[i]), (int64_t)0);
+    const int64_t end = min(min(pos + p.wr, s1[i]), p.kvLen - 1);
+    if (row < p.qLen && lo <= end) first = min(first, (int)lo), last = max(last, (int)end);
+  }
+}
+
 // PADDED: the head is narrower than the 64 columns the tile holds (see the file header);
 // p.hd is the real size, `shift` = (kvh * hd) & 7 the head's first column inside the box.
 // PAIR: two CTAs of a cluster share every K/V tile (see the file header).
 template <int HD, bool PADDED, bool PAIR>
 __global__ void __launch_bounds__(kThreads3, 1)
 prefill_tc3_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
-                   const __grid_constant__ CUtensorMap mapV, const AttnParams p, int* status) {
+                   const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapO,
+                   const AttnParams p, int* status) {
   using C = Cfg3<HD, PAIR>;
   constexpr int BK = BK3, KP = C::KP, VP = C::VP, NS = C::SLOTS;
   static_assert(!PADDED || (HD == 64 && !PAIR), "narrow heads are padded to 64 columns, one CTA");
@@ -206,7 +265,8 @@ prefill_tc3_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
   __shared__ Barriers3 bars;
   __shared__ uint32_t sTmemBase;
   __shared__ int sAbort;
-  __shared__ int sLoMin[8], sEndMax[8];
+  __shared__ int sLoMin[8], sEndMax[8];   // a pair's range of keys, by warp
+  __shared__ int sUnit[2];                // one CTA alone: first key tile and number of key tiles
   __shared__ float sMref[BM];          // the rows' reference points (log2 domain)
   __shared__ float sL[2][BM];          // the warpgroups' row sums, for the epilogue
   __shared__ volatile int sMaxDone[4];  // per warp of a warpgroup: tiles whose max phase is over
@@ -228,34 +288,57 @@ prefill_tc3_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
   const uint32_t sQ = smemBase;
   const uint32_t sRing = sQ + C::Q_BYTES;
 
-  // One CTA alone: the Q tile needs nothing but the CTA's coordinates, so the producer's lane
-  // sets up its barrier and starts its copy before the rest of the set-up (tensor memory,
-  // the rows' bands, which read sequence lengths from memory) instead of after it.
-  constexpr bool EARLY_Q = !PAIR && !PADDED;
-  // (In a padded batch the units past a sequence's end see no key and must not pay for a Q
-  // tile: the lane looks the length up first.)
-  bool earlyQ = false;
-  if (EARLY_Q && tid == 8 * 32) {
-    mbar_init(smem_u32(&bars.fullQ), 1);
-    fence_barrier_init();
-    earlyQ = true;
-    if (RT_TC3_CHECK_EMPTY && p.seqStride > 0 && !p.segs) {
-      const int64_t b0 = row0 / p.seqStride;
-      earlyQ = row0 - b0 * p.seqStride < p.seqLens[b0];
+  const int xKV = PADDED ? ((kvh * hd) & ~7) : kvh * HD;
+
+  // One CTA alone: the producer warp works the unit's key range out by itself (four rows per
+  // lane) and starts the copies of Q and of the first K tile before the rest of the set-up —
+  // tensor memory, the rows' bands — instead of after the barrier that ends it: the first S of
+  // a unit at head size 128 is there 4340 cycles after the block's start, 5020 before (of 24000
+  // for nine key tiles).
+  if (!PAIR && warp == 8) {
+    if (lane == 0) {
+      if (!PADDED) prefetch_tensormap(&mapQ);
+      prefetch_tensormap(&mapK);
+      prefetch_tensormap(&mapV);
+      mbar_init(smem_u32(&bars.fullQ), 1);
+      for (int s = 0; s < kMaxSlots; s++) {
+        mbar_init(smem_u32(&bars.full[s]), 1);
+        mbar_init(smem_u32(&bars.empty[s]), 1);
+      }
+      fence_barrier_init();
     }
-    if (earlyQ) {
-      prefetch_tensormap(&mapQ);
-      mbar_expect_tx(smem_u32(&bars.fullQ), C::Q_BYTES);
-      for (int c = 0; c < C::CHUNKS; c++)
-        tma_load_2d(sQ + c * (BM * 128), &mapQ, h * HD + c * 64, (int)row0, smem_u32(&bars.fullQ));
+    int wl, we;
+    rows_range(p, row0, lane, wl, we);
+    wl = __reduce_min_sync(0xffffffffu, wl);
+    we = __reduce_max_sync(0xffffffffu, we);
+    if (lane == 0) {
+      const int first = we >= 0 ? wl / BK : 0;
+      sUnit[0] = first;
+      sUnit[1] = we >= 0 ? we / BK - first + 1 : 0;
+      if (we >= 0) {   // (in a padded batch the units past a sequence's end ask for nothing)
+        if (!PADDED) {
+          mbar_expect_tx(smem_u32(&bars.fullQ), C::Q_BYTES);
+          for (int c = 0; c < C::CHUNKS; c++)
+            tma_load_2d(sQ + c * (BM * 128), &mapQ, h * HD + c * 64, (int)row0, smem_u32(&bars.fullQ));
+        }
+        for (int part = 0; part < KP; part++) {
+          mbar_expect_tx(smem_u32(&bars.full[part]), C::K_BYTES);
+          for (int c = 0; c < C::K_CHUNKS; c++)
+            tma_load_2d(sRing + part * C::SLOT_BYTES + c * (C::K_ROWS * 128), &mapK,
+                        xKV + (part * C::K_CHUNKS + c) * 64, first * BK, smem_u32(&bars.full[part]));
+        }
+      }
     }
+    __syncwarp();
   }
   if (tid == 0) {
     sAbort = 0;
-    if (!EARLY_Q) mbar_init(smem_u32(&bars.fullQ), 1);
-    for (int s = 0; s < kMaxSlots; s++) {
-      mbar_init(smem_u32(&bars.full[s]), 1);
-      mbar_init(smem_u32(&bars.empty[s]), 1);
+    if (PAIR) {
+      mbar_init(smem_u32(&bars.fullQ), 1);
+      for (int s = 0; s < kMaxSlots; s++) {
+        mbar_init(smem_u32(&bars.full[s]), 1);
+        mbar_init(smem_u32(&bars.empty[s]), 1);
+      }
     }
     for (int b = 0; b < 2; b++) {
       mbar_init(smem_u32(&bars.sFull[b]), 1);
@@ -278,12 +361,42 @@ prefill_tc3_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
     }
   }
 
-  // Band of this thread's row, then of the whole unit (one row tile, or the pair's two):
-  // the two CTAs of a pair walk the same key tiles, so each works the range out for both —
-  // warps 0-3 from its own rows, warps 4-7 from the other CTA's.
+  // Band of this thread's row.  The two CTAs of a pair walk the same key tiles, so each works
+  // the range out for both — warps 0-3 from its own rows, warps 4-7 from the other CTA's.
   const int rowInTile = tid & 127;
   int lo = 1, end = 0;  // empty
   if (warp < 8) {
+    // Q of a narrow head by hand: 16-byte units of the swizzled K-major layout, the head's
+    // columns at [shift, shift + hd), zeros beside them and in rows past the end.  A head
+    // starts on four elements of the tile, so a unit is two quads that are inside or outside
+    // as a whole; they are read as such (as pairs where q's rows start on four bytes only),
+    // all of a thread's before the first is used: element by element, after the barrier, this
+    // took 4000 of a unit's 26000 cycles (head size 52, nine key tiles).
+    constexpr int kUnits = PADDED ? BM * 8 / 256 : 1;
+    uint2 v[kUnits][2];
+    if (PADDED) {
+      const __half* qg = static_cast<const __half*>(p.q) + (int64_t)h * hd;
+      const bool quads = (reinterpret_cast<uintptr_t>(p.q) & 7u) == 0 && p.qStride % 4 == 0;
+      auto load = [&](auto read) {
+#pragma unroll
+        for (int i = 0; i < kUnits; i++) {
+          const int u = tid + 256 * i, c0 = (u & 7) * 8 - shift;
+          const int64_t row = row0 + (u >> 3);
+#pragma unroll
+          for (int e = 0; e < 2; e++) {
+            const int c = c0 + 4 * e;
+            v[i][e] = make_uint2(0u, 0u);
+            if (row < p.qLen && c >= 0 && c < hd) v[i][e] = read(qg + row * p.qStride + c);
+          }
+        }
+      };
+      if (quads) load([](const __half* src) { return *reinterpret_cast<const uint2*>(src); });
+      else
+        load([](const __half* src) {
+          const uint32_t* w = reinterpret_cast<const uint32_t*>(src);
+          return make_uint2(w[0], w[1]);
+        });
+    }
     const int64_t row = row0 + rowInTile;
     if (row < p.qLen) {
       int64_t l64, e64;
@@ -293,23 +406,29 @@ prefill_tc3_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
         end = (int)e64;
       }
     }
-    int olo = lo, oend = end;   // the row this thread contributes to the unit's range
-    if (PAIR && warp >= 4) {
-      const int64_t other = (int64_t)(unit * 2 + (1 - cta)) * BM + rowInTile;
-      olo = 1, oend = 0;
-      if (other < p.qLen) {
-        int64_t l64, e64;
-        row_band(p, other, l64, e64);
-        if (l64 <= e64) olo = (int)l64, oend = (int)e64;
-      }
-    }
-    if (warp < 4 || PAIR) {
-      int wl = olo <= oend ? olo : INT_MAX, we = olo <= oend ? oend : -1;
+    if (PADDED) {
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        wl = min(wl, __shfl_xor_sync(0xffffffffu, wl, o));
-        we = max(we, __shfl_xor_sync(0xffffffffu, we, o));
+      for (int i = 0; i < kUnits; i++) {
+        const int u = tid + 256 * i, r = u >> 3;
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sQ + r * 128 + (((u & 7) ^ (r & 7)) << 4)),
+                     "r"(v[i][0].x), "r"(v[i][0].y), "r"(v[i][1].x), "r"(v[i][1].y)
+                     : "memory");
       }
+      fence_proxy_async();  // generic-proxy stores -> visible to the tensor core after the barrier
+    }
+    if (PAIR) {
+      int olo = lo, oend = end;   // the row this thread contributes to the pair's range
+      if (warp >= 4) {
+        const int64_t other = (int64_t)(unit * 2 + (1 - cta)) * BM + rowInTile;
+        olo = 1, oend = 0;
+        if (other < p.qLen) {
+          int64_t l64, e64;
+          row_band(p, other, l64, e64);
+          if (l64 <= e64) olo = (int)l64, oend = (int)e64;
+        }
+      }
+      const int wl = __reduce_min_sync(0xffffffffu, olo <= oend ? olo : INT_MAX);
+      const int we = __reduce_max_sync(0xffffffffu, olo <= oend ? oend : -1);
       if (lane == 0) {
         sLoMin[warp] = wl;
         sEndMax[warp] = we;
@@ -326,14 +445,20 @@ prefill_tc3_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
   tc_fence_after_sync();
   TC_TRACE(99, 0);
   const uint32_t tmem = sTmemBase;
-  int tileLo = INT_MAX, tileEnd = -1;
+  int kt0, nTiles;
+  if (PAIR) {
+    int tileLo = INT_MAX, tileEnd = -1;
 #pragma unroll
-  for (int w8 = 0; w8 < (PAIR ? 8 : 4); w8++) {
-    tileLo = min(tileLo, sLoMin[w8]);
-    tileEnd = max(tileEnd, sEndMax[w8]);
+    for (int w8 = 0; w8 < 8; w8++) {
+      tileLo = min(tileLo, sLoMin[w8]);
+      tileEnd = max(tileEnd, sEndMax[w8]);
+    }
+    kt0 = tileEnd >= 0 ? tileLo / BK : 0;
+    nTiles = tileEnd >= 0 ? tileEnd / BK - kt0 + 1 : 0;
+  } else {
+    kt0 = sUnit[0];
+    nTiles = sUnit[1];
   }
-  const int kt0 = tileEnd >= 0 ? tileLo / BK : 0;
-  const int nTiles = tileEnd >= 0 ? tileEnd / BK - kt0 + 1 : 0;
 
   if (warp >= 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsOther3));
@@ -343,27 +468,24 @@ prefill_tc3_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
       // own ring (which both CTAs walk in step: same sequence numbers, same slots); all
       // completions are counted on the even CTA's barriers, where the byte counts expected
       // are the pair's.
-      // (a unit that sees no key leaves only after the Q tile it asked for has landed)
-      if (EARLY_Q && lane == 0 && nTiles == 0 && earlyQ) mbar_wait(smem_u32(&bars.fullQ), 0, &sAbort);
       if (lane == 0 && nTiles > 0) {
-        prefetch_tensormap(&mapK);
-        prefetch_tensormap(&mapV);
         auto load = [&](uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
           if (PAIR) tma_load_2d_pair(dst, map, x, y, bar);
           else tma_load_2d(dst, map, x, y, bar);
         };
-        if (!PADDED && !earlyQ) {
+        if (PAIR) {
           prefetch_tensormap(&mapQ);
+          prefetch_tensormap(&mapK);
+          prefetch_tensormap(&mapV);
           if (leader) mbar_expect_tx(smem_u32(&bars.fullQ), C::CTAS * C::Q_BYTES);
           for (int c = 0; c < C::CHUNKS; c++)
             load(sQ + c * (BM * 128), &mapQ, h * HD + c * 64, (int)row0, smem_u32(&bars.fullQ));
         }
-        const int xKV = PADDED ? ((kvh * hd) & ~7) : kvh * HD;
-        int seq = 0;
+        int seq = PAIR ? 0 : KP;   // (one CTA alone: K(0) is on its way)
         bool ok = true;
         auto slot_for = [&](int& slot) {  // claims the next ring slot, waiting for its release
           slot = seq % NS;
-          if (seq >= NS) ok = mbar_wait(smem_u32(&bars.empty[slot]), ((seq / NS) - 1) & 1, &sAbort);
+          if (seq >= NS) ok = mbar_poll(smem_u32(&bars.empty[slot]), ((seq / NS) - 1) & 1, &sAbort);
           seq++;
           return ok;
         };
@@ -390,11 +512,12 @@ prefill_tc3_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
               load(dst + c * (C::V_ROWS * 128), &mapV, x0 + c * 64, key0 + part * C::V_ROWS, bar);
           }
         };
-        load_k(0);
+        if (PAIR) load_k(0);
         for (int j = 0; j < nTiles && ok; j++) {
           if (j + 1 < nTiles) load_k(j + 1);
           if (ok) load_v(j);
         }
+        if (!ok) sAbort = 1;
       }
     } else if (warp == 9 && leader) {
       // ------------------------------ MMA issuer: S = Q K^T ----------------------
@@ -406,12 +529,12 @@ prefill_tc3_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
         constexpr uint32_t kLboK = (16u >> 4) << 16;
         auto desc = [](uint32_t lo32) { return ((uint64_t)kDescHi << 32) | lo32; };
         auto wait = [&](uint64_t* bar, int parity) {
-          return __all_sync(0xffffffffu, mbar_wait(smem_u32(bar), (uint32_t)parity, &sAbort)) != 0;
+          return mbar_poll_warp(smem_u32(bar), (uint32_t)parity, &sAbort);
         };
         // descriptors carry the 18-bit offset inside the CTA's window, not the CTA's rank bits
         const uint32_t aLo = ((sQ & 0x3ffffu) >> 4) | kLboK;
         const int kSteps = PADDED ? (shift + hd + 15) / 16 : HD / 16;  // K = 16 per instruction
-        bool ok = wait(&bars.fullQ, 0);
+        bool ok = PADDED || wait(&bars.fullQ, 0);   // (a narrow head's Q was staged before the barrier)
 #pragma unroll 1
         for (int j = 0; j < nTiles && ok; j++) {
           const int b = j & 1;
@@ -455,6 +578,7 @@ prefill_tc3_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
             TC_TRACE(12, j);
           }
         }
+        if (!ok) sAbort = 1;
       }
     } else if (warp == 10 && leader) {
       // ------------------------------ MMA issuer: O += P V ------------------------
@@ -463,7 +587,7 @@ prefill_tc3_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
         constexpr uint32_t kLboV = ((uint32_t)(C::V_ROWS * 128) >> 4) << 16;  // next 64 columns of hd
         auto desc = [](uint32_t lo32) { return ((uint64_t)kDescHi << 32) | lo32; };
         auto wait = [&](uint64_t* bar, int parity) {
-          return __all_sync(0xffffffffu, mbar_wait(smem_u32(bar), (uint32_t)parity, &sAbort)) != 0;
+          return mbar_poll_warp(smem_u32(bar), (uint32_t)parity, &sAbort);
         };
         const uint32_t idescO = PAIR ? instr_desc_pair(HD, true)
                                      : instr_desc(PADDED ? ((shift + hd + 15) & ~15) : HD, true);
@@ -507,6 +631,7 @@ prefill_tc3_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
             __syncwarp();
           }
         }
+        if (!ok) sAbort = 1;
       }
     }
   } else {
@@ -524,37 +649,13 @@ prefill_tc3_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
     };
     bool ok = true;
 
-    if (PADDED && nTiles > 0) {
-      // Q tile by hand: 16-byte units of the swizzled K-major layout, the head's columns at
-      // [shift, shift + hd), zeros beside them and in rows past the end.
-      const __half* qg = static_cast<const __half*>(p.q) + (int64_t)h * hd;
-      for (int u = tid; u < BM * 8; u += 256) {
-        const int r = u >> 3, unit8 = u & 7;
-        const int64_t row = row0 + r;
-        __align__(16) __half vals[8];
-#pragma unroll
-        for (int e = 0; e < 8; e++) {
-          const int c = unit8 * 8 + e - shift;
-          vals[e] = (row < p.qLen && c >= 0 && c < hd) ? qg[row * p.qStride + c] : __half(0.f);
-        }
-        const uint32_t addr = sQ + r * 128 + ((unit8 ^ (r & 7)) << 4);
-        const uint4 v4 = *reinterpret_cast<const uint4*>(vals);
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v4.x), "r"(v4.y),
-                     "r"(v4.z), "r"(v4.w)
-                     : "memory");
-      }
-      fence_proxy_async();  // generic-proxy stores -> visible to the tensor core
-      named_barrier_sync(2, 256);
-      if (tid == 0) mbar_arrive(smem_u32(&bars.fullQ));
-    }
-
     float seen = p.sinks ? p.sinks[h] : kNegSeed;  // the reference point this thread's l is relative to
     float l = (p.sinks && g == 0) ? 1.f : 0.f;
 #pragma unroll 1
     for (int j = g; j < nTiles && ok; j += 2) {
       const int key0 = (kt0 + j) * BK;
       TC_TRACE(0, j);
-      ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&bars.sFull[g]), (j >> 1) & 1, &sAbort));
+      ok = mbar_poll_warp(smem_u32(&bars.sFull[g]), (j >> 1) & 1, &sAbort);
       if (!ok) break;  // the whole warp leaves together
       tc_fence_after_sync();
       TC_TRACE(1, j);
@@ -586,120 +687,22 @@ prefill_tc3_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
         for (int c = 0; c < BK; c++)
           sv[c] = ((unsigned)(c - c0) <= span) ? sv[c] : 0xff800000u;  // -inf
       }
-      // Row maximum: four independent chains of 3-input max.
+      // Row maximum: four independent chains of 3-input max, gathered while the special-
+      // function unit works on the first half's exponentials.
       float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-      for (int c = 0; c < BK; c += 8) {
+      float2 sum2[4];
+      uint32_t pk[32];
+      auto foldMax = [&](int c) {  // columns c .. c+7
 #pragma unroll
         for (int u = 0; u < 4; u++)
           mx4[u] = max3(mx4[u], __uint_as_float(sv[c + 2 * u]), __uint_as_float(sv[c + 2 * u + 1]));
-      }
-      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * kLog2e;
-      TC_TRACE(21, j);
-
-      // ---- max phase, in tile order across the two warpgroups ----
-      if (j > 0) {
-        // (an acquire load pairs with the release store below: what the other warpgroup's
-        // warp wrote before it — reference points, its rescale of O — is visible after it)
-        bool arrived = false;
-        const uint32_t doneAddr = smem_u32(const_cast<int*>(&sMaxDone[w]));
-        for (int i = 0; i < (1 << 22); i++) {
-          int done;
-#if RT_TC3_RELAXED
-          (void)doneAddr;
-          done = sMaxDone[w];
-#else
-          asm volatile("ld.acquire.cta.shared::cta.s32 %0, [%1];" : "=r"(done) : "r"(doneAddr) : "memory");
-#endif
-          if (done >= j) { arrived = true; break; }
-          if ((i & 63) == 63) {
-            if (sAbort) break;
-            __nanosleep(64);
-          }
-        }
-        ok = __all_sync(0xffffffffu, arrived);
-        if (!ok) {
-          sAbort = 1;
-          break;
-        }
-        tc_fence_after_sync();
-      }
-      TC_TRACE(22, j);
-      float mref = sMref[rowInTile];
-      if (mref != seen) {  // the other warpgroup moved the reference point since this one last looked
-        l *= fast_exp2(seen - mref);
-        seen = mref;
-      }
-      const bool grow = mx > mref + kRescaleThreshold;
-      if (__any_sync(0xffffffffu, grow)) {
-        // A row whose reference point is still the seed has seen no key in any tile so far:
-        // its accumulator row is exactly zero and needs no pass (the rows of a band's first,
-        // partly masked tile meet their first keys in the second one).  When only such rows
-        // have grown, they alone move; the pass over O, when there is one, moves every row.
-        const bool pass = j > 0 && __any_sync(0xffffffffu, grow && mref != kNegSeed);
-        const float mnew = (pass || j == 0 || mref == kNegSeed) ? fmaxf(mref, mx) : mref;
-        const float f = fast_exp2(mref - mnew);
-        if (pass) {
-          // O holds the tiles up to j-1 once P V(j-1) has landed (the products complete in order)
-          ok = __all_sync(0xffffffffu,
-                          mbar_wait(smem_u32(&bars.pvDone[(j - 1) & 1]), ((j - 1) >> 1) & 1, &sAbort));
-          if (!ok) break;
-          tc_fence_after_sync();
-          constexpr int oCols = PADDED ? 64 : HD;
+      };
+      auto clearSums = [&]() {
 #pragma unroll
-          for (int c = 0; c < oCols; c += 32) {
-            uint32_t o[32];
-            tmem_ld32(oCol + c, o);
-            tmem_wait_ld();
-#pragma unroll
-            for (int x = 0; x < 32; x++) o[x] = __float_as_uint(__uint_as_float(o[x]) * f);
-            tmem_st32(oCol + c, o);
-          }
-          tmem_wait_st();
-          tc_fence_before_sync();
-        }
-        l *= f;
-        mref = seen = mnew;
-        sMref[rowInTile] = mnew;
-      }
-      __syncwarp();
-#if RT_TC3_RELAXED
-      if (lane == 0) sMaxDone[w] = j + 1;
-#else
-      if (lane == 0)
-        asm volatile("st.release.cta.shared::cta.s32 [%0], %1;" ::"r"(
-                         smem_u32(const_cast<int*>(&sMaxDone[w]))),
-                     "r"(j + 1)
-                     : "memory");
-#endif
-      TC_TRACE(3, j);
-
-      // ---- exponentials, P in two halves ----
-      // P's own columns were last read by P V(j-2).
-      if (j >= 2) {
-#if RT_TC3_RELAXED
-        // (nearly always complete by now: one look by one lane, the full wait only if not)
-        const uint32_t pvBar = smem_u32(&bars.pvDone[g]);
-        const uint32_t pvPar = ((j >> 1) - 1) & 1;
-        int done = 0;
-        if (lane == 0) done = mbar_test_wait(pvBar, pvPar);
-        if (!__shfl_sync(0xffffffffu, done, 0)) {
-          ok = __all_sync(0xffffffffu, mbar_wait(pvBar, pvPar, &sAbort));
-          if (!ok) break;
-        }
-#else
-        ok = __all_sync(0xffffffffu,
-                        mbar_wait(smem_u32(&bars.pvDone[g]), ((j >> 1) - 1) & 1, &sAbort));
-        if (!ok) break;
-#endif
-      }
-      TC_TRACE(6, j);
-      float2 sum2[4] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f),
-                        make_float2(0.f, 0.f)};
-      const float2 scale2 = make_float2(kLog2e, kLog2e), shift2 = make_float2(-mref, -mref);
-#pragma unroll
-      for (int half = 0; half < 2; half++) {
-        uint32_t pk[32];
+        for (int u = 0; u < 4; u++) sum2[u] = make_float2(0.f, 0.f);
+      };
+      auto expHalf = [&](int half, bool withMax) {
+        const float2 scale2 = make_float2(kLog2e, kLog2e), shift2 = make_float2(-seen, -seen);
 #pragma unroll
         for (int c = 0; c < 64; c += 2) {
           const int cc = half * 64 + c;
@@ -709,21 +712,109 @@ prefill_tc3_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
           sum2[(c >> 1) & 3] = add2(sum2[(c >> 1) & 3], pe);
           const __half2 hp = __floats2half2_rn(pe.x, pe.y);
           pk[c / 2] = *reinterpret_cast<const uint32_t*>(&hp);
+          if (withMax && (c & 3) == 0) foldMax(2 * c);  // 16 steps x 8 columns = all 128
         }
-        TC_TRACE(7 + half, j);
+      };
+      clearSums();
+      // The exponentials of a warpgroup's first tile wait for a reference point; later tiles
+      // start against the one last seen, and the half is computed again if it has moved.
+      const bool early = HD < 256 && j > 1;
+      if (early) {
+        expHalf(0, true);
+      } else {
+#pragma unroll
+        for (int c = 0; c < BK; c += 8) foldMax(c);
+      }
+      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * kLog2e;
+      TC_TRACE(21, j);
+
+      // ---- max phase, in tile order across the two warpgroups ----
+      if (j > 0) {
+        // (an acquire load pairs with the release store below: what the other warpgroup's
+        // warp wrote before it — reference points, its rescale of O — is visible after it)
+        ok = counter_poll_warp(smem_u32(const_cast<int*>(&sMaxDone[w])), j, &sAbort);
+        if (!ok) break;
+        tc_fence_after_sync();
+      }
+      TC_TRACE(22, j);
+      float mref = sMref[rowInTile];
+      const bool grow = mx > mref + kRescaleThreshold;
+      if (__any_sync(0xffffffffu, grow || mref != seen || !early)) {
+        if (mref != seen) {  // the other warpgroup moved the reference point since this one last looked
+          l *= fast_exp2(seen - mref);
+          seen = mref;
+        }
+        if (__any_sync(0xffffffffu, grow)) {
+          // A row whose reference point is still the seed has seen no key in any tile so far:
+          // its accumulator row is exactly zero and needs no pass (the rows of a band's first,
+          // partly masked tile meet their first keys in the second one).  When only such rows
+          // have grown, they alone move; the pass over O, when there is one, moves every row.
+          const bool pass = j > 0 && __any_sync(0xffffffffu, grow && mref != kNegSeed);
+          const float mnew = (pass || j == 0 || mref == kNegSeed) ? fmaxf(mref, mx) : mref;
+          const float f = fast_exp2(mref - mnew);
+          if (pass) {
+            // O holds the tiles up to j-1 once P V(j-1) has landed (the products complete in order)
+            ok = mbar_poll_warp(smem_u32(&bars.pvDone[(j - 1) & 1]), ((j - 1) >> 1) & 1, &sAbort);
+            if (!ok) break;
+            tc_fence_after_sync();
+            constexpr int oCols = PADDED ? 64 : HD;
+#pragma unroll
+            for (int c = 0; c < oCols; c += 32) {
+              tmem_ld32(oCol + c, pk);
+              tmem_wait_ld();
+#pragma unroll
+              for (int x = 0; x < 32; x++) pk[x] = __float_as_uint(__uint_as_float(pk[x]) * f);
+              tmem_st32(oCol + c, pk);
+            }
+            tmem_wait_st();
+            tc_fence_before_sync();
+          }
+          l *= f;
+          mref = seen = mnew;
+          sMref[rowInTile] = mnew;
+        }
+        clearSums();
+        __syncwarp();
+        if (lane == 0)
+          asm volatile("st.release.cta.shared::cta.s32 [%0], %1;" ::"r"(
+                           smem_u32(const_cast<int*>(&sMaxDone[w]))),
+                       "r"(j + 1)
+                       : "memory");
+        expHalf(0, false);
+      } else if (lane == 0) {
+        asm volatile("st.release.cta.shared::cta.s32 [%0], %1;" ::"r"(
+                         smem_u32(const_cast<int*>(&sMaxDone[w]))),
+                     "r"(j + 1)
+                     : "memory");
+      }
+      TC_TRACE(3, j);
+
+      // ---- P in two halves ----
+      // P's own columns were last read by P V(j-2).
+      if (j >= 2) {
+        ok = mbar_poll_warp(smem_u32(&bars.pvDone[g]), ((j >> 1) - 1) & 1, &sAbort);
+        if (!ok) break;
+      }
+      TC_TRACE(6, j);
+      auto publish = [&](int half) {
         tmem_st32(pCol + half * 32, pk);
         tmem_wait_st();
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) arrive(&bars.pReady[g][half]);
         TC_TRACE(4 + half, j);
-      }
+      };
+      publish(0);
+      expHalf(1, false);
+      publish(1);
       const float2 s01 = add2(add2(sum2[0], sum2[1]), add2(sum2[2], sum2[3]));
       l += s01.x + s01.y;
     }
 
+    if (!ok) sAbort = 1;
+
     // ---- epilogue: both warpgroups, half of the output columns each ----
-    // (every softmax thread passes the two barriers, also after a failed wait)
+    // (every softmax thread passes the barriers, also after a failed wait)
     named_barrier_sync(2, 256);
     {
       const float mfin = sMref[rowInTile];
@@ -732,74 +823,102 @@ prefill_tc3_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
     }
     named_barrier_sync(2, 256);
     l = sL[0][rowInTile] + sL[1][rowInTile];
-    const int64_t row = row0 + rowInTile;
-    __half* out = static_cast<__half*>(p.out) + row * ((int64_t)p.qHeads * hd) + (int64_t)h * hd;
-    const bool wide = !PADDED && (reinterpret_cast<uintptr_t>(p.out) & 31u) == 0;   // rows start on 32 bytes
-    if (nTiles > 0 && ok && !sAbort) {
-      ok = mbar_wait(smem_u32(&bars.pvDone[(nTiles - 1) & 1]), ((nTiles - 1) >> 1) & 1, &sAbort);
-      if (ok) {
+    // The unit's rows go out through the Q tile's shared memory, which the last S has left:
+    // one bulk tensor store per 64 columns (rows past the end are outside the map), or, for
+    // a narrow head, whose columns start on eight bytes, quads in the order of memory.  A
+    // thread that stores its own row sends each piece of 32 bytes to another row's sectors:
+    // 2000 cycles a unit at head size 128, 3500 at 256, 3900 in 4-byte pieces at 52.
+    bool good = ok && !sAbort;
+    if (nTiles > 0) {
+      if (good) {
+        good = mbar_poll(smem_u32(&bars.pvDone[(nTiles - 1) & 1]), ((nTiles - 1) >> 1) & 1, &sAbort);
+        if (!good) sAbort = 1;
+      }
+      good = __all_sync(0xffffffffu, good);
+      if (good) {
         tc_fence_after_sync();
         const float invL = (l > 0.f && lo <= end) ? 1.f / l : 0.f;  // a row that saw no key: zeros
-        constexpr int oCols = PADDED ? 64 : HD;
-        constexpr int perGroup = oCols / 2;
+        constexpr int perGroup = (PADDED ? 64 : HD) / 2;
 #pragma unroll
-        for (int c = g * perGroup; c < (g + 1) * perGroup; c += 32) {
+        for (int c = 0; c < perGroup; c += 32) {
+          const int col = g * perGroup + c;
           uint32_t o[32];
-          tmem_ld32(oCol + c, o);
+          tmem_ld32(oCol + col, o);
           tmem_wait_ld();
-          if (row < p.qLen) {
-            if (PADDED) {
+          uint32_t wds[16];
 #pragma unroll
-              for (int x = 0; x < 32; x += 2) {
-                const int col = c + x - shift;  // even: shift is 0 or 4
-                if (col >= 0 && col < hd)
-                  *reinterpret_cast<__half2*>(out + col) = __floats2half2_rn(
-                      __uint_as_float(o[x]) * invL, __uint_as_float(o[x + 1]) * invL);
-              }
-            } else {
-              uint4 pkd[4];
-              uint32_t* wds = reinterpret_cast<uint32_t*>(pkd);
+          for (int x = 0; x < 32; x += 2) {
+            const __half2 hp = __floats2half2_rn(__uint_as_float(o[x]) * invL,
+                                                 __uint_as_float(o[x + 1]) * invL);
+            wds[x / 2] = *reinterpret_cast<const uint32_t*>(&hp);
+          }
+          if (PADDED) {
+            const uint32_t base = sQ + rowInTile * (hd * 2);
 #pragma unroll
-              for (int x = 0; x < 32; x += 2) {
-                const __half2 hp = __floats2half2_rn(__uint_as_float(o[x]) * invL,
-                                                     __uint_as_float(o[x + 1]) * invL);
-                wds[x / 2] = *reinterpret_cast<const uint32_t*>(&hp);
-              }
-              if (RT_TC3_WIDE_STORES && wide) {
-                // a row's piece is then one full 32-byte sector per request instead of half of
-                // one (the stores of a warp go to 32 different rows)
-#pragma unroll
-                for (int v = 0; v < 2; v++)
-                  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(
-                                   out + c + 16 * v),
-                               "r"(wds[8 * v]), "r"(wds[8 * v + 1]), "r"(wds[8 * v + 2]), "r"(wds[8 * v + 3]),
-                               "r"(wds[8 * v + 4]), "r"(wds[8 * v + 5]), "r"(wds[8 * v + 6]), "r"(wds[8 * v + 7])
-                               : "memory");
-              } else {
-#pragma unroll
-                for (int v = 0; v < 4; v++) reinterpret_cast<uint4*>(out + c)[v] = pkd[v];
-              }
+            for (int x = 0; x < 32; x += 4) {
+              const int at = col + x - shift;   // a quad is inside the head or outside as a whole
+              if (at >= 0 && at < hd)
+                asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(base + at * 2), "r"(wds[x / 2]),
+                             "r"(wds[x / 2 + 1])
+                             : "memory");
             }
+          } else {
+            const uint32_t base = sQ + (col >> 6) * (BM * 128) + rowInTile * 128;
+#pragma unroll
+            for (int v = 0; v < 4; v++)
+              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(
+                               base + (((((col & 63) >> 3) + v) ^ (rowInTile & 7)) << 4)),
+                           "r"(wds[4 * v]), "r"(wds[4 * v + 1]), "r"(wds[4 * v + 2]), "r"(wds[4 * v + 3])
+                           : "memory");
+          }
+        }
+        if (!PADDED) fence_proxy_async();
+      }
+      // At head sizes of 128 and more a warpgroup stores the chunks it has written itself.
+      constexpr bool own = !PADDED && HD >= 128;
+      if (own) named_barrier_sync(3 + g, 128);
+      else named_barrier_sync(2, 256);
+      if (!PADDED && good && w == 0 && (own || g == 0) && elect_one()) {
+        constexpr int chunks = own ? C::CHUNKS / 2 : C::CHUNKS;
+#pragma unroll
+        for (int c = 0; c < chunks; c++) {
+          const int chunk = (own ? g * chunks : 0) + c;
+          tma_store_2d(&mapO, sQ + chunk * (BM * 128), h * HD + chunk * 64, (int)row0);
+        }
+        bulk_commit();
+        bulk_wait_read<0>();
+      }
+    }
+    if (PADDED && good) {
+      // (zeros where no row of the unit sees a key)
+      __half* base = static_cast<__half*>(p.out) + (int64_t)h * hd;
+      const int64_t pitch = (int64_t)p.qHeads * hd;
+      const bool quads = (reinterpret_cast<uintptr_t>(p.out) & 7u) == 0;
+      const int perRow = hd / 4;
+      for (int u = tid; u < BM * perRow; u += 256) {
+        const int r = u / perRow, c = (u - r * perRow) * 4;
+        if (row0 + r < p.qLen) {
+          uint2 v = make_uint2(0u, 0u);
+          if (nTiles > 0)
+            asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(sQ + u * 8));
+          __half* dst = base + (row0 + r) * pitch + c;
+          if (quads) {
+            *reinterpret_cast<uint2*>(dst) = v;
+          } else {
+            reinterpret_cast<uint32_t*>(dst)[0] = v.x;
+            reinterpret_cast<uint32_t*>(dst)[1] = v.y;
           }
         }
       }
     } else if (nTiles == 0) {
-      // No row of this unit sees a key (in a padded batch: every unit past a sequence's end).
-      if (PADDED) {
-        if (row < p.qLen)
-          for (int c = g * (hd / 2); c < (g + 1) * (hd / 2); c += 2)
-            *reinterpret_cast<__half2*>(out + c) = __floats2half2_rn(0.f, 0.f);
-      } else {
-        // 16-byte stores, consecutive threads on consecutive pieces of a row: a thread per
-        // row writing its own row in 4-byte pieces made such a unit cost ~9 us of store
-        // traffic, a third of a padded batch's time.
-        constexpr int kPerRow = HD / 8;
-        __half* base = static_cast<__half*>(p.out) + row0 * ((int64_t)p.qHeads * HD) + (int64_t)h * HD;
-        for (int i = tid; i < BM * kPerRow; i += 256) {
-          const int r = i / kPerRow, c = i - r * kPerRow;
-          if (row0 + r < p.qLen)
-            reinterpret_cast<uint4*>(base + (int64_t)r * p.qHeads * HD)[c] = make_uint4(0u, 0u, 0u, 0u);
-        }
+      // No row of this unit sees a key (in a padded batch: every unit past a sequence's end):
+      // 16-byte stores, consecutive threads on consecutive pieces of a row.
+      constexpr int kPerRow = HD / 8;
+      __half* base = static_cast<__half*>(p.out) + row0 * ((int64_t)p.qHeads * HD) + (int64_t)h * HD;
+      for (int i = tid; i < BM * kPerRow; i += 256) {
+        const int r = i / kPerRow, c = i - r * kPerRow;
+        if (row0 + r < p.qLen)
+          reinterpret_cast<uint4*>(base + (int64_t)r * p.qHeads * HD)[c] = make_uint4(0u, 0u, 0u, 0u);
       }
     }
   }
@@ -820,7 +939,7 @@ prefill_tc3_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
 template <int HD, bool PADDED, bool PAIR>
 cudaError_t launch3(const AttnParams& p, int* status, cudaStream_t s, std::string* err) {
   using C = Cfg3<HD, PAIR>;
-  CUtensorMap mq, mk, mv;
+  CUtensorMap mq, mk, mv, mo;
   // The narrow-head form reads Q with plain loads; its K/V maps span the real columns,
   // so a box that runs past the last head reads zeros there.
   const int64_t qCols = (int64_t)p.qHeads * p.hd, kvCols = (int64_t)p.kvHeads * p.hd;
@@ -828,7 +947,8 @@ cudaError_t launch3(const AttnParams& p, int* status, cudaStream_t s, std::strin
       !make_map(&mk, p.k, p.kvLen, kvCols, p.kvStride, C::K_ROWS, err) ||
       !make_map(&mv, p.v, p.kvLen, kvCols, p.kvStride, C::V_ROWS, err))
     return cudaErrorInvalidValue;
-  if (PADDED) mq = mk;  // unused by the kernel; a valid map all the same
+  if (PADDED) mq = mo = mk;  // unused by the kernel; valid maps all the same
+  else if (!make_map(&mo, p.out, p.qLen, qCols, qCols, BM, err)) return cudaErrorInvalidValue;
   auto kern = prefill_tc3_kernel<HD, PADDED, PAIR>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
   if (e != cudaSuccess) return e;
@@ -845,7 +965,7 @@ cudaError_t launch3(const AttnParams& p, int* status, cudaStream_t s, std::strin
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = PAIR ? 1 : 0;
-  e = cudaLaunchKernelEx(&cfg, kern, mq, mk, mv, p, status);
+  e = cudaLaunchKernelEx(&cfg, kern, mq, mk, mv, mo, p, status);
   return e != cudaSuccess ? e : cudaGetLastError();
 }
 

@@ -34,22 +34,16 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// One poll of a barrier phase.  The time hint lets the hardware park the thread until the
-// phase completes or the time is up, instead of returning to a spinning loop at once:
-// waiting warps then leave the issue slots to the working ones (measured: +2 % on the
-// large causal prefill).
-#ifndef RT_MBAR_SUSPEND_NS
-#define RT_MBAR_SUSPEND_NS 20000
-#endif
-constexpr uint32_t kSuspendNs = RT_MBAR_SUSPEND_NS;
+// One look at a barrier phase that may suspend the thread for a moment (measured on a phase
+// that does not complete: 1.3 us).
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
-      : "r"(bar), "r"(parity), "r"(kSuspendNs)
+      : "r"(bar), "r"(parity)
       : "memory");
   return ok != 0;
 }
@@ -67,19 +61,27 @@ __device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Polls up to kWaitLimit times.  Each poll may suspend for up to kSuspendNs, so a wait
-// that never completes ends after at most about five seconds (and after some
-// milliseconds if the hardware returns from every poll at once).  `abortFlag` is a
-// CTA-shared word: once any thread has given up, the others stop waiting too.
-constexpr uint32_t kWaitLimit = 1u << 18;
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abortFlag) {
+// Polls up to kWaitLimit times, so a wait that never completes ends after about a second and
+// a half.  `abortFlag` is a CTA-shared word: once a thread that has given up has set it, the
+// others stop waiting too.  The caller sets it: with the store (or a sleep) in this function
+// the compiler's code for it made a wait whose phase is already complete cost 184 cycles on
+// an idle SM, without them 64, and the pipelines pass three to five such waits per tile.
+// (A time hint, which parks the thread for longer, costs 30 of these cycles.)
+constexpr uint32_t kWaitLimit = 1u << 20;
+__device__ __forceinline__ bool mbar_poll(uint32_t bar, uint32_t parity, volatile int* abortFlag) {
   for (uint32_t i = 0; i < kWaitLimit; i++) {
     if (mbar_try_wait(bar, parity)) return true;
-    if ((i & 31u) == 31u) {
-      if (*abortFlag) return false;
-      __nanosleep(32);
-    }
+    if ((i & 31u) == 31u && *abortFlag) return false;
   }
+  return false;
+}
+// The same for a converged warp, whose lanes agree on the outcome.
+__device__ __forceinline__ bool mbar_poll_warp(uint32_t bar, uint32_t parity, volatile int* abortFlag) {
+  return __all_sync(0xffffffffu, mbar_poll(bar, parity, abortFlag));
+}
+// The same with the flag set here, for code outside the pipelines' loops.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abortFlag) {
+  if (mbar_poll(bar, parity, abortFlag)) return true;
   *abortFlag = 1;
   return false;
 }
@@ -111,6 +113,23 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
       "{%2, %3, %4}], [%5];" ::"r"(dst),
       "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar)
       : "memory");
+}
+// Tiled TMA store (rows and columns outside the map are left out) and its groups.
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t src, int x, int y) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(map),
+               "r"(src), "r"(x), "r"(y)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_commit() {
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+template <int N>
+__device__ __forceinline__ void bulk_wait_read() {
+  asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
+}
+template <int N>
+__device__ __forceinline__ void bulk_wait() {
+  asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory");
 }
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");

@@ -141,6 +141,60 @@ def test_scores_that_shrink_then_jump(alt):
     oracle.assert_close(out, want, "f16")
 
 
+@pytest.mark.parametrize("hd", [40, 128, 256])
+@pytest.mark.parametrize("key", [3 * 128 + 7, 3 * 128 + 120, 4 * 128 + 7, 4 * 128 + 120, 899])
+def test_a_jump_in_either_half_of_either_warpgroups_tile(alt, hd, key):
+    """One key that towers over all others for some rows, after the exponentials of its tile's
+    first half have begun against the old reference point; one row in a warp, and every row."""
+    import runntime_b200 as rt
+    T = 900
+    rng = np.random.default_rng(key)
+    q = oracle.round_f16((rng.standard_normal((T, hd)) * 0.2).astype(np.float32))
+    q[512:640] = oracle.round_f16(np.abs(q[512:640]) + 0.25)
+    k = oracle.round_f16((rng.standard_normal((T, hd)) * 0.2).astype(np.float32))
+    k[key] = oracle.round_f16(q[300] * (600.0 / hd) + 60.0 / hd)
+    v = oracle.round_f16(rng.standard_normal((T, hd)).astype(np.float32))
+    opts = dict(qHeads=1, kvHeads=1, headDim=hd, windowLeft=INF, windowRight=INF)
+    out = rt.toArray(rt.sdpa(alt.upload(q, [T, hd], "f16"), alt.upload(k, [T, hd], "f16"),
+                             alt.upload(v, [T, hd], "f16"), opts), alt)
+    assert alt.dispatches[-1] == "prefill_tc3"
+    want = oracle.sdpa_ref(q, k, v, qHeads=1, kvHeads=1, headDim=hd)
+    oracle.assert_close(out, want, "f16")
+
+
+@pytest.mark.parametrize("hd", [4, 36, 52, 60])
+@pytest.mark.parametrize("qOff,outOff", [(0, 2), (2, 0), (2, 2), (4, 4)])
+def test_narrow_heads_at_addresses_of_four_and_eight_bytes(alt, hd, qOff, outOff):
+    """Q is read and the output written in quads where the address allows, in pairs elsewhere;
+    rows past the end and between sequences; nothing beside the output is touched."""
+    import torch
+    from runntime_b200.engine import prefill_batched
+    heads, S, lens = 8, 200, [200, 1, 77]
+    dev = torch.device("cuda", 0)
+    g = torch.Generator(device=dev).manual_seed(hd)
+    n, w = len(lens) * S, heads * hd
+    k, v = (torch.randn(n, w, generator=g, device=dev).half() for _ in range(2))
+    q = (torch.randn(n * w + 8, generator=g, device=dev) * hd ** -0.5).half()[qOff:qOff + n * w].view(n, w)
+    room = torch.full((n * w + 8,), 7.0, device=dev, dtype=torch.float16)
+    out = room[outOff:outOff + n * w].view(n, w)
+    alt.setStream(torch.cuda.current_stream().cuda_stream)
+    try:
+        prefill_batched(alt, q, k, v, out, dtype="f16", batch=len(lens), seqStride=S,
+                        seqLens=torch.tensor(lens, dtype=torch.int32, device=dev), qHeads=heads,
+                        kvHeads=heads, headDim=hd, windowLeft=None, windowRight=0)
+        alt.sync()
+    finally:
+        alt.setStream(None)
+    got = out.float().cpu().numpy()
+    for b, length in enumerate(lens):
+        part = slice(b * S, b * S + length)
+        want = oracle.sdpa_ref(*(t[part].float().cpu().numpy() for t in (q, k, v)), qHeads=heads,
+                               kvHeads=heads, headDim=hd, windowRight=0)
+        oracle.assert_close(got[part].reshape(want.shape), want, "f16")
+        assert (got[b * S + length:(b + 1) * S] == 0).all()
+    assert (room[:outOff] == 7).all() and (room[outOff + n * w:] == 7).all()
+
+
 def test_matches_the_other_kernels(alt):
     from runntime_b200._lib import OPT_PREFILL_TC
     c = _c(qLen=900, kvLen=900, qHeads=4, kvHeads=2, headDim=128, windowLeft=400, windowRight=0,
