@@ -121,6 +121,15 @@ SYMBOLS = {
                                C.c_int64, C.c_int64, C.c_int32]),
 }
 
+# What csrc/host.cpp calls, in the order of its table.
+HOST_CALLS = ("rt_matmul", "rt_rope", "rt_slice", "rt_attn", "rt_attn_route", "rt_attn_decode",
+              "rt_argmax_dot", "rt_kv_append", "rt_softmax", "rt_local_attention")
+
+try:
+    from . import _host as host   # constructors and eval loop in native code
+except ImportError:               # not built: the Python they stand for runs
+    host = None
+
 _lib = None
 
 
@@ -137,6 +146,8 @@ def load():
         for name, (res, args) in SYMBOLS.items():
             fn = getattr(lib, name)
             fn.restype, fn.argtypes = res, args
+        if host is not None:
+            host.bind_library(lib, tuple(C.cast(getattr(lib, n), C.c_void_p).value for n in HOST_CALLS))
         _lib = lib
     return _lib
 

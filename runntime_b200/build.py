@@ -1,4 +1,5 @@
-"""Builds librt_attn.so (the CUDA kernels and the C ABI) for sm_100a with nvcc.
+"""Builds librt_attn.so (the CUDA kernels and the C ABI) for sm_100a with nvcc, and _host.so
+(csrc/host.cpp) with the C++ compiler.
 
 nvcc cross-compiles without a GPU.  The library links the static CUDA runtime
 and resolves driver entry points at run time, so it loads (and its symbols can
@@ -10,11 +11,13 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "librt_attn.so")
+HOST = os.path.join(HERE, "_host.so")   # the constructors and the eval loop in native code (CPython extension)
 SOURCES = ["api.cu", "prefill_simt.cu", "prefill_rows.cu", "prefill_f32_tc.cu", "prefill_mma.cu", "prefill_tc.cu", "prefill_tc2.cu", "prefill_tc3.cu", "prefill_tc4.cu", "decode.cu", "exchange.cu", "misc.cu", "softmax.cu",
            "local_attn.cu", "local_attn_tc.cu", "matmul.cu",
            "matmul_tc.cu", "matmul_f32_tc.cu"]
@@ -33,6 +36,19 @@ def _nvcc() -> str:
     raise RuntimeError("nvcc not found; set NVCC")
 
 
+def build_host() -> str:
+    """Compile the CPython extension if it is missing or older than its sources.  Python runs in
+    its place where it is missing."""
+    src, header = os.path.join(CSRC, "host.cpp"), os.path.join(ROOT, "include", "rt_attn.h")
+    if os.path.exists(HOST) and os.path.getmtime(HOST) >= max(
+            os.path.getmtime(f) for f in (src, header, os.path.abspath(__file__))):
+        return HOST
+    subprocess.check_call(["/usr/bin/g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
+                           "-Wall", "-I", sysconfig.get_paths()["include"], "-I", os.path.join(ROOT, "include"),
+                           src, "-o", HOST])
+    return HOST
+
+
 def _stale() -> bool:
     if not os.path.exists(LIB):
         return True
@@ -47,6 +63,8 @@ def build(force: bool = False, verbose: bool = False, defines=(), target: str = 
     """Compile the library if it is missing or older than its sources.  ``defines``
     (extra -D macros) and ``target`` build a variant beside the product library, for
     kernel experiments."""
+    if target == LIB:
+        build_host()
     if not force and not defines and target == LIB and not _stale():
         return LIB
     objdir = (os.path.join(HERE, "build") if target == LIB else

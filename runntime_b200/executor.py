@@ -26,7 +26,7 @@ from typing import Dict, List, Optional, Sequence
 import numpy as np
 
 from . import _lib
-from ._lib import AttnArgs, DecodeArgs, DTYPE_CODE, WINDOW_INF, check
+from ._lib import AttnArgs, DecodeArgs, DTYPE_CODE, WINDOW_INF, check, host
 from .errors import RunntimeError
 from .value import DeviceBuffer, Value, ValueMeta, elemBytes, matrix, materialized
 
@@ -416,9 +416,21 @@ def _fused_extras(f: dict) -> dict:
     return ex
 
 
+def _plan_extras(k, v, q, vSlice) -> dict:
+    """The extras of a fused attn node from the nodes of its plan (None where it has none)."""
+    plan = {"k": k, "v": v}
+    if q is not None:
+        plan["rope"] = (q, k.pending.inputs[1])
+    if vSlice is not None:
+        plan["vSlice"] = vSlice
+    return {"fusedAppend": _fused_extras(plan)}
+
+
 def evalValues(targets: Sequence[Value], ex: CudaExecutor) -> None:
     """Dispatches every pending node the targets depend on, once, in dependency
     order; intermediates go back to the pool after their last consumer."""
+    if host is not None and host.evaluate(targets, ex, _plan_extras):
+        return   # (csrc/host.cpp: the loop below for a CudaExecutor, in native code)
     # Values are compared and hashed by identity, so they are the keys themselves.
     order = _collect_pending(targets)
     fuse = _fusable_appends(order, targets)
@@ -479,6 +491,10 @@ def _release(inputs, left, aliased, elided, ex, after=()) -> None:
                 # (views of a caller-owned buffer and values never materialized stay)
                 ex.releaseOutput(i.buffer, i.shape)
                 i.markReleased()
+
+
+if host is not None:
+    host.bind_executor(CudaExecutor, Value.markReleased.__defaults__[0], check)
 
 
 def toArray(value: Value, ex: CudaExecutor) -> np.ndarray:

@@ -10,12 +10,24 @@ import json
 import math
 from typing import Optional, Sequence
 
-from ._lib import WINDOW_INF
-from .value import Value, ValueMeta, pending
+from ._lib import WINDOW_INF, host
+from .value import DeviceBuffer, PendingOp, Value, ValueMeta, pending
 
 FLOAT_DTYPES = ("f32", "f16")
 MAX_HEAD_DIM = 512          # widest head with more than one query row
 MAX_DECODE_HEAD_DIM = 128   # widest head with one query row
+
+
+class _Deferring:
+    """Stands for csrc/host.cpp where it is not built: every constructor below runs its Python."""
+
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
+# The plain accepted cases of the constructors in native code.  Each answers with the node that
+# the Python below it would make, or with None for everything else: the Python decides.
+_native = host if host is not None else _Deferring()
 
 
 def _js(x) -> str:
@@ -74,6 +86,9 @@ def sdpa(q: Value, k: Value, v: Value, opts: dict) -> Value:
     ``[start, end)`` of keys; ``keyBias`` raises the scores of one key range by a constant;
     ``sinks`` gives every head an extra term in the softmax denominator.  Scores are used
     as they come: callers fold 1/sqrt(headDim) into q or k."""
+    node = _native.sdpa(q, k, v, opts)
+    if node is not None:
+        return node
     qHeads, kvHeads, headDim = opts["qHeads"], opts["kvHeads"], opts["headDim"]
     sinks: Optional[Value] = opts.get("sinks")
     segments: Optional[Value] = opts.get("segments")
@@ -146,6 +161,9 @@ def sdpaPacked(qkv: Value, opts: dict) -> Value:
     q, k and v are the three column blocks of ONE tensor ``qkv [T, (qHeads +
     2*kvHeads)*headDim]`` — the fused projection's output is attended to where it lies, no
     slicing.  More than one row, heads up to 128 wide, no key bias; otherwise ``sdpa``."""
+    node = _native.sdpaPacked(qkv, opts)
+    if node is not None:
+        return node
     qHeads, kvHeads, headDim = opts["qHeads"], opts["kvHeads"], opts["headDim"]
     sinks: Optional[Value] = opts.get("sinks")
     segments: Optional[Value] = opts.get("segments")
@@ -196,6 +214,9 @@ def rope(x: Value, cos: Value, sin: Value, opts: dict) -> Value:
     from f32 tables ``cos, sin [T, headDim]`` that hold each pair's value twice and may
     carry a scale.  ``srcStart``/``width`` pick a column window of a wider row — the q
     or the k part of a fused qkv projection — so that no slice is needed first."""
+    node = _native.rope(x, cos, sin, opts)
+    if node is not None:
+        return node
     headDim = opts["headDim"]
     t, xw, dtype = want2d("rope", x, FLOAT_DTYPES)
     srcStart = opts.get("srcStart")
@@ -222,11 +243,19 @@ def rope(x: Value, cos: Value, sin: Value, opts: dict) -> Value:
 ACT_CODE = {"none": 0, "tanh": 1, "gelu": 2, "silu": 3, "relu": 4, "geluTanh": 5, "elu": 6}
 
 
+if host is not None:
+    host.bind_ops(Value, ValueMeta, PendingOp, DeviceBuffer, ACT_CODE, WINDOW_INF, MAX_HEAD_DIM,
+                  MAX_DECODE_HEAD_DIM)
+
+
 def matmul(a: Value, b: Value, opts: Optional[dict] = None) -> Value:
     """2D matrix multiply, a [M,K] x b [K,N] to [M,N], with the fused bias,
     activation and addend epilogue: act(a·b + bias) + addend.  ``baseRow`` views K
     rows of a taller fused b.  Plain f32/f16 weights only (quantized weights are
     not built).  packages/runntime/src/core/graph/ops/matmul.ts:28-99."""
+    node = _native.matmul(a, b, opts)
+    if node is not None:
+        return node
     opts = opts or {}
     if any(opts.get(k) for k in ("scales", "bits", "groupSize")) or b.shape.dtype == "quantW":
         raise ValueError("matmul: quantW weights are not supported by this build")
@@ -266,6 +295,9 @@ def argmaxDot(w: Value, x: Value) -> Value:
     """Fused gemv and argmax for greedy decoding: w [V,N] · x [1,N] to the argmax
     row index, lowest on ties; always f32
     (packages/runntime/src/core/graph/ops/matmul.ts:316-333)."""
+    node = _native.argmaxDot(w, x)
+    if node is not None:
+        return node
     _, n, wDtype = want2d("argmaxDot.w", w, FLOAT_DTYPES)
     xr, xn, xDtype = want2d("argmaxDot.x", x, FLOAT_DTYPES)
     if xr != 1:
@@ -357,6 +389,9 @@ def slice(x: Value, dim, start, end) -> Value:  # noqa: A001 - the reference's n
     """Narrows a 2-D x to [start, end) along dim, like torch's narrow: how v is
     cut out of a fused qkv row and k | v out of the fused cross projection
     (packages/runntime/src/core/graph/ops/shape.ts:69-135)."""
+    node = _native.slice(x, dim, start, end)
+    if node is not None:
+        return node
     dims = x.shape.dims
     if dims is None or len(dims) != 2:
         got = "undefined" if dims is None else ",".join(str(d) for d in dims)
@@ -393,6 +428,9 @@ def writeRows(dst: Value, src: Value, startRow) -> Value:
     caller-owned buffer behind dst and returns a [startRow + r, cols] view of
     that same buffer.  Built for KV-cache appends: rows past the view keep
     whatever they held."""
+    node = _native.writeRows(dst, src, startRow)
+    if node is not None:
+        return node
     dstRows, dstCols, dtype = want2d("writeRows.dst", dst, FLOAT_DTYPES)
     srcRows, srcCols, srcDtype = want2d("writeRows.src", src, FLOAT_DTYPES)
     if srcDtype != dtype:
