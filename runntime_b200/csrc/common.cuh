@@ -109,6 +109,7 @@ struct DecodeParams {
   int32_t keySlots;     // keys processed concurrently by one CTA
   int32_t stages;       // smem ring depth (bulk path)
   int32_t mergeAfter;   // the splits are merged by a second launch
+  int32_t mma;          // f16 on the tensor cores (decode_mma_kernel)
   int32_t lanesPerRow;  // threads that share one (key, head) pair, each a slice of the head (1, 2, 4)
   // fused rope (null tables = off) and row strides of q / kNew / vNew, in elements
   const float* ropeCos;

@@ -11,6 +11,9 @@
 // arrive for the sequence merges them, without waiting, or, where they are more than
 // one CTA reads in a few microseconds, a second launch does (see plan_decode).
 //
+// f16 caches with several query heads per kv head, or many wide heads and few keys, are read by
+// eight warps on the tensor cores instead (decode_mma_kernel).
+//
 // The KV-cache append is fused: the new K/V row is stored to the cache by the
 // CTA of split 0 and attended to straight from its source.
 //
@@ -57,6 +60,7 @@ constexpr int kMaxStages = 8;
 // the whole SM.
 constexpr size_t kSmemBudget = 200 * 1024;
 constexpr size_t kSmemBudgetTwoPerSm = 108 * 1024;
+constexpr size_t kSmemBudgetMma = 220 * 1024;   // three stages of 16 keys, 8 heads of 128
 
 __host__ __device__ constexpr int q_stride(int hdp) { return ((hdp / 4) & 1) ? hdp : hdp + 4; }
 
@@ -585,7 +589,10 @@ decode_kernel(const DecodeParams p) {
     for (int it = 0; it < ntiles; it++) {
       const int s = it % stages;
       if (it >= stages) {
-        if (!mbar_wait(smem_u32(&sEmpty[s]), ((it / stages) - 1) & 1, &sAbort)) break;
+        if (!mbar_park(smem_u32(&sEmpty[s]), ((it / stages) - 1) & 1, &sAbort)) {
+          sAbort = 1;
+          break;
+        }
       }
       const int64_t k0 = s0 + (int64_t)it * KS;
       const int nk = (int)min((int64_t)KS, s1 - k0);
@@ -772,8 +779,8 @@ decode_kernel(const DecodeParams p) {
     if (stages >= 4) {
       for (; it + 1 < ntiles; it += 2) {
         const int sa = it % stages, sb = (it + 1) % stages;
-        if (!mbar_wait(smem_u32(&sFull[sa]), (it / stages) & 1, &sAbort) ||
-            !mbar_wait(smem_u32(&sFull[sb]), ((it + 1) / stages) & 1, &sAbort)) {
+        if (!mbar_park(smem_u32(&sFull[sa]), (it / stages) & 1, &sAbort) ||
+            !mbar_park(smem_u32(&sFull[sb]), ((it + 1) / stages) & 1, &sAbort)) {
           ok = false;
           break;
         }
@@ -809,7 +816,7 @@ decode_kernel(const DecodeParams p) {
     T* tK = reinterpret_cast<T*>(ring + (size_t)s * 2 * tileBytes);
     T* tV = reinterpret_cast<T*>(ring + (size_t)s * 2 * tileBytes + tileBytes);
     if (BULK) {
-      if (!mbar_wait(smem_u32(&sFull[s]), (it / stages) & 1, &sAbort)) { ok = false; break; }
+      if (!mbar_park(smem_u32(&sFull[s]), (it / stages) & 1, &sAbort)) { ok = false; break; }
       if (it == 0) DEC_TRACE(2);
     } else {
       named_barrier_sync(1, kConsumers);
@@ -831,6 +838,7 @@ decode_kernel(const DecodeParams p) {
     }
   }
 
+  if (!ok) sAbort = 1;
   DEC_TRACE(3);
   // This block has streamed its keys: once every block has, the next kernel's blocks may
   // take the freed slots (they wait for this grid to finish before they read anything).
@@ -952,6 +960,512 @@ decode_kernel(const DecodeParams p) {
   if (p.xWorld > 0) exchange_rows(p, b, hqReal, kvh0 * group, tid, epoch, gridDim.z);
 }
 
+// ---- f16 on the tensor cores -------------------------------------------------------------
+// A warp takes one kv head and 16 or 32 keys of the tile at a time: S = q K^T with the (up to
+// eight) query heads of the kv head as the rows of an m16n8k16 and the keys as its columns, then
+// O = P V with S's fragments as the A operand.  P is held in two halves, p = hi + lo, as rows g and
+// g + 8 of that operand (22 bits; scaled by 2^12 so that small probabilities keep theirs), and
+// the accumulators are emptied into f32 sums every 32 columns and every 16 or 32 keys, so nothing
+// is rounded more than on the FP32 pipes.  The order of a contraction is free, so a thread's
+// operands are 8 or 16 contiguous bytes of a key's row: columns for the scores, key pairs (by
+// byte permutes) for the output.
+// What bounds the FP32-pipe form with several query heads per kv head is that every key is read
+// and converted once per query head, by two warps per scheduler: 16 sequences of 2000 keys, 32
+// heads of 128 on 8, took 103 us at 1.3 TB/s; here 36 (mma_better has more of both sides).
+template <int HD>
+struct Mma {
+  static constexpr int VEC = HD % 8 == 0 ? 8 : 4;               // halves per load
+  static constexpr int STEPS = (HD + 15) / 16;                  // of the scores' contraction
+  static constexpr int CHUNKS = (HD + 8 * VEC - 1) / (8 * VEC); // of 8 * VEC output columns
+  static constexpr int NB = HD <= 64 ? 2 : 1;                   // blocks of 16 keys at a time
+  static constexpr int KEYS = 16 * NB;
+};
+constexpr float kPScale = 4096.f, kPScaleLog2 = 12.f;
+
+__device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                          uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+      "{%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// VEC halves as 32-bit words, zeros where `there` is false.
+template <int VEC>
+__device__ __forceinline__ void load_words(const __half* p, bool there, uint32_t (&w)[VEC / 2]) {
+#pragma unroll
+  for (int i = 0; i < VEC / 2; i++) w[i] = 0u;
+  if (there) {
+    if constexpr (VEC == 8) {
+      const uint4 v = *reinterpret_cast<const uint4*>(p);
+      w[0] = v.x, w[1] = v.y, w[2] = v.z, w[3] = v.w;
+    } else {
+      const uint2 v = *reinterpret_cast<const uint2*>(p);
+      w[0] = v.x, w[1] = v.y;
+    }
+  }
+}
+
+// A thread's part of q: row g of the A operand, the columns its K loads will cover.
+template <int HD>
+__device__ __forceinline__ void mma_query(const __half* q, bool there, int t, uint32_t (&qa)[Mma<HD>::STEPS][2]) {
+  constexpr int VEC = Mma<HD>::VEC;
+#pragma unroll
+  for (int st = 0; st < Mma<HD>::STEPS; st++)
+#pragma unroll
+    for (int r = 0; r < 2; r++) {
+      const int col = VEC == 8 ? 32 * (st >> 1) + 8 * t + 4 * (st & 1) + 2 * r : 16 * st + 4 * t + 2 * r;
+      qa[st][r] = there && col < HD ? *reinterpret_cast<const uint32_t*>(q + col) : 0u;
+    }
+}
+
+// KEYS keys from k and v on, `pitch` elements apart, of which the first nk count.
+template <int HD>
+__device__ __forceinline__ void mma_keys(const __half* k, const __half* v, int pitch, int nk, int g, int t,
+                                         const uint32_t (&qa)[Mma<HD>::STEPS][2], float& m, float& l,
+                                         float (&o)[Mma<HD>::CHUNKS][Mma<HD>::VEC][2]) {
+  using C = Mma<HD>;
+  constexpr int VEC = C::VEC, NB = C::NB, PER = VEC / 4;   // steps per load
+  float sc[2 * NB][2];
+#pragma unroll
+  for (int i = 0; i < 2 * NB; i++) {
+    const __half* row = k + (8 * i + g) * pitch + VEC * t;
+    sc[i][0] = sc[i][1] = 0.f;
+#pragma unroll
+    for (int st = 0; st < C::STEPS; st += 2) {
+      float c[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int u = st; u < st + 2 && u < C::STEPS; u += PER) {
+        uint32_t w[VEC / 2];
+        load_words<VEC>(row + 16 * u, VEC == 8 || 16 * u + 4 * t < HD, w);
+#pragma unroll
+        for (int e = 0; e < PER; e++) mma_16816(c, qa[u + e][0], 0u, qa[u + e][1], 0u, w[2 * e], w[2 * e + 1]);
+      }
+      sc[i][0] += c[0];
+      sc[i][1] += c[1];
+    }
+  }
+  // this thread: head g, keys 8 i + 2 t and + 1
+  float mx = -INFINITY;
+#pragma unroll
+  for (int i = 0; i < 2 * NB; i++)
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+      sc[i][e] = 8 * i + 2 * t + e < nk ? sc[i][e] : -INFINITY;
+      mx = fmaxf(mx, sc[i][e]);
+    }
+  mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+  mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+  const float top = fmaxf(m, mx * kLog2e), alpha = fast_exp2(m - top), base = kPScaleLog2 - top;
+  m = top;
+  l *= alpha;
+  uint32_t hi[2 * NB], lo[2 * NB];
+#pragma unroll
+  for (int i = 0; i < 2 * NB; i++) {
+    const float p0 = fast_exp2(fmaf(sc[i][0], kLog2e, base)), p1 = fast_exp2(fmaf(sc[i][1], kLog2e, base));
+    l += p0 + p1;
+    const __half2 h = __floats2half2_rn(p0, p1);
+    const float2 f = __half22float2(h);
+    const __half2 r = __floats2half2_rn(p0 - f.x, p1 - f.y);
+    hi[i] = *reinterpret_cast<const uint32_t*>(&h);
+    lo[i] = *reinterpret_cast<const uint32_t*>(&r);
+  }
+#pragma unroll
+  for (int c = 0; c < C::CHUNKS; c++) {
+    const int col = c * 8 * VEC + VEC * g;
+    uint32_t w[NB][4][VEC / 2];
+#pragma unroll
+    for (int b = 0; b < NB; b++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const int key = 16 * b + 2 * t + (j & 1) + 8 * (j >> 1);
+        load_words<VEC>(v + key * pitch + col, key < nk && (HD % (8 * VEC) == 0 || col < HD), w[b][j]);
+      }
+#pragma unroll
+    for (int e = 0; e < VEC; e++) {
+      float d[4] = {0.f, 0.f, 0.f, 0.f};
+      const uint32_t sel = e & 1 ? 0x7632u : 0x5410u;
+#pragma unroll
+      for (int b = 0; b < NB; b++)
+        mma_16816(d, hi[2 * b], lo[2 * b], hi[2 * b + 1], lo[2 * b + 1],
+                  __byte_perm(w[b][0][e / 2], w[b][1][e / 2], sel), __byte_perm(w[b][2][e / 2], w[b][3][e / 2], sel));
+      o[c][e][0] = fmaf(o[c][e][0], alpha, d[0] + d[2]);
+      o[c][e][1] = fmaf(o[c][e][1], alpha, d[1] + d[3]);
+    }
+  }
+}
+
+// One head over the keys [k0, k0 + n) and, if `kn` is given, an appended row, key by key: what the
+// tensor cores cannot give where a value is infinite (hi * inf + lo * inf is NaN).  The warp's
+// lanes share the columns; the row goes to r = (l, columns), the maximum is returned.
+template <int HD>
+__device__ __noinline__ float exact_head(const __half* q, const __half* k, const __half* v, int64_t pitch, int64_t s0,
+                                         int64_t s1, int tile, int off, const __half* kn, const __half* vn, float m,
+                                         float l, float* r) {
+  constexpr int kCols = (HD + 31) / 32;
+  const int lane = threadIdx.x & 31;
+  float acc[kCols];
+#pragma unroll
+  for (int c = 0; c < kCols; c++) acc[c] = 0.f;
+  auto key = [&](const __half* kr, const __half* vr) {
+    float s = 0.f;
+    for (int x = lane; x < HD; x += 32) s = fmaf(__half2float(q[x]), __half2float(kr[x]), s);
+    s = warp_sum(s) * kLog2e;
+    if (s > m) {
+      const float c = fast_exp2(m - s);
+      l *= c;
+#pragma unroll
+      for (int i = 0; i < kCols; i++) acc[i] *= c;
+      m = s;
+    }
+    const float pe = fast_exp2(s - m);
+    l += pe;
+#pragma unroll
+    for (int i = 0; i < kCols; i++)
+      if (lane + 32 * i < HD) acc[i] = fmaf(pe, __half2float(vr[lane + 32 * i]), acc[i]);
+  };
+  for (int64_t at = s0 + off; at < s1; at += tile)   // this warp's keys of every tile
+    for (int64_t j = at; j < s1 && j < at + Mma<HD>::KEYS; j++) key(k + j * pitch, v + j * pitch);
+  if (kn) key(kn, vn);
+  if (lane == 0) r[0] = l;
+#pragma unroll
+  for (int i = 0; i < kCols; i++)
+    if (lane + 32 * i < HD) r[1 + lane + 32 * i] = acc[i];
+  __syncwarp();
+  return m;
+}
+
+// ---- f16 on the tensor cores: the kernel ---------------------------------------------------
+// The same streaming as decode_kernel — producer warp, ring of bulk copies, append by split 0, last
+// CTA or a second launch merges the splits — with eight consumer warps that each take a kv head
+// and KEYS keys of every tile (slots = 8 / kvPerCta warps share a head).  The appended row is
+// attended to from the cache row the block has just stored.
+template <int HD>
+__global__ void __launch_bounds__(kConsumers + 32, HD <= 64 ? 2 : 1) decode_mma_kernel(const DecodeParams p) {
+  using T = __half;
+  using M = Mma<HD>;
+  constexpr int MS = 1 + HD;   // a row of the block's merge: l, columns
+  extern __shared__ __align__(128) unsigned char smemRaw[];
+  __shared__ int sAbort, sAbortSeen, sIsLast;
+  __shared__ float sHeadTop[kConsumers], sHeadSum[kConsumers];
+  __shared__ __align__(8) uint64_t sFull[kMaxStages], sEmpty[kMaxStages];
+
+  const int tid = threadIdx.x;
+  DEC_TRACE(0);
+  asm volatile("griddepcontrol.wait;" ::: "memory");   // (launched as a programmatic dependent)
+  const int split = blockIdx.x, zb = blockIdx.z, by = blockIdx.y;
+  int b = by;
+  if (p.xWorld > 1) {   // the sequences this rank merges itself come last
+    b += p.xRot;
+    if (b >= p.batch) b -= p.batch;
+  }
+  const bool sec = p.hasSecond && by >= p.batch;   // the second attention's blocks
+  if (sec) b = by - p.batch;
+  const int group = p.qHeads / p.kvHeads, kvh0 = zb * p.kvPerCta, hq = p.kvPerCta * group;
+  const int KS = p.keySlots, sliceElems = p.kvPerCta * HD, rowElems = p.kvHeads * HD;
+  const int32_t* lens = sec ? p.s2.kvLens : p.kvLens;
+  const int64_t seqStride = sec ? p.s2.cacheSeqStride : p.cacheSeqStride;
+  const void* const* kPtrs = sec ? p.s2.kPtrs : p.kPtrs;
+  const void* const* vPtrs = sec ? p.s2.vPtrs : p.vPtrs;
+  const T* kBase = kPtrs ? static_cast<const T*>(kPtrs[b])
+                         : static_cast<const T*>(sec ? p.s2.kCache : p.kCache) + (int64_t)b * seqStride;
+  const T* vBase = vPtrs ? static_cast<const T*>(vPtrs[b])
+                         : static_cast<const T*>(sec ? p.s2.vCache : p.vCache) + (int64_t)b * seqStride;
+  const bool misaligned =
+      kPtrs && ((reinterpret_cast<uintptr_t>(kBase) | reinterpret_cast<uintptr_t>(vBase)) & 15u);
+  kBase += kvh0 * HD;
+  vBase += kvh0 * HD;
+  const T* qg = static_cast<const T*>(sec ? p.s2.q : p.q) + (int64_t)b * (sec ? p.s2.qRowStride : p.qRowStride) +
+                kvh0 * group * HD;
+  // (finished rows that the exchange between GPUs sends on are staged; see decode_kernel)
+  float* partialsOut = p.partialsOut;
+  uint32_t epoch = 0;
+  if (p.xWorld > 0) {
+    epoch = *reinterpret_cast<volatile uint32_t*>(p.xStep) + 1u;
+    partialsOut = p.xStage;
+  }
+
+  // L: visible rows of this cache; Lg: the sequence's length (see decode_kernel).
+  int64_t lo, end, L = 0, Lg = 0;
+  bool hasNew = p.kNew != nullptr && !sec;
+  if (p.useRange) {
+    lo = p.lo;
+    end = p.end;
+  } else {
+    Lg = L = lens ? lens[b] : sec ? p.s2.kvLen : p.kvLen;
+    if (p.kvSharded) {
+      const int64_t local = Lg - p.shardStart;
+      hasNew = hasNew && local >= 1 && local <= p.cacheRows;
+      L = local < 0 ? 0 : local > p.cacheRows ? p.cacheRows : local;
+    } else if (L > (sec ? p.s2.cacheRows : p.cacheRows) || misaligned) {
+      if (tid == 0) atomicOr(p.status, kStatusBadState);
+      Lg = L = 0;
+      hasNew = false;
+    }
+    end = L - 1;
+    lo = Lg - 1 - (sec ? p.s2.wl : p.wl) - p.shardStart;
+    if (lo < 0) lo = 0;
+    if (hasNew) end -= 1;  // row L-1 is the appended one
+    if (L <= 0) { lo = 1; end = -1; }
+  }
+  const int64_t n = end >= lo ? end - lo + 1 : 0;
+  int64_t chunk = (n + p.splits - 1) / p.splits;
+  chunk = (chunk + KS - 1) / KS * KS;
+  const int64_t s0 = lo + (int64_t)split * chunk, s1 = min(s0 + chunk, end + 1);
+  const int ntiles = s1 > s0 ? (int)((s1 - s0 + KS - 1) / KS) : 0;
+
+  // Shared memory: q, the ring (used again for the merge at the end).
+  T* sQ = reinterpret_cast<T*>(smemRaw);
+  unsigned char* ring = smemRaw + ((hq * HD * (int)sizeof(T) + 127) / 128) * 128;
+  const int tileBytes = ((KS * sliceElems * (int)sizeof(T) + 127) / 128) * 128, stages = p.stages;
+  if (tid == 0) {
+    sAbort = 0;
+    sIsLast = 0;
+    for (int s = 0; s < stages; s++) {
+      mbar_init(smem_u32(&sFull[s]), 1);
+      mbar_init(smem_u32(&sEmpty[s]), kConsumerWarps);
+    }
+    fence_barrier_init();
+  }
+  __syncthreads();
+
+  if (tid >= kConsumers) {
+    // ---------------- producer warp ----------------
+    const int lane = tid - kConsumers;
+    const uint32_t rowBytes = (uint32_t)sliceElems * sizeof(T);
+    for (int it = 0; it < ntiles; it++) {
+      const int s = it % stages;
+      if (it >= stages && !mbar_park(smem_u32(&sEmpty[s]), ((it / stages) - 1) & 1, &sAbort)) {
+        sAbort = 1;
+        break;
+      }
+      const int64_t k0 = s0 + (int64_t)it * KS;
+      const int nk = (int)min((int64_t)KS, s1 - k0);
+      const uint32_t bar = smem_u32(&sFull[s]);
+      const uint32_t dK = smem_u32(ring + (size_t)s * 2 * tileBytes), dV = dK + tileBytes;
+      if (lane == 0) mbar_expect_tx(bar, 2u * nk * rowBytes);
+      __syncwarp();
+      if (sliceElems == rowElems) {
+        if (lane == 0) {
+          bulk_g2s(dK, kBase + k0 * rowElems, nk * rowBytes, bar);
+          bulk_g2s(dV, vBase + k0 * rowElems, nk * rowBytes, bar);
+        }
+      } else {
+        for (int r = lane; r < nk; r += 32) {
+          bulk_g2s(dK + r * rowBytes, kBase + (k0 + r) * rowElems, rowBytes, bar);
+          bulk_g2s(dV + r * rowBytes, vBase + (k0 + r) * rowElems, rowBytes, bar);
+        }
+      }
+    }
+    return;
+  }
+
+  // ---------------- consumers ----------------
+  // q and, in split 0, the appended row: rotated and rounded to f16 as the separate rope dispatch
+  // stores them; the row goes to the cache.
+  const bool roped = p.ropeCos != nullptr && !p.useRange && !sec;
+  const bool appendHere = hasNew && split == 0 && !p.useRange && L >= 1;
+  const int64_t ropeRow = p.ropeByPos ? (Lg >= 1 ? Lg - 1 : 0) : b;
+  const float* rc = roped ? p.ropeCos + ropeRow * HD : nullptr;
+  const float* rs = roped ? p.ropeSin + ropeRow * HD : nullptr;
+  for (int idx = tid; idx < hq * (HD / 2); idx += kConsumers) {
+    T r0 = qg[2 * idx], r1 = qg[2 * idx + 1];
+    if (roped) {
+      const int x = idx % (HD / 2) * 2;
+      float f0, f1;
+      rope_pair(to_f32<T>(r0), to_f32<T>(r1), rc[x], rs[x], f0, f1);
+      r0 = from_f32<T>(f0), r1 = from_f32<T>(f1);
+    }
+    sQ[2 * idx] = r0;
+    sQ[2 * idx + 1] = r1;
+  }
+  if (appendHere) {
+    const T* kn = static_cast<const T*>(p.kNew) + (int64_t)b * p.kNewRowStride + kvh0 * HD;
+    const T* vn = static_cast<const T*>(p.vNew) + (int64_t)b * p.vNewRowStride + kvh0 * HD;
+    T* kc = const_cast<T*>(kBase) + (L - 1) * rowElems;
+    T* vc = const_cast<T*>(vBase) + (L - 1) * rowElems;
+    constexpr int kBatch = 4;   // loads ahead of any of their stores, which may alias them for the compiler
+    for (int i0 = tid; i0 < sliceElems / 2; i0 += kBatch * kConsumers) {
+      T k0[kBatch], k1[kBatch], v0[kBatch], v1[kBatch];
+      float c[kBatch], sn[kBatch];
+#pragma unroll
+      for (int i = 0; i < kBatch; i++) {
+        const int idx = i0 + i * kConsumers, x = idx % (HD / 2) * 2;
+        if (idx < sliceElems / 2) {
+          k0[i] = kn[2 * idx], k1[i] = kn[2 * idx + 1];
+          v0[i] = vn[2 * idx], v1[i] = vn[2 * idx + 1];
+          if (roped) c[i] = rc[x], sn[i] = rs[x];
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < kBatch; i++) {
+        const int at = 2 * (i0 + i * kConsumers);
+        if (at >= sliceElems) break;
+        if (roped) {
+          float r0, r1;
+          rope_pair(to_f32<T>(k0[i]), to_f32<T>(k1[i]), c[i], sn[i], r0, r1);
+          k0[i] = from_f32<T>(r0), k1[i] = from_f32<T>(r1);
+        }
+        kc[at] = k0[i], kc[at + 1] = k1[i];
+        vc[at] = v0[i], vc[at + 1] = v1[i];
+      }
+    }
+  }
+  named_barrier_sync(1, kConsumers);
+  DEC_TRACE(1);
+
+  const int lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int kvl = (tid >> 5) % p.kvPerCta, slot = (tid >> 5) / p.kvPerCta, slots = kConsumerWarps / p.kvPerCta;
+  const bool sink = slot == 0 && split == 0 && p.sinks, append = appendHere && slot == 0;
+  const int64_t newRow = (L - 1) * rowElems + kvl * HD;
+  uint32_t qa[M::STEPS][2];
+  mma_query<HD>(sQ + (kvl * group + g) * HD, g < group, t, qa);
+  float m = kNegSeed, l = 0.f, o[M::CHUNKS][M::VEC][2];
+#pragma unroll
+  for (int c = 0; c < M::CHUNKS; c++)
+#pragma unroll
+    for (int e = 0; e < M::VEC; e++) o[c][e][0] = o[c][e][1] = 0.f;
+  if (sink && g < group) {
+    m = p.sinks[(kvh0 + kvl) * group + g];   // log2-space: sink * ln2 * log2e
+    l = t == 0 ? kPScale : 0.f;              // (a head's sum is spread over the four threads of a row)
+  }
+  bool ok = true;
+  for (int it = 0; it < ntiles; it++) {
+    const int s = it % stages;
+    ok = __all_sync(0xffffffffu, mbar_park(smem_u32(&sFull[s]), (it / stages) & 1, &sAbort));
+    if (!ok) break;   // the whole warp leaves together
+    if (it == 0) DEC_TRACE(2);
+    const int first = slot * M::KEYS, nk = (int)min((int64_t)KS, s1 - (s0 + (int64_t)it * KS)) - first;
+    const T* tK = reinterpret_cast<const T*>(ring + (size_t)s * 2 * tileBytes) + first * sliceElems + kvl * HD;
+    if (nk > 0) mma_keys<HD>(tK, tK + tileBytes / (int)sizeof(T), sliceElems, nk, g, t, qa, m, l, o);
+    __syncwarp();
+    if (lane == 0) mbar_arrive(smem_u32(&sEmpty[s]));
+  }
+  if (!ok) sAbort = 1;
+  DEC_TRACE(3);
+  // (this block has streamed its keys: the next kernel's blocks may take the freed slots)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (append && ok) mma_keys<HD>(kBase + newRow, vBase + newRow, 0, 1, g, t, qa, m, l, o);
+
+  // Whether a wait ran out is decided once for the whole block.
+  named_barrier_sync(1, kConsumers);
+  if (tid == 0) sAbortSeen = sAbort;
+  named_barrier_sync(1, kConsumers);
+  if (sAbortSeen) {
+    if (tid == 0) {
+      atomicOr(p.status, kStatusWaitTimeout);
+      if (p.mergeAfter) p.counters[by * gridDim.z + zb] = 1;
+    }
+    for (int i = 0; i < 64; i++) __nanosleep(4000);
+    return;
+  }
+
+  // ---- merge the warps that share a head (log-sum-exp), as decode_kernel merges its slots ----
+  float* sTop = reinterpret_cast<float*>(ring);   // [slots][hq] maxima
+  float* sM = sTop + slots * hq;                  // [slots][hq][MS]
+  l += __shfl_xor_sync(0xffffffffu, l, 1);
+  l += __shfl_xor_sync(0xffffffffu, l, 2);
+  // An output that is not finite is computed again, key by key.
+  float probe = 0.f;
+#pragma unroll
+  for (int c = 0; c < M::CHUNKS; c++)
+#pragma unroll
+    for (int e = 0; e < M::VEC; e++)
+#pragma unroll
+      for (int x = 0; x < 2; x++)
+        if (c * 8 * M::VEC + M::VEC * (2 * t + x) + e < HD) probe = fmaf(o[c][e][x], 0.f, probe);
+  const bool redo = __any_sync(0xffffffffu, g < group && probe != 0.f);
+  if (redo) {
+    for (int hh = kvl * group; hh < (kvl + 1) * group; hh++) {
+      const int at = slot * hq + hh;
+      const float top = exact_head<HD>(sQ + hh * HD, kBase + kvl * HD, vBase + kvl * HD, rowElems, s0, s1, KS,
+                                       slot * M::KEYS, append ? kBase + newRow : nullptr, vBase + newRow,
+                                       sink ? p.sinks[kvh0 * group + hh] : kNegSeed, sink ? 1.f : 0.f, sM + at * MS);
+      if (lane == 0) sTop[at] = top;
+    }
+  } else if (g < group && t == 0) {
+    sTop[slot * hq + kvl * group + g] = m;
+  }
+  named_barrier_sync(1, kConsumers);
+  auto top_of = [&](int hh) {
+    float top = kNegSeed;
+    for (int s = 0; s < slots; s++) top = fmaxf(top, sTop[s * hq + hh]);
+    return top;
+  };
+  if (redo) {
+    for (int hh = kvl * group; hh < (kvl + 1) * group; hh++) {
+      const float top = top_of(hh), w = fast_exp2(sTop[slot * hq + hh] - top);
+      float* r = sM + (slot * hq + hh) * MS;
+      for (int x = lane; x < MS; x += 32) r[x] *= w;
+      if (slot == 0 && lane == 0) sHeadTop[hh] = top;
+    }
+  } else if (g < group) {
+    const int hh = kvl * group + g;
+    const float top = top_of(hh), w = fast_exp2(m - top) * (1.f / kPScale);
+    float* r = sM + (slot * hq + hh) * MS;
+    if (t == 0) r[0] = l * w;
+#pragma unroll
+    for (int c = 0; c < M::CHUNKS; c++)
+#pragma unroll
+      for (int e = 0; e < M::VEC; e++)
+#pragma unroll
+        for (int x = 0; x < 2; x++) {
+          const int col = c * 8 * M::VEC + M::VEC * (2 * t + x) + e;
+          if (col < HD) r[1 + col] = o[c][e][x] * w;
+        }
+    if (slot == 0 && t == 0) sHeadTop[hh] = top;
+  }
+  named_barrier_sync(1, kConsumers);
+
+  constexpr int stride = 2 + HD;  // partials row in global memory
+  const bool whole = p.splits == 1;
+  const int64_t head0 = (int64_t)b * p.qHeads + kvh0 * group;
+  float* rowF = !whole ? p.scratch + (((int64_t)by * p.splits + split) * p.qHeads + kvh0 * group) * stride
+                       : partialsOut ? partialsOut + head0 * stride : nullptr;
+  T* rowT = static_cast<T*>(sec ? p.s2.out : p.out) + head0 * HD;
+  for (int hh = tid; hh < hq; hh += kConsumers) {
+    const float top = sHeadTop[hh];
+    float sum = 0.f;
+    for (int s = 0; s < slots; s++) sum += sM[(s * hq + hh) * MS];
+    sHeadSum[hh] = sum;
+    if (rowF) {
+      // finished rows carry the maximum in natural-log units, split rows in log2 units
+      rowF[hh * stride] = !whole ? top : sum > 0.f ? top * 0.6931471805599453f : kNegSeed;
+      rowF[hh * stride + 1] = sum;
+    }
+  }
+  named_barrier_sync(1, kConsumers);
+  for (int i = tid; i < hq * HD; i += kConsumers) {
+    const int hh = i / HD, x = i - hh * HD;
+    const float* r = sM + hh * MS + 1 + x;
+    float v = 0.f;
+    for (int s = 0; s < slots; s++) v += r[s * hq * MS];
+    if (rowF) {
+      rowF[hh * stride + 2 + x] = v;
+    } else {
+      const float sum = sHeadSum[hh];
+      rowT[i] = from_f32<T>(v * (sum > 0.f ? 1.f / sum : 0.f));
+    }
+  }
+  DEC_TRACE(4);
+  if (whole) {
+    if (p.xWorld > 0) exchange_rows(p, b, hq, kvh0 * group, tid, epoch, gridDim.z);
+    return;
+  }
+  if (p.mergeAfter) return;   // a launch of its own merges the splits
+  __threadfence();
+  named_barrier_sync(1, kConsumers);
+  if (tid == 0) sIsLast = atomicAdd(&p.counters[by * gridDim.z + zb], 1u) == (unsigned)p.splits - 1;
+  named_barrier_sync(1, kConsumers);
+  if (!sIsLast) return;
+  __threadfence();
+  merge_splits<T>(HD, p.splits, p.qHeads, p.scratch + ((int64_t)by * p.splits * p.qHeads + kvh0 * group) * stride,
+                  rowT, partialsOut ? partialsOut + head0 * stride : nullptr, hq, sM, slots * hq * MS);
+  if (tid == 0) p.counters[by * gridDim.z + zb] = 0;  // ready for the next launch
+  if (p.xWorld > 0) exchange_rows(p, b, hq, kvh0 * group, tid, epoch, gridDim.z);
+}
+
 // The merge of the splits as a launch of its own, one block per (sequence, query head):
 // what the last block of a sequence does when there is little of it.
 constexpr int kMergeThreads = 128;
@@ -1010,12 +1524,15 @@ size_t smem_bytes(const DecodeParams& p, int esize, int hdp, bool bulk) {
   const int group = p.qHeads / p.kvHeads;
   const int hqMax = p.kvPerCta * group;
   const bool staged = p.lanesPerRow <= 1;   // see the kernel's carve-up
-  const size_t qBytes = staged ? (((size_t)hqMax * q_stride(hdp) * 4 + 127) / 128) * 128 : 0;
+  const size_t qBytes = p.mma   ? (((size_t)hqMax * p.hd * esize + 127) / 128) * 128
+                        : staged ? (((size_t)hqMax * q_stride(hdp) * 4 + 127) / 128) * 128
+                                 : 0;
   const size_t tileBytes = (((size_t)p.keySlots * p.kvPerCta * p.hd * esize + 127) / 128) * 128;
   const size_t ringBytes = (size_t)(bulk ? p.stages : 1) * 2 * tileBytes;
   const int lanes = p.lanesPerRow > 1 ? p.lanesPerRow : 1;
-  const size_t mergeBytes = (size_t)p.keySlots * hqMax * lanes * (2 + hdp / lanes) * 4;
-  const size_t newBytes = (staged && p.kNew) ? 2 * ((((size_t)p.kvPerCta * p.hd * esize) + 127) / 128) * 128 : 0;
+  const int slots = p.mma ? kConsumerWarps / p.kvPerCta : p.keySlots;
+  const size_t mergeBytes = (size_t)slots * hqMax * lanes * (2 + hdp / lanes) * 4;
+  const size_t newBytes = (staged && p.kNew && !p.mma) ? 2 * ((((size_t)p.kvPerCta * p.hd * esize) + 127) / 128) * 128 : 0;
   return qBytes + newBytes + (ringBytes > mergeBytes ? ringBytes : mergeBytes);
 }
 
@@ -1040,16 +1557,14 @@ bool bulk_ok(const DecodeParams& p, int esize) {
   return true;
 }
 
-template <typename T, int HDP, bool EXACT, int VEC, bool BULK, int R = 1>
-cudaError_t launch_one(const DecodeParams& p, size_t smem, cudaStream_t s) {
-  auto kern = decode_kernel<T, HDP, EXACT, VEC, BULK, R>;
+cudaError_t launch_kernel(void (*kern)(DecodeParams), bool bulk, const DecodeParams& p, size_t smem, cudaStream_t s) {
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   const int zBlocks = (p.kvHeads + p.kvPerCta - 1) / p.kvPerCta;
   dim3 grid(p.splits, p.batch * (p.hasSecond ? 2 : 1), zBlocks);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
-  cfg.blockDim = dim3(BULK ? kConsumers + 32 : kConsumers);
+  cfg.blockDim = dim3(bulk ? kConsumers + 32 : kConsumers);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
@@ -1060,12 +1575,25 @@ cudaError_t launch_one(const DecodeParams& p, size_t smem, cudaStream_t s) {
   return cudaLaunchKernelEx(&cfg, kern, p);
 }
 
+template <typename T, int HDP, bool EXACT, int VEC, bool BULK, int R = 1>
+cudaError_t launch_one(const DecodeParams& p, size_t smem, cudaStream_t s) {
+  return launch_kernel(decode_kernel<T, HDP, EXACT, VEC, BULK, R>, BULK, p, smem, s);
+}
+
 template <typename T>
 cudaError_t launch_typed(const DecodeParams& p, cudaStream_t s) {
   constexpr int esize = sizeof(T);
   constexpr int V = sizeof(T) == 2 ? 8 : 4;   // widest vector for the exact paths
   if (bulk_ok(p, esize)) {
     const size_t smem = smem_bytes(p, esize, p.hd, true);
+    if (p.mma) {
+      switch (p.hd) {
+        case 36: return launch_kernel(decode_mma_kernel<36>, true, p, smem, s);
+        case 52: return launch_kernel(decode_mma_kernel<52>, true, p, smem, s);
+        case 64: return launch_kernel(decode_mma_kernel<64>, true, p, smem, s);
+        case 128: return launch_kernel(decode_mma_kernel<128>, true, p, smem, s);
+      }
+    }
     switch (p.hd) {
       case 36: return launch_one<T, 36, true, 4, true>(p, smem, s);
       case 52: return launch_one<T, 52, true, 4, true>(p, smem, s);
@@ -1077,12 +1605,27 @@ cudaError_t launch_typed(const DecodeParams& p, cudaStream_t s) {
                                   : launch_one<T, 128, true, V, true>(p, smem, s);
     }
   }
-  if (p.lanesPerRow > 1) return cudaErrorInvalidValue;   // the plan promised the bulk path
+  if (p.lanesPerRow > 1 || p.mma) return cudaErrorInvalidValue;   // the plan promised the bulk path
   const int hdp = padded_hd(p.hd);
   const size_t smem = smem_bytes(p, esize, hdp, false);
   if (hdp == 32) return launch_one<T, 32, false, 1, false>(p, smem, s);
   if (hdp == 64) return launch_one<T, 64, false, 1, false>(p, smem, s);
   return launch_one<T, 128, false, 1, false>(p, smem, s);
+}
+
+// Which f16 calls go to the tensor cores.  With several query heads on a kv head the FP32 pipes
+// read and convert every key once per query head and are what bounds the step; measured (B200, us):
+// 16 sequences of up to 1000 keys, 16 heads of 128 on 8: 28.2 / 23.0; 64 x 1000, 8 of 128 on 1: 48.1 / 18.3;
+// 64 x 2000, 8 of 52 on 2: 32.6 / 19.1; 64 x 1000, 32 of 64 on 8: 56.8 / 38.0; at worst 38.2 / 38.8.
+// With one query head each it is a wash, but for many wide heads and short caches, where a block
+// of the other kernel holds all heads of two keys at a time (32 heads of 128: 60 x 100 keys 38.9 / 29.2,
+// 32 x 300 40.9 / 36.1, 118 MB); long ones stream better in its whole rows (6 x 2600, 192 MB: 53.1 / 53.8,
+// 16 x 1024, 201 MB: 53.2 / 59.6).
+bool mma_better(const DecodeParams& p, int group) {
+  if (group > 8 || (p.kvHeads % 8 && p.kvHeads != 4 && p.kvHeads != 2 && p.kvHeads != 1)) return false;
+  if (group > 1) return true;
+  const int64_t keys = p.useRange ? p.end - p.lo + 1 : p.kvLen;
+  return p.hd == 128 && p.kvHeads > 8 && p.batch * keys * p.kvHeads * p.hd * 4 <= (160ll << 20);
 }
 
 }  // namespace
@@ -1149,7 +1692,36 @@ bool plan_decode(DecodeParams& p, int dtype, int smCount, std::string* err) {
   // 270 / 286 / 234 / 248 us with two; the same crossing at 8 heads and at head size 64.
   Geom g{};
   int ctasPerSm = 1;
-  for (;; lanes = 1) {
+  // f16 on the tensor cores: eight warps deal with eight kv heads, or with fewer of them and more
+  // keys.
+  auto mma_geometry = [&](size_t budget) {
+    Geom of{};
+    of.kvPerCta = p.kvHeads % 8 == 0 ? 8 : p.kvHeads;
+    const int slots = kConsumerWarps / of.kvPerCta;
+    of.keySlots = (p.hd <= 64 ? 32 : 16) * slots;
+    of.tile = 2ull * of.kvPerCta * p.hd * esize * of.keySlots + 256;
+    const size_t qBytes = (size_t)of.kvPerCta * group * p.hd * esize + 128;
+    const size_t rest = budget > qBytes ? budget - qBytes : 0;
+    of.stages = (int)(rest / of.tile);
+    if (of.stages > kMaxStages) of.stages = kMaxStages;
+    of.fits = of.stages >= 3 && (size_t)slots * of.kvPerCta * group * (2 + p.hd) * 4 <= rest;
+    return of;
+  };
+  p.mma = 0;
+  if (dtype == RT_F16 && exact_hd(p.hd) && mma_better(p, group)) {
+    g = mma_geometry(kSmemBudgetMma);
+    p.kvPerCta = g.kvPerCta;
+    if (g.fits && bulk_ok(p, esize)) {
+      p.mma = 1;
+      p.lanesPerRow = 1;
+      const Geom two = mma_geometry(kSmemBudgetTwoPerSm);
+      if (p.hd <= 64 && two.fits && (int64_t)p.batch * (p.kvHeads / g.kvPerCta) * (p.hasSecond ? 2 : 1) > smCount) {
+        g = two;
+        ctasPerSm = 2;
+      }
+    }
+  }
+  for (; !p.mma; lanes = 1) {
     const bool twoFit = hdp / lanes <= 64;
     const Geom one = geometry(kSmemBudget, lanes);
     g = one;

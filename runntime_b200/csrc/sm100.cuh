@@ -65,8 +65,7 @@ __device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
 // a half.  `abortFlag` is a CTA-shared word: once a thread that has given up has set it, the
 // others stop waiting too.  The caller sets it: with the store (or a sleep) in this function
 // the compiler's code for it made a wait whose phase is already complete cost 184 cycles on
-// an idle SM, without them 64, and the pipelines pass three to five such waits per tile.
-// (A time hint, which parks the thread for longer, costs 30 of these cycles.)
+// an idle SM, without them 64, and the prefill pipelines pass three to five such waits per tile.
 constexpr uint32_t kWaitLimit = 1u << 20;
 __device__ __forceinline__ bool mbar_poll(uint32_t bar, uint32_t parity, volatile int* abortFlag) {
   for (uint32_t i = 0; i < kWaitLimit; i++) {
@@ -79,9 +78,31 @@ __device__ __forceinline__ bool mbar_poll(uint32_t bar, uint32_t parity, volatil
 __device__ __forceinline__ bool mbar_poll_warp(uint32_t bar, uint32_t parity, volatile int* abortFlag) {
   return __all_sync(0xffffffffu, mbar_poll(bar, parity, abortFlag));
 }
+
+// The same for waits that are long as a rule: a time hint parks the thread (for 4 us at most,
+// measured) instead of returning it to the loop, which costs 30 cycles where the phase is
+// complete and leaves the issue slots to the working warps where it is not.  A decode block's
+// waits are of this kind: eight sequences of 448 keys, 8 heads of 52, 12.0 us with the hint,
+// 13.4 without; 16 of 600 keys 11.8 and 13.0.
+constexpr uint32_t kSuspendNs = 20000;
+__device__ __forceinline__ bool mbar_park(uint32_t bar, uint32_t parity, volatile int* abortFlag) {
+  for (uint32_t i = 0; i < kWaitLimit / 4; i++) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity), "r"(kSuspendNs)
+        : "memory");
+    if (ok) return true;
+    if ((i & 31u) == 31u && *abortFlag) return false;
+  }
+  return false;
+}
 // The same with the flag set here, for code outside the pipelines' loops.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abortFlag) {
-  if (mbar_poll(bar, parity, abortFlag)) return true;
+  if (mbar_park(bar, parity, abortFlag)) return true;
   *abortFlag = 1;
   return false;
 }
