@@ -431,6 +431,26 @@ RT_API int rt_slice(rt_ctx* ctx, const void* x, void* out, int64_t rows, int64_t
                     int64_t rowStart, int64_t rowEnd, int64_t colStart, int64_t colEnd,
                     int32_t dtype);
 
+/* ---- several column windows at once ---------------------------------------------
+ * Each window is what rt_rope (with tables) or rt_slice over columns (cosT and sinT
+ * NULL; headDim unused) makes of columns [start, start+width) of x [rows, cols], all
+ * in one launch where their alignment allows 8-byte accesses: q and k rotated and v
+ * cut out of a fused qkv projection.  The outputs must not overlap each other or
+ * any input. */
+#define RT_MAX_WINDOWS 4
+typedef struct {
+  const void* x;
+  const float* cosT;
+  const float* sinT;
+  void* out;              /* [rows, width] */
+  int64_t rows;
+  int64_t cols;
+  int64_t start;
+  int64_t width;
+  int32_t headDim;
+} rt_window;
+RT_API int rt_windows(rt_ctx* ctx, const rt_window* windows, int32_t count, int32_t dtype);
+
 /* ---- writeRows: the KV-cache append as its own op ----------------------------
  * dst rows [startRow, startRow+rows) = src (packages/runntime/src/core/graph/
  * ops/shape.ts:236-259; kernel packages/runntime/src/core/kernels/shape/

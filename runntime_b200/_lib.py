@@ -76,6 +76,15 @@ class DecodeArgs(C.Structure):
     ]
 
 
+class Window(C.Structure):
+    """rt_window: a column window, rotated or cut out."""
+    _fields_ = [
+        ("x", C.c_void_p), ("cosT", C.c_void_p), ("sinT", C.c_void_p), ("out", C.c_void_p),
+        ("rows", C.c_int64), ("cols", C.c_int64), ("start", C.c_int64), ("width", C.c_int64),
+        ("headDim", C.c_int32),
+    ]
+
+
 # name -> (restype, argtypes); every symbol include/rt_attn.h declares.
 SYMBOLS = {
     "rt_ctx_create": (C.c_int, [C.c_int, C.POINTER(C.c_void_p)]),
@@ -117,13 +126,14 @@ SYMBOLS = {
                              C.c_int32, C.c_int32, C.c_int32]),
     "rt_slice": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int64,
                            C.c_int64, C.c_int64, C.c_int64, C.c_int32]),
+    "rt_windows": (C.c_int, [C.c_void_p, C.POINTER(Window), C.c_int32, C.c_int32]),
     "rt_kv_append": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64,
                                C.c_int64, C.c_int64, C.c_int32]),
 }
 
 # What csrc/host.cpp calls, in the order of its table.
 HOST_CALLS = ("rt_matmul", "rt_rope", "rt_slice", "rt_attn", "rt_attn_route", "rt_attn_decode",
-              "rt_argmax_dot", "rt_kv_append", "rt_softmax", "rt_local_attention")
+              "rt_argmax_dot", "rt_kv_append", "rt_softmax", "rt_local_attention", "rt_windows")
 
 try:
     from . import _host as host   # constructors and eval loop in native code

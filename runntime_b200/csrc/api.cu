@@ -1,5 +1,6 @@
 // The C ABI: context, buffers, argument validation and kernel routing.
 // Declarations and the reference interfaces they replace are in rt_attn.h.
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <mutex>
@@ -24,8 +25,9 @@ struct rt_ctx {
     size_t clear;   // bytes to clear after a wait that ran out: all of counters, none of scratch
   };
   std::vector<Outgrown> outgrown;   // smaller scratch and counters of before
-  int* statusDev;
-  int* statusHost;   // pinned: the status word comes back on the stream, without a second wait
+  int* status;       // pinned host memory that kernels write to when something goes wrong: a wait for the
+                     // stream is all it takes to read it (a copy of it cost every read-back 3 us)
+  int* work;         // device: the persistent prefill kernel's queue (units drawn, CTAs finished)
   int64_t launches;
   int useTc;
   int waitPolls;   // polls of the cross-GPU merge's wait before it gives up
@@ -35,9 +37,7 @@ struct rt_ctx {
 namespace {
 
 constexpr uint32_t kLive = 0x52544358u;  // 'RTCX'
-// statusDev: the status word, then the two words of the persistent prefill kernel's work
-// queue (units drawn, CTAs finished), zero between launches.
-constexpr int kStatusWords = 3;
+constexpr int kWorkWords = 2;   // zero between launches
 constexpr uint32_t kDead = 0x44454144u;  // 'DEAD'
 
 thread_local std::string tlsError;
@@ -261,7 +261,7 @@ int run_decode(rt_ctx* ctx, rt::DecodeParams& p, int dtype) {
   }
   p.scratch = ctx->scratch;
   p.counters = ctx->counters;
-  p.status = ctx->statusDev;
+  p.status = ctx->status;
   RT_CUDA(ctx, rt::launch_decode(p, dtype, ctx->stream));
   ctx->launches += p.mergeAfter ? 2 : 1;
   return RT_OK;
@@ -303,12 +303,13 @@ int rt_ctx_create(int device, rt_ctx** out) {
   ctx->waitPolls = 1 << 20;   // about a second with the kernel's sleeps
   if ((e = cudaSetDevice(device)) != cudaSuccess ||
       (e = cudaStreamCreateWithFlags(&ctx->own, cudaStreamNonBlocking)) != cudaSuccess ||
-      (e = cudaMallocHost(&ctx->statusHost, sizeof(int))) != cudaSuccess ||
-      (e = cudaMalloc(&ctx->statusDev, kStatusWords * sizeof(int))) != cudaSuccess ||
-      (e = cudaMemset(ctx->statusDev, 0, kStatusWords * sizeof(int))) != cudaSuccess) {
+      (e = cudaMallocHost(&ctx->status, sizeof(int))) != cudaSuccess ||
+      (e = cudaMalloc(&ctx->work, kWorkWords * sizeof(int))) != cudaSuccess ||
+      (e = cudaMemset(ctx->work, 0, kWorkWords * sizeof(int))) != cudaSuccess) {
     delete ctx;
     return fail(nullptr, RT_EXECUTION_FAILED, "context setup: %s", cudaGetErrorString(e));
   }
+  *ctx->status = 0;
   ctx->stream = ctx->own;
   *out = ctx;
   return RT_OK;
@@ -321,13 +322,13 @@ int rt_ctx_destroy(rt_ctx* ctx) {
   if (ctx->counters) cudaFree(ctx->counters);
   for (const auto& o : ctx->outgrown) cudaFree(o.block);
   ctx->outgrown.clear();
-  cudaFree(ctx->statusDev);
-  cudaFreeHost(ctx->statusHost);
+  cudaFree(ctx->work);
+  cudaFreeHost(ctx->status);
   cudaStreamDestroy(ctx->own);
   ctx->scratch = nullptr;
   ctx->counters = nullptr;
-  ctx->statusDev = nullptr;
-  ctx->statusHost = nullptr;
+  ctx->work = nullptr;
+  ctx->status = nullptr;
   ctx->magic = kDead;
   std::lock_guard<std::mutex> lock(gGraveyardMutex);
   gGraveyard.push_back(ctx);
@@ -364,14 +365,14 @@ const char* rt_last_error(const rt_ctx* ctx) {
   return tlsError.c_str();
 }
 
-// Waits for the stream and for the copy of the status word that is on it; what the word says.
+// Waits for the stream; what the status word then says.
 static int finish(rt_ctx* ctx) {
   RT_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  const int status = *ctx->statusHost;
+  const int status = *const_cast<volatile int*>(ctx->status);
   if (status != 0) {
-    // (with the status word, the work counter of the persistent prefill kernel, which a
-    // block that gave up never rewound)
-    cudaMemset(ctx->statusDev, 0, kStatusWords * sizeof(int));
+    *ctx->status = 0;
+    // (the work counter of the persistent prefill kernel, which a block that gave up never rewound)
+    cudaMemset(ctx->work, 0, kWorkWords * sizeof(int));
     // A block that gave up never counted itself in: the arrival counters of the split
     // merge are no longer zero, and the next split launch would pick the wrong last block.
     if (ctx->counters) cudaMemset(ctx->counters, 0, ctx->counterCount * sizeof(unsigned));
@@ -387,13 +388,8 @@ static int finish(rt_ctx* ctx) {
   return RT_OK;
 }
 
-static cudaError_t copy_status(rt_ctx* ctx) {
-  return cudaMemcpyAsync(ctx->statusHost, ctx->statusDev, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
-}
-
 int rt_sync(rt_ctx* ctx) {
   RT_ENTER(ctx);
-  RT_CUDA(ctx, copy_status(ctx));
   return finish(ctx);
 }
 
@@ -429,7 +425,6 @@ int rt_buf_upload(rt_ctx* ctx, void* device_ptr, size_t offset, const void* host
 int rt_buf_download(rt_ctx* ctx, const void* device_ptr, size_t offset, void* host, size_t bytes) {
   RT_ENTER(ctx);
   if (!device_ptr || !host) return fail(ctx, RT_INVALID_ARGUMENT, "rt_buf_download: NULL pointer");
-  RT_CUDA(ctx, copy_status(ctx));   // ahead of the data, whose copy to pageable memory waits
   RT_CUDA(ctx, cudaMemcpyAsync(host, static_cast<const char*>(device_ptr) + offset, bytes,
                                cudaMemcpyDeviceToHost, ctx->stream));
   return finish(ctx);
@@ -506,11 +501,11 @@ int rt_attn(rt_ctx* ctx, const rt_attn_args* a) {
     RT_CUDA(ctx, rt::launch_prefill_f32_tc(p, ctx->stream));
   } else if (kernel != 0) {
     std::string err;
-    cudaError_t e = kernel == 5   ? rt::launch_prefill_tc4(p, ctx->statusDev, ctx->statusDev + 1, ctx->smCount,
+    cudaError_t e = kernel == 5   ? rt::launch_prefill_tc4(p, ctx->status, ctx->work, ctx->smCount,
                                                            ctx->stream, &err)
-                    : kernel >= 3 ? rt::launch_prefill_tc3(p, kernel == 4, ctx->statusDev, ctx->stream, &err)
-                    : kernel == 2 ? rt::launch_prefill_tc2(p, ctx->statusDev, ctx->stream, &err)
-                                  : rt::launch_prefill_tc(p, a->dtype, ctx->statusDev, ctx->stream, &err);
+                    : kernel >= 3 ? rt::launch_prefill_tc3(p, kernel == 4, ctx->status, ctx->stream, &err)
+                    : kernel == 2 ? rt::launch_prefill_tc2(p, ctx->status, ctx->stream, &err)
+                                  : rt::launch_prefill_tc(p, a->dtype, ctx->status, ctx->stream, &err);
     if (e != cudaSuccess)
       return fail(ctx, RT_EXECUTION_FAILED, "prefill_tc launch: %s %s", cudaGetErrorString(e),
                   err.c_str());
@@ -580,7 +575,7 @@ int rt_attn_decode(rt_ctx* ctx, const rt_decode_args* a) {
   const int owned = rt::owner_count(x.rank, a->batch, x.world);
   RT_CUDA(ctx, rt::launch_merge_exchanged(x.partials[x.rank], x.flags[x.rank], x.step, x.world, per,
                                           owned, first, a->qHeads, a->headDim, a->out, a->dtype,
-                                          ctx->statusDev, ctx->waitPolls, ctx->stream));
+                                          ctx->status, ctx->waitPolls, ctx->stream));
   if (owned > 0) ctx->launches++;
   return RT_OK;
 }
@@ -601,10 +596,8 @@ int rt_attn_merge_partials(rt_ctx* ctx, const float* partials, int32_t parts, in
   return RT_OK;
 }
 
-int rt_rope(rt_ctx* ctx, const void* x, const float* cosT, const float* sinT, void* out,
-            int64_t rows, int64_t cols, int32_t headDim, int64_t srcStart, int64_t width,
-            int32_t dtype) {
-  RT_ENTER(ctx);
+static int check_rope(rt_ctx* ctx, const void* x, const float* cosT, const float* sinT, const void* out,
+                      int64_t rows, int64_t cols, int32_t headDim, int64_t srcStart, int64_t width, int32_t dtype) {
   if (!x || !cosT || !sinT || !out) return fail(ctx, RT_INVALID_ARGUMENT, "rope: NULL pointer");
   if (dtype != RT_F32 && dtype != RT_F16)
     return fail(ctx, RT_INVALID_ARGUMENT, "rope: bad dtype %d", dtype);
@@ -623,6 +616,15 @@ int rt_rope(rt_ctx* ctx, const void* x, const float* cosT, const float* sinT, vo
   if (width % headDim != 0)
     return fail(ctx, RT_INVALID_ARGUMENT, "rope: width %lld must be a multiple of headDim %d",
                 (long long)width, headDim);
+  return RT_OK;
+}
+
+int rt_rope(rt_ctx* ctx, const void* x, const float* cosT, const float* sinT, void* out,
+            int64_t rows, int64_t cols, int32_t headDim, int64_t srcStart, int64_t width,
+            int32_t dtype) {
+  RT_ENTER(ctx);
+  const int s = check_rope(ctx, x, cosT, sinT, out, rows, cols, headDim, srcStart, width, dtype);
+  if (s != RT_OK) return s;
   RT_CUDA(ctx, rt::launch_rope(x, cosT, sinT, out, rows, cols, headDim, srcStart, width, dtype,
                                ctx->stream));
   ctx->launches++;
@@ -650,7 +652,7 @@ int rt_matmul(rt_ctx* ctx, const void* a, const void* b, const void* bias, const
   if (ctx->useTc && rt::matmul_tc_supported(a, bp, out, m, k, n, dtype)) {
     std::string err;
     cudaError_t e = rt::launch_matmul_tc(a, bp, bias, addend, out, m, k, n, activation,
-                                         ctx->statusDev, ctx->stream, &err);
+                                         ctx->status, ctx->stream, &err);
     if (e != cudaSuccess)
       return fail(ctx, RT_EXECUTION_FAILED, "matmul_tc launch: %s %s", cudaGetErrorString(e),
                   err.c_str());
@@ -682,11 +684,16 @@ int rt_argmax_dot(rt_ctx* ctx, const void* w, const void* x, float* out, int64_t
   if (rows < 1 || cols < 1 || rows > 0xffffffffll)
     return fail(ctx, RT_INVALID_ARGUMENT, "argmaxDot: empty or oversized tensor (%lld x %lld)",
                 (long long)rows, (long long)cols);
-  int s = ensure_scratch(ctx, 64, 1);
+  // One word of scratch per block; under a capture, where none can be made, as many blocks as the scratch
+  // at hand has words for (eight words are asked for in any case).
+  int blocks = rt::argmax_dot_blocks(rows, cols);
+  if (capturing(ctx->stream) && ctx->scratchBytes < blocks * sizeof(uint64_t) && ctx->scratchBytes >= 64)
+    blocks = (int)(ctx->scratchBytes / sizeof(uint64_t));
+  int s = ensure_scratch(ctx, std::max<size_t>(blocks * sizeof(uint64_t), 64), 1);
   if (s != RT_OK) return s;
-  RT_CUDA(ctx, rt::launch_argmax_dot(w, x, out, rows, cols, dtype,
-                                     reinterpret_cast<unsigned long long*>(ctx->scratch), ctx->stream));
-  ctx->launches += 2;
+  RT_CUDA(ctx, rt::launch_argmax_dot(w, x, out, rows, cols, dtype, reinterpret_cast<unsigned long long*>(ctx->scratch),
+                                     ctx->counters, blocks, ctx->stream));
+  ctx->launches++;
   return RT_OK;
 }
 
@@ -719,7 +726,7 @@ int rt_local_attention(rt_ctx* ctx, const void* qkv, const float* rel, const flo
   if (ctx->useTc && rt::local_attn_tc_supported(qkv, rel, out, rows, heads, headDim, dtype)) {
     std::string err;
     cudaError_t e = rt::launch_local_attn_tc(qkv, rel, qScale, out, rows, heads, headDim, window, kScale,
-                                             softcap, ctx->statusDev, ctx->stream, &err);
+                                             softcap, ctx->status, ctx->stream, &err);
     if (e != cudaSuccess)
       return fail(ctx, RT_EXECUTION_FAILED, "local_attn_tc launch: %s %s", cudaGetErrorString(e),
                   err.c_str());
@@ -755,9 +762,8 @@ int rt_softmax(rt_ctx* ctx, const void* x, void* out, const float* segments, int
   return RT_OK;
 }
 
-int rt_slice(rt_ctx* ctx, const void* x, void* out, int64_t rows, int64_t cols, int64_t rowStart,
-             int64_t rowEnd, int64_t colStart, int64_t colEnd, int32_t dtype) {
-  RT_ENTER(ctx);
+static int check_slice(rt_ctx* ctx, const void* x, const void* out, int64_t rows, int64_t cols, int64_t rowStart,
+                       int64_t rowEnd, int64_t colStart, int64_t colEnd, int32_t dtype) {
   if (!x || !out) return fail(ctx, RT_INVALID_ARGUMENT, "slice: NULL pointer");
   if (dtype != RT_F32 && dtype != RT_F16)
     return fail(ctx, RT_INVALID_ARGUMENT, "slice: bad dtype %d", dtype);
@@ -770,11 +776,38 @@ int rt_slice(rt_ctx* ctx, const void* x, void* out, int64_t rows, int64_t cols, 
   if (colStart < 0 || colEnd > cols || colStart >= colEnd)
     return fail(ctx, RT_INVALID_ARGUMENT, "slice: bad range [%lld, %lld) for %lld cols",
                 (long long)colStart, (long long)colEnd, (long long)cols);
+  return RT_OK;
+}
+
+int rt_slice(rt_ctx* ctx, const void* x, void* out, int64_t rows, int64_t cols, int64_t rowStart,
+             int64_t rowEnd, int64_t colStart, int64_t colEnd, int32_t dtype) {
+  RT_ENTER(ctx);
+  const int s = check_slice(ctx, x, out, rows, cols, rowStart, rowEnd, colStart, colEnd, dtype);
+  if (s != RT_OK) return s;
   const int es = elem_size(dtype);
   RT_CUDA(ctx, rt::launch_slice(x, out, rowEnd - rowStart, cols * es,
                                 (rowStart * cols + colStart) * es, (colEnd - colStart) * es,
                                 ctx->stream));
   ctx->launches++;
+  return RT_OK;
+}
+
+int rt_windows(rt_ctx* ctx, const rt_window* w, int32_t count, int32_t dtype) {
+  RT_ENTER(ctx);
+  if (!w) return fail(ctx, RT_INVALID_ARGUMENT, "rt_windows: windows is NULL");
+  if (count < 1 || count > RT_MAX_WINDOWS)
+    return fail(ctx, RT_INVALID_ARGUMENT, "rt_windows: takes 1..%d windows, got %d", RT_MAX_WINDOWS, count);
+  for (int i = 0; i < count; i++) {
+    const rt_window& o = w[i];
+    const int s = o.cosT || o.sinT ? check_rope(ctx, o.x, o.cosT, o.sinT, o.out, o.rows, o.cols, o.headDim, o.start,
+                                                o.width, dtype)
+                                   : check_slice(ctx, o.x, o.out, o.rows, o.cols, 0, o.rows, o.start,
+                                                 o.start + o.width, dtype);
+    if (s != RT_OK) return s;
+  }
+  int launches = 0;
+  RT_CUDA(ctx, rt::launch_windows(w, count, dtype, &launches, ctx->stream));
+  ctx->launches += launches;
   return RT_OK;
 }
 

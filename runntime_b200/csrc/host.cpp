@@ -62,6 +62,7 @@ struct Entry {
   decltype(&rt_kv_append) kvAppend;
   decltype(&rt_softmax) softmax;
   decltype(&rt_local_attention) localAttention;
+  decltype(&rt_windows) windows;
 } gEntry;
 
 // ---- small pieces ------------------------------------------------------------------------
@@ -555,6 +556,15 @@ bool release(Evaluation& e, Exec& x, PyObject* inputs) {
   return true;
 }
 
+// Raises what check() makes of a status that is not RT_OK.
+bool report(Exec& x, int status) {
+  if (status == 0) return true;
+  Ref code(PyLong_FromLong(status));
+  Ref r(code ? PyObject_CallFunctionObjArgs(gCheck, code.p, x.ctxObject.p, nullptr) : nullptr);
+  if (r) PyErr_SetString(PyExc_SystemError, "a failed call was not reported");
+  return false;
+}
+
 // -1: an exception is set; 0: left to the executor's dispatch(); 1: done.
 int dispatch(Evaluation& e, Exec& x, const Node& n, PyObject* out) {
   char *o = nullptr, *in[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -726,15 +736,72 @@ int dispatch(Evaluation& e, Exec& x, const Node& n, PyObject* out) {
     default:
       return 0;
   }
-  if (status != 0) {
-    Ref code(PyLong_FromLong(status));
-    Ref r(code ? PyObject_CallFunctionObjArgs(gCheck, code.p, x.ctxObject.p, nullptr) : nullptr);
-    if (r) PyErr_SetString(PyExc_SystemError, "a failed call was not reported");
-    return -1;
-  }
+  if (!report(x, status)) return -1;
   Ref text(route ? PyUnicode_FromString(route) : Py_NewRef(name));
   if (!text || PyList_Append(x.names.p, text.p) < 0) return -1;
   return 1;
+}
+
+// Ropes and column slices that follow one another over the same tensor (q and k rotated, v cut out
+// of a fused qkv projection) from place `i` of the order on: one call for up to four of them, whose
+// outputs come from acquire().  -1: an exception is set; 0: not here; else how many were run.
+int dispatch_windows(Evaluation& e, Exec& x, size_t i) {
+  rt_window w[RT_MAX_WINDOWS] = {};
+  PyObject* source = input(e.order[i], 0);
+  Meta m;
+  int n = 0;
+  for (; n < RT_MAX_WINDOWS && i + n < e.order.size(); n++) {
+    const Node& d = e.order[i + n];
+    const bool rope = d.op == kRope;
+    if (d.elided || !(rope || d.op == kSliceCols) || inputs_of(d) != (rope ? 3 : 1) || input(d, 0) != source) break;
+    long long a[3];
+    char *p, *cs = nullptr, *sn = nullptr;
+    if (!read_matrix(source, m) || slot(source, gReleasedAt) != Py_None || !buffer_ptr(slot(source, gBufferAt), p) ||
+        !attr(d, 0, a[0]) || !attr(d, 1, a[1]) || (rope && !attr(d, 2, a[2])))
+      break;
+    if (rope) {
+      PyObject *c = input(d, 1), *s = input(d, 2);
+      if (Py_TYPE(c) != gValue || Py_TYPE(s) != gValue || slot(c, gReleasedAt) != Py_None ||
+          slot(s, gReleasedAt) != Py_None || !buffer_ptr(slot(c, gBufferAt), cs) || !buffer_ptr(slot(s, gBufferAt), sn))
+        break;
+    }
+    w[n].x = p;
+    w[n].cosT = reinterpret_cast<float*>(cs);
+    w[n].sinT = reinterpret_cast<float*>(sn);
+    w[n].rows = m.rows;
+    w[n].cols = m.cols;
+    w[n].start = rope ? a[1] : a[0];
+    w[n].width = rope ? a[2] : a[1] - a[0];
+    w[n].headDim = rope ? (int32_t)a[0] : 0;
+  }
+  if (n < 2) return 0;
+  Ref disposed(PyObject_GetAttr(x.self, s__disposed));
+  if (!disposed) return -1;
+  if (disposed.p != Py_False) return 0;
+  Ref out[RT_MAX_WINDOWS];
+  for (int k = 0; k < n; k++) {
+    char* o;
+    out[k].p = acquire(x, slot(e.order[i + k].v, gShapeAt));
+    if (!out[k]) return -1;
+    if (!buffer_ptr(out[k].p, o)) {
+      PyErr_SetString(PyExc_TypeError, "acquireOutput gave no DeviceBuffer");
+      return -1;
+    }
+    w[k].out = o;
+  }
+  int status;
+  Py_BEGIN_ALLOW_THREADS;
+  status = gEntry.windows(x.ctx, w, n, m.dtype);
+  Py_END_ALLOW_THREADS;
+  if (!report(x, status)) return -1;
+  for (int k = 0; k < n; k++) {
+    Node& d = e.order[i + k];
+    if (PyList_Append(x.names.p, d.op == kRope ? s_rope : s_sliceCols) < 0) return -1;
+    set_slot(d.v, gBufferAt, out[k].p);
+  }
+  for (int k = 0; k < n; k++)
+    if (!release(e, x, e.order[i + k].inputs)) return -1;
+  return n;
 }
 
 // dispatch() of the executor, with the arguments the Python loop gives it.
@@ -804,8 +871,17 @@ PyObject* evaluate_graph(PyObject* const* args, Py_ssize_t nargs) {
     return nullptr;
   if (!PyDict_CheckExact(x.pool.p) || !PySet_CheckExact(x.live.p) || !PyList_CheckExact(x.names.p)) Py_RETURN_FALSE;
 
-  for (Node& m : e.order) {
+  for (size_t i = 0; i < e.order.size(); i++) {
+    Node& m = e.order[i];
     if (m.elided) continue;
+    if (m.op == kRope || m.op == kSliceCols) {
+      const int ran = dispatch_windows(e, x, i);
+      if (ran < 0) return nullptr;
+      if (ran > 0) {
+        i += ran - 1;
+        continue;
+      }
+    }
     if (m.op == kWriteRows) {
       PyObject* out = slot(input(m, 0), gBufferAt);
       Ref keep(Py_NewRef(out));
@@ -826,8 +902,8 @@ PyObject* evaluate_graph(PyObject* const* args, Py_ssize_t nargs) {
     if (!release(e, x, m.inputs)) return nullptr;
     if (m.fused.on) {
       if (!release(e, x, e.order[m.fused.k].inputs) || !release(e, x, e.order[m.fused.v].inputs)) return nullptr;
-      for (int i : {m.fused.ropeQ, m.fused.ropeK, m.fused.vSlice})
-        if (i >= 0 && !release(e, x, e.order[i].inputs)) return nullptr;
+      for (int k : {m.fused.ropeQ, m.fused.ropeK, m.fused.vSlice})
+        if (k >= 0 && !release(e, x, e.order[k].inputs)) return nullptr;
     }
   }
   Py_RETURN_TRUE;

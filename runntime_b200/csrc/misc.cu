@@ -1,6 +1,7 @@
 // Small kernels beside attention: the standalone KV-cache append (writeRows),
 // the rotary embedding that precedes it, and the cross-device merge of
 // (m, l, acc) partials.
+#include <algorithm>
 #include <type_traits>
 #include "common.cuh"
 
@@ -236,6 +237,47 @@ __global__ void rope_vec_kernel(const T* __restrict__ x, const float* __restrict
   }
 }
 
+// Up to four column windows in one launch, blockIdx.y each: rotated as above or, without tables,
+// copied.  A pass over a short clip is bound by its launches (3.5 to 4 us each on the host): two
+// rotations and a slice of 415 rows by 288 columns took three of them, 12.3 us; one takes 4, its
+// kernel 1.8.
+struct Windows {
+  rt_window w[RT_MAX_WINDOWS];
+};
+template <typename T, int V>
+__global__ void windows_kernel(const Windows ws) {
+  using Word = typename std::conditional<V * sizeof(T) == 16, uint4, uint2>::type;
+  asm volatile("griddepcontrol.wait;" ::: "memory");   // (a programmatic dependent)
+  const rt_window& w = ws.w[blockIdx.y];
+  const int64_t units = w.width / V, total = w.rows * units, stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
+    const int64_t row = i / units, col = (i - row * units) * V;
+    Word raw = *reinterpret_cast<const Word*>(static_cast<const T*>(w.x) + row * w.cols + w.start + col);
+    if (w.cosT) {
+      const int64_t at = row * w.headDim + (int)col % w.headDim;
+      T* v = reinterpret_cast<T*>(&raw);
+#pragma unroll
+      for (int e = 0; e < V; e += 4) {  // tables are pair-duplicated: entries 0, 2 of a float4
+        const float4 c = *reinterpret_cast<const float4*>(w.cosT + at + e);
+        const float4 sn = *reinterpret_cast<const float4*>(w.sinT + at + e);
+        float r0, r1, r2, r3;
+        rope_pair(to_f32<T>(v[e]), to_f32<T>(v[e + 1]), c.x, sn.x, r0, r1);
+        rope_pair(to_f32<T>(v[e + 2]), to_f32<T>(v[e + 3]), c.z, sn.z, r2, r3);
+        v[e] = from_f32<T>(r0), v[e + 1] = from_f32<T>(r1), v[e + 2] = from_f32<T>(r2), v[e + 3] = from_f32<T>(r3);
+      }
+    }
+    *reinterpret_cast<Word*>(static_cast<T*>(w.out) + row * w.width + col) = raw;
+  }
+}
+
+// Whether a window can be walked in groups of V elements.
+bool window_aligned(const rt_window& w, int v, int esize) {
+  const uintptr_t bytes = (uintptr_t)v * esize;
+  const auto on = [](const void* p, uintptr_t b) { return reinterpret_cast<uintptr_t>(p) % b == 0; };
+  if (w.start % v || w.cols % v || w.width % v || !on(w.x, bytes) || !on(w.out, bytes)) return false;
+  return !w.cosT || (w.headDim % v == 0 && on(w.cosT, 16) && on(w.sinT, 16));
+}
+
 template <typename T>
 void rope_launch(const void* x, const float* cosT, const float* sinT, void* out, int64_t rows,
                  int64_t srcCols, int hd, int64_t srcStart, int64_t width, unsigned blocks,
@@ -304,6 +346,50 @@ cudaError_t launch_slice(const void* x, void* out, int64_t rows, int64_t srcColB
   else if ((mis & 3) == 0) run(uint32_t{});
   else run(uint16_t{});
   return cudaGetLastError();
+}
+
+// Large windows go one by one: a launch is little beside them, and rope_vec_kernel reads a row's
+// tables once for all heads.  q, k and v of 8 heads of 36 halves: 8000 rows 12.3 us one by one, 9.6
+// together; 16000 18.5 and 15.9; 64000 56.3 and 61.8.
+constexpr int64_t kWindowBytes = 8 << 20;
+cudaError_t launch_windows(const rt_window* w, int count, int dtype, int* launches, cudaStream_t s) {
+  const int esize = dtype == RT_F16 ? 2 : 4, wide = 16 / esize;
+  bool by16 = true, by4 = true, small = true;
+  int64_t most = 0;
+  for (int i = 0; i < count; i++) {
+    by16 = by16 && window_aligned(w[i], wide, esize);
+    by4 = by4 && window_aligned(w[i], 4, esize);
+    most = std::max(most, w[i].rows * w[i].width);
+  }
+  small = most * esize <= kWindowBytes;
+  if (!small || !(by16 || by4)) {
+    for (int i = 0; i < count; i++) {
+      const rt_window& o = w[i];
+      const cudaError_t e =
+          o.cosT ? launch_rope(o.x, o.cosT, o.sinT, o.out, o.rows, o.cols, o.headDim, o.start, o.width, dtype, s)
+                 : launch_slice(o.x, o.out, o.rows, o.cols * esize, o.start * esize, o.width * esize, s);
+      if (e != cudaSuccess) return e;
+      ++*launches;
+    }
+    return cudaSuccess;
+  }
+  Windows ws{};
+  for (int i = 0; i < count; i++) ws.w[i] = w[i];
+  const int v = by16 ? wide : 4;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)std::min<int64_t>((most / v + 255) / 256, 148 * 8), (unsigned)count);
+  cfg.blockDim = dim3(256);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  ++*launches;
+  if (dtype == RT_F16)
+    return by16 ? cudaLaunchKernelEx(&cfg, windows_kernel<__half, 8>, ws)
+                : cudaLaunchKernelEx(&cfg, windows_kernel<__half, 4>, ws);
+  return cudaLaunchKernelEx(&cfg, windows_kernel<float, 4>, ws);
 }
 
 cudaError_t launch_write_rows(void* dst, const void* src, int64_t dstOffsetBytes, int64_t bytes,

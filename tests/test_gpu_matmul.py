@@ -146,3 +146,27 @@ def test_argmax_dot_takes_the_lowest_index_on_ties(ex):
     x = np.ones((1, 8), np.float32)
     got = rt.toArray(rt.argmaxDot(ex.upload(w, [4096, 8]), ex.upload(x, [1, 8])), ex)
     assert int(got[0]) == 77
+
+
+@pytest.mark.parametrize("dtype", ["f16", "f32"])
+@pytest.mark.parametrize("rows,cols", [(1, 8), (3, 8), (32, 264), (33, 1), (127, 300), (23680, 24), (23681, 24), (50000, 17)])
+def test_argmax_dot_over_warps_blocks_and_rounds(ex, dtype, rows, cols):
+    """Fewer rows than a warp's four, a block's thirty-two or one round of all blocks, and more; the
+    same row whatever block finds it, twice in a row on the same scratch."""
+    import runntime_b200 as rt
+    rng = np.random.default_rng(rows)
+    w = oracle.round_f16(rng.standard_normal((rows, cols)).astype(np.float32))
+    x = oracle.round_f16(rng.standard_normal((1, cols)).astype(np.float32))
+    W, X = ex.upload(w, [rows, cols], dtype), ex.upload(x, [1, cols], dtype)
+    for at in (rows - 1, rows // 2, 0):
+        big = w.copy()
+        big[at] = oracle.round_f16(x[0] * 40)
+        B = ex.upload(big, [rows, cols], dtype)
+        before = ex.launchCount()
+        assert rt.toArray(rt.argmaxDot(B, X), ex)[0] == at
+        assert ex.launchCount() == before + 1
+    got = int(rt.toArray(rt.argmaxDot(W, X), ex)[0])
+    scores = w.astype(np.float64) @ x[0].astype(np.float64)
+    # (the f32 sum of `cols` products is off by at most cols/2 ulps of the largest partial sum)
+    slack = cols * 2.0 ** -24 * np.abs(w[got] * x[0]).sum() * 2
+    assert scores[got] >= scores.max() - slack

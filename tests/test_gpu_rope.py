@@ -219,3 +219,32 @@ def test_slice_and_chunk(ex, dtype):
     for i, p in enumerate(parts):
         assert np.array_equal(ex.readback(p.buffer, p.shape).reshape(rows, -1),
                               x[:, i * 52:(i + 1) * 52])
+
+
+@pytest.mark.parametrize("dtype", ["f16", "f32"])
+@pytest.mark.parametrize("rows,heads,hd", [(1, 8, 36), (415, 8, 36), (37, 8, 52), (130, 4, 64), (5, 3, 128), (9, 2, 20),
+                                           (7, 3, 6), (2100, 8, 64), (9000, 8, 64)])
+def test_windows_of_one_tensor_in_one_launch(ex, dtype, rows, heads, hd):
+    """q and k rotated and v cut out of a fused row: what the operators give one by one, bit for
+    bit, in one launch where the windows are small and start on four elements."""
+    import runntime_b200 as rt
+    w = heads * hd
+    x = ex.upload(oracle.random_f32(rows * 3 * w, 1), [rows, 3 * w], dtype)
+    cos, sin = (ex.upload(oracle.random_f32(rows * hd, s), [rows, hd]) for s in (2, 3))
+
+    def nodes():
+        return [rt.rope(x, cos, sin, dict(headDim=hd, srcStart=0, width=w)),
+                rt.rope(x, cos, sin, dict(headDim=hd, srcStart=w, width=w)),
+                rt.slice(x, 1, 2 * w, 3 * w), rt.slice(x, 1, w - hd, w + 2 * hd),
+                rt.rope(x, cos, sin, dict(headDim=hd, srcStart=2 * w, width=w))]
+
+    alone = [rt.toArray(n, ex) for n in nodes()]
+    together = nodes()
+    before = ex.launchCount()
+    rt.evalValues(together, ex)
+    launches = ex.launchCount() - before
+    if rt._lib.host is not None:
+        # (the fifth is a call of its own; large windows and unaligned ones go one by one)
+        assert launches == (2 if hd % 4 == 0 and rows * w * (2 if dtype == "f16" else 4) <= 8 << 20 else 5)
+    for a, t in zip(alone, together):
+        assert np.array_equal(a, rt.toArray(t, ex))
