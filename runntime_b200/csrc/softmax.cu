@@ -185,7 +185,7 @@ __device__ __forceinline__ void kept_range(const float* segs, int64_t row, int64
 }
 
 // One row.  V: elements per chunk.
-template <typename T, By BY, int V>
+template <typename T, By BY, int V, int TH = kThreads>   // TH: threads of the CTA
 __device__ __forceinline__ void softmax_row(const T* __restrict__ x, T* __restrict__ out, int64_t row, int64_t cols,
                                             int64_t lo64, int64_t hi64, float* sM, float* sS) {
   using C = Chunk<T, V>;
@@ -193,9 +193,9 @@ __device__ __forceinline__ void softmax_row(const T* __restrict__ x, T* __restri
   using I = std::conditional_t<V == 1, int64_t, int>;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int t = BY == By::Cta ? threadIdx.x : lane;      // for the kept columns
-  const int span = BY == By::Cta ? kThreads : 32;
+  const int span = BY == By::Cta ? TH : 32;
   const int zt = BY == By::Warp ? lane : threadIdx.x;    // for the zeros
-  const int zspan = BY == By::Warp ? 32 : kThreads;
+  const int zspan = BY == By::Warp ? 32 : TH;
   const bool keeps = BY != By::WarpInCta || warp == 0;
 
   // The row begins `mis` elements into its first chunk (the same for x and out: see the
@@ -287,7 +287,7 @@ __device__ __forceinline__ void softmax_row(const T* __restrict__ x, T* __restri
   s = warp_sum(s * __expf(m - top));
   m = top;
   if (BY == By::Cta) {
-    constexpr int kWarps = kThreads / 32;
+    constexpr int kWarps = TH / 32;
     if (lane == 0) sM[warp] = m, sS[warp] = s;
     __syncthreads();
     const float mw = sM[lane % kWarps];
@@ -327,6 +327,47 @@ softmax_cta_kernel(const T* __restrict__ x, T* __restrict__ out, const float* __
   kept_range(segs, blockIdx.x, cols, wl, wr, lo, hi);
   if (hi - lo <= kWarpKept) softmax_row<T, By::WarpInCta, V>(x, out, blockIdx.x, cols, lo, hi, nullptr, nullptr);
   else softmax_row<T, By::Cta, V>(x, out, blockIdx.x, cols, lo, hi, sM, sS);
+}
+
+// Long half-precision rows that start anywhere, four to a CTA: where all four keep few columns each
+// warp takes a row of its own, else the CTA takes them in turn.  A CTA per row spends a narrow row's time
+// waiting for one warp's scores, statistics and stores in turn (20.6 us for 11.5 at the copy
+// rate); four at once overlap them.  The last quarter of the rows go one to a CTA, so that a launch whose
+// rows are wide does not end on a few CTAs with four of them (n columns, segments, us, a CTA per
+// row and this: 6007, 24 22.4, 18.5; 6007, 6 42.4, 28.7; 7001, 60 27.0, 22.6; 10239, 9 61.9, 53.8; 6007, 1 71.9, 70.1;
+// 9001, 1 149.9, 149.7).  With fewer rows than the chip takes four at a time wide ones lose (4097, 1
+// 41.7, 45.7), as do rows of more than 20 KB, whose zeros are better written by eight warps (f32 6007, 24
+// 30.1, 32.7), and f32 ones (4097, 1 41.2, 49.4).
+constexpr int kGroupRows = 4, kGroup = 32 * kGroupRows, kGroupMinRows = 5000, kGroupRowBytes = 20480;
+template <int V>
+__global__ void __launch_bounds__(kGroup, 10)
+softmax_group_kernel(const __half* __restrict__ x, __half* __restrict__ out, const float* __restrict__ segs,
+                     int64_t cols, int64_t wl, int64_t wr, int groups) {
+  using T = __half;
+  __shared__ float sM[2][kGroupRows], sS[2][kGroupRows];
+  const bool group = (int)blockIdx.x < groups;
+  int64_t row = group ? (int64_t)blockIdx.x * kGroupRows : (int64_t)groups * (kGroupRows - 1) + blockIdx.x;
+  int64_t lo, hi;
+  if (group) {
+    const int64_t mine = row + (threadIdx.x >> 5);
+    kept_range(segs, mine, cols, wl, wr, lo, hi);
+    if (__syncthreads_and(hi - lo <= kWarpKept)) {
+      softmax_row<T, By::Warp, V>(x, out, mine, cols, lo, hi, nullptr, nullptr);
+      return;
+    }
+  } else {
+    kept_range(segs, row, cols, wl, wr, lo, hi);
+    if (hi - lo <= kWarpKept) {
+      softmax_row<T, By::WarpInCta, V, kGroup>(x, out, row, cols, lo, hi, nullptr, nullptr);
+      return;
+    }
+  }
+#pragma unroll 1
+  for (int r = 0; r < (group ? kGroupRows : 1); r++, row++) {
+    // (two sets of sums: a row's are read while the next one's are written)
+    kept_range(segs, row, cols, wl, wr, lo, hi);
+    softmax_row<T, By::Cta, V, kGroup>(x, out, row, cols, lo, hi, sM[r & 1], sS[r & 1]);
+  }
 }
 
 // A row by a warp, element by element.
@@ -371,6 +412,14 @@ cudaError_t softmax_chunked(const T* x, T* out, const float* segs, int64_t rows,
   const int64_t blocks = warpRows ? (rows + kThreads / 32 - 1) / (kThreads / 32) : rows;
   if (blocks > 0x7fffffffll) return cudaErrorInvalidValue;
   const unsigned g = (unsigned)blocks;
+  if constexpr (sizeof(T) == 2 && V > 1) {
+    if (segs && rows >= kGroupMinRows && cols > kWarpRowCols && cols * 2 <= kGroupRowBytes) {
+      const int groups = (int)(rows / 4 * 3 / kGroupRows);
+      softmax_group_kernel<V><<<(unsigned)(rows - (int64_t)groups * (kGroupRows - 1)), kGroup, 0, s>>>(
+          x, out, segs, cols, wl, wr, groups);
+      return cudaGetLastError();
+    }
+  }
   if (warpRows) softmax_warp_kernel<T, V><<<g, kThreads, 0, s>>>(x, out, segs, rows, cols, wl, wr);
   else softmax_cta_kernel<T, V><<<g, kThreads, 0, s>>>(x, out, segs, cols, wl, wr);
   return cudaGetLastError();

@@ -182,3 +182,35 @@ def test_masked_rows_of_a_warp(ex, dtype, n, parts):
     segs[3], segs[4], segs[5] = (0, n // 2), (n // 2 - 1, n), (n, n)
     got = rt.toArray(rt.softmax(ex.upload(x, [n, n], dtype), dict(segments=ex.upload(segs, [n, 2]))), ex)
     close(got, oracle.softmax_ref(x, segs), dtype)
+
+
+@pytest.mark.parametrize("n,shift", [(5001, 0), (5003, 3), (5002, 4)])
+def test_long_half_precision_rows_in_groups(ex, n, shift):
+    """Four rows to a block: all narrow (a warp each), all wide, one wide among narrow ones, rows
+    that keep nothing, ranges at either end; the rows that have a block of their own; what the
+    output held is overwritten and nothing around it."""
+    import ctypes as C
+    import torch
+    from runntime_b200._lib import WINDOW_INF, check
+    g = torch.Generator(device="cuda").manual_seed(n)
+    src = torch.empty(n * n + 16, device="cuda").normal_(0, 3, generator=g).half()
+    out = torch.full((n * n + 16,), 7.0, device="cuda", dtype=torch.float16)
+    x = src[shift:shift + n * n].view(n, n)
+    kinds = [[(0, 40), (9, 1033), (n - 1024, n), (n - 1, n)], [(0, n), (1, n), (0, n - 1), (3, 1028)],
+             [(5, 60), (0, 1025), (7, 7), (0, 0)], [(n, n), (0, 0), (4, 4), (1, 1)],
+             [(8, 1032), (n - 1033, n - 9), (0, 1024), (2, 3)]]
+    segs = [kinds[(r // 4) % len(kinds)][r % 4] for r in range(n)]
+    dev = torch.tensor(segs, dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
+    check(ex._lib.rt_softmax(ex.ctx, C.c_void_p(x.data_ptr()), C.c_void_p(out.data_ptr() + 2 * shift),
+                             C.c_void_p(dev.data_ptr()), n, n, WINDOW_INF, WINDOW_INF, 1), ex.ctx)
+    ex.sync()
+    at = torch.arange(n, device="cuda")
+    lo, hi = dev[:, :1].long(), dev[:, 1:].long()
+    keep = (at[None] >= lo) & (at[None] < hi)
+    want = torch.softmax(x.double().masked_fill(~keep, -math.inf), 1).nan_to_num(0.0) if n else None
+    got = out[shift:shift + n * n].view(n, n).double()
+    # one rounding to f16, and exponentials of approximate scores (2^-21 of the value)
+    assert ((got - want).abs() <= want * 2.0 ** -10 + 2.0 ** -24).all()
+    assert (got[~keep] == 0).all()
+    assert (out[:shift] == 7).all() and (out[shift + n * n:] == 7).all()
