@@ -171,7 +171,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         const int row0 = tile / tilesN * GBM, col0 = tile % tilesN * BN;
         for (int k = 0; k < nk; k++, it++) {
           const int s = it % G::kStages;
-          if (it >= G::kStages && !mbar_wait(smem_u32(&sEmpty[s]), ((it / G::kStages) - 1) & 1, &sAbort)) {
+          if (it >= G::kStages && !mbar_poll(smem_u32(&sEmpty[s]), ((it / G::kStages) - 1) & 1, &sAbort)) {
             ok = false;
             break;
           }
@@ -184,6 +184,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
             tma_load_2d(dB + c * GBK * 2, &mapB, col0 + c, k * GBK, bar);
         }
       }
+      if (!ok) sAbort = 1;
       grid_launch_dependents();
     }
   } else if (warp == 9) {
@@ -196,10 +197,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
     int it = 0, t = 0;
     for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, t++) {
       const int b = t & 1;
-      if (t >= 2) ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&sAccEmpty[b]), ((t >> 1) - 1) & 1, &sAbort)) != 0;
+      if (t >= 2) ok = mbar_poll_warp(smem_u32(&sAccEmpty[b]), ((t >> 1) - 1) & 1, &sAbort);
       for (int k = 0; k < nk && ok; k++, it++) {
         const int s = it % G::kStages;
-        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&sFull[s]), (it / G::kStages) & 1, &sAbort)) != 0;
+        ok = mbar_poll_warp(smem_u32(&sFull[s]), (it / G::kStages) & 1, &sAbort);
         if (!ok) break;
         tc_fence_after_sync();
         if (elect_one()) {
@@ -217,6 +218,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         __syncwarp();
       }
     }
+    if (!ok) sAbort = 1;
   } else if (warp == 10) {
     // ------------------------------ addend loads ------------------------------
     if (addMode == 1 && elect_one()) {
@@ -225,8 +227,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         const int row0 = tile / tilesN * GBM, col0 = tile % tilesN * BN;
         const int g = t % G::kStagings;
         if (t >= G::kStagings &&
-            !mbar_wait(smem_u32(&sStgFree[g]), ((t / G::kStagings) - 1) & 1, &sAbort))
+            !mbar_poll(smem_u32(&sStgFree[g]), ((t / G::kStagings) - 1) & 1, &sAbort)) {
+          sAbort = 1;
           break;
+        }
         const uint32_t bar = smem_u32(&sAddFull[g]);
         mbar_expect_tx(bar, G::kStaging);
 #pragma unroll
@@ -245,9 +249,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__
         const int c = tid;
         sBias[b][c] = (bias && col0 + c < N) ? __half2float(bias[col0 + c]) : 0.f;
       }
-      bool ok = mbar_wait(smem_u32(&sAccFull[b]), (t >> 1) & 1, &sAbort);
+      bool ok = mbar_poll(smem_u32(&sAccFull[b]), (t >> 1) & 1, &sAbort);
       if (ok && addMode == 1)
-        ok = mbar_wait(smem_u32(&sAddFull[g]), (t / G::kStagings) & 1, &sAbort);
+        ok = mbar_poll(smem_u32(&sAddFull[g]), (t / G::kStagings) & 1, &sAbort);
+      if (!ok) sAbort = 1;
       // (also: this tile's bias is in place, and the store that last used the staging buffer
       // has read it — thread 0 waited for that before it came here)
       if (!readout_all(ok)) break;
@@ -441,6 +446,16 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_con
   tc_fence_after_sync();
   const uint32_t tmem = sTmemBase;
   SK_MARK(1);
+  // The first weights may be asked into the L2 meanwhile, whoever wrote them last ([8, 4096] x [4096, 4096]
+  // 15.9 -> 15.6 us among launches, x [4096, 12288] 19.6 -> 19.2; twice as many steps take the bandwidth
+  // from the grid that is still at work: 17.8 and 23.4).
+  constexpr int kPrefetchSteps = 6;
+  if (warp == 4 && elect_one()) {
+    for (int it = 0; it < min(nk, kPrefetchSteps); it++) {
+      tma_prefetch_2d(&mapB, (int)col0, (it0 + it) * SKK);
+      tma_prefetch_2d(&mapB, (int)col0 + 64, (it0 + it) * SKK);
+    }
+  }
   // Everything above touched no global memory; what follows reads tensors the grid before
   // this one may have written (a, addend) and overwrites out, which it may still read.
   grid_dependency_wait();
@@ -453,8 +468,10 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_con
       prefetch_tensormap(&mapB);
       for (int it = 0; it < nk; it++) {
         const int s = it % SKSTAGES;
-        if (it >= SKSTAGES && !mbar_wait(smem_u32(&sEmpty[s]), ((it / SKSTAGES) - 1) & 1, &sAbort))
+        if (it >= SKSTAGES && !mbar_park(smem_u32(&sEmpty[s]), ((it / SKSTAGES) - 1) & 1, &sAbort)) {
+          sAbort = 1;
           break;
+        }
         const uint32_t bar = smem_u32(&sFull[s]);
         const uint32_t dB = smemBase + s * kSkStage, dA = dB + kSkB;
         const int k0 = (it0 + it) * SKK;
@@ -475,7 +492,7 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_con
     bool ok = true;
     for (int it = 0; it < nk && ok; it++) {
       const int s = it % SKSTAGES;
-      ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&sFull[s]), (it / SKSTAGES) & 1, &sAbort)) != 0;
+      ok = __all_sync(0xffffffffu, mbar_park(smem_u32(&sFull[s]), (it / SKSTAGES) & 1, &sAbort));
       if (!ok) break;
       tc_fence_after_sync();
       if (it == 0) SK_MARK(2);
@@ -496,6 +513,7 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_con
       }
       __syncwarp();
     }
+    if (!ok) sAbort = 1;
   }
 
   // Accumulator of this CTA: thread = column, 16 values = rows of a.
@@ -503,7 +521,8 @@ gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_con
 #pragma unroll
   for (int m = 0; m < SKM; m++) acc[m] = 0.f;
   if (warp < 4 && nk > 0) {
-    const bool ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&sAcc), 0, &sAbort)) != 0;
+    const bool ok = __all_sync(0xffffffffu, mbar_park(smem_u32(&sAcc), 0, &sAbort));
+    if (!ok) sAbort = 1;
     if (ok) {
       tc_fence_after_sync();
       uint32_t raw[SKM];
