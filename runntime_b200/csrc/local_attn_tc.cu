@@ -145,6 +145,7 @@ local_attn_tc_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_cons
                      const float* __restrict__ qScale, __half* __restrict__ out, int64_t rows, int heads,
                      int window, float kScale, float softcap, int* status) {
   using L = Local<HD, WP>;
+  grid_dependency_wait();
   constexpr int NT = (16 + WP) / 8, KS = HD / 16;       // key tiles of a warp, steps of the head
   // Steps that an accumulator adds up before it joins the f32 sum.  (The widest form has no registers for
   // the sums of two: 4 bytes spilled, [9000, 3 x 8 x 128] with a window of 32 4 % slower.)
@@ -440,10 +441,9 @@ cudaError_t launch(const void* qkv, const float* rel, const float* qScale, void*
   // rows once and walks every step-th tile.
   const int64_t tiles = (rows + kRows - 1) / kRows, most = 3 * 148 / heads;
   const int64_t perHead = tiles < most ? tiles : most < 1 ? 1 : most;
-  kern<<<(unsigned)(perHead * heads), kLocalThreads, L::kSmem, s>>>(
-      mq, mkv, static_cast<const __half*>(qkv), rel, qScale, static_cast<__half*>(out), rows, heads, window, kScale,
-      softcap, status);
-  return cudaGetLastError();
+  return launch_dependent(kern, dim3((unsigned)(perHead * heads)), dim3(kLocalThreads), L::kSmem, s, mq, mkv,
+                          static_cast<const __half*>(qkv), rel, qScale, static_cast<__half*>(out), rows, heads, window,
+                          kScale, softcap, status);
 }
 
 }  // namespace

@@ -32,6 +32,7 @@ matmul_f32_tc_kernel(const float* __restrict__ a, const float* __restrict__ b, c
                      const float* __restrict__ addend, float* __restrict__ out, int64_t M, int64_t K, int64_t N,
                      int act) {
   extern __shared__ __align__(16) float ring[];
+  grid_dependency_wait();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t4 = lane & 3;      // fragment row and column
   const int wm = (warp & 1) * 32, wn = (warp >> 1) * 32;
@@ -166,10 +167,9 @@ cudaError_t launch_matmul_f32_tc(const void* a, const void* b, const void* bias,
   cudaError_t e = cudaFuncSetAttribute(matmul_f32_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
   if (e != cudaSuccess) return e;
   const dim3 grid((unsigned)((N + TN - 1) / TN), (unsigned)((M + TM - 1) / TM));
-  matmul_f32_tc_kernel<<<grid, kThreads, kSmem, s>>>(
-      static_cast<const float*>(a), static_cast<const float*>(b), static_cast<const float*>(bias),
-      static_cast<const float*>(addend), static_cast<float*>(out), M, K, N, act);
-  return cudaGetLastError();
+  return launch_dependent(matmul_f32_tc_kernel, grid, dim3(kThreads), kSmem, s, static_cast<const float*>(a),
+                          static_cast<const float*>(b), static_cast<const float*>(bias),
+                          static_cast<const float*>(addend), static_cast<float*>(out), M, K, N, act);
 }
 
 }  // namespace rt

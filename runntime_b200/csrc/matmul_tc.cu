@@ -33,17 +33,6 @@ namespace {
 using namespace sm100;
 using namespace tc;
 
-// Programmatic dependent launch: a grid launched with the stream-serialization attribute
-// may start while the grid before it in the stream drains; grid_dependency_wait() returns
-// once that grid has completed and its writes are visible (at once if there is none);
-// grid_launch_dependents() lets the next such grid start its prologue.
-__device__ __forceinline__ void grid_dependency_wait() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-__device__ __forceinline__ void grid_launch_dependents() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
 constexpr int GBM = 128, GBK = 64;
 constexpr int kReadThreads = 256;                   // two warpgroups, half of a tile's columns each
 constexpr int kGemmThreads = kReadThreads + 96;

@@ -88,6 +88,7 @@ template <int HDP>
 __global__ void __launch_bounds__(kThreads, F32Tc<HDP>::kCtas)
 prefill_f32_tc_kernel(const AttnParams p, int tilesPerSeq) {
   using S = F32Tc<HDP>;
+  grid_dependency_wait();
   extern __shared__ __align__(16) float smem[];
   uint4* sQ = reinterpret_cast<uint4*>(smem);         // [16-column block][row set][hi g, hi g+8, lo g, lo g+8][lane]
   uint4* sP = reinterpret_cast<uint4*>(smem + S::kQ); // [8-key block][row set][hi, lo][lane]
@@ -446,8 +447,7 @@ cudaError_t launch(const AttnParams& p, cudaStream_t s) {
   if (e != cudaSuccess) return e;
   const int64_t perSeq = p.seqStride > 0 ? (p.seqStride + BQ - 1) / BQ : 0;
   const int64_t tiles = p.seqStride > 0 ? p.qLen / p.seqStride * perSeq : (p.qLen + BQ - 1) / BQ;
-  kern<<<(unsigned)(tiles * p.qHeads), kThreads, smem, s>>>(p, (int)perSeq);
-  return cudaGetLastError();
+  return launch_dependent(kern, dim3((unsigned)(tiles * p.qHeads)), dim3(kThreads), smem, s, p, (int)perSeq);
 }
 
 }  // namespace

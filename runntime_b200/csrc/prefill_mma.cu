@@ -80,6 +80,7 @@ prefill_mma_kernel(const AttnParams p, int tilesPerSeq) {
   const __half* __restrict__ k = static_cast<const __half*>(p.k) + (int64_t)kvh * hd;
   const __half* __restrict__ v = static_cast<const __half*>(p.v) + (int64_t)kvh * hd;
 
+  grid_dependency_wait();
   for (int i = tid; i < BQ * W; i += kThreads) {
     const int r = i / W, x = (i % W) * E;
     const bool in = row0 + r < rowEnd && x < hd;
@@ -92,10 +93,15 @@ prefill_mma_kernel(const AttnParams p, int tilesPerSeq) {
     sEnd[tid] = end;
   }
   __syncthreads();
-  int64_t tileLo = INT64_MAX, tileEnd = -1;   // keys some row of the CTA sees
-#pragma unroll 8
-  for (int r = 0; r < BQ; r++)
-    if (sLo[r] <= sEnd[r]) tileLo = min(tileLo, sLo[r]), tileEnd = max(tileEnd, sEnd[r]);
+  int64_t tileLo, tileEnd;   // keys some row of the CTA sees
+  {
+    const bool a = sLo[lane] <= sEnd[lane], b = sLo[lane + 32] <= sEnd[lane + 32];
+    // (key numbers are below 2^30: see prefill_mma_supported)
+    const int first = min(a ? (int)sLo[lane] : INT32_MAX, b ? (int)sLo[lane + 32] : INT32_MAX);
+    const int last = max(a ? (int)sEnd[lane] : -1, b ? (int)sEnd[lane + 32] : -1);
+    tileLo = __reduce_min_sync(0xffffffffu, first);
+    tileEnd = __reduce_max_sync(0xffffffffu, last);
+  }
   const int span = tileEnd >= tileLo ? (int)(tileEnd - tileLo + 1) : 0;   // keys from here on relative to tileLo
   const int tiles = (span + BK - 1) / BK;
   // ... rows g and g + 8 of this warp, and the warp's whole range
@@ -258,8 +264,7 @@ cudaError_t launch(const AttnParams& p, cudaStream_t s) {
   static_assert(kSmem <= 48 * 1024, "no opt-in to more shared memory");
   const int64_t perSeq = p.seqStride > 0 ? (p.seqStride + BQ - 1) / BQ : 0;
   const int64_t tiles = p.seqStride > 0 ? p.qLen / p.seqStride * perSeq : (p.qLen + BQ - 1) / BQ;
-  prefill_mma_kernel<CB><<<(unsigned)(tiles * p.qHeads), kThreads, kSmem, s>>>(p, (int)perSeq);
-  return cudaGetLastError();
+  return launch_dependent(prefill_mma_kernel<CB>, dim3((unsigned)(tiles * p.qHeads)), dim3(kThreads), kSmem, s, p, (int)perSeq);
 }
 
 int piece_bytes(const AttnParams& p) {

@@ -307,6 +307,7 @@ prefill_tc3_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
       }
       fence_barrier_init();
     }
+    grid_dependency_wait();
     int wl, we;
     rows_range(p, row0, lane, wl, we);
     wl = __reduce_min_sync(0xffffffffu, wl);
@@ -365,6 +366,7 @@ prefill_tc3_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
   // the range out for both — warps 0-3 from its own rows, warps 4-7 from the other CTA's.
   const int rowInTile = tid & 127;
   int lo = 1, end = 0;  // empty
+  if (warp < 8 || PAIR) grid_dependency_wait();   // (the producer has waited by itself where it loads before here)
   if (warp < 8) {
     // Q of a narrow head by hand: 16-byte units of the swizzled K-major layout, the head's
     // columns at [shift, shift + hd), zeros beside them and in rows past the end.  A head
@@ -958,13 +960,15 @@ cudaError_t launch3(const AttnParams& p, int* status, cudaStream_t s, std::strin
   cfg.blockDim = dim3(kThreads3);
   cfg.dynamicSmemBytes = C::SMEM;
   cfg.stream = s;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = C::CTAS;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = PAIR ? 1 : 0;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = PAIR ? attr : attr + 1;
+  cfg.numAttrs = PAIR ? 2 : 1;
   e = cudaLaunchKernelEx(&cfg, kern, mq, mk, mv, mo, p, status);
   return e != cudaSuccess ? e : cudaGetLastError();
 }

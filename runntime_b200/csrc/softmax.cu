@@ -75,6 +75,7 @@ template <typename T, bool WARP>
 __global__ void __launch_bounds__(kThreads)
 softmax_quad_kernel(const T* __restrict__ x, T* __restrict__ out, const float* __restrict__ segs,
                int64_t rows, int64_t cols, int64_t wl, int64_t wr) {
+  grid_dependency_wait();
   using Q = Quad<T>;
   using QV = typename Q::type;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -322,6 +323,7 @@ template <typename T, int V>
 __global__ void __launch_bounds__(kThreads, kCtas)
 softmax_cta_kernel(const T* __restrict__ x, T* __restrict__ out, const float* __restrict__ segs, int64_t cols,
                    int64_t wl, int64_t wr) {
+  grid_dependency_wait();
   __shared__ float sM[kThreads / 32], sS[kThreads / 32];
   int64_t lo, hi;
   kept_range(segs, blockIdx.x, cols, wl, wr, lo, hi);
@@ -344,6 +346,7 @@ __global__ void __launch_bounds__(kGroup, 10)
 softmax_group_kernel(const __half* __restrict__ x, __half* __restrict__ out, const float* __restrict__ segs,
                      int64_t cols, int64_t wl, int64_t wr, int groups) {
   using T = __half;
+  grid_dependency_wait();
   __shared__ float sM[2][kGroupRows], sS[2][kGroupRows];
   const bool group = (int)blockIdx.x < groups;
   int64_t row = group ? (int64_t)blockIdx.x * kGroupRows : (int64_t)groups * (kGroupRows - 1) + blockIdx.x;
@@ -375,6 +378,7 @@ template <typename T, bool MASKED>
 __global__ void __launch_bounds__(kThreads)
 softmax_element_kernel(const T* __restrict__ x, T* __restrict__ out, const float* __restrict__ segs, int64_t rows,
                        int64_t cols, int64_t wl, int64_t wr) {
+  grid_dependency_wait();
   const int lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
   if (row >= rows) return;
@@ -398,6 +402,7 @@ template <typename T, int V>
 __global__ void __launch_bounds__(kThreads, kCtas)
 softmax_warp_kernel(const T* __restrict__ x, T* __restrict__ out, const float* __restrict__ segs, int64_t rows,
                     int64_t cols, int64_t wl, int64_t wr) {
+  grid_dependency_wait();
   const int64_t row = (int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
   if (row >= rows) return;
   int64_t lo, hi;
@@ -415,14 +420,13 @@ cudaError_t softmax_chunked(const T* x, T* out, const float* segs, int64_t rows,
   if constexpr (sizeof(T) == 2 && V > 1) {
     if (segs && rows >= kGroupMinRows && cols > kWarpRowCols && cols * 2 <= kGroupRowBytes) {
       const int groups = (int)(rows / 4 * 3 / kGroupRows);
-      softmax_group_kernel<V><<<(unsigned)(rows - (int64_t)groups * (kGroupRows - 1)), kGroup, 0, s>>>(
-          x, out, segs, cols, wl, wr, groups);
-      return cudaGetLastError();
+      return launch_dependent(softmax_group_kernel<V>, dim3((unsigned)(rows - (int64_t)groups * (kGroupRows - 1))),
+                              dim3(kGroup), 0, s, x, out, segs, cols, wl, wr, groups);
     }
   }
-  if (warpRows) softmax_warp_kernel<T, V><<<g, kThreads, 0, s>>>(x, out, segs, rows, cols, wl, wr);
-  else softmax_cta_kernel<T, V><<<g, kThreads, 0, s>>>(x, out, segs, cols, wl, wr);
-  return cudaGetLastError();
+  if (warpRows)
+    return launch_dependent(softmax_warp_kernel<T, V>, dim3(g), dim3(kThreads), 0, s, x, out, segs, rows, cols, wl, wr);
+  return launch_dependent(softmax_cta_kernel<T, V>, dim3(g), dim3(kThreads), 0, s, x, out, segs, cols, wl, wr);
 }
 
 // The widest chunk at whose boundaries x and out agree: 16 bytes unless a caller's own memory
@@ -437,17 +441,15 @@ cudaError_t softmax_typed(const void* x, void* out, const float* segs, int64_t r
     const bool warpRows = cols <= kWarpRowCols;
     const int64_t blocks = warpRows ? (rows + kThreads / 32 - 1) / (kThreads / 32) : rows;
     if (blocks > 0x7fffffffll) return cudaErrorInvalidValue;
-    if (warpRows) softmax_quad_kernel<T, true><<<(unsigned)blocks, kThreads, 0, s>>>(xi, oi, segs, rows, cols, wl, wr);
-    else softmax_quad_kernel<T, false><<<(unsigned)blocks, kThreads, 0, s>>>(xi, oi, segs, rows, cols, wl, wr);
-    return cudaGetLastError();
+    if (warpRows) return launch_dependent(softmax_quad_kernel<T, true>, dim3((unsigned)blocks), dim3(kThreads), 0, s, xi, oi, segs, rows, cols, wl, wr);
+    return launch_dependent(softmax_quad_kernel<T, false>, dim3((unsigned)blocks), dim3(kThreads), 0, s, xi, oi, segs, rows, cols, wl, wr);
   }
   if (cols <= (segs ? kElementCols : kWarpRowCols)) {
     const int64_t blocks = (rows + kThreads / 32 - 1) / (kThreads / 32);
     if (blocks > 0x7fffffffll) return cudaErrorInvalidValue;
     const unsigned g = (unsigned)blocks;
-    if (segs) softmax_element_kernel<T, true><<<g, kThreads, 0, s>>>(xi, oi, segs, rows, cols, wl, wr);
-    else softmax_element_kernel<T, false><<<g, kThreads, 0, s>>>(xi, oi, segs, rows, cols, wl, wr);
-    return cudaGetLastError();
+    if (segs) return launch_dependent(softmax_element_kernel<T, true>, dim3(g), dim3(kThreads), 0, s, xi, oi, segs, rows, cols, wl, wr);
+    return launch_dependent(softmax_element_kernel<T, false>, dim3(g), dim3(kThreads), 0, s, xi, oi, segs, rows, cols, wl, wr);
   }
   const uintptr_t apart = reinterpret_cast<uintptr_t>(x) ^ reinterpret_cast<uintptr_t>(out);
   const bool shortRows = cols < (1ll << 31) - 4096;
