@@ -275,10 +275,13 @@ prefill_tc3_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_consta
   TC_TRACE_DECL
   // Long rows first under a causal mask; the two CTAs of a pair take adjacent row tiles.
   const int cta = PAIR ? (int)cluster_ctarank() : 0;
-  const int unit = (int)(gridDim.x / C::CTAS) - 1 - (int)(blockIdx.x / C::CTAS);
+  // One CTA alone: the query heads that share a kv head are neighbours in the grid, so that a K
+  // or V tile is read from memory once for all of them.
+  const int group = PAIR ? 1 : p.qHeads / p.kvHeads;
+  const int unit = (int)(gridDim.x / (C::CTAS * group)) - 1 - (int)(blockIdx.x / (C::CTAS * group));
   const int qTile = unit * C::CTAS + cta;
   const bool leader = cta == 0;
-  const int h = blockIdx.y;
+  const int h = (int)blockIdx.y * group + (PAIR ? 0 : (int)(blockIdx.x % (unsigned)group));
   const int kvh = h / (p.qHeads / p.kvHeads);
   const int64_t row0 = (int64_t)qTile * BM;
   const int hd = PADDED ? p.hd : HD;
@@ -956,7 +959,8 @@ cudaError_t launch3(const AttnParams& p, int* status, cudaStream_t s, std::strin
   if (e != cudaSuccess) return e;
   const unsigned tiles = (unsigned)((p.qLen + BM - 1) / BM);
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((tiles + C::CTAS - 1) / C::CTAS * C::CTAS, (unsigned)p.qHeads);
+  const unsigned group = PAIR ? 1u : (unsigned)(p.qHeads / p.kvHeads);
+  cfg.gridDim = dim3((tiles + C::CTAS - 1) / C::CTAS * C::CTAS * group, (unsigned)p.qHeads / group);
   cfg.blockDim = dim3(kThreads3);
   cfg.dynamicSmemBytes = C::SMEM;
   cfg.stream = s;
