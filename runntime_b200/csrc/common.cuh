@@ -350,7 +350,7 @@ bool prefill_tc4_supported(const AttnParams& p, int dtype);
 cudaError_t launch_prefill_tc4(const AttnParams& p, int* status, int* work, int smCount,
                                cudaStream_t s, std::string* err);
 // Fills kvPerCta/keySlots/stages/splits/mergeAfter; returns false with a message when the shape cannot run.
-bool plan_decode(DecodeParams& p, int dtype, int smCount, std::string* err);
+bool plan_decode(DecodeParams& p, int dtype, int smCount, std::string* err, bool tensorCores = true);
 cudaError_t launch_decode(const DecodeParams& p, int dtype, cudaStream_t s);
 cudaError_t launch_merge_partials(const float* partials, int parts, int64_t units, int hd,
                                   void* out, int dtype, cudaStream_t s);

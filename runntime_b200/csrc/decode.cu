@@ -1633,7 +1633,7 @@ bool mma_better(const DecodeParams& p, int group) {
 
 }  // namespace
 
-bool plan_decode(DecodeParams& p, int dtype, int smCount, std::string* err) {
+bool plan_decode(DecodeParams& p, int dtype, int smCount, std::string* err, bool tensorCores) {
   const int esize = dtype == RT_F16 ? 2 : 4;
   const int group = p.qHeads / p.kvHeads;
   if (group > kConsumers) {
@@ -1711,7 +1711,7 @@ bool plan_decode(DecodeParams& p, int dtype, int smCount, std::string* err) {
     return of;
   };
   p.mma = 0;
-  if (dtype == RT_F16 && exact_hd(p.hd) && mma_better(p, group)) {
+  if (tensorCores && dtype == RT_F16 && exact_hd(p.hd) && mma_better(p, group)) {
     g = mma_geometry(kSmemBudgetMma);
     p.kvPerCta = g.kvPerCta;
     if (g.fits && bulk_ok(p, esize)) {
@@ -1942,6 +1942,16 @@ int rt_attn_decode_noalloc(const rt_decode_args* a, void* cuda_stream) {
   const size_t fit = kStaticScratchFloats / perSplit;
   if (a->splits == 0 && (size_t)p.splits > fit && fit >= 2) {
     p.splits = (int)fit;   // the plan's own choice: as many as the area holds
+    if (!plan_decode(p, a->dtype, smCount, &err)) return static_fail(RT_INVALID_ARGUMENT, err);
+  }
+  if (a->splits == 0 && p.mma && fit < 2) {
+    // No room for two splits: what runs is what the FP32 kernel would run unsplit, whichever kernel
+    // it then is.  (By their own plan the tensor cores would split, and so refuse, 275 sequences of
+    // 2048 keys with 64 heads of 36 on 32.)
+    DecodeParams simt = p;
+    simt.splits = 0;
+    if (!plan_decode(simt, a->dtype, smCount, &err, false)) return static_fail(RT_INVALID_ARGUMENT, err);
+    p.splits = simt.splits;
     if (!plan_decode(p, a->dtype, smCount, &err)) return static_fail(RT_INVALID_ARGUMENT, err);
   }
   const size_t needFloats = p.splits > 1 ? p.splits * perSplit : 0;

@@ -106,3 +106,34 @@ def test_no_less_precise_than_f32_sums(ex):
         # (a handful of results lie so near the middle of two halves that 24 bits decide either way)
         assert (got[b] != nearest).mean() < 0.01
         assert np.linalg.norm(got[b] - want) <= np.linalg.norm(nearest - want) * 1.01
+
+
+@pytest.mark.parametrize("heads,kv,hd,batch,rows,runs", [
+    (64, 32, 36, 275, 2048, True),    # the FP32 kernel would not split it, the tensor cores would: they take it whole
+    (16, 8, 128, 300, 1000, False),   # both would split it
+    (8, 1, 128, 1024, 8192, False),   # only the FP32 kernel would
+])
+def test_where_the_fixed_scratch_holds_no_splits(heads, kv, hd, batch, rows, runs):
+    import ctypes as C
+    import torch
+    import runntime_b200._lib as L
+    lib = L.load()
+    s = _state(heads, kv, hd, rows, 1)
+    g = torch.Generator(device=s["q"].device).manual_seed(3)
+    q = (torch.randn(batch, heads * hd, generator=g, device=s["q"].device) * hd ** -0.5).half()
+    out = torch.full_like(q, 9.0)
+    k, v = (torch.full((batch,), s[x].data_ptr(), dtype=torch.int64, device=q.device) for x in "kv")   # one cache for all
+    a = L.DecodeArgs()
+    a.q, a.out, a.kCachePtrs, a.vCachePtrs = q.data_ptr(), out.data_ptr(), k.data_ptr(), v.data_ptr()
+    a.dtype, a.batch, a.cacheRows, a.kvLen = L.DTYPE_CODE["f16"], batch, rows, rows
+    a.qHeads, a.kvHeads, a.headDim, a.windowLeft = heads, kv, hd, L.WINDOW_INF
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    assert lib.rt_attn_decode_noalloc(C.byref(a), stream) == (0 if runs else 6)   # 6: INVALID_ARGUMENT
+    assert lib.rt_attn_decode_noalloc_status(stream) == 0
+    if not runs:
+        assert (out == 9.0).all()
+        return
+    for b in (0, batch - 1):
+        want = sdpa_ref(q[b:b + 1].float().cpu().numpy(), s["k"][0].float().cpu().numpy(), s["v"][0].float().cpu().numpy(),
+                        qHeads=heads, kvHeads=kv, headDim=hd, qPosOffset=rows - 1, windowRight=0)
+        oracle.assert_close(out[b].float().cpu().numpy(), want.reshape(-1), "f16", f"sequence {b}")
