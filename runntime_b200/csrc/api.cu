@@ -246,7 +246,14 @@ int run_decode(rt_ctx* ctx, rt::DecodeParams& p, int dtype) {
   if (p.splits > 1) {
     const size_t sets = p.hasSecond ? 2 : 1;   // a second attention has its own partials and counters
     const size_t perSplit = sets * p.batch * p.qHeads * (2 + p.hd) * sizeof(float);
-    const size_t counters = sets * p.batch * ((p.kvHeads + p.kvPerCta - 1) / p.kvPerCta);
+    size_t counters = sets * p.batch * ((p.kvHeads + p.kvPerCta - 1) / p.kvPerCta);
+    if (!chosen && p.mma && counters > ctx->counterCount && capturing(ctx->stream)) {
+      // The tensor cores' blocks hold fewer heads and so need more counters, which cannot be made
+      // under a capture: the FP32 kernel takes the call.
+      if (!rt::plan_decode(p, dtype, ctx->smCount, &err, false))
+        return fail(ctx, RT_INVALID_ARGUMENT, "%s", err.c_str());
+      counters = sets * p.batch * ((p.kvHeads + p.kvPerCta - 1) / p.kvPerCta);
+    }
     const bool grows = p.splits * perSplit > ctx->scratchBytes || counters > ctx->counterCount;
     if (chosen && grows && capturing(ctx->stream)) {
       // Nothing can be allocated under a capture: as many splits as the scratch at hand holds.

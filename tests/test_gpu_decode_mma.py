@@ -137,3 +137,37 @@ def test_where_the_fixed_scratch_holds_no_splits(heads, kv, hd, batch, rows, run
         want = sdpa_ref(q[b:b + 1].float().cpu().numpy(), s["k"][0].float().cpu().numpy(), s["v"][0].float().cpu().numpy(),
                         qHeads=heads, kvHeads=kv, headDim=hd, qPosOffset=rows - 1, windowRight=0)
         oracle.assert_close(out[b].float().cpu().numpy(), want.reshape(-1), "f16", f"sequence {b}")
+
+
+def test_given_splits_under_capture_with_the_other_kernels_counters():
+    """32 heads of 128 are one block of the FP32 kernel and four of this one: a context warmed by the
+    former has counters for too few of the latter, and none can be made under a capture."""
+    import torch
+    import runntime_b200 as rt
+    heads, hd, rows, batch = 32, 128, 200, 4
+    s = _state(heads, heads, hd, rows, batch)
+    ex = rt.CudaExecutor(0)
+    lens = torch.tensor([200, 1, 130, 64], dtype=torch.int32, device=s["q"].device)
+    out = torch.empty_like(s["q"])
+    from runntime_b200.engine import decode_batched
+    kw = dict(batch=batch, cacheRows=rows, qHeads=heads, kvHeads=heads, headDim=hd, kvLen=rows, kvLens=lens, splits=3)
+    stream = torch.cuda.Stream()
+    try:
+        ex.setStream(stream.cuda_stream)
+        f = {x: s[x].float() for x in ("q", "k", "v")}
+        torch.cuda.synchronize()
+        decode_batched(ex, f["q"], torch.empty_like(f["q"]), f["k"], f["v"], dtype="f32", **kw)
+        ex.sync()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            decode_batched(ex, s["q"], out, s["k"], s["v"], dtype="f16", **kw)
+        graph.replay()
+        torch.cuda.synchronize()
+        for b, n in enumerate(lens.tolist()):
+            want = sdpa_ref(s["q"][b:b + 1].float().cpu().numpy(), s["k"][b, :n].float().cpu().numpy(),
+                            s["v"][b, :n].float().cpu().numpy(), qHeads=heads, kvHeads=heads, headDim=hd,
+                            qPosOffset=n - 1, windowRight=0)
+            oracle.assert_close(out[b].float().cpu().numpy(), want.reshape(-1), "f16", f"length {n}")
+        del graph
+    finally:
+        ex.dispose()
