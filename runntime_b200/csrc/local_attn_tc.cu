@@ -28,8 +28,8 @@
 // What bounds it: instructions, about 2 000 per warp and 16 rows, at 12 warps per SM (issue slots 46 %
 // busy, DRAM 40 %).
 // [32769, 3 x 8 x 128], window 12: 528 us for one warp per row on the FP32 pipes (local_attn.cu), 98 us
-// with the soft cap on the scores' own fragments and the bias rows split for every tile, 74 us; the
-// slab and the output at the copy rate are 40 us.
+// with the soft cap on the scores' own fragments and the bias rows split for every tile, 74 us (73
+// as a dependent launch); the slab and the output at the copy rate are 40 us.
 #include "common.cuh"
 #include "sm100.cuh"
 #include "tc_common.cuh"

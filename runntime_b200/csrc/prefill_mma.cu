@@ -11,7 +11,8 @@
 // three key tiles, so the kernel is the latency of one CTA's chain (loads, MMA, tensor memory, softmax,
 // MMA, read-out), most of a 128 x 128 tile of packed segments is masked, and half of its 64
 // columns are padding.  Here four CTAs per SM overlap their chains and a 16-row warp skips what it
-// does not see.  32 paragraphs of 16..256 tokens, 12 heads of 32: 33.9 us there, 20.6 here.
+// does not see.  32 paragraphs of 16..256 tokens, 12 heads of 32: 33.9 us there, 20.6 here
+// when this was written; among other launches 24.7, and 19.4 as a dependent launch whose key range is one redux.
 // What bounds it: the exponentials and the fragments' way through shared memory, at 16 warps per SM.
 #include "common.cuh"
 #include "sm100.cuh"

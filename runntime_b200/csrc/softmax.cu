@@ -5,7 +5,7 @@
 // packages/runntime/src/core/kernels/reduce/softmax.ts:111-186).
 //
 // HBM-bound: one read of the kept scores and one write of the row.  A row is handled by one
-// warp (narrow rows, eight per CTA) or by one CTA; the first pass keeps a running (max, sum) per
+// warp (narrow rows, eight per CTA), by one CTA, or with three others (softmax_group_kernel); the first pass keeps a running (max, sum) per
 // thread, the second re-reads the row (it is in L1/L2 by then) and writes exp(x - max) / sum.
 //
 // Rows that start on four elements are taken four at a time.  Any other row begins in the middle of
@@ -13,7 +13,7 @@
 // first and last chunk go element by element, and the zeros outside the kept range, which need no
 // statistics, are stored while the first scores are on their way.  Element by element, chunks, us: f16
 // [6007, 6007] with 24 segments (75 MB, 11 us at the copy rate) 55.5, 20.8 (55.3, 24.6 through the
-// operator), with one 74.6, 71.9; f32
+// operator; 17.2 with four rows to a CTA and as a dependent launch), with one 74.6, 71.9; f32
 // 51.4, 31.0 with 24.  On aligned rows the quads are the faster ones: f16 [12288, 12288] with 2
 // segments 119 against 141, [2500, 2500] with 3 12.4 against 18.7.
 #include "common.cuh"
