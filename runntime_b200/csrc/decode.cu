@@ -524,21 +524,22 @@ decode_kernel(const DecodeParams p) {
     end = p.end;
   } else {
     Lg = L = aLens ? aLens[b] : aKvLen;
-    if (p.kvSharded) {
+    if (misaligned || (!p.kvSharded && L > aCacheRows)) {
+      // A length past the cache's capacity (the host checks only the scalar kvLen; this one
+      // lives on the device): writeRows would refuse it ('rows exceed dst capacity').  The
+      // sequence is treated as empty — nothing appended, nothing read, zeros out — and the
+      // status word reports it.  The same for a cache pointer the bulk copies cannot take,
+      // whether the cache holds the whole sequence or a shard of it.
+      if (tid == 0) atomicOr(p.status, kStatusBadState);
+      Lg = L = 0;
+      hasNew = false;
+    } else if (p.kvSharded) {
       // This cache holds rows [shardStart, shardStart + cacheRows) of the sequence: it sees
       // what falls inside, and takes the appended row (global row Lg-1) only if that is one
       // of its own.
       const int64_t local = Lg - p.shardStart;
       hasNew = hasNew && local >= 1 && local <= p.cacheRows;
       L = local < 0 ? 0 : local > p.cacheRows ? p.cacheRows : local;
-    } else if (L > aCacheRows || misaligned) {
-      // A length past the cache's capacity (the host checks only the scalar kvLen; this one
-      // lives on the device): writeRows would refuse it ('rows exceed dst capacity').  The
-      // sequence is treated as empty — nothing appended, nothing read, zeros out — and the
-      // status word reports it.  The same for a cache pointer the bulk copies cannot take.
-      if (tid == 0) atomicOr(p.status, kStatusBadState);
-      Lg = L = 0;
-      hasNew = false;
     }
     end = L - 1;
     lo = Lg - 1 - aWl - p.shardStart;
@@ -1194,14 +1195,14 @@ __global__ void __launch_bounds__(kConsumers + 32, HD <= 64 ? 2 : 1) decode_mma_
     end = p.end;
   } else {
     Lg = L = lens ? lens[b] : sec ? p.s2.kvLen : p.kvLen;
-    if (p.kvSharded) {
-      const int64_t local = Lg - p.shardStart;
-      hasNew = hasNew && local >= 1 && local <= p.cacheRows;
-      L = local < 0 ? 0 : local > p.cacheRows ? p.cacheRows : local;
-    } else if (L > (sec ? p.s2.cacheRows : p.cacheRows) || misaligned) {
+    if (misaligned || (!p.kvSharded && L > (sec ? p.s2.cacheRows : p.cacheRows))) {
       if (tid == 0) atomicOr(p.status, kStatusBadState);
       Lg = L = 0;
       hasNew = false;
+    } else if (p.kvSharded) {
+      const int64_t local = Lg - p.shardStart;
+      hasNew = hasNew && local >= 1 && local <= p.cacheRows;
+      L = local < 0 ? 0 : local > p.cacheRows ? p.cacheRows : local;
     }
     end = L - 1;
     lo = Lg - 1 - (sec ? p.s2.wl : p.wl) - p.shardStart;

@@ -279,6 +279,52 @@ def test_caches_allocated_one_by_one(ex, heads, hd):
         ex.setStream(None)
 
 
+@pytest.mark.parametrize("heads,kvHeads,hd,dtype", [(16, 8, 64, "f16"), (9, 9, 36, "f32"), (9, 9, 128, "f16")])
+@pytest.mark.parametrize("splits", [1, 2])
+def test_a_shard_that_does_not_start_on_16_bytes(ex, heads, kvHeads, hd, dtype, splits):
+    """Shards allocated one by one, one of them one element off: its sequence comes out as having no
+    key, takes no row, and the status says so (tensor-core kernel and FP32 kernel)."""
+    import torch
+    import runntime_b200 as rt
+    from runntime_b200.engine import decode_batched
+    batch, rows, start, lens = 3, 96, 64, [160, 130, 100]      # the shard: rows 64..159
+    dev, td = torch.device("cuda", 0), torch.float16 if dtype == "f16" else torch.float32
+    g = torch.Generator(device=dev).manual_seed(hd)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=dev).to(td)  # noqa: E731
+    q, kn, vn = rnd(batch, heads * hd) * hd ** -0.5, rnd(batch, kvHeads * hd), rnd(batch, kvHeads * hd)
+    size = rows * kvHeads * hd
+    ks, vs = ([rnd(size + 8) for _ in range(batch)] for _ in range(2))
+    kept = [t.clone() for t in ks + vs]
+    ld = torch.tensor(lens, dtype=torch.int32, device=dev)
+
+    def run(offK, offV):
+        for t, old in zip(ks + vs, kept):
+            t.copy_(old)
+        at = lambda ts, off: torch.tensor([t.data_ptr() + (off * t.element_size() if b == 1 else 0)  # noqa: E731
+                                           for b, t in enumerate(ts)], dtype=torch.int64, device=dev)
+        part = torch.full((batch, heads, 2 + hd), 7.0, device=dev)
+        decode_batched(ex, q, None, None, None, dtype=dtype, batch=batch, cacheRows=rows, qHeads=heads,
+                       kvHeads=kvHeads, headDim=hd, kvLen=max(lens), kvLens=ld, kNew=kn, vNew=vn,
+                       kCachePtrs=at(ks, offK), vCachePtrs=at(vs, offV), partialsOut=part, kvSharded=True,
+                       shardStart=start, splits=splits)
+        return part
+
+    ex.setStream(torch.cuda.current_stream().cuda_stream)
+    try:
+        good = run(0, 0)
+        ex.sync()
+        assert (good[:, :, 1] > 0).all()
+        for offs in ((1, 0), (0, 1)):
+            part = run(*offs)
+            with pytest.raises(rt.RunntimeError, match="not 16-byte aligned"):
+                ex.sync()
+            assert (part[1, :, 1:] == 0).all()
+            assert torch.equal(part[::2], good[::2])
+            assert torch.equal(ks[1], kept[1]) and torch.equal(vs[1], kept[batch + 1])   # nothing appended
+    finally:
+        ex.setStream(None)
+
+
 def test_batched_cross_attention_and_window(ex):
     import torch
     from runntime_b200.engine import decode_batched
