@@ -964,15 +964,27 @@ decode_kernel(const DecodeParams p) {
 // ---- f16 on the tensor cores -------------------------------------------------------------
 // A warp takes one kv head and 16 or 32 keys of the tile at a time: S = q K^T with the (up to
 // eight) query heads of the kv head as the rows of an m16n8k16 and the keys as its columns, then
-// O = P V with S's fragments as the A operand.  P is held in two halves, p = hi + lo, as rows g and
-// g + 8 of that operand (22 bits; scaled by 2^12 so that small probabilities keep theirs), and
-// the accumulators are emptied into f32 sums every 32 columns and every 16 or 32 keys, so nothing
-// is rounded more than on the FP32 pipes.  The order of a contraction is free, so a thread's
+// O = P V with S's fragments as the A operand.  The order of a contraction is free, so a thread's
 // operands are 8 or 16 contiguous bytes of a key's row: columns for the scores, key pairs (by
 // byte permutes) for the output.
+// The tensor core adds f32 sums up by cutting off what an FMA would round, so little is left to it:
+//   - q is split in two (rows g and g + 8), and no more than 16 columns go into one accumulator;
+//   - a probability, p = exp(s - m) in f32 as on the FP32 pipes, is scaled by a power of two to the top of
+//     a half's range and held as hi + lo (rows g and g + 8 again), 22 to 24 bits of it; the scale is
+//     the block of keys' own, and what is smaller than its largest one by 2^28 or more waits for another pass,
+//     so small ones keep as many bits as large ones;
+//   - no more than 16 keys go into one accumulator, the rest is f32;
+//   - a sink joins the sums at their end, so that a dominating one takes no bits from the keys.
+// Error of the f32 partials (2-norm, against 64 bits; the FP32 pipes / here): 32 heads of 128 on 8, 50 / 487 /
+// 4000 keys 1.9 / 4.8 / 13 e-7 and 1.4 / 2.0 / 3.8 e-7, scores four times as steep 3.2 / 6.2 / 18 and
+// 2.3 / 3.7 / 6.1, a sink of e^20 4.5 / 15 / 76 and 4.6 / 5.2 / 6.2; the log of the sum within the same
+// few e-7 of both.  What stays larger: all-positive values of heads of 36 or 52, four on each of 8 kv heads, over
+// 4000 keys (2.0 and 2.4), whose keys the other kernel deals out to more threads.
 // What bounds the FP32-pipe form with several query heads per kv head is that every key is read
 // and converted once per query head, by two warps per scheduler: 16 sequences of 2000 keys, 32
-// heads of 128 on 8, took 103 us at 1.3 TB/s; here 36 (mma_better has more of both sides).
+// heads of 128 on 8, take 75.9 us among launches; here 34.9 (mma_better has more of both sides).  This form
+// is bound by its instructions at heads of up to 64 (96 registers a thread, so that nine warps fit
+// twice per SM, spill 64 to 84 bytes a thread), and by the copies above.
 template <int HD>
 struct Mma {
   static constexpr int VEC = HD % 8 == 0 ? 8 : 4;               // halves per load
@@ -981,7 +993,10 @@ struct Mma {
   static constexpr int NB = HD <= 64 ? 2 : 1;                   // blocks of 16 keys at a time
   static constexpr int KEYS = 16 * NB;
 };
-constexpr float kPScale = 4096.f, kPScaleLog2 = 12.f;
+// A probability in two halves: p * 2^e rounded, between 2^-14 (the least normal half) and 2^kPTop, and what
+// that left of it times kPLow.
+constexpr int kPTop = 14;
+constexpr float kPLeast = 1.f / 16384, kPLow = 4096.f;
 
 __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                           uint32_t b0, uint32_t b1) {
@@ -1008,23 +1023,44 @@ __device__ __forceinline__ void load_words(const __half* p, bool there, uint32_t
   }
 }
 
-// A thread's part of q: row g of the A operand, the columns its K loads will cover.
+// A thread's part of q, the columns its K loads will cover.  An element's upper six bits go to row g of
+// the A operand and the other five to row g + 8, so that products of 17 and 16 bits are what the tensor
+// core adds up and cuts off.  Heads of 128 hold both (8 sequences of 8000 keys, 8 heads of 128 on one: 54.4
+// us split at each use, 52.5); narrower ones have no registers for that (64 x 8000, 8 of 52 on 2 56.9
+// held, 53.9).
 template <int HD>
-__device__ __forceinline__ void mma_query(const __half* q, bool there, int t, uint32_t (&qa)[Mma<HD>::STEPS][2]) {
-  constexpr int VEC = Mma<HD>::VEC;
+struct MmaQuery {
+  static constexpr bool HELD = HD > 64;
+  uint32_t upper[Mma<HD>::STEPS][2], lower[HELD ? Mma<HD>::STEPS : 1][2];
+  static __device__ __forceinline__ uint32_t high(uint32_t q) { return q & 0xffe0ffe0u; }
+  static __device__ __forceinline__ uint32_t rest(uint32_t q) {
+    const uint32_t h = high(q);
+    const __half2 d = __hsub2(*reinterpret_cast<const __half2*>(&q), *reinterpret_cast<const __half2*>(&h));
+    return *reinterpret_cast<const uint32_t*>(&d);
+  }
+  __device__ __forceinline__ MmaQuery(const __half* q, bool there, int t) {
+    constexpr int VEC = Mma<HD>::VEC;
 #pragma unroll
-  for (int st = 0; st < Mma<HD>::STEPS; st++)
+    for (int st = 0; st < Mma<HD>::STEPS; st++)
 #pragma unroll
-    for (int r = 0; r < 2; r++) {
-      const int col = VEC == 8 ? 32 * (st >> 1) + 8 * t + 4 * (st & 1) + 2 * r : 16 * st + 4 * t + 2 * r;
-      qa[st][r] = there && col < HD ? *reinterpret_cast<const uint32_t*>(q + col) : 0u;
-    }
-}
+      for (int r = 0; r < 2; r++) {
+        const int col = VEC == 8 ? 32 * (st >> 1) + 8 * t + 4 * (st & 1) + 2 * r : 16 * st + 4 * t + 2 * r;
+        const uint32_t v = there && col < HD ? *reinterpret_cast<const uint32_t*>(q + col) : 0u;
+        upper[st][r] = HELD ? high(v) : v;
+        if constexpr (HELD) lower[st][r] = rest(v);
+      }
+  }
+  __device__ __forceinline__ uint32_t up(int st, int r) const { return HELD ? upper[st][r] : high(upper[st][r]); }
+  __device__ __forceinline__ uint32_t low(int st, int r) const {
+    if constexpr (HELD) return lower[st][r];
+    else return rest(upper[st][r]);
+  }
+};
 
 // KEYS keys from k and v on, `pitch` elements apart, of which the first nk count.
 template <int HD>
 __device__ __forceinline__ void mma_keys(const __half* k, const __half* v, int pitch, int nk, int g, int t,
-                                         const uint32_t (&qa)[Mma<HD>::STEPS][2], float& m, float& l,
+                                         const MmaQuery<HD>& qa, float& m, float& l,
                                          float (&o)[Mma<HD>::CHUNKS][Mma<HD>::VEC][2]) {
   using C = Mma<HD>;
   constexpr int VEC = C::VEC, NB = C::NB, PER = VEC / 4;   // steps per load
@@ -1032,20 +1068,22 @@ __device__ __forceinline__ void mma_keys(const __half* k, const __half* v, int p
 #pragma unroll
   for (int i = 0; i < 2 * NB; i++) {
     const __half* row = k + (8 * i + g) * pitch + VEC * t;
-    sc[i][0] = sc[i][1] = 0.f;
+    float part[4][2] = {};   // of 32 columns each
 #pragma unroll
-    for (int st = 0; st < C::STEPS; st += 2) {
-      float c[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int st = 0; st < C::STEPS; st += PER) {
+      uint32_t w[VEC / 2];
+      load_words<VEC>(row + 16 * st, VEC == 8 || 16 * st + 4 * t < HD, w);
 #pragma unroll
-      for (int u = st; u < st + 2 && u < C::STEPS; u += PER) {
-        uint32_t w[VEC / 2];
-        load_words<VEC>(row + 16 * u, VEC == 8 || 16 * u + 4 * t < HD, w);
-#pragma unroll
-        for (int e = 0; e < PER; e++) mma_16816(c, qa[u + e][0], 0u, qa[u + e][1], 0u, w[2 * e], w[2 * e + 1]);
+      for (int e = 0; e < PER; e++) {
+        float c[4] = {0.f, 0.f, 0.f, 0.f};
+        mma_16816(c, qa.up(st + e, 0), qa.low(st + e, 0), qa.up(st + e, 1), qa.low(st + e, 1), w[2 * e], w[2 * e + 1]);
+        part[(st + e) / 2][0] += c[0] + c[2];
+        part[(st + e) / 2][1] += c[1] + c[3];
       }
-      sc[i][0] += c[0];
-      sc[i][1] += c[1];
     }
+#pragma unroll
+    for (int e = 0; e < 2; e++)
+      sc[i][e] = C::STEPS > 4 ? (part[0][e] + part[1][e]) + (part[2][e] + part[3][e]) : part[0][e] + part[1][e];
   }
   // this thread: head g, keys 8 i + 2 t and + 1
   float mx = -INFINITY;
@@ -1058,41 +1096,68 @@ __device__ __forceinline__ void mma_keys(const __half* k, const __half* v, int p
     }
   mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
   mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-  const float top = fmaxf(m, mx * kLog2e), alpha = fast_exp2(m - top), base = kPScaleLog2 - top;
+  mx *= kLog2e;
+  const float top = fmaxf(m, mx);
+  float alpha = fast_exp2(m - top);
   m = top;
   l *= alpha;
-  uint32_t hi[2 * NB], lo[2 * NB];
 #pragma unroll
   for (int i = 0; i < 2 * NB; i++) {
-    const float p0 = fast_exp2(fmaf(sc[i][0], kLog2e, base)), p1 = fast_exp2(fmaf(sc[i][1], kLog2e, base));
-    l += p0 + p1;
-    const __half2 h = __floats2half2_rn(p0, p1);
-    const float2 f = __half22float2(h);
-    const __half2 r = __floats2half2_rn(p0 - f.x, p1 - f.y);
-    hi[i] = *reinterpret_cast<const uint32_t*>(&h);
-    lo[i] = *reinterpret_cast<const uint32_t*>(&r);
+    sc[i][0] = fast_exp2(fmaf(sc[i][0], kLog2e, -top)), sc[i][1] = fast_exp2(fmaf(sc[i][1], kLog2e, -top));
+    l += sc[i][0] + sc[i][1];
   }
+  // The largest of these probabilities goes to the top of a half's range; those that would be below its
+  // normal numbers wait for another pass, 28 powers of two further down.
+  int at = kPTop + (int)fminf(top - mx, 100.f);
+  for (bool more = true; more; alpha = 1.f) {
+    const float up = __int_as_float((at + 127) << 23), down = __int_as_float((127 - at) << 23);
+    uint32_t hi[2 * NB], lo[2 * NB];
+    bool small = false;
 #pragma unroll
-  for (int c = 0; c < C::CHUNKS; c++) {
-    const int col = c * 8 * VEC + VEC * g;
-    uint32_t w[NB][4][VEC / 2];
+    for (int i = 0; i < 2 * NB; i++) {
+      float y[2];
 #pragma unroll
-    for (int b = 0; b < NB; b++)
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const int key = 16 * b + 2 * t + (j & 1) + 8 * (j >> 1);
-        load_words<VEC>(v + key * pitch + col, key < nk && (HD % (8 * VEC) == 0 || col < HD), w[b][j]);
+      for (int e = 0; e < 2; e++) {
+        const float x = sc[i][e] * up;
+        const bool later = __float_as_uint(x) - 1u < __float_as_uint(kPLeast) - 1u;   // 0 < x < kPLeast
+        small |= later;
+        y[e] = later ? 0.f : x;
+        sc[i][e] = later ? sc[i][e] : 0.f;
       }
+      const __half2 h = __floats2half2_rn(y[0], y[1]);
+      const float2 f = __half22float2(h);
+      const __half2 r = __floats2half2_rn((y[0] - f.x) * kPLow, (y[1] - f.y) * kPLow);
+      hi[i] = *reinterpret_cast<const uint32_t*>(&h);
+      lo[i] = *reinterpret_cast<const uint32_t*>(&r);
+    }
+    more = __any_sync(0xffffffffu, small && at < 126);   // (the same in all lanes: at most five passes)
+    at = min(at + 28, 126);
 #pragma unroll
-    for (int e = 0; e < VEC; e++) {
-      float d[4] = {0.f, 0.f, 0.f, 0.f};
-      const uint32_t sel = e & 1 ? 0x7632u : 0x5410u;
+    for (int c = 0; c < C::CHUNKS; c++) {
+      const int col = c * 8 * VEC + VEC * g;
+      uint32_t w[NB][4][VEC / 2];
 #pragma unroll
       for (int b = 0; b < NB; b++)
-        mma_16816(d, hi[2 * b], lo[2 * b], hi[2 * b + 1], lo[2 * b + 1],
-                  __byte_perm(w[b][0][e / 2], w[b][1][e / 2], sel), __byte_perm(w[b][2][e / 2], w[b][3][e / 2], sel));
-      o[c][e][0] = fmaf(o[c][e][0], alpha, d[0] + d[2]);
-      o[c][e][1] = fmaf(o[c][e][1], alpha, d[1] + d[3]);
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          const int key = 16 * b + 2 * t + (j & 1) + 8 * (j >> 1);
+          load_words<VEC>(v + key * pitch + col, key < nk && (HD % (8 * VEC) == 0 || col < HD), w[b][j]);
+        }
+#pragma unroll
+      for (int e = 0; e < VEC; e++) {
+        const uint32_t sel = e & 1 ? 0x7632u : 0x5410u;
+        float x0 = 0.f, x1 = 0.f;
+#pragma unroll
+        for (int b = 0; b < NB; b++) {
+          float d[4] = {0.f, 0.f, 0.f, 0.f};
+          mma_16816(d, hi[2 * b], lo[2 * b], hi[2 * b + 1], lo[2 * b + 1],
+                    __byte_perm(w[b][0][e / 2], w[b][1][e / 2], sel), __byte_perm(w[b][2][e / 2], w[b][3][e / 2], sel));
+          x0 += fmaf(d[2], 1.f / kPLow, d[0]);
+          x1 += fmaf(d[3], 1.f / kPLow, d[1]);
+        }
+        o[c][e][0] = fmaf(o[c][e][0], alpha, x0 * down);
+        o[c][e][1] = fmaf(o[c][e][1], alpha, x1 * down);
+      }
     }
   }
 }
@@ -1320,17 +1385,12 @@ __global__ void __launch_bounds__(kConsumers + 32, HD <= 64 ? 2 : 1) decode_mma_
   const int kvl = (tid >> 5) % p.kvPerCta, slot = (tid >> 5) / p.kvPerCta, slots = kConsumerWarps / p.kvPerCta;
   const bool sink = slot == 0 && split == 0 && p.sinks, append = appendHere && slot == 0;
   const int64_t newRow = (L - 1) * rowElems + kvl * HD;
-  uint32_t qa[M::STEPS][2];
-  mma_query<HD>(sQ + (kvl * group + g) * HD, g < group, t, qa);
+  const MmaQuery<HD> qa(sQ + (kvl * group + g) * HD, g < group, t);
   float m = kNegSeed, l = 0.f, o[M::CHUNKS][M::VEC][2];
 #pragma unroll
   for (int c = 0; c < M::CHUNKS; c++)
 #pragma unroll
     for (int e = 0; e < M::VEC; e++) o[c][e][0] = o[c][e][1] = 0.f;
-  if (sink && g < group) {
-    m = p.sinks[(kvh0 + kvl) * group + g];   // log2-space: sink * ln2 * log2e
-    l = t == 0 ? kPScale : 0.f;              // (a head's sum is spread over the four threads of a row)
-  }
   bool ok = true;
   for (int it = 0; it < ntiles; it++) {
     const int s = it % stages;
@@ -1348,6 +1408,18 @@ __global__ void __launch_bounds__(kConsumers + 32, HD <= 64 ? 2 : 1) decode_mma_
   // (this block has streamed its keys: the next kernel's blocks may take the freed slots)
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (append && ok) mma_keys<HD>(kBase + newRow, vBase + newRow, 0, 1, g, t, qa, m, l, o);
+  // A sink joins the finished sums: as the first reference point a dominating one would leave the
+  // probabilities no bits.
+  if (sink && g < group) {
+    const float x = p.sinks[(kvh0 + kvl) * group + g];   // log2-space: sink * ln2 * log2e
+    const float top = m > x ? m : x, f = fast_exp2(m - top);   // (a NaN stays one)
+    l = l * f + (t == 0 ? fast_exp2(x - top) : 0.f);     // (a head's sum is spread over the four threads of a row)
+    m = top;
+#pragma unroll
+    for (int c = 0; c < M::CHUNKS; c++)
+#pragma unroll
+      for (int e = 0; e < M::VEC; e++) o[c][e][0] *= f, o[c][e][1] *= f;
+  }
 
   // Whether a wait ran out is decided once for the whole block.
   named_barrier_sync(1, kConsumers);
@@ -1403,7 +1475,7 @@ __global__ void __launch_bounds__(kConsumers + 32, HD <= 64 ? 2 : 1) decode_mma_
     }
   } else if (g < group) {
     const int hh = kvl * group + g;
-    const float top = top_of(hh), w = fast_exp2(m - top) * (1.f / kPScale);
+    const float top = top_of(hh), w = fast_exp2(m - top);
     float* r = sM + (slot * hq + hh) * MS;
     if (t == 0) r[0] = l * w;
 #pragma unroll

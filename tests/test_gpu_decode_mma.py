@@ -13,7 +13,8 @@ pytestmark = pytest.mark.gpu
 
 # (query heads, kv heads, head size): one warp per kv head, two, four and eight; head blocks;
 # the largest group; one query head each
-SHAPES = [(16, 8, 36), (8, 4, 52), (6, 2, 64), (8, 1, 128), (64, 8, 128), (32, 16, 128), (32, 32, 128), (24, 24, 128)]
+SHAPES = [(16, 8, 36), (8, 4, 52), (6, 2, 64), (8, 1, 128), (64, 8, 128), (32, 16, 128), (32, 32, 128), (24, 24, 128),
+          (32, 8, 36), (16, 2, 36), (64, 8, 52), (5, 1, 52), (56, 8, 64)]
 LENS = [1, 2, 15, 16, 17, 31, 33, 64, 65, 127, 130, 300]
 
 
@@ -66,7 +67,7 @@ def test_against_oracle(ex, heads, kv, hd, splits, append, sinks, window):
         oracle.assert_close(got[b], want.reshape(-1), "f16", f"length {n}")
 
 
-@pytest.mark.parametrize("heads,kv,hd", [(16, 8, 36), (8, 2, 64), (32, 8, 128), (32, 32, 128)])
+@pytest.mark.parametrize("heads,kv,hd", [(16, 8, 36), (8, 2, 64), (32, 8, 128), (32, 32, 128), (8, 2, 36), (32, 4, 52)])
 @pytest.mark.parametrize("splits", [1, 2])
 def test_infinities_and_nan_stay_where_they_are(ex, heads, kv, hd, splits):
     """Infinite values give infinite columns of their own head, whatever half of a probability they
@@ -106,6 +107,114 @@ def test_no_less_precise_than_f32_sums(ex):
         # (a handful of results lie so near the middle of two halves that 24 bits decide either way)
         assert (got[b] != nearest).mean() < 0.01
         assert np.linalg.norm(got[b] - want) <= np.linalg.norm(nearest - want) * 1.01
+
+
+def _partials(ex, q, k, v, kv, group, hd, sinks, **opts):
+    import torch
+    from runntime_b200.engine import decode_batched
+    batch, rows = k.shape[:2]
+    part = torch.empty(batch, kv * group, 2 + hd, device=k.device)
+    ex.setStream(torch.cuda.current_stream().cuda_stream)
+    try:
+        decode_batched(ex, q.reshape(batch, -1).contiguous(), None, k.reshape(batch, rows, -1).contiguous(),
+                       v.reshape(batch, rows, -1).contiguous(), dtype="f16", batch=batch, cacheRows=rows,
+                       qHeads=kv * group, kvHeads=kv, headDim=hd, kvLen=rows, partialsOut=part,
+                       sinks=None if sinks is None else sinks.reshape(-1).contiguous(), **opts)
+        ex.sync()
+    finally:
+        ex.setStream(None)
+    return part
+
+
+@pytest.mark.parametrize("kv,group,hd", [(8, 8, 36), (2, 4, 36), (2, 4, 52), (8, 8, 52), (8, 4, 64), (2, 4, 64),
+                                         (8, 2, 128), (8, 4, 128), (8, 8, 128)])
+@pytest.mark.parametrize("rows", [50, 487, 3000])
+@pytest.mark.parametrize("kind,scale", [("flat", .1), ("plain", 1), ("steep", 4), ("steeper", 16), ("sink", 1),
+                                        ("top", 1)])
+def test_partials_no_less_precise_than_the_f32_kernels(ex, kv, group, hd, rows, kind, scale):
+    """The f32 rows that leave the kernel against 64 bits.  The yardstick is the FP32 kernel on the same
+    heads: it takes the call with 3 or 9 kv heads, these among them.  sink: e^20 times what the keys come to;
+    top: a key that outweighs the others by about 2^40 and whose values are zeros, so that the
+    output is what the others come to."""
+    import torch
+    dev, batch, more = torch.device("cuda", 0), 16, 9 if kv == 8 else 3
+    g = torch.Generator(device=dev).manual_seed(hd + rows)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=dev)  # noqa: E731
+    q = (rnd(batch, more, group, hd) * hd ** -0.5 * scale).half()
+    k, v, sinks = rnd(batch, rows, more, hd).half(), rnd(batch, rows, more, hd).half(), None
+    if kind == "sink":
+        sinks = rnd(more, group) * 2 + 30
+    if kind == "top":     # one query head of a group, in turn, along the key
+        at = torch.arange(batch, device=dev)
+        qt = q[at, :, at % group].float()
+        k[at, at * 3] = (qt * (28 / qt.square().sum(-1, keepdim=True))).half()
+        v[at, at * 3] = 0
+    own = lambda t, d: t.narrow(d, 0, kv)  # noqa: E731
+    s = torch.einsum("bkgd,bnkd->bkgn", own(q, 1).double(), own(k, 2).double())
+    m = s.amax(-1, keepdim=True)
+    if sinks is not None:
+        sk = (own(sinks, 0).double() * math.log(2)).view(1, kv, group, 1)
+        m = torch.maximum(m, sk)
+    w = torch.exp(s - m)
+    total = w.sum(-1, keepdim=True) + (0 if sinks is None else torch.exp(sk - m))
+    want = (torch.einsum("bkgn,bnkd->bkgd", w, own(v, 2).double()) / total).reshape(batch, kv * group, hd)
+    wantLog = (m + torch.log(total)).reshape(batch, kv * group)
+
+    def errors(part):
+        part = part.double()
+        e = (part[..., 2:] / part[..., 1:2] - want).norm(dim=-1) / want.norm(dim=-1)
+        z = part[..., 0] + torch.log(part[..., 1]) - wantLog
+        return e.square().mean().sqrt().item(), z.square().mean().sqrt().item()
+
+    for splits in (1, 3):
+        mine = errors(_partials(ex, own(q, 1), own(k, 2), own(v, 2), kv, group, hd,
+                                None if sinks is None else own(sinks, 0), splits=splits))
+        f32 = _partials(ex, q, k, v, more, group, hd, sinks, splits=splits)
+        f32 = errors(f32.view(batch, more, group, -1)[:, :kv].reshape(batch, kv * group, -1))
+        # (both are sums of independent roundings: in another order, the FP32 kernel's own differ by up to
+        # 1.3; half an ulp of the numbers compared.  Under one key the output is divided by that key's
+        # weight, and so carries its score's last rounding: half an ulp of 28)
+        assert mine[0] <= 1.3 * f32[0] + 2.0 ** -24 * (28 if kind == "top" else 1), (splits, mine, f32)
+        assert mine[1] <= 1.3 * f32[1] + 2.0 ** -24 * max(1.0, wantLog.abs().max().item()), (splits, mine, f32)
+
+
+@pytest.mark.parametrize("heads,kv,hd", [(32, 8, 128), (8, 1, 128), (8, 2, 52), (64, 8, 36), (32, 32, 128)])
+@pytest.mark.parametrize("splits", [0, 2])
+def test_shards_with_append_merge_to_the_whole(ex, heads, kv, hd, splits):
+    """Caches cut into shards of 96 rows, rope and the appended row included: each shard's partials,
+    merged, are the attention over the whole sequence; the row goes to one shard."""
+    import torch
+    from runntime_b200.engine import decode_batched, merge_partials
+    lens, per, parts = [250, 1, 96, 97, 192, 193], 96, 3
+    batch, rows = len(lens), per * parts
+    s = _state(heads, kv, hd, rows, batch, seed=heads + hd)
+    dev = s["q"].device
+    g = torch.Generator(device=dev).manual_seed(1)
+    angle = torch.rand(rows, hd // 2, generator=g, device=dev).repeat_interleave(2, 1) * 6
+    cos, sin = angle.cos().contiguous(), angle.sin().contiguous()
+    dl = torch.tensor(lens, dtype=torch.int32, device=dev)
+    kw = dict(dtype="f16", batch=batch, qHeads=heads, kvHeads=kv, headDim=hd, kvLen=max(lens), kvLens=dl, kNew=s["kn"],
+              vNew=s["vn"], ropeCos=cos, ropeSin=sin, ropeByPosition=True)
+    shards = [(s["k"][:, r * per:(r + 1) * per].contiguous(), s["v"][:, r * per:(r + 1) * per].contiguous())
+              for r in range(parts)]
+    parted = torch.empty(parts, batch, heads, 2 + hd, device=dev)
+    whole, out = torch.empty_like(s["q"]), torch.empty_like(s["q"])
+    ex.setStream(torch.cuda.current_stream().cuda_stream)
+    try:
+        for r, (k, v) in enumerate(shards):
+            decode_batched(ex, s["q"], None, k, v, cacheRows=per, kvSharded=True, shardStart=r * per,
+                           partialsOut=parted[r], splits=splits, **kw)
+        merge_partials(ex, parted, parts, batch * heads, hd, out, "f16")
+        decode_batched(ex, s["q"], whole, s["k"], s["v"], cacheRows=rows, splits=splits, **kw)
+        ex.sync()
+    finally:
+        ex.setStream(None)
+    assert torch.equal(torch.cat([k for k, _ in shards], 1), s["k"])
+    assert torch.equal(torch.cat([v for _, v in shards], 1), s["v"])
+    for b, n in enumerate(lens):
+        assert (parted[(n - 1) // per + 1:, b, :, 1] == 0).all()      # shards past the sequence's end
+    # (two orders of f32 sums, each rounded to f16 once: an ulp)
+    assert ((out.float() - whole.float()).abs() <= 2.0 ** -10 * whole.float().abs() + 2.0 ** -14).all()
 
 
 @pytest.mark.parametrize("heads,kv,hd,batch,rows,runs", [
