@@ -1689,19 +1689,30 @@ cudaError_t launch_typed(const DecodeParams& p, cudaStream_t s) {
   return launch_one<T, 128, false, 1, false>(p, smem, s);
 }
 
-// Which f16 calls go to the tensor cores.  With several query heads on a kv head the FP32 pipes
-// read and convert every key once per query head and are what bounds the step; measured (B200, us):
-// 16 sequences of up to 1000 keys, 16 heads of 128 on 8: 28.2 / 23.0; 64 x 1000, 8 of 128 on 1: 48.1 / 18.3;
-// 64 x 2000, 8 of 52 on 2: 32.6 / 19.1; 64 x 1000, 32 of 64 on 8: 56.8 / 38.0; at worst 38.2 / 38.8.
-// With one query head each it is a wash, but for many wide heads and short caches, where a block
-// of the other kernel holds all heads of two keys at a time (32 heads of 128: 60 x 100 keys 38.9 / 29.2,
-// 32 x 300 40.9 / 36.1, 118 MB); long ones stream better in its whole rows (6 x 2600, 192 MB: 53.1 / 53.8,
-// 16 x 1024, 201 MB: 53.2 / 59.6).
+// Which f16 calls go to the tensor cores, by measurement (B200, us among launches, FP32 pipes / tensor cores).
+// With several query heads on a kv head the FP32 pipes read and convert every key once per query
+// head: 16 sequences of 2000 keys, 32 heads of 128 on 8: 75.9 / 34.9; 64 x 100, 8 of 128 on one: 14.2 / 6.8;
+// 64 x 2000, 32 of 64 on 8: 112.8 / 64.3; 64 x 448, 64 of 36 on 8: 46.6 / 27.1.
+//   - Heads of less than 64 need four query heads on a warp's kv head, or two where a block's warps
+//     share kv heads: 64 x 2000, 16 of 36 on 8 43.6 / 52.7, of 52 51.0 / 59.7; 8 of 52 on 4 30.2 / 32.3, 64 x 100 8.4 / 7.9.
+//   - Few keys of few sequences, heads of 128 and one kv head to a warp: a tile is 16 keys, the other
+//     kernel's 4 to 16 spread over more blocks.  100 keys, 16 heads on 8, 1 / 16 sequences: 12.7 / 15.5, 13.8 / 17.0;
+//     65 keys, 32 on 8, one: 11.8 / 14.1, 16: 14.5 / 14.0; 16 keys, 32 on 8: 11.4 / 9.4.
+//   - With one query head each it is a wash, but for many wide heads and short caches, where a block
+//     of the other kernel holds all heads of two keys at a time (32 heads of 128: 64 x 100 keys 37.3 / 32.3,
+//     4 x 448 19.0 / 16.6); long ones stream better in its whole rows (16 x 2000, 524 MB: 87.7 / 88).
 bool mma_better(const DecodeParams& p, int group) {
   if (group > 8 || (p.kvHeads % 8 && p.kvHeads != 4 && p.kvHeads != 2 && p.kvHeads != 1)) return false;
+  const int heads = p.kvHeads < 8 ? p.kvHeads : 8;   // kv heads of a block
+  if (p.hd < 64) return group > 1 && group * (8 / heads) >= 4;
+  const int64_t rows = p.useRange ? p.end - p.lo + 1 : p.kvLen;
+  const int64_t keys = !p.useRange && rows - 1 > p.wl ? (int64_t)p.wl + 1 : rows;
+  if (p.hd == 128 && heads == 8 && keys > 16 && keys <= 128 && keys * group <= 520) {
+    const int64_t blocks = (int64_t)p.batch * (p.kvHeads / heads) * (p.hasSecond ? 2 : 1);
+    if (blocks * group <= 32) return false;
+  }
   if (group > 1) return true;
-  const int64_t keys = p.useRange ? p.end - p.lo + 1 : p.kvLen;
-  return p.hd == 128 && p.kvHeads > 8 && p.batch * keys * p.kvHeads * p.hd * 4 <= (160ll << 20);
+  return p.hd == 128 && p.kvHeads > 8 && p.batch * rows * p.kvHeads * p.hd * 4 <= (160ll << 20);
 }
 
 }  // namespace
