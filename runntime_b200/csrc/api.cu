@@ -241,25 +241,33 @@ rt::AttnParams to_params(const rt_attn_args* a) {
 int run_decode(rt_ctx* ctx, rt::DecodeParams& p, int dtype) {
   std::string err;
   const bool chosen = p.splits <= 0;   // by the plan, not by the caller
+  bool tensorCores = true;
   if (!rt::plan_decode(p, dtype, ctx->smCount, &err))
     return fail(ctx, RT_INVALID_ARGUMENT, "%s", err.c_str());
   if (p.splits > 1) {
     const size_t sets = p.hasSecond ? 2 : 1;   // a second attention has its own partials and counters
     const size_t perSplit = sets * p.batch * p.qHeads * (2 + p.hd) * sizeof(float);
-    size_t counters = sets * p.batch * ((p.kvHeads + p.kvPerCta - 1) / p.kvPerCta);
-    if (!chosen && p.mma && counters > ctx->counterCount && capturing(ctx->stream)) {
+    auto counters_of = [&](const rt::DecodeParams& d) { return sets * d.batch * ((d.kvHeads + d.kvPerCta - 1) / d.kvPerCta); };
+    size_t counters = counters_of(p);
+    if (p.mma && counters > ctx->counterCount && capturing(ctx->stream)) {
       // The tensor cores' blocks hold fewer heads and so need more counters, which cannot be made
-      // under a capture: the FP32 kernel takes the call.
-      if (!rt::plan_decode(p, dtype, ctx->smCount, &err, false))
+      // under a capture: the FP32 kernel takes the call where it can split it (always, with given splits).
+      rt::DecodeParams simt = p;
+      if (chosen) simt.splits = 0;
+      if (!rt::plan_decode(simt, dtype, ctx->smCount, &err, false))
         return fail(ctx, RT_INVALID_ARGUMENT, "%s", err.c_str());
-      counters = sets * p.batch * ((p.kvHeads + p.kvPerCta - 1) / p.kvPerCta);
+      if (!chosen || (simt.splits > 1 && counters_of(simt) <= ctx->counterCount && ctx->scratchBytes >= 2 * perSplit)) {
+        p = simt;
+        counters = counters_of(p);
+        tensorCores = false;
+      }
     }
     const bool grows = p.splits * perSplit > ctx->scratchBytes || counters > ctx->counterCount;
     if (chosen && grows && capturing(ctx->stream)) {
       // Nothing can be allocated under a capture: as many splits as the scratch at hand holds.
       const size_t fit = counters > ctx->counterCount ? 0 : ctx->scratchBytes / perSplit;
       p.splits = fit > 1 ? (int)fit : 1;
-      if (!rt::plan_decode(p, dtype, ctx->smCount, &err))
+      if (!rt::plan_decode(p, dtype, ctx->smCount, &err, tensorCores))
         return fail(ctx, RT_INVALID_ARGUMENT, "%s", err.c_str());
     } else {
       const int s = ensure_scratch(ctx, p.splits * perSplit, counters);

@@ -69,3 +69,29 @@ def check_sdpa(ex, c: SdpaCase, dtype: str = "f32", route: str | None = None):
     want = sdpa_ref_inputs(x)
     oracle.assert_close(got, want, dtype, f"{c} [{dtype}]")
     return got, want
+
+
+def capture(call, stream):
+    """A CUDA graph of ``call`` on ``stream``, and the grids of its kernels in the order of capture."""
+    import ctypes as C
+    import torch
+
+    class Params(C.Structure):   # CUDA_KERNEL_NODE_PARAMS_v2
+        _fields_ = [("func", C.c_void_p), ("grid", C.c_uint * 3), ("block", C.c_uint * 3), ("shared", C.c_uint),
+                    ("kernelParams", C.c_void_p), ("extra", C.c_void_p), ("kern", C.c_void_p), ("ctx", C.c_void_p)]
+
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph, stream=stream):
+        call()
+    cu, handle, n = C.CDLL("libcuda.so.1"), C.c_void_p(graph.raw_cuda_graph()), C.c_size_t(0)
+    assert cu.cuGraphGetNodes(handle, None, C.byref(n)) == 0
+    nodes, grids = (C.c_void_p * n.value)(), []
+    assert cu.cuGraphGetNodes(handle, nodes, C.byref(n)) == 0
+    for node in nodes:
+        kind, p = C.c_int(), Params()
+        assert cu.cuGraphNodeGetType(C.c_void_p(node), C.byref(kind)) == 0
+        if kind.value == 0:      # a kernel
+            assert cu.cuGraphKernelNodeGetParams_v2(C.c_void_p(node), C.byref(p)) == 0
+            grids.append(tuple(p.grid))
+    graph.instantiate()
+    return graph, grids

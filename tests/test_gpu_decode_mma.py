@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 import oracle
-from gpu_harness import ex  # noqa: F401
+from gpu_harness import capture, ex  # noqa: F401
 from oracle import sdpa_ref
 
 pytestmark = pytest.mark.gpu
@@ -248,9 +248,11 @@ def test_where_the_fixed_scratch_holds_no_splits(heads, kv, hd, batch, rows, run
         oracle.assert_close(out[b].float().cpu().numpy(), want.reshape(-1), "f16", f"sequence {b}")
 
 
-def test_given_splits_under_capture_with_the_other_kernels_counters():
+@pytest.mark.parametrize("splits", [3, 0])
+def test_splits_under_capture_with_the_other_kernels_counters(splits):
     """32 heads of 128 are one block of the FP32 kernel and four of this one: a context warmed by the
-    former has counters for too few of the latter, and none can be made under a capture."""
+    former has counters for too few of the latter, and none can be made under a capture.  The FP32 kernel
+    then takes the call, and splits it."""
     import torch
     import runntime_b200 as rt
     heads, hd, rows, batch = 32, 128, 200, 4
@@ -259,17 +261,18 @@ def test_given_splits_under_capture_with_the_other_kernels_counters():
     lens = torch.tensor([200, 1, 130, 64], dtype=torch.int32, device=s["q"].device)
     out = torch.empty_like(s["q"])
     from runntime_b200.engine import decode_batched
-    kw = dict(batch=batch, cacheRows=rows, qHeads=heads, kvHeads=heads, headDim=hd, kvLen=rows, kvLens=lens, splits=3)
+    kw = dict(batch=batch, cacheRows=rows, qHeads=heads, kvHeads=heads, headDim=hd, kvLen=rows, kvLens=lens)
     stream = torch.cuda.Stream()
     try:
         ex.setStream(stream.cuda_stream)
         f = {x: s[x].float() for x in ("q", "k", "v")}
         torch.cuda.synchronize()
-        decode_batched(ex, f["q"], torch.empty_like(f["q"]), f["k"], f["v"], dtype="f32", **kw)
+        decode_batched(ex, f["q"], torch.empty_like(f["q"]), f["k"], f["v"], dtype="f32", splits=3, **kw)
         ex.sync()
-        graph = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(graph, stream=stream):
-            decode_batched(ex, s["q"], out, s["k"], s["v"], dtype="f16", **kw)
+        graph, grids = capture(lambda: decode_batched(ex, s["q"], out, s["k"], s["v"], dtype="f16", splits=splits, **kw),
+                               stream)
+        assert grids[0][1:] == (batch, 1)      # all heads in a block: the FP32 kernel
+        assert grids[0][0] == splits if splits else grids[0][0] > 1
         graph.replay()
         torch.cuda.synchronize()
         for b, n in enumerate(lens.tolist()):
@@ -277,6 +280,33 @@ def test_given_splits_under_capture_with_the_other_kernels_counters():
                             s["v"][b, :n].float().cpu().numpy(), qHeads=heads, kvHeads=heads, headDim=hd,
                             qPosOffset=n - 1, windowRight=0)
             oracle.assert_close(out[b].float().cpu().numpy(), want.reshape(-1), "f16", f"length {n}")
+        del graph
+    finally:
+        ex.dispose()
+
+
+def test_splits_under_capture_without_scratch_for_the_other_kernel():
+    """Too few counters, and no scratch for two splits of either kernel: the tensor cores take the call whole."""
+    import torch
+    import runntime_b200 as rt
+    from runntime_b200.engine import decode_batched
+    heads, hd, rows, batch = 32, 128, 200, 4
+    s = _state(heads, heads, hd, rows, batch)
+    out, stream, ex = torch.empty_like(s["q"]), torch.cuda.Stream(), rt.CudaExecutor(0)
+    torch.cuda.synchronize()
+    try:
+        ex.setStream(stream.cuda_stream)
+        graph, grids = capture(lambda: decode_batched(
+            ex, s["q"], out, s["k"], s["v"], dtype="f16", batch=batch, cacheRows=rows, qHeads=heads, kvHeads=heads,
+            headDim=hd, kvLen=rows), stream)
+        assert grids == [(1, batch, 4)]
+        graph.replay()
+        torch.cuda.synchronize()
+        for b in range(batch):
+            want = sdpa_ref(s["q"][b:b + 1].float().cpu().numpy(), s["k"][b].float().cpu().numpy(),
+                            s["v"][b].float().cpu().numpy(), qHeads=heads, kvHeads=heads, headDim=hd, windowRight=0,
+                            qPosOffset=rows - 1)
+            oracle.assert_close(out[b].float().cpu().numpy(), want.reshape(-1), "f16", f"sequence {b}")
         del graph
     finally:
         ex.dispose()
