@@ -699,15 +699,15 @@ int rt_argmax_dot(rt_ctx* ctx, const void* w, const void* x, float* out, int64_t
   if (rows < 1 || cols < 1 || rows > 0xffffffffll)
     return fail(ctx, RT_INVALID_ARGUMENT, "argmaxDot: empty or oversized tensor (%lld x %lld)",
                 (long long)rows, (long long)cols);
-  // One word of scratch per block; under a capture, where none can be made, as many blocks as the scratch
-  // at hand has words for (eight words are asked for in any case).
-  int blocks = rt::argmax_dot_blocks(rows, cols);
-  if (capturing(ctx->stream) && ctx->scratchBytes < blocks * sizeof(uint64_t) && ctx->scratchBytes >= 64)
-    blocks = (int)(ctx->scratchBytes / sizeof(uint64_t));
-  int s = ensure_scratch(ctx, std::max<size_t>(blocks * sizeof(uint64_t), 64), 1);
+  // One word of scratch per block, or, under a capture, where none can be made, as many as the scratch at
+  // hand has (eight words are asked for in any case).
+  int words = rt::argmax_dot_blocks(rows, cols);
+  if (ctx->scratchBytes < words * sizeof(uint64_t) && ctx->scratchBytes >= 64 && capturing(ctx->stream))
+    words = (int)(ctx->scratchBytes / sizeof(uint64_t));
+  int s = ensure_scratch(ctx, std::max<size_t>(words * sizeof(uint64_t), 64), 1);
   if (s != RT_OK) return s;
   RT_CUDA(ctx, rt::launch_argmax_dot(w, x, out, rows, cols, dtype, reinterpret_cast<unsigned long long*>(ctx->scratch),
-                                     ctx->counters, blocks, ctx->stream));
+                                     ctx->counters, words, ctx->stream));
   ctx->launches++;
   return RT_OK;
 }

@@ -378,10 +378,10 @@ bool matmul_f32_tc_supported(const void* a, const void* b, const void* addend, c
                              int64_t K, int64_t N, int dtype);
 cudaError_t launch_matmul_f32_tc(const void* a, const void* b, const void* bias, const void* addend, void* out,
                                  int64_t M, int64_t K, int64_t N, int act, cudaStream_t s);
-int argmax_dot_blocks(int64_t V, int64_t N);   // of the launch below, a word of scratch each
+int argmax_dot_blocks(int64_t V, int64_t N);   // of the launch below, which meet in as many words of scratch or fewer
 cudaError_t launch_windows(const rt_window* w, int count, int dtype, int* launches, cudaStream_t s);
 cudaError_t launch_argmax_dot(const void* w, const void* x, float* out, int64_t V, int64_t N, int dtype,
-                              unsigned long long* scratch, unsigned* counter, int blocks, cudaStream_t s);
+                              unsigned long long* scratch, unsigned* counter, int words, cudaStream_t s);
 cudaError_t launch_local_attn(const void* qkv, const float* rel, const float* qScale, void* out,
                               int64_t rows, int heads, int hd, int window, float kScale,
                               float softcap, int dtype, cudaStream_t s);

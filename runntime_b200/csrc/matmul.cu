@@ -362,7 +362,7 @@ __device__ __forceinline__ unsigned long long argmax_key(float v, uint32_t idx) 
 template <typename T, int U>   // U: rows of a warp at a time
 __global__ void __launch_bounds__(256)
 argmax_dot_kernel(const T* w, const T* x, int64_t V, int64_t N,
-                  unsigned long long* best, unsigned* counter, float* out, bool vec) {
+                  unsigned long long* best, int words, unsigned* counter, float* out, bool vec) {
   constexpr int VV = 16 / sizeof(T);
   __shared__ unsigned long long sBest[8];
   __shared__ bool sLast;
@@ -408,7 +408,8 @@ argmax_dot_kernel(const T* w, const T* x, int64_t V, int64_t N,
   __syncthreads();
   if (threadIdx.x == 0) {
     for (int i = 1; i < 8; i++) mine = sBest[i] > mine ? sBest[i] : mine;
-    best[blockIdx.x] = mine;
+    if (words == (int)gridDim.x) best[blockIdx.x] = mine;
+    else atomicMax(best + blockIdx.x % words, mine);   // (fewer words than blocks: cleared by the host)
     __threadfence();
     sLast = atomicAdd(counter, 1u) == gridDim.x - 1;
   }
@@ -416,7 +417,7 @@ argmax_dot_kernel(const T* w, const T* x, int64_t V, int64_t N,
   if (!sLast) return;
   __threadfence();
   mine = 0ull;
-  for (int i = threadIdx.x; i < (int)gridDim.x; i += 256) {
+  for (int i = threadIdx.x; i < words; i += 256) {
     const unsigned long long key = __ldcg(best + i);
     if (key > mine) mine = key;
   }
@@ -527,7 +528,12 @@ int argmax_dot_blocks(int64_t V, int64_t N) {
 }
 
 cudaError_t launch_argmax_dot(const void* w, const void* x, float* out, int64_t V, int64_t N, int dtype,
-                              unsigned long long* scratch, unsigned* counter, int blocks, cudaStream_t s) {
+                              unsigned long long* scratch, unsigned* counter, int words, cudaStream_t s) {
+  const int blocks = argmax_dot_blocks(V, N);
+  if (words < blocks) {
+    const cudaError_t e = cudaMemsetAsync(scratch, 0, words * sizeof(unsigned long long), s);
+    if (e != cudaSuccess) return e;
+  }
   const int vv = 16 / (dtype == RT_F16 ? 2 : 4);
   const bool vec = N % vv == 0 && reinterpret_cast<uintptr_t>(w) % 16 == 0 &&
                    reinterpret_cast<uintptr_t>(x) % 16 == 0;
@@ -542,8 +548,8 @@ cudaError_t launch_argmax_dot(const void* w, const void* x, float* out, int64_t 
   cfg.numAttrs = 1;
   auto launch = [&](auto kern, auto one) {
     using T = decltype(one);
-    return cudaLaunchKernelEx(&cfg, kern, static_cast<const T*>(w), static_cast<const T*>(x), V, N, scratch, counter,
-                              out, vec);
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<const T*>(w), static_cast<const T*>(x), V, N, scratch, words,
+                              counter, out, vec);
   };
   if (dtype == RT_F16)
     return N > kArgmaxWide ? launch(argmax_dot_kernel<__half, 1>, __half{}) : launch(argmax_dot_kernel<__half, 4>, __half{});

@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 import oracle
-from gpu_harness import ex  # noqa: F401
+from gpu_harness import capture, ex  # noqa: F401
 
 pytestmark = pytest.mark.gpu
 
@@ -170,3 +170,41 @@ def test_argmax_dot_over_warps_blocks_and_rounds(ex, dtype, rows, cols):
     # (the f32 sum of `cols` products is off by at most cols/2 ulps of the largest partial sum)
     slack = cols * 2.0 ** -24 * np.abs(w[got] * x[0]).sum() * 2
     assert scores[got] >= scores.max() - slack
+
+
+@pytest.mark.parametrize("dtype", ["f16", "f32"])
+@pytest.mark.parametrize("rows,cols", [(9999, 24), (40000, 17), (3001, 1040)])
+def test_argmax_dot_under_capture_with_little_scratch(dtype, rows, cols):
+    """A context warmed by a short product has scratch for fewer words than a long one has blocks, and none can
+    be made under a capture: the blocks share them, and are as many as with scratch enough."""
+    import torch
+    import runntime_b200 as rt
+    from runntime_b200._lib import DTYPE_CODE, check
+    td = torch.float16 if dtype == "f16" else torch.float32
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    w = torch.randn(rows, cols, generator=g, device="cuda").to(td)
+    x = torch.randn(cols, generator=g, device="cuda").to(td)
+    out, stream, grids = torch.zeros(1, device="cuda"), torch.cuda.Stream(), []
+    torch.cuda.synchronize()
+    for warm in (8, rows):
+        e = rt.CudaExecutor(0)
+        try:
+            e.setStream(stream.cuda_stream)
+            call = lambda n: check(e._lib.rt_argmax_dot(e.ctx, w.data_ptr(), x.data_ptr(), out.data_ptr(), n, cols,  # noqa: E731
+                                                        DTYPE_CODE[dtype]), e.ctx)
+            call(warm)
+            e.sync()
+            graph, grid = capture(lambda: call(rows), stream)
+            grids.append(grid)
+            for at in (rows - 1, rows // 2, 0):
+                row = w[at].clone()
+                w[at] = x * 40
+                torch.cuda.synchronize()
+                graph.replay()
+                torch.cuda.synchronize()
+                assert int(out.item()) == at
+                w[at] = row
+            del graph
+        finally:
+            e.dispose()
+    assert grids[0] == grids[1] and len(grids[0]) == 1
