@@ -430,6 +430,9 @@ __device__ __forceinline__ float warp_sum(float x) {
 // may start while the grid before it in the stream drains; grid_dependency_wait() returns
 // once that grid has completed and its writes are visible (at once if there is none);
 // grid_launch_dependents() lets the next such grid start its prologue.
+// A kernel that may be resident while the one before it still writes promises the compiler nothing
+// about its tensors before the wait: its parameters are not __restrict__, which would let loads be
+// moved above the wait or through the cache of constant data.
 __device__ __forceinline__ void grid_dependency_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }

@@ -141,8 +141,7 @@ __device__ __noinline__ void exact_row(const __half* qkv, const float* rel, cons
 template <int HD, int WP>
 __global__ void __launch_bounds__(kLocalThreads, 3)
 local_attn_tc_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapKV,
-                     const __half* __restrict__ qkv, const float* __restrict__ rel,
-                     const float* __restrict__ qScale, __half* __restrict__ out, int64_t rows, int heads,
+                     const __half* qkv, const float* rel, const float* qScale, __half* out, int64_t rows, int heads,
                      int window, float kScale, float softcap, int* status) {
   using L = Local<HD, WP>;
   grid_dependency_wait();

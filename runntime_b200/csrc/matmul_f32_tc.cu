@@ -28,9 +28,8 @@ constexpr int kAFloats = TM * kAPitch, kStage = kAFloats + TK * kBPitch;
 constexpr int kSmem = 4 * kStages * kStage;
 
 __global__ void __launch_bounds__(kThreads, 3)
-matmul_f32_tc_kernel(const float* __restrict__ a, const float* __restrict__ b, const float* __restrict__ bias,
-                     const float* __restrict__ addend, float* __restrict__ out, int64_t M, int64_t K, int64_t N,
-                     int act) {
+matmul_f32_tc_kernel(const float* a, const float* b, const float* bias, const float* addend, float* out, int64_t M,
+                     int64_t K, int64_t N, int act) {
   extern __shared__ __align__(16) float ring[];
   grid_dependency_wait();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;

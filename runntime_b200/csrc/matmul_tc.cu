@@ -106,7 +106,7 @@ template <int BN, int ACT>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                const __grid_constant__ CUtensorMap mapAdd, const __grid_constant__ CUtensorMap mapOut,
-               const __half* __restrict__ bias, const __half* __restrict__ addend, int addMode,
+               const __half* bias, const __half* addend, int addMode,
                int64_t M, int64_t K, int64_t N, int tilesN, int tiles, int* status) {
   using G = Gemm<BN>;
   extern __shared__ unsigned char smemRaw[];
@@ -400,8 +400,7 @@ __device__ unsigned long long gSkTrace[4096 * 8];
 // rowsPad: 8 or 16, the rows of a that are exchanged and stored (M <= rowsPad).
 __global__ void __launch_bounds__(kSkThreads, RT_SK_MIN_CTAS)
 gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
-                      const __half* __restrict__ bias, const __half* __restrict__ addend,
-                      __half* __restrict__ out, int M, int64_t K, int64_t N, int stepsPerRank,
+                      const __half* bias, const __half* addend, __half* out, int M, int64_t K, int64_t N, int stepsPerRank,
                       int rowsPad, int act, int* status) {
   extern __shared__ unsigned char smemRaw[];
   __shared__ __align__(8) uint64_t sFull[SKSTAGES], sEmpty[SKSTAGES], sAcc;

@@ -69,11 +69,9 @@ __global__ void merge_partials_kernel(const float* __restrict__ partials, int pa
 // (`limit` polls, about a second by default), then the block records the failure in *status
 // and writes zeros.  Output rows: sequences [firstSeq, firstSeq + owned) of `out`.
 template <typename T>
-__global__ void merge_exchanged_kernel(const float* __restrict__ buffer,
-                                       const uint32_t* __restrict__ flags,
-                                       const uint32_t* __restrict__ step, int world, int per,
-                                       int owned, int firstSeq, int heads, int hd,
-                                       T* __restrict__ out, int* status, int limit) {
+__global__ void merge_exchanged_kernel(const float* buffer, const uint32_t* flags, const uint32_t* step, int world,
+                                       int per, int owned, int firstSeq, int heads, int hd, T* out, int* status,
+                                       int limit) {
   __shared__ int sOk;
   // A programmatic dependent of the decode kernel: resident early, reading nothing before
   // that grid has finished; the kernel after this one may be made resident at once.

@@ -77,11 +77,11 @@ prefill_mma_kernel(const AttnParams p, int tilesPerSeq) {
   }
   rowEnd = min(rowEnd, row0 + BQ);
   const int kvh = h / (p.qHeads / p.kvHeads);
+  grid_dependency_wait();
   const __half* __restrict__ q = static_cast<const __half*>(p.q) + (int64_t)h * hd;
   const __half* __restrict__ k = static_cast<const __half*>(p.k) + (int64_t)kvh * hd;
   const __half* __restrict__ v = static_cast<const __half*>(p.v) + (int64_t)kvh * hd;
 
-  grid_dependency_wait();
   for (int i = tid; i < BQ * W; i += kThreads) {
     const int r = i / W, x = (i % W) * E;
     const bool in = row0 + r < rowEnd && x < hd;

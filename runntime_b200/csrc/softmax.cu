@@ -73,8 +73,7 @@ __device__ __forceinline__ void combine(float& m, float& s, float m2, float s2) 
 // Rows that start on four elements: quads.  WARP: one warp per row, else one CTA per row.
 template <typename T, bool WARP>
 __global__ void __launch_bounds__(kThreads)
-softmax_quad_kernel(const T* __restrict__ x, T* __restrict__ out, const float* __restrict__ segs,
-               int64_t rows, int64_t cols, int64_t wl, int64_t wr) {
+softmax_quad_kernel(const T* x, T* out, const float* segs, int64_t rows, int64_t cols, int64_t wl, int64_t wr) {
   grid_dependency_wait();
   using Q = Quad<T>;
   using QV = typename Q::type;
@@ -321,7 +320,7 @@ __device__ __forceinline__ void softmax_row(const T* __restrict__ x, T* __restri
 
 template <typename T, int V>
 __global__ void __launch_bounds__(kThreads, kCtas)
-softmax_cta_kernel(const T* __restrict__ x, T* __restrict__ out, const float* __restrict__ segs, int64_t cols,
+softmax_cta_kernel(const T* x, T* out, const float* segs, int64_t cols,
                    int64_t wl, int64_t wr) {
   grid_dependency_wait();
   __shared__ float sM[kThreads / 32], sS[kThreads / 32];
@@ -343,7 +342,7 @@ softmax_cta_kernel(const T* __restrict__ x, T* __restrict__ out, const float* __
 constexpr int kGroupRows = 4, kGroup = 32 * kGroupRows, kGroupMinRows = 5000, kGroupRowBytes = 20480;
 template <int V>
 __global__ void __launch_bounds__(kGroup, 10)
-softmax_group_kernel(const __half* __restrict__ x, __half* __restrict__ out, const float* __restrict__ segs,
+softmax_group_kernel(const __half* x, __half* out, const float* segs,
                      int64_t cols, int64_t wl, int64_t wr, int groups) {
   using T = __half;
   grid_dependency_wait();
@@ -376,7 +375,7 @@ softmax_group_kernel(const __half* __restrict__ x, __half* __restrict__ out, con
 // A row by a warp, element by element.
 template <typename T, bool MASKED>
 __global__ void __launch_bounds__(kThreads)
-softmax_element_kernel(const T* __restrict__ x, T* __restrict__ out, const float* __restrict__ segs, int64_t rows,
+softmax_element_kernel(const T* x, T* out, const float* segs, int64_t rows,
                        int64_t cols, int64_t wl, int64_t wr) {
   grid_dependency_wait();
   const int lane = threadIdx.x & 31;
@@ -400,7 +399,7 @@ softmax_element_kernel(const T* __restrict__ x, T* __restrict__ out, const float
 
 template <typename T, int V>
 __global__ void __launch_bounds__(kThreads, kCtas)
-softmax_warp_kernel(const T* __restrict__ x, T* __restrict__ out, const float* __restrict__ segs, int64_t rows,
+softmax_warp_kernel(const T* x, T* out, const float* segs, int64_t rows,
                     int64_t cols, int64_t wl, int64_t wr) {
   grid_dependency_wait();
   const int64_t row = (int64_t)blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
