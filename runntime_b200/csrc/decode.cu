@@ -1695,24 +1695,24 @@ cudaError_t launch_typed(const DecodeParams& p, cudaStream_t s) {
 // 64 x 2000, 32 of 64 on 8: 112.8 / 64.3; 64 x 448, 64 of 36 on 8: 46.6 / 27.1.
 //   - Heads of less than 64 need four query heads on a warp's kv head, or two where a block's warps
 //     share kv heads: 64 x 2000, 16 of 36 on 8 43.6 / 52.7, of 52 51.0 / 59.7; 8 of 52 on 4 30.2 / 32.3, 64 x 100 8.4 / 7.9.
-//   - Few keys of few sequences, heads of 128 and one kv head to a warp: a tile is 16 keys, the other
-//     kernel's 4 to 16 spread over more blocks.  100 keys, 16 heads on 8, 1 / 16 sequences: 12.7 / 15.5, 13.8 / 17.0;
-//     65 keys, 32 on 8, one: 11.8 / 14.1, 16: 14.5 / 14.0; 16 keys, 32 on 8: 11.4 / 9.4.
-//   - With one query head each it is a wash, but for many wide heads and short caches, where a block
-//     of the other kernel holds all heads of two keys at a time (32 heads of 128: 64 x 100 keys 37.3 / 32.3,
-//     4 x 448 19.0 / 16.6); long ones stream better in its whole rows (16 x 2000, 524 MB: 87.7 / 88).
+//     At worst 16 x 448, 32 of 36 on 8: 14.5 / 16.9, 16 of 64 on 8, one of 448 11.4 / 12.4.
+//   - With one query head each, wide heads and many of them gain from tiles of 16 keys and 8 heads where the
+//     other kernel's hold all heads of two to four keys: up to 64 MB (32 heads of 128, 64 x 50 keys
+//     29.4 / 22.9, 4 x 400 19.6 / 15.8; 16 heads up to 48), and up to 160 where the blocks are few (4 x 2500 40.7 / 40.4, 64 heads, 4 x 800
+//     34.8 / 30.9) or fill the chip once or twice (32 x 256 33.1 / 32.2, 64 x 160 48.4 / 43.8).  Else a wave of them is half
+//     empty (24 x 256 28.7 / 31.9, 16 x 600 37.5 / 41.2), or long rows stream as well (16 x 2000 87.7 / 88).
 bool mma_better(const DecodeParams& p, int group) {
   if (group > 8 || (p.kvHeads % 8 && p.kvHeads != 4 && p.kvHeads != 2 && p.kvHeads != 1)) return false;
   const int heads = p.kvHeads < 8 ? p.kvHeads : 8;   // kv heads of a block
   if (p.hd < 64) return group > 1 && group * (8 / heads) >= 4;
-  const int64_t rows = p.useRange ? p.end - p.lo + 1 : p.kvLen;
-  const int64_t keys = !p.useRange && rows - 1 > p.wl ? (int64_t)p.wl + 1 : rows;
-  if (p.hd == 128 && heads == 8 && keys > 16 && keys <= 128 && keys * group <= 520) {
-    const int64_t blocks = (int64_t)p.batch * (p.kvHeads / heads) * (p.hasSecond ? 2 : 1);
-    if (blocks * group <= 32) return false;
-  }
   if (group > 1) return true;
-  return p.hd == 128 && p.kvHeads > 8 && p.batch * rows * p.kvHeads * p.hd * 4 <= (160ll << 20);
+  if (p.hd != 128 || p.kvHeads <= 8) return false;
+  constexpr int64_t kSms = 148;
+  const int64_t blocks = (int64_t)p.batch * (p.kvHeads / heads) * (p.hasSecond ? 2 : 1);
+  const int64_t rows = p.useRange ? p.end - p.lo + 1 : p.kvLen, bytes = p.batch * rows * p.kvHeads * p.hd * 4;
+  const bool fills = blocks <= 2 * kSms && blocks * 20 >= (blocks + kSms - 1) / kSms * kSms * 17;   // 85 %
+  const bool wide = p.kvHeads >= 32;
+  return bytes <= ((wide ? 64ll : 48ll) << 20) || (bytes <= (160ll << 20) && (blocks <= (wide ? 48 : 8) || fills));
 }
 
 }  // namespace
@@ -1851,7 +1851,10 @@ bool plan_decode(DecodeParams& p, int dtype, int smCount, std::string* err, bool
       nmax = nmax < 1 ? 1 : nmax > p.cacheRows ? p.cacheRows : nmax;
     }
     if (!p.useRange && p.wl < nmax) nmax = (int64_t)p.wl + 1;
-    int64_t maxS = nmax / keySlots;   // at least one tile per split
+    // At least one full tile per split, or, for the tensor cores' tiles of 16 keys and more, a begun one:
+    // a few keys over a whole number of tiles else make two of every split (100 keys, 16 heads of 128 on 8,
+    // 16.1 us in six splits of up to two tiles, 10.7 in seven of one).
+    int64_t maxS = (nmax + (p.mma ? keySlots - 1 : 0)) / keySlots;
     if (maxS > 64) maxS = 64;
     if (maxS < 1) maxS = 1;
     // Cost in eighths of one tile's streaming time: every CTA pays a fixed set-up,
