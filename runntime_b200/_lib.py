@@ -133,7 +133,7 @@ SYMBOLS = {
 
 # What csrc/host.cpp calls, in the order of its table.
 HOST_CALLS = ("rt_matmul", "rt_rope", "rt_slice", "rt_attn", "rt_attn_route", "rt_attn_decode",
-              "rt_argmax_dot", "rt_kv_append", "rt_softmax", "rt_local_attention", "rt_windows")
+              "rt_argmax_dot", "rt_kv_append", "rt_softmax", "rt_windows")
 
 try:
     from . import _host as host   # constructors and eval loop in native code

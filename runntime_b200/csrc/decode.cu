@@ -1549,9 +1549,6 @@ merge_kernel(const DecodeParams p) {
   const int h = blockIdx.x, b = blockIdx.y, hd = p.hd, stride = 2 + hd, splits = p.splits;
   const int zBlocks = (p.kvHeads + p.kvPerCta - 1) / p.kvPerCta;
   const int zb = h / (p.qHeads / p.kvHeads) / p.kvPerCta;
-#if RT_SK_EARLY
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-#endif
   asm volatile("griddepcontrol.wait;" ::: "memory");   // the attention's partials are complete
   if (__ldcg(p.counters + b * zBlocks + zb) != 0) return;   // a block gave up: its rows are no partials
   const int64_t row = (int64_t)b * p.qHeads + h;

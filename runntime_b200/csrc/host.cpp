@@ -42,7 +42,7 @@ PyObject *gMethodName[kMethods], *gMethod[kMethods];   // the executor's own, to
 
 #define RT_STRINGS(X)                                                                              \
   X(attn) X(matmul) X(rope) X(softmax) X(writeRows) X(sliceRows) X(sliceCols) X(argmaxDot)         \
-  X(localAttention) X(f16) X(f32) X(qHeads) X(kvHeads) X(headDim) X(windowLeft) X(windowRight)     \
+  X(f16) X(f32) X(qHeads) X(kvHeads) X(headDim) X(windowLeft) X(windowRight)     \
   X(qPosOffset) X(sinks) X(segments) X(maxSegment) X(keyBias) X(srcStart) X(width) X(baseRow)      \
   X(bias) X(addend) X(activation) X(scales) X(bits) X(groupSize) X(value)                          \
   X(dispatches) X(_pool) X(_live) X(_ctx) X(_lib) X(_disposed) X(ctx)
@@ -61,7 +61,6 @@ struct Entry {
   decltype(&rt_argmax_dot) argmaxDot;
   decltype(&rt_kv_append) kvAppend;
   decltype(&rt_softmax) softmax;
-  decltype(&rt_local_attention) localAttention;
   decltype(&rt_windows) windows;
 } gEntry;
 
@@ -347,7 +346,7 @@ PyObject* op_argmax_dot(PyObject*, PyObject* const* args, Py_ssize_t n) {
 
 // ---- the eval driver ---------------------------------------------------------------------
 
-enum Op { kOther, kMatmul, kAttn, kWriteRows, kRope, kSliceRows, kSliceCols, kSoftmax, kArgmaxDot, kLocal };
+enum Op { kOther, kMatmul, kAttn, kWriteRows, kRope, kSliceRows, kSliceCols, kSoftmax, kArgmaxDot };
 
 struct Fused {   // what executor.py's _fusable_appends plans for an attn node
   int k = -1, v = -1, ropeQ = -1, ropeK = -1, vSlice = -1;
@@ -382,7 +381,6 @@ Op op_of(PyObject* name) {
   if (is_str(name, s_writeRows)) return kWriteRows;
   if (is_str(name, s_argmaxDot)) return kArgmaxDot;
   if (is_str(name, s_softmax)) return kSoftmax;
-  if (is_str(name, s_localAttention)) return kLocal;
   if (is_str(name, s_sliceRows)) return kSliceRows;
   return kOther;
 }
