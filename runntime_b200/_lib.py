@@ -156,10 +156,15 @@ def load():
         for name, (res, args) in SYMBOLS.items():
             fn = getattr(lib, name)
             fn.restype, fn.argtypes = res, args
-        if host is not None:
-            host.bind_library(lib, tuple(C.cast(getattr(lib, n), C.c_void_p).value for n in HOST_CALLS))
+        bind_host(lib)
         _lib = lib
     return _lib
+
+
+def bind_host(lib) -> None:
+    """The library that csrc/host.cpp calls; executors of another one run in Python."""
+    if host is not None:
+        host.bind_library(lib, tuple(C.cast(getattr(lib, n), C.c_void_p).value for n in HOST_CALLS))
 
 
 def check(status: int, ctx=None):

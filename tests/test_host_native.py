@@ -1,8 +1,10 @@
 """The constructors and the eval loop in native code (csrc/host.cpp) against the Python they
 stand for: the same nodes, the same refusals, the same calls of the C ABI in the same order, the
 same buffers in the pool.  The library is a stub that writes its calls down (no GPU)."""
+import contextlib
 import ctypes as C
 import math
+import os
 import shutil
 import subprocess
 
@@ -85,13 +87,25 @@ def stub(tmp_path_factory):
     return str(d / "stub.so")
 
 
-@pytest.fixture
-def lib(stub, monkeypatch):
+@contextlib.contextmanager
+def stubbed(stub, monkeypatch):
+    """The stub in the library's place; afterwards the native code calls the one that was there again."""
+    before = L._lib
     monkeypatch.setattr(L, "LIB_PATH", stub)
     monkeypatch.setattr(L, "_lib", None)
     lib = L.load()
     lib.stub_log.restype, lib.stub_reset.argtypes = C.c_char_p, [C.c_int]
-    yield lib
+    try:
+        yield lib
+    finally:
+        if before is not None:
+            L.bind_host(before)
+
+
+@pytest.fixture
+def lib(stub, monkeypatch):
+    with stubbed(stub, monkeypatch) as lib:
+        yield lib
 
 
 def python_only(monkeypatch):
@@ -305,3 +319,36 @@ def test_overridden_executors_and_released_values_stay_with_python(lib):
     with pytest.raises(rt.RunntimeError, match="executor was disposed"):
         rt.evalValues([y], ex)
     rt.evalValues([val(2, 2)], ex)   # nothing to do
+
+
+def test_the_real_library_is_bound_again_after_the_stub(stub):
+    if not os.path.exists(L.LIB_PATH):
+        pytest.skip("librt_attn.so is not built")
+    real = L.load()
+    ex = X.CudaExecutor.__new__(X.CudaExecutor)
+    ex._lib = real
+    with pytest.MonkeyPatch.context() as m:
+        with stubbed(stub, m):
+            assert L.host.evaluate([val(2, 2)], ex, None) is False     # (left to Python: another library)
+    assert L.load() is real and L.host.evaluate([val(2, 2)], ex, None) is True
+
+
+@pytest.mark.gpu
+def test_graphs_run_in_native_code_on_the_gpu(monkeypatch):
+    """An evaluation of plain operators is the native code's, not the Python that stands in for it."""
+    import numpy as np
+    ex, said = rt.CudaExecutor(0), []
+
+    class Watched:
+        @staticmethod
+        def evaluate(*a):
+            said.append(L.host.evaluate(*a))
+            return said[-1]
+
+    try:
+        monkeypatch.setattr(X, "host", Watched)
+        x, w = ex.upload(np.eye(4, 8), [4, 8], "f16"), ex.upload(np.ones((8, 6)), [8, 6], "f16")
+        got = rt.toArray(rt.slice(rt.matmul(x, w), 1, 1, 3), ex)
+        assert said == [True] and (got == 1).all()
+    finally:
+        ex.dispose()
