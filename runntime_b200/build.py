@@ -1,5 +1,5 @@
-"""Builds librt_attn.so (the CUDA kernels and the C ABI) for sm_100a with nvcc, and _host.so
-(csrc/host.cpp) with the C++ compiler.
+"""Builds librt_attn.so (the CUDA kernels and the C ABI) for sm_100a with nvcc, and the extension
+_host (csrc/host.cpp) for the running interpreter with the C++ compiler.
 
 nvcc cross-compiles without a GPU.  The library links the static CUDA runtime
 and resolves driver entry points at run time, so it loads (and its symbols can
@@ -12,12 +12,15 @@ import shutil
 import subprocess
 import sys
 import sysconfig
+import warnings
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "librt_attn.so")
-HOST = os.path.join(HERE, "_host.so")   # the constructors and the eval loop in native code (CPython extension)
+# The constructors and the eval loop in native code: a CPython extension, and so named after the
+# interpreter it is compiled for (another one does not import it).
+HOST = os.path.join(HERE, "_host" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 SOURCES = ["api.cu", "prefill_simt.cu", "prefill_rows.cu", "prefill_f32_tc.cu", "prefill_mma.cu", "prefill_tc.cu", "prefill_tc2.cu", "prefill_tc3.cu", "prefill_tc4.cu", "decode.cu", "exchange.cu", "misc.cu", "softmax.cu",
            "local_attn.cu", "local_attn_tc.cu", "matmul.cu",
            "matmul_tc.cu", "matmul_f32_tc.cu"]
@@ -36,17 +39,26 @@ def _nvcc() -> str:
     raise RuntimeError("nvcc not found; set NVCC")
 
 
-def build_host() -> str:
-    """Compile the CPython extension if it is missing or older than its sources.  Python runs in
-    its place where it is missing."""
+def build_host() -> bool:
+    """Compile the CPython extension if it is missing or older than its sources.  Where it cannot be
+    compiled (no Python.h, no C++ compiler) none is left behind and Python runs in its place."""
     src, header = os.path.join(CSRC, "host.cpp"), os.path.join(ROOT, "include", "rt_attn.h")
     if os.path.exists(HOST) and os.path.getmtime(HOST) >= max(
             os.path.getmtime(f) for f in (src, header, os.path.abspath(__file__))):
-        return HOST
-    subprocess.check_call(["/usr/bin/g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
-                           "-Wall", "-I", sysconfig.get_paths()["include"], "-I", os.path.join(ROOT, "include"),
-                           src, "-o", HOST])
-    return HOST
+        return True
+    fresh = f"{HOST}.{os.getpid()}"
+    try:
+        subprocess.check_call(["/usr/bin/g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
+                               "-Wall", "-I", sysconfig.get_paths()["include"], "-I", os.path.join(ROOT, "include"),
+                               src, "-o", fresh])
+        os.replace(fresh, HOST)
+        return True
+    except (OSError, subprocess.CalledProcessError) as e:
+        for f in (fresh, HOST):
+            if os.path.exists(f):
+                os.remove(f)
+        warnings.warn(f"csrc/host.cpp was not built, the Python it stands for runs: {e}")
+        return False
 
 
 def _stale() -> bool:

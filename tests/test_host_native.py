@@ -3,6 +3,7 @@ stand for: the same nodes, the same refusals, the same calls of the C ABI in the
 same buffers in the pool.  The library is a stub that writes its calls down (no GPU)."""
 import contextlib
 import ctypes as C
+import importlib.util
 import math
 import os
 import shutil
@@ -11,7 +12,7 @@ import subprocess
 import pytest
 
 import runntime_b200 as rt
-from runntime_b200 import _lib as L, executor as X, ops
+from runntime_b200 import _lib as L, build as B, executor as X, ops
 from runntime_b200.value import DeviceBuffer, ValueMeta, materialized
 
 INF = math.inf
@@ -331,6 +332,28 @@ def test_the_real_library_is_bound_again_after_the_stub(stub):
         with stubbed(stub, m):
             assert L.host.evaluate([val(2, 2)], ex, None) is False     # (left to Python: another library)
     assert L.load() is real and L.host.evaluate([val(2, 2)], ex, None) is True
+
+
+def test_an_extension_that_does_not_compile_leaves_none_behind(tmp_path, monkeypatch):
+    """A stale one goes, the rest is built all the same."""
+    (tmp_path / "host.cpp").write_text("#error\n")
+    stale = tmp_path / "_host.so"
+    stale.write_bytes(b"old")
+    os.utime(stale, (0, 0))
+    monkeypatch.setattr(B, "CSRC", str(tmp_path))
+    monkeypatch.setattr(B, "HOST", str(stale))
+    monkeypatch.setattr(B, "_stale", lambda: False)
+    with pytest.warns(UserWarning, match="host.cpp was not built"):
+        assert B.build() == B.LIB
+    assert sorted(p.name for p in tmp_path.iterdir()) == ["host.cpp"]
+
+
+def test_the_extension_is_named_after_the_interpreter(tmp_path, monkeypatch):
+    assert L.host.__file__ == B.HOST
+    monkeypatch.setattr(B, "HOST", str(tmp_path / os.path.basename(B.HOST)))
+    assert B.build_host() and [p.name for p in tmp_path.iterdir()] == [os.path.basename(B.HOST)]
+    spec = importlib.util.spec_from_file_location("_host", B.HOST)
+    assert hasattr(importlib.util.module_from_spec(spec), "evaluate")
 
 
 @pytest.mark.gpu
