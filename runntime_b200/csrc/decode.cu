@@ -982,9 +982,10 @@ decode_kernel(const DecodeParams p) {
 // 4000 keys (2.0 and 2.4), whose keys the other kernel deals out to more threads.
 // What bounds the FP32-pipe form with several query heads per kv head is that every key is read
 // and converted once per query head, by two warps per scheduler: 16 sequences of 2000 keys, 32
-// heads of 128 on 8, take 75.9 us among launches; here 34.9 (mma_better has more of both sides).  This form
-// is bound by its instructions at heads of up to 64 (96 registers a thread, so that nine warps fit
-// twice per SM, spill 64 to 84 bytes a thread), and by the copies above.
+// heads of 128 on 8, take 75.9 us among launches; here 34.9 (mma_better has more of both sides).  What bounds
+// this form is the latency of nine warps, once per SM at heads of 128 (that case: DRAM 51 % busy, issue slots
+// 35 %, per issue 1.5 warps waiting for shared memory, 1.4 for the pipe, 1.2 for global loads), and its instructions at
+// heads of up to 64, twice per SM (96 registers a thread, 64 to 84 bytes of them spilled).
 template <int HD>
 struct Mma {
   static constexpr int VEC = HD % 8 == 0 ? 8 : 4;               // halves per load

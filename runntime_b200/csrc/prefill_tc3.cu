@@ -18,11 +18,12 @@
 // the same reference point and the accumulator is rescaled by exactly one of them.
 // Up to head size 128 a tile's exponentials start before its max phase, against the
 // reference point last seen, and the maximum is gathered beside them; if the point has
-// moved, what was computed is computed again before anything is published.  (Together with
-// cheaper waits: 64 x 8192 rows causal, 8 heads of 128, 9440 -> 9220 us, the power limit
-// being what is left there; 16 x 2048 rows in a +-512 window 164 -> 140; head size 256,
-// where the one S buffer makes the order of the max phases matter more and the maximum
-// comes first, 32 sequences in that window 162 -> 139.)
+// moved, what was computed is computed again before anything is published.  (At head size 256
+// the one S buffer makes the order of the max phases matter more, and the maximum comes first.
+// Through the operator, in turn with the version before the early exponentials, the cheaper
+// waits, the output through shared memory and the grid order below: 64 x 8192 rows causal, 8 heads
+// of 128, 9626 -> 9323 us, the power limit being what is left there; 32 sequences of 512..2048,
+// 3 heads of 256 on one, +-512 window, 180 -> 156.)
 //
 // Head sizes: 64 and 128 (two S buffers), 256 (the accumulator takes half of tensor
 // memory, so there is ONE S buffer — free again as soon as its scores are in a warpgroup's

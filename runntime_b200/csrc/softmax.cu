@@ -337,7 +337,9 @@ softmax_cta_kernel(const T* x, T* out, const float* segs, int64_t cols,
 // rows are wide does not end on a few CTAs with four of them (n columns, segments, us, a CTA per
 // row and this: 6007, 24 22.4, 18.5; 6007, 6 42.4, 28.7; 7001, 60 27.0, 22.6; 10239, 9 61.9, 53.8; 6007, 1 71.9, 70.1;
 // 9001, 1 149.9, 149.7).  With fewer rows than the chip takes four at a time wide ones lose (4097, 1
-// 41.7, 45.7), as do rows of more than 20 KB, whose zeros are better written by eight warps (f32 6007, 24
+// 41.7, 45.7; 2101, 1 15.7, 25.0), narrow ones would gain (2101, 24 9.1, 5.0; 4097, 24 14.4, 9.7), and the host, which
+// has the ranges on the device only, cannot tell them apart; so the line lies where no rows lose (4999, 1
+// 53.9, 54.0).  Rows of more than 20 KB lose, whose zeros are better written by eight warps (f32 6007, 24
 // 30.1, 32.7), and f32 ones (4097, 1 41.2, 49.4).
 constexpr int kGroupRows = 4, kGroup = 32 * kGroupRows, kGroupMinRows = 5000, kGroupRowBytes = 20480;
 template <int V>
