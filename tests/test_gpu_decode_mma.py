@@ -92,6 +92,26 @@ def test_infinities_and_nan_stay_where_they_are(ex, heads, kv, hd, splits):
     assert (np.abs(got[ok] - want[ok]) <= 2.0 ** -10 * np.abs(want[ok]) + 2.0 ** -14).all()
 
 
+@pytest.mark.parametrize("heads,kv,hd", [(16, 2, 36), (8, 2, 64), (32, 8, 128)])
+@pytest.mark.parametrize("splits", [1, 2])
+def test_a_key_of_minus_infinity_weighs_nothing(ex, heads, kv, hd, splits):
+    """Its score is -inf for a query that is positive there, also for one whose lower bits are zeros (the
+    part of it that the tensor core multiplies the infinity with)."""
+    lens, at = [40, 40], (7, 33)
+    s = _state(heads, kv, hd, 64, 2, seed=11)
+    q, k = s["q"].view(2, heads, hd), s["k"].view(2, 64, kv, hd)
+    q[0, :, 2], q[1, :, 2] = 0.5, 0.3337
+    for b in range(2):
+        k[b, at[b], :, 2] = -math.inf
+    got = _decode(ex, s, heads, kv, hd, lens, splits=splits)
+    for b, n in enumerate(lens):
+        left = [i for i in range(n) if i != at[b]]
+        want = sdpa_ref(s["q"][b:b + 1].float().cpu().numpy(), s["k"][b, left].float().cpu().numpy(),
+                        s["v"][b, left].float().cpu().numpy(), qHeads=heads, kvHeads=kv, headDim=hd, qPosOffset=n - 2,
+                        windowRight=0)
+        oracle.assert_close(got[b], want.reshape(-1), "f16", f"sequence {b}")
+
+
 def test_no_less_precise_than_f32_sums(ex):
     """Long caches and steep scores: the error against 64 bits is that of rounding the result."""
     heads, kv, hd, n = 16, 4, 128, 3000
